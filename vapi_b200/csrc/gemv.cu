@@ -885,96 +885,112 @@ VAPI_EXPORT int vapi_skinny_linear_conv(const void* W, int H, int K, int M, cons
 
 // ---------------------------------------------------------------------------------------------
 // The same product on the true 32-bit path: float weights, float tokens, float FMA and nothing
-// else (no tensor cores, no reduced-precision mode), for the decode steps of that path.  A warp
-// owns a few weight rows and walks K in 16-byte pieces, a chunk of K at a time; the tokens' pieces
-// of a chunk are used for all rows of all warps of the block.  The sum over K is formed per (token, row) in an order that depends on K alone:
-// lane-strided partial sums, then a butterfly over the lanes, so a token's result does not
-// depend on what else is in the batch.
-constexpr int F32_WARPS = 8;
-// rows of the weight a warp owns, and 16-byte pieces of each row that a lane asks for together
-// (fewer of both for nine to sixteen tokens, whose sums take the registers)
-__host__ __device__ constexpr int f32_rows(int mt) { return mt <= 8 ? 4 : 2; }
-__host__ __device__ constexpr int f32_depth(int mt) { return mt <= 8 ? 4 : 2; }
+// else (no tensor cores, no reduced-precision mode), for the decode steps of that path.
+//
+// Bound by reading the weights once, and by what is in flight: a block of four warps owns four weight rows and shares their
+// K, warp w takes the pieces w, w + 4, ... of 128 k, a lane 16 bytes of a piece of each row.  So even the narrowest product
+// of a model (2,048 rows) is 2,048 warps, the grid of many short blocks leaves no long last wave, and four blocks a
+// multiprocessor with f32_depth pieces of four rows a lane in flight keep about 100 KB on their way (before: eight warps of four
+// rows each, one round of loads between two barriers: 64 blocks for 2,048 rows).  The tokens' pieces come from L1, which
+// the weights pass by; a 16-byte load serves four rows x 4 FMAs.  Measured with a flushed L2, 8 tokens: 2,048 x 2,048 14 us,
+// 16,384 x 2,048 43 us, 2,048 x 8,192 29 us, 65,536 x 2,048 125 us (4.3 TB/s); 3 tokens: 65,536 x 2,048 86 us (6.2 TB/s).
+// One or two warps a row group instead of four: 25 or 18 us at 2,048 x 2,048, 84 or 48 us at 2,048 x 8,192, and 143 us at 65,536.
+// A lane's partial sums, the exchange over the lanes and the sum over the four warps add in an order that depends on K
+// alone, so a token's result does not depend on what else is in the batch.
+constexpr int F32_WARPS = 4, F32_ROWS = 4;
+// pieces of the four rows that a lane has in flight (the sums of many tokens take the registers)
+__host__ __device__ constexpr int f32_depth(int mt) { return mt <= 4 ? 4 : (mt <= 8 ? 3 : 2); }
 
-// The tokens' rows travel through shared memory, a chunk of K at a time (two buffers, filled by
-// asynchronous copies one chunk ahead), so that they are read from L2 once per block, not once per warp.
+__device__ __forceinline__ float4 f32_stream(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
 template <int MT>
-__global__ void __launch_bounds__(F32_WARPS * 32)
-skinny_linear_f32_kernel(const float* __restrict__ W, const float* __restrict__ act, const float* __restrict__ bias,
-                         float* __restrict__ out, int N, int K, int M, long long out_stride) {
-    constexpr int F32_ROWS = f32_rows(MT), F32_DEPTH = f32_depth(MT);
-    constexpr int F32_CHUNK = 32 * F32_DEPTH;             // pieces of K in a chunk
-    __shared__ float4 abuf[2][MT][F32_CHUNK];
+__global__ void __launch_bounds__(F32_WARPS * 32, MT <= 8 ? 4 : 3)
+skinny_linear_f32_kernel(const float* __restrict__ W, const float* act /*(the kernel before this one writes it)*/,
+                         const float* __restrict__ bias, float* out, int N, int K, int M, long long out_stride) {
+    constexpr int D = f32_depth(MT), C = F32_ROWS * MT, MG = MT < 8 ? MT : 8;    // (MG tokens at a time: registers)
+    __shared__ float part[F32_WARPS][C];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long n0 = ((long long)blockIdx.x * F32_WARPS + warp) * F32_ROWS;
+    const long long n0 = (long long)blockIdx.x * F32_ROWS;
     pdl_trigger();
-    float acc[F32_ROWS][MT];
-#pragma unroll
-    for (int r = 0; r < F32_ROWS; ++r)
-#pragma unroll
-        for (int m = 0; m < MT; ++m) acc[r][m] = 0.f;
     const int k4 = K >> 2;
-    const int chunks = (k4 + F32_CHUNK - 1) / F32_CHUNK;
+    const int first = warp * 32 + lane;                                 // this lane's 16-byte pieces of a row: first, first + step, ...
+    constexpr int step = F32_WARPS * 32;
+    const int steps = (k4 - warp * 32 + step - 1) / step;               // (the same for the whole warp; <= 0: none)
     const float4* wrow[F32_ROWS];
 #pragma unroll
-    for (int r = 0; r < F32_ROWS; ++r) wrow[r] = reinterpret_cast<const float4*>(W + (size_t)(n0 + r < N ? n0 + r : 0) * K);
-    float4 w[F32_DEPTH][F32_ROWS];
-    auto fetch = [&](int c0) {          // this lane's pieces of a chunk of its rows
+    for (int r = 0; r < F32_ROWS; ++r) wrow[r] = reinterpret_cast<const float4*>(W + (size_t)(n0 + r < N ? n0 + r : n0) * K);
+    float acc[C];
 #pragma unroll
-        for (int u = 0; u < F32_DEPTH; ++u)
+    for (int i = 0; i < C; ++i) acc[i] = 0.f;
+    float4 w[D][F32_ROWS];
+    auto fetch = [&](float4 (&dst)[F32_ROWS], int c) {
 #pragma unroll
-            for (int r = 0; r < F32_ROWS; ++r)
-                w[u][r] = (c0 + 32 * u < k4 && n0 < N) ? __ldcs(wrow[r] + c0 + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = 0; r < F32_ROWS; ++r) dst[r] = c < k4 ? f32_stream(wrow[r] + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
-    auto stage = [&](int chunk, int buf) {     // the tokens' pieces of a chunk, by the whole block
-        for (int idx = threadIdx.x; idx < MT * F32_CHUNK; idx += F32_WARPS * 32) {
-            const int m = idx / F32_CHUNK, c = idx - m * F32_CHUNK, cg = chunk * F32_CHUNK + c;
-            const bool ok = m < M && cg < k4;
-            gv_cp16(&abuf[buf][m][c], reinterpret_cast<const float4*>(act + (size_t)(ok ? m : 0) * K) + (ok ? cg : 0), ok ? 16 : 0);
-        }
-        gv_commit();
-    };
-    fetch(lane);                         // the weights do not depend on the kernel before this one
+#pragma unroll
+    for (int d = 0; d < D; ++d) fetch(w[d], first + d * step);          // the weights do not depend on the kernel before this one
     pdl_wait();
-    stage(0, 0);
-    for (int ch = 0; ch < chunks; ++ch) {
-        if (ch + 1 < chunks) stage(ch + 1, (ch + 1) & 1);
-        else gv_commit();
-        gv_wait<1>();
-        __syncthreads();                 // chunk ch of the tokens is in place for every warp
-        if (ch > 0) fetch(ch * F32_CHUNK + lane);
+    for (int i = 0; i < steps; i += D) {
 #pragma unroll
-        for (int u = 0; u < F32_DEPTH; ++u) {
+        for (int d = 0; d < D; ++d) {
+            const int c = first + (i + d) * step;
+            if (i + d < steps) {
 #pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                const float4 a = abuf[ch & 1][m][lane + 32 * u];
+                for (int g = 0; g < MT; g += MG) {
+                    float4 a[MG];
 #pragma unroll
-                for (int r = 0; r < F32_ROWS; ++r) {
-                    acc[r][m] = fmaf(w[u][r].x, a.x, acc[r][m]);
-                    acc[r][m] = fmaf(w[u][r].y, a.y, acc[r][m]);
-                    acc[r][m] = fmaf(w[u][r].z, a.z, acc[r][m]);
-                    acc[r][m] = fmaf(w[u][r].w, a.w, acc[r][m]);
+                    for (int m = 0; m < MG; ++m)
+                        a[m] = c < k4 ? *(reinterpret_cast<const float4*>(act + (size_t)(g + m < M ? g + m : 0) * K) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int r = 0; r < F32_ROWS; ++r)
+#pragma unroll
+                        for (int m = 0; m < MG; ++m) {
+                            float s = acc[r * MT + g + m];
+                            s = fmaf(w[d][r].x, a[m].x, s);
+                            s = fmaf(w[d][r].y, a[m].y, s);
+                            s = fmaf(w[d][r].z, a[m].z, s);
+                            acc[r * MT + g + m] = fmaf(w[d][r].w, a[m].w, s);
+                        }
+                }
+                fetch(w[d], c + D * step);
+            }
+        }
+    }
+    // the C sums over the 32 lanes: halves are exchanged while there is more than one left, so the lanes end with C / 32 (or one
+    // of C, in 32 / C lanes) each
+    int n = C;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int j = 0; j < C / 2; ++j) {
+                if (j < n) {
+                    const float keep = up ? acc[j + n] : acc[j], give = up ? acc[j] : acc[j + n];
+                    acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
                 }
             }
+        } else {
+            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
         }
-        __syncthreads();                 // everyone is done with this buffer before it is filled again
     }
-    gv_wait<0>();
-    if (n0 >= N) return;
+    if (C >= 32) {
 #pragma unroll
-    for (int r = 0; r < F32_ROWS; ++r)
-#pragma unroll
-        for (int m = 0; m < MT; ++m) acc[r][m] = warp_sum(acc[r][m]);
-    if (lane == 0) {
-#pragma unroll
-        for (int r = 0; r < F32_ROWS; ++r) {
-            if (n0 + r < N) {
-                const float b = bias ? bias[n0 + r] : 0.f;
-#pragma unroll
-                for (int m = 0; m < MT; ++m)
-                    if (m < M) out[(size_t)m * out_stride + n0 + r] = acc[r][m] + b;
-            }
-        }
+        for (int j = 0; j < (C >= 32 ? C / 32 : 1); ++j) part[warp][lane * (C / 32) + j] = acc[j];
+    } else if (lane % (32 / (C < 32 ? C : 32)) == 0) {
+        part[warp][lane / (32 / (C < 32 ? C : 32))] = acc[0];
+    }
+    __syncthreads();
+    // the four warps in order; neighbouring threads write neighbouring features of a token
+    if (threadIdx.x < C) {
+        const int r = threadIdx.x % F32_ROWS, m = threadIdx.x / F32_ROWS, i = r * MT + m;
+        if (n0 + r < N && m < M)
+            out[(size_t)m * out_stride + n0 + r] = part[0][i] + part[1][i] + part[2][i] + part[3][i] + (bias ? bias[n0 + r] : 0.f);
     }
 }
 
@@ -986,8 +1002,7 @@ VAPI_EXPORT int vapi_skinny_linear_f32(const float* W, int N, int K, int M, cons
     if (N <= 0 || K <= 0 || K % 4 != 0) return fail(-1, "skinny_linear_f32: K=%d must be a positive multiple of 4 (N=%d)", K, N);
     if (!W || !act || !out) return fail(-1, "skinny_linear_f32: missing array");
     if ((((uintptr_t)W | (uintptr_t)act) & 15) != 0) return fail(-1, "skinny_linear_f32: operands must be 16-byte aligned");
-    const int mt = M <= 1 ? 1 : (M <= 4 ? 4 : (M <= 8 ? 8 : 16));
-    const int blocks = (N + F32_WARPS * f32_rows(mt) - 1) / (F32_WARPS * f32_rows(mt));
+    const int blocks = (N + F32_ROWS - 1) / F32_ROWS;
     cudaError_t e;
     if (M <= 1) e = launch(skinny_linear_f32_kernel<1>, blocks, F32_WARPS * 32, 0, stream, W, act, bias, out, N, K, M, out_stride);
     else if (M <= 4) e = launch(skinny_linear_f32_kernel<4>, blocks, F32_WARPS * 32, 0, stream, W, act, bias, out, N, K, M, out_stride);
