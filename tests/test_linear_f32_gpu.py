@@ -1,0 +1,76 @@
+"""The float32 product on the tensor cores (csrc/linear_f32.cu) against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from vapi_b200 import ops as o
+    o.strict_fp32()
+    return o
+
+
+def _bound(a, w):
+    """Elementwise: a piece of 64 k is 6 x 4 tensor-core additions of 16 products, each of which may drop what lies below the
+    last of 24 bits (2^-23 of the sum so far), the pieces are K / 64 float additions, the split leaves out 2^-25, and
+    the bias is one more rounding; all against the sum of the magnitudes."""
+    K = a.shape[1]
+    return (2 * 24 + -(-K // 64) + 8 + 2) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t()) + 1e-30
+
+
+# one row and one tile; edges of the 64 / 128 token and 128 feature tiles; K below a stage, ragged, not a multiple of 8; K shared by
+# two to eight blocks; more tiles than multiprocessors
+@pytest.mark.parametrize("M,N,K", [(1, 1, 4), (17, 6, 12), (33, 129, 60), (64, 128, 64), (65, 127, 68), (128, 256, 516), (129, 300, 1028),
+                                   (31, 130, 4160), (200, 1536, 2052), (64, 2048, 8192), (513, 5000, 130 * 4)])
+def test_float32_product_is_no_further_from_the_exact_one_than_its_bound(ops, M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N)
+    a = torch.randn(M, K, generator=g, device="cuda") * torch.exp(2 * torch.randn(M, K, generator=g, device="cuda"))
+    w = torch.randn(N, K, generator=g, device="cuda")
+    b = torch.randn(N, generator=g, device="cuda")
+    want = a.double() @ w.double().t()
+    got = ops.linear_f32(a, w, b)
+    assert ((got.double() - want - b.double()).abs() <= _bound(a, w) + 2.0 ** -23 * b.double().abs()).all()
+    assert torch.equal(ops.linear_f32(a, w), ops.linear_f32(a, w))
+    before = ops.launch_count
+    via = ops.linear(a, w, b)
+    assert M <= 16 or (ops.launch_count == before + 2 and torch.equal(via, got))
+
+
+@pytest.mark.parametrize("M,N,K", [(70, 300, 256), (40, 130, 2048), (300, 20000, 68)])
+def test_float32_product_of_what_cannot_be_split(ops, M, N, K):
+    """Infinities, NaN and magnitudes next to the largest float, in tokens and in weights, in the first and the last row, in tiles of one
+    block and of several: what plain FMAs give, and nothing else changes."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    a2, w2 = a.clone(), w.clone()
+    a2[0, 0], a2[3, K - 1], a2[M - 1, K // 2], a2[5, 1] = float("inf"), float("nan"), -float("inf"), 3.0e38
+    w2[0, 2], w2[N - 1, K - 1], w2[N // 2, 0], w2[7, 9] = float("inf"), float("nan"), 2.0e38, 0.0
+    # the huge finite ones never meet in one sum, and the huge weight does not overflow beside the other sign's infinity: what a
+    # float sum makes of that depends on its order, and the float64 product below does not show it
+    a2[5, 0], w2[N // 2, 1], a2[M - 1, 0] = 0.0, 0.0, 0.5
+    clean = ops.linear_f32(a, w)
+    got, want = ops.linear_f32(a2, w2), a2.double() @ w2.double().t()
+    big = want.abs() >= 2.0 ** 128 * (1 - 2.0 ** -25)         # (what rounds to a float's infinity)
+    want = torch.where(big, want.sign() * float("inf"), want)
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    assert torch.equal(torch.isinf(got), torch.isinf(want))
+    fin = torch.isfinite(want)
+    err = torch.where(fin, (got.double() - want).abs(), torch.zeros_like(want))
+    scale = torch.where(fin, (torch.nan_to_num(a2, 0, 0, 0).double().abs() @ torch.nan_to_num(w2, 0, 0, 0).double().abs().t()), torch.ones_like(want))
+    assert (err <= (K + 60) * 2.0 ** -24 * scale).all()       # (a plain sum of K products is K roundings)
+    rows = torch.ones(M, dtype=torch.bool, device="cuda")
+    rows[[0, 3, 5, M - 1]] = False
+    cols = torch.ones(N, dtype=torch.bool, device="cuda")
+    cols[[0, 7, N // 2, N - 1]] = False
+    assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
+
+
+def test_float32_product_of_tiny_and_exact_numbers(ops):
+    """Numbers of eight bits have empty lower planes; small whole numbers come out exactly; small magnitudes keep their bits."""
+    g = torch.Generator(device="cuda").manual_seed(4)
+    a = torch.randint(-9, 10, (90, 200), generator=g, device="cuda").float()
+    w = torch.randint(-9, 10, (150, 200), generator=g, device="cuda").float()
+    assert torch.equal(ops.linear_f32(a, w).double(), a.double() @ w.double().t())
+    assert torch.equal(ops.linear_f32(a * 2.0 ** -60, w).double(), (a.double() @ w.double().t()) * 2.0 ** -60)

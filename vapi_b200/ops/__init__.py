@@ -670,6 +670,39 @@ def skinny_linear_f32(weight: torch.Tensor, act: torch.Tensor, bias: Optional[to
     return out
 
 
+def linear_f32_applies(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether the split product on the tensor cores takes this float32 product: 16-byte rows of the weight and the
+    tokens (inner size a multiple of 4, both contiguous and aligned)."""
+    return (use_tc and weight.is_cuda and weight.dtype == torch.float32 and x.dtype == torch.float32 and weight.dim() == 2
+            and x.dim() == 2 and x.shape[0] > 0 and weight.shape[0] > 0 and x.shape[1] == weight.shape[1] > 0
+            and weight.shape[1] % 4 == 0 and weight.is_contiguous() and x.is_contiguous()
+            and weight.data_ptr() % 16 == 0 and x.data_ptr() % 16 == 0)
+
+
+def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
+               status: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``x @ weight.T (+ bias)`` in float32 for any number of rows: every float is the exact sum of three bfloat16, six of
+    the nine products are taken on the tensor cores and added up in float32, no further from the exact result than float
+    FMAs (csrc/linear_f32.cu)."""
+    _cuda(x, weight, bias, status)
+    N, K = weight.shape
+    M = x.shape[0]
+    if weight.dtype != torch.float32 or not weight.is_contiguous():
+        raise KernelError("linear_f32 needs a contiguous float32 weight")
+    if x.dtype != torch.float32 or tuple(x.shape) != (M, K) or not x.is_contiguous():
+        raise KernelError(f"linear_f32: token operand {tuple(x.shape)} / {x.dtype} does not fit a weight of {N}x{K}")
+    _f32(bias, "bias")
+    _i32(status, "status")
+    out = torch.empty((M, N), dtype=torch.float32, device=weight.device)
+    kp = -(-K // 8) * 8
+    planes = torch.empty(3 * M * kp, dtype=torch.bfloat16, device=weight.device)
+    bad = torch.empty(M, dtype=torch.int32, device=weight.device)
+    lib = _lib("linear_f32")
+    _check(lib, lib.vapi_linear_f32(_p(weight), N, K, M, _p(x), _p(planes), _p(bad), _p(bias), _p(out), ctypes.c_longlong(N),
+                                    _p(status), _stream()), launches=2)
+    return out
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """``x @ weight.T (+ bias)``.  The library matrix product, except for decode-sized
@@ -692,6 +725,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if (x.dtype == torch.float32 and out_dtype in (None, torch.float32) and skinny_f32_applies(x.shape[0], weight)
             and x.is_contiguous() and x.data_ptr() % 16 == 0):
         return skinny_linear_f32(weight, x, bias)
+    if out_dtype in (None, torch.float32) and linear_f32_applies(x, weight):
+        return linear_f32(x, weight, bias)
     if weight.dtype != x.dtype:
         y = torch.mm(x.to(torch.float32), weight.to(torch.float32).t())
         if bias is not None:
