@@ -326,7 +326,7 @@ VAPI_EXPORT int vapi_paged_attention(const void* q, long long q_row_stride, cons
         // prompt portions on tcgen05; in a mixed step the short sequences (decode tokens) go to the
         // flash kernel, whose small blocks suit them: each kernel skips the other's sequences
         const int min_q = (impl == 3 || num_seqs == 1) ? 1 : FT_MIN_Q;
-        rc = launch_flash_tc(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, num_seqs, max_q,
+        rc = launch_flash_tc(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, n, num_seqs, max_q,
                              nh, nkv, page_size, num_pages, scale, window, min_q, status, stream);
         if (rc != 0 || min_q == 1) return rc;
         // (of the shorter ones, those of at most 16 rows - decode tokens, whose contexts can be long -

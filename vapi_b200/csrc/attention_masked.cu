@@ -385,7 +385,7 @@ VAPI_EXPORT int vapi_masked_attention(const void* q, long long q_row_stride, con
         if (tc_ok) {
             const int min_q = num_seqs == 1 ? 1 : FT_MIN_Q;
 #define MA_TC(SIG)                                                                                                            \
-    rc = launch_flash_tc<SIG>(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, num_seqs, max_q, nh, nkv, \
+    rc = launch_flash_tc<SIG>(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, n, num_seqs, max_q, nh, nkv, \
                               page_size, num_pages, scale, window, min_q, status, stream, chunk, sinks, gate, gate_stride, keep, \
                               form);                                                                                          \
     if (rc != 0 || min_q == 1) return rc;                                                                                     \

@@ -56,7 +56,7 @@ struct FaTcParams {
     __nv_bfloat16* out;
     int nh, nkv, page_size, num_pages;
     float scale_log2e;
-    int window, min_q;
+    int window, min_q, num_seqs;
     int* status;
     // mask_chunk > 0: a query also sees only keys of its own block of mask_chunk positions; sinks: exp(sink[head])
     // joins the softmax's denominator; gate: the output of (token, head) is multiplied by
@@ -79,6 +79,38 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return y;
 }
 
+// The row tiles of all sequences that this kernel takes stand in one list, sequence after sequence, longest tiles (the last
+// rows) of a sequence first: entry `want` of it as (sequence, row tile); false behind its end.  For whole warps.  A grid of
+// (longest sequence's tiles) x sequences instead is mostly blocks with nothing to do when one portion stands beside many
+// decode tokens, and each of them holds a multiprocessor's 99 KB until it has seen that (31 decode tokens beside a portion of
+// 777, 32 / 8 heads: 6,400 blocks for 200 tiles).
+__device__ __forceinline__ bool ft_tile(const int* cu_q, int num_seqs, int min_q, int n_rep, int want, int& s, int& tile) {
+    const int lane = threadIdx.x & 31;
+    int before = 0;
+    for (int c = 0; c < num_seqs; c += 32) {
+        int t = 0;
+        if (c + lane < num_seqs) {
+            const int qlen = cu_q[c + lane + 1] - cu_q[c + lane];
+            t = qlen >= min_q ? (qlen * n_rep + FT_ROWS - 1) / FT_ROWS : 0;
+        }
+        int upto = t;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, before + upto > want);
+        if (hit) {
+            const int src = __ffs(hit) - 1;
+            s = c + src;
+            tile = before + __shfl_sync(0xffffffffu, upto, src) - 1 - want;
+            return true;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return false;
+}
+
 template <bool SIG>
 __global__ void __launch_bounds__(FT_THREADS, 2)
 flash_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const FaTcParams p) {
@@ -92,17 +124,17 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const FaTcParams p) {
     int* flags = reinterpret_cast<int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int s = blockIdx.z, g = blockIdx.y;
+    const int g = blockIdx.y, n_rep = p.nh / p.nkv;
     pdl_trigger();
     // index data was copied from the host before the step's first kernel: safe before the wait
-    const int q0 = p.cu_q[s], qlen = p.cu_q[s + 1] - q0, klen = p.seqlens_k[s];
-    const int n_rep = p.nh / p.nkv;
-    const int rows_total = qlen * n_rep;
-    const int tile_start = ((int)gridDim.x - 1 - (int)blockIdx.x) * FT_ROWS;     // longest tiles first
-    if (qlen < p.min_q || tile_start >= rows_total) {
+    int s = 0, tile = 0;
+    if (!ft_tile(p.cu_q, p.num_seqs, p.min_q, n_rep, (int)blockIdx.x, s, tile)) {
         pdl_wait();
         return;
     }
+    const int q0 = p.cu_q[s], qlen = p.cu_q[s + 1] - q0, klen = p.seqlens_k[s];
+    const int rows_total = qlen * n_rep;
+    const int tile_start = tile * FT_ROWS;
     const int last_row = min(rows_total, tile_start + FT_ROWS) - 1;
     const int base_pos = klen - qlen;
     const int p_min = base_pos + tile_start / n_rep;
@@ -405,13 +437,15 @@ static int make_kv_map(CUtensorMap* map, const void* cache, long long rows) {
 
 template <bool SIG = false>
 static int launch_flash_tc(const void* q, long long q_row_stride, const void* cache, const int* block_table,
-                           int table_stride, const int* cu_q, const int* seqlens_k, void* out, int num_seqs,
+                           int table_stride, const int* cu_q, const int* seqlens_k, void* out, int n, int num_seqs,
                            int max_q, int nh, int nkv, int page_size, int num_pages, float scale, int window,
                            int min_q, int* status, cudaStream_t stream, int mask_chunk = 0, const float* sinks = nullptr,
                            const void* gate = nullptr, long long gate_stride = 0, int keep = 0,
                            const ScoreForm& form = ScoreForm()) {
     const int n_rep = nh / nkv;
-    const long long tiles = ((long long)max_q * n_rep + FT_ROWS - 1) / FT_ROWS;
+    // tiles of all sequences together: at most those of n tokens in one piece and a ragged one a sequence
+    const long long longest = ((long long)max_q * n_rep + FT_ROWS - 1) / FT_ROWS, whole = (long long)n * n_rep / FT_ROWS + num_seqs;
+    const long long tiles = longest * num_seqs < whole ? longest * num_seqs : whole;
     if (tiles > 0x7fffffffLL || nkv > 65535 || num_seqs > 65535)
         return fail(-1, "paged_attention: the step exceeds the grid (%lld row tiles, %d kv heads, %d sequences)", tiles, nkv, num_seqs);
     if (!(scale > 0.f)) return fail(-1, "paged_attention: the tcgen05 kernel needs a positive scale");
@@ -429,11 +463,11 @@ static int launch_flash_tc(const void* q, long long q_row_stride, const void* ca
     FaTcParams p;
     p.q = (const __nv_bfloat16*)q; p.q_row_stride = q_row_stride; p.block_table = block_table; p.table_stride = table_stride;
     p.cu_q = cu_q; p.seqlens_k = seqlens_k; p.out = (__nv_bfloat16*)out; p.nh = nh; p.nkv = nkv; p.page_size = page_size;
-    p.num_pages = num_pages; p.scale_log2e = scale * 1.4426950408889634f; p.window = window; p.min_q = min_q; p.status = status;
+    p.num_pages = num_pages; p.scale_log2e = scale * 1.4426950408889634f; p.window = window; p.min_q = min_q; p.num_seqs = num_seqs; p.status = status;
     p.mask_chunk = mask_chunk; p.keep = keep; p.sinks = sinks; p.gate = (const __nv_bfloat16*)gate; p.gate_stride = gate_stride;
     p.sig = sigmoid_form(scale, form.softcap); p.score_bias = form.bias; p.out_scale = form.out_scale;
     p.out_stride = form.out_stride > 0 ? form.out_stride : (long long)nh * FT_HD;
-    dim3 grid((unsigned)tiles, nkv, num_seqs);
+    dim3 grid((unsigned)tiles, nkv);
     return check_launch("paged_attention (tcgen05)", launch(flash_tc_kernel<SIG>, grid, FT_THREADS, FT_SMEM, stream, map, p));
 }
 
