@@ -35,7 +35,7 @@ def test_float32_product_is_no_further_from_the_exact_one_than_its_bound(ops, M,
     assert torch.equal(ops.linear_f32(a, w), ops.linear_f32(a, w))
     before = ops.launch_count
     via = ops.linear(a, w, b)
-    assert M <= 16 or (ops.launch_count == before + 2 and torch.equal(via, got))
+    assert M <= 16 or N * K < 1 << 20 or (ops.launch_count == before + 2 and torch.equal(via, got))
 
 
 @pytest.mark.parametrize("M,N,K", [(70, 300, 256), (40, 130, 2048), (300, 20000, 68)])

@@ -670,12 +670,18 @@ def skinny_linear_f32(weight: torch.Tensor, act: torch.Tensor, bias: Optional[to
     return out
 
 
+#: numbers in a float32 weight from which on products of more than 16 rows go to csrc/linear_f32.cu
+LINEAR_F32_LEAST = 1 << 20
+
+
 def linear_f32_applies(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether the split product on the tensor cores takes this float32 product: 16-byte rows of the weight and the
-    tokens (inner size a multiple of 4, both contiguous and aligned)."""
+    tokens (inner size a multiple of 4, both contiguous and aligned), and a weight large enough that its two launches
+    pay: 17 x 100 x 36 takes 12 us against the library's 8, 129 tokens x 1536 x 1024 30 against 31 to 33, and from there
+    on it is ahead (33 tokens x 1536 x 1536 26 against 45)."""
     return (use_tc and weight.is_cuda and weight.dtype == torch.float32 and x.dtype == torch.float32 and weight.dim() == 2
             and x.dim() == 2 and x.shape[0] > 0 and weight.shape[0] > 0 and x.shape[1] == weight.shape[1] > 0
-            and weight.shape[1] % 4 == 0 and weight.is_contiguous() and x.is_contiguous()
+            and weight.shape[1] % 4 == 0 and weight.numel() >= LINEAR_F32_LEAST and weight.is_contiguous() and x.is_contiguous()
             and weight.data_ptr() % 16 == 0 and x.data_ptr() % 16 == 0)
 
 
