@@ -1,0 +1,55 @@
+"""The float32 prompt attention on the tensor cores (csrc/attention_f32.cuh) beside the general kernel and the plain form."""
+import pytest
+import torch
+
+from test_kernels_gpu import _attention_case
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from vapi_b200 import ops as o
+    o.strict_fp32()
+    return o
+
+
+# tiles of 64 rows and 64 keys and their edges, decode tokens beside portions, rows that no whole token fills, split keys, windows
+@pytest.mark.parametrize("nh,nkv,page", [(8, 2, 64), (32, 8, 128), (3, 1, 64), (40, 1, 192)])
+@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("window", [0, 1, 70])
+def test_float_attention_of_portions(ops, nh, nkv, page, splits, window):
+    _attention_case(ops, torch.float32, nh, nkv, 64, page, [(17, 17), (1, 130), (64, 64), (65, 129), (1, 1), (30, 400), (128, 128), (2, 63)],
+                    window=window, splits=splits)
+    _attention_case(ops, torch.float32, nh, nkv, 64, page, [(70, 300)] + [(1, 5 + i) for i in range(40)], window=window, splits=splits, planted=True)
+
+
+def _random_case(seed, n, klen, nh, nkv):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    pages = -(-klen // 64)
+    q = torch.randn(n, nh * 64, generator=g, device="cuda")
+    cache = torch.randn(pages, 2, nkv, 64, 64, generator=g, device="cuda")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    return q, cache, (torch.arange(pages, device="cuda").int()[None], i32([0, n]), i32([klen]), n, 1, n, klen, nh, nkv, 64, 0.125)
+
+
+def test_float_attention_is_no_further_from_the_exact_one(ops):
+    q, cache, args = _random_case(1, 200, 700, 4, 2)
+    got, general = (ops.paged_attention(q, 256, cache, *args, splits=1, impl=impl).double() for impl in ("auto", "general"))
+    k, v = (cache.double()[:, i].transpose(0, 1).reshape(2, -1, 64)[:, :700].repeat_interleave(2, 0) for i in (0, 1))
+    s = torch.einsum("nhd,hkd->hnk", q.double().view(200, 4, 64), k) * 0.125
+    s = s.masked_fill(torch.arange(700, device="cuda")[None, :] > 500 + torch.arange(200, device="cuda")[:, None], float("-inf"))
+    want = torch.einsum("hnk,hkd->nhd", s.softmax(-1), v).reshape(200, 256)
+    err, before = ((t - want).norm() / want.norm() for t in (got, general))
+    assert err < 3e-7 and err <= 1.05 * before, (err, before)
+
+
+def test_float_attention_of_what_cannot_be_split(ops):
+    """Infinities, NaN and magnitudes next to the largest float in queries, keys and values give what the general kernel gives."""
+    q, cache, args = _random_case(2, 100, 260, 4, 2)
+    q[3, 5], q[50, 70] = float("inf"), float("nan")
+    cache[1, 0, 0, 7, 3], cache[2, 0, 1, 9, 60], cache[3, 1, 0, 5, 0] = -float("inf"), 3.0e38, float("inf")
+    got, want = (ops.paged_attention(q, 256, cache, *args, splits=1, impl=impl) for impl in ("auto", "general"))
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    fin = torch.isfinite(want)
+    torch.testing.assert_close(got[fin], want[fin], atol=2e-5, rtol=2e-5)

@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "attention_mma.cuh"
 #include "attention_tc.cuh"
+#include "attention_f32.cuh"
 #include "attention_decode.cuh"
 
 using namespace vapi;
@@ -368,6 +369,12 @@ VAPI_EXPORT int vapi_paged_attention(const void* q, long long q_row_stride, cons
     } else if (fast) {
         if (d == 64) { if (few_rows) VAPI_FLASH(64, 1, 3); else VAPI_FLASH(64, 4, 3); }
         else         { if (few_rows) VAPI_FLASH(128, 1, 3); else VAPI_FLASH(128, 4, 3); }
+    } else if (dtype == VAPI_F32 && impl == 0 && d == FF_HD && !few_rows && page_size % FF_BK == 0 && q_row_stride % 4 == 0 &&
+               (((uintptr_t)q | (uintptr_t)cache) & 15) == 0 && (((uintptr_t)out | (uintptr_t)part_o) & 7) == 0) {
+        // (few rows - decode tokens - leave three of the kernel's four warps without work: four steps of 8 requests at 1,024 tokens
+        // took 7.6 ms here and take 7.0 ms on the general kernel)
+        rc = launch_flash_f32(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, part_o, part_ml, n, num_seqs,
+                              max_q, nh, nkv, page_size, num_pages, scale, window, splits, status, stream);
     } else if (dtype == VAPI_F32) {
         if (d <= 64) VAPI_ATT(float, 64); else if (d <= 128) VAPI_ATT(float, 128); else VAPI_ATT(float, 256);
     } else if (dtype == VAPI_BF16) {

@@ -79,19 +79,19 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return y;
 }
 
-// The row tiles of all sequences that this kernel takes stand in one list, sequence after sequence, longest tiles (the last
+// The row tiles (of `rows` rows) of all sequences that a kernel takes stand in one list, sequence after sequence, longest tiles (the last
 // rows) of a sequence first: entry `want` of it as (sequence, row tile); false behind its end.  For whole warps.  A grid of
 // (longest sequence's tiles) x sequences instead is mostly blocks with nothing to do when one portion stands beside many
 // decode tokens, and each of them holds a multiprocessor's 99 KB until it has seen that (31 decode tokens beside a portion of
 // 777, 32 / 8 heads: 6,400 blocks for 200 tiles).
-__device__ __forceinline__ bool ft_tile(const int* cu_q, int num_seqs, int min_q, int n_rep, int want, int& s, int& tile) {
+__device__ __forceinline__ bool ft_tile(const int* cu_q, int num_seqs, int min_q, int n_rep, int rows, int want, int& s, int& tile) {
     const int lane = threadIdx.x & 31;
     int before = 0;
     for (int c = 0; c < num_seqs; c += 32) {
         int t = 0;
         if (c + lane < num_seqs) {
             const int qlen = cu_q[c + lane + 1] - cu_q[c + lane];
-            t = qlen >= min_q ? (qlen * n_rep + FT_ROWS - 1) / FT_ROWS : 0;
+            t = qlen >= min_q ? (qlen * n_rep + rows - 1) / rows : 0;
         }
         int upto = t;
 #pragma unroll
@@ -128,7 +128,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const FaTcParams p) {
     pdl_trigger();
     // index data was copied from the host before the step's first kernel: safe before the wait
     int s = 0, tile = 0;
-    if (!ft_tile(p.cu_q, p.num_seqs, p.min_q, n_rep, (int)blockIdx.x, s, tile)) {
+    if (!ft_tile(p.cu_q, p.num_seqs, p.min_q, n_rep, FT_ROWS, (int)blockIdx.x, s, tile)) {
         pdl_wait();
         return;
     }
