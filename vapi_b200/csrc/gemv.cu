@@ -892,14 +892,17 @@ VAPI_EXPORT int vapi_skinny_linear_conv(const void* W, int H, int K, int M, cons
 // of a model (2,048 rows) is 2,048 warps, the grid of many short blocks leaves no long last wave, and four blocks a
 // multiprocessor with f32_depth pieces of four rows a lane in flight keep about 100 KB on their way (before: eight warps of four
 // rows each, one round of loads between two barriers: 64 blocks for 2,048 rows).  The tokens' pieces come from L1, which
-// the weights pass by; a 16-byte load serves four rows x 4 FMAs.  Measured with a flushed L2, 8 tokens: 2,048 x 2,048 14 us,
-// 16,384 x 2,048 43 us, 2,048 x 8,192 29 us, 65,536 x 2,048 125 us (4.3 TB/s); 3 tokens: 65,536 x 2,048 86 us (6.2 TB/s).
-// One or two warps a row group instead of four: 25 or 18 us at 2,048 x 2,048, 84 or 48 us at 2,048 x 8,192, and 143 us at 65,536.
+// the weights pass by; a 16-byte load serves four rows x 4 FMAs.  In a captured chain of products, 8 tokens:
+// 2,048 x 2,048 6.3 us, 16,384 x 2,048 33, 2,048 x 8,192 17.6, 65,536 x 2,048 120 (4.5 TB/s); 3 tokens: 65,536 x 2,048 80 us
+// (6.7 TB/s).  One or two warps a row group instead of four (one launch, L2 flushed): 25 or 18 against 14 us at 2,048 x 2,048,
+// 84 or 48 against 29 at 2,048 x 8,192, and 143 against 125 at 65,536.
 // A lane's partial sums, the exchange over the lanes and the sum over the four warps add in an order that depends on K
 // alone, so a token's result does not depend on what else is in the batch.
 constexpr int F32_WARPS = 4, F32_ROWS = 4;
-// pieces of the four rows that a lane has in flight (the sums of many tokens take the registers)
-__host__ __device__ constexpr int f32_depth(int mt) { return mt <= 4 ? 4 : (mt <= 8 ? 3 : 2); }
+// pieces of the four rows that a lane has in flight.  The sums of many tokens take the registers, and what they leave is worth
+// more as room between the tokens' loads and their use: 2,048 x 8,192, 8 tokens 18.8 us with three pieces, 17.6 with two; 16
+// tokens 43.6 with two, 37.5 with one.
+__host__ __device__ constexpr int f32_depth(int mt) { return mt <= 4 ? 4 : (mt <= 8 ? 2 : 1); }
 
 __device__ __forceinline__ float4 f32_stream(const float4* p) {
     float4 v;
