@@ -24,6 +24,17 @@ def test_float_attention_of_portions(ops, nh, nkv, page, splits, window):
     _attention_case(ops, torch.float32, nh, nkv, 64, page, [(70, 300)] + [(1, 5 + i) for i in range(40)], window=window, splits=splits, planted=True)
 
 
+# decode steps: one token a sequence, up to four q heads a kv head; slices that end inside 32 and 128 keys, empty slices, windows that begin inside
+# a tile, pages of 32 to 192
+@pytest.mark.parametrize("nh,nkv,page", [(8, 2, 64), (3, 1, 32), (4, 4, 96), (32, 8, 192)])
+@pytest.mark.parametrize("splits", [1, 2, 7])
+@pytest.mark.parametrize("window", [0, 1, 33, 200])
+def test_float_attention_of_decode_tokens(ops, nh, nkv, page, splits, window):
+    lens = [(1, 1), (1, 31), (1, 32), (1, 33), (1, 127), (1, 128), (1, 129), (1, 500), (1, 1000)]
+    _attention_case(ops, torch.float32, nh, nkv, 64, page, lens, window=window, splits=splits)
+    _attention_case(ops, torch.float32, nh, nkv, 64, page, lens, window=window, splits=splits, planted=window == 0)
+
+
 def _random_case(seed, n, klen, nh, nkv):
     g = torch.Generator(device="cuda").manual_seed(seed)
     pages = -(-klen // 64)

@@ -375,6 +375,10 @@ VAPI_EXPORT int vapi_paged_attention(const void* q, long long q_row_stride, cons
         // took 7.6 ms here and take 7.0 ms on the general kernel)
         rc = launch_flash_f32(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, part_o, part_ml, n, num_seqs,
                               max_q, nh, nkv, page_size, num_pages, scale, window, splits, status, stream);
+    } else if (dtype == VAPI_F32 && impl == 0 && d == FF_HD && max_q == 1 && nh / nkv <= DF_ROWS && page_size % 32 == 0 && q_row_stride % 4 == 0 &&
+               (((uintptr_t)q | (uintptr_t)cache) & 15) == 0) {
+        rc = launch_decode_f32(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, part_o, part_ml, num_seqs,
+                               nh, nkv, page_size, num_pages, scale, window, splits, status, stream);
     } else if (dtype == VAPI_F32) {
         if (d <= 64) VAPI_ATT(float, 64); else if (d <= 128) VAPI_ATT(float, 128); else VAPI_ATT(float, 256);
     } else if (dtype == VAPI_BF16) {
