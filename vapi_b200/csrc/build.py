@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -81,7 +82,6 @@ def find_nvcc() -> str:
 
 def _headers(name: str) -> List[str]:
     """The package's own headers that ``name``.cu includes, directly or through another."""
-    import re
     seen: List[str] = []
     todo = [_source(name)]
     while todo:
@@ -104,6 +104,27 @@ def _digest(name: str) -> str:
     flags = HOST_FLAGS if _is_host(name) else ARCH_FLAGS + COMMON_FLAGS + _ENV_FLAGS
     h.update(" ".join(flags + EXTRA.get(name, [])).encode())
     return h.hexdigest()[:12]
+
+
+_EXPORT = re.compile(r"^\s*VAPI_EXPORT\s+([\w\s\*]+?)\b(vapi_\w+)\s*\(([^)]*)\)", re.M)
+
+
+def exports(name: str) -> Dict[str, List[str]]:
+    """The C functions of ``name``.cu: name -> [type of the result, types of the parameters ...], a pointer of any kind (and
+    a stream) as ``ptr``.  Whoever loads the library declares them with it, so that plain numbers can be passed."""
+    with open(_source(name), "r", encoding="utf-8") as f:
+        text = re.sub(r"//[^\n]*|/\*.*?\*/", "", f.read(), flags=re.S)
+
+    def kind(decl: str) -> str:
+        if "*" in decl or "cudaStream_t" in decl:
+            return "ptr"
+        words = [w for w in decl.split() if w != "const"]
+        return " ".join(words[:-1] if len(words) > 1 and words[-1] not in ("int", "long", "float", "double") else words)
+
+    out: Dict[str, List[str]] = {}
+    for result, fn, params in _EXPORT.findall(text):
+        out[fn] = [kind(result)] + [kind(p) for p in params.split(",") if p.strip() and p.strip() != "void"]
+    return out
 
 
 def _build_dirs() -> List[str]:

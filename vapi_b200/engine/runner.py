@@ -194,7 +194,8 @@ class ModelRunner:
             ctx.pos[pe.name] = pe.prepare(ctx)
         views = self.views(ctx)
         ctx.fused = (self._stream_form and self.device.type == "cuda" and self.dtype == torch.bfloat16 and ops.use_skinny
-                     and (ctx.n <= (ops.TC_MAX_ROWS if ops.use_tc else ops.SKINNY_MAX_ROWS)
+                     and (ctx.n <= (ops.SKINNY_MAX_ROWS if not ops.use_tc else ops.TC_MAX_ROWS if ctx.max_q <= 1
+                                    else max(ops.TC_MAX_ROWS, ops.STREAM_PROMPT_MAX_ROWS))
                           or 0 < ops.PROMPT_MIN_ROWS <= ctx.n))
         if ctx.fused:
             return self._forward_few_rows(ctx, views)
@@ -222,7 +223,7 @@ class ModelRunner:
         return self.plan.embedding.forward(ctx)
 
     def _forward_few_rows(self, ctx: StepContext, views: List[CacheView]) -> Optional[torch.Tensor]:
-        """The same model for a step of at most 16 rows (decode): every block runs in its
+        """The same model for a step of few rows (decode, short prompts): every block runs in its
         stream form, see :meth:`PreNormBlock.forward_stream`."""
         from ..parts.base import StreamState
         plan = self.plan

@@ -23,6 +23,10 @@ from ..csrc import build as _build
 F32, BF16 = 0, 1
 _DT = {torch.float32: F32, torch.bfloat16: BF16}
 
+#: how the types of the libraries' functions (csrc/build.py: exports) are declared: a call then takes plain numbers, where
+#: every pointer had to be wrapped in an object of its own
+_CTYPES = {"ptr": ctypes.c_void_p, "int": ctypes.c_int, "long long": ctypes.c_longlong, "float": ctypes.c_float, "void": None}
+
 _libs: Dict[str, ctypes.CDLL] = {}
 _lock = threading.Lock()
 loaded_libraries: Dict[str, str] = {}
@@ -41,6 +45,9 @@ def _lib(name: str) -> ctypes.CDLL:
         if lib is None:
             path = _build.build(name)
             lib = ctypes.CDLL(path)
+            for fn, (result, *params) in _build.exports(name).items():
+                f = getattr(lib, fn)
+                f.argtypes, f.restype = [_CTYPES[p] for p in params], _CTYPES[result]
             lib.vapi_last_error.restype = ctypes.c_char_p
             _libs[name] = lib
             loaded_libraries[name] = path
@@ -118,16 +125,16 @@ def _cuda(*ts: Optional[torch.Tensor]) -> None:
             raise KernelError("vapi_b200 kernels run on CUDA tensors only; there is no CPU fallback")
 
 
-def _p(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def _p(t: Optional[torch.Tensor]) -> Optional[int]:
+    return None if t is None else t.data_ptr()
 
 
 _held_stream = threading.local()
 
 
-def _stream() -> ctypes.c_void_p:
+def _stream() -> int:
     h = getattr(_held_stream, "handle", None)
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream if h is None else h)
+    return torch.cuda.current_stream().cuda_stream if h is None else h
 
 
 class one_stream:
@@ -411,6 +418,13 @@ def skinny_linear(weight: torch.Tensor, *, act: Optional[torch.Tensor] = None,
 #: beats the library's product plus separate norm / SwiGLU / add kernels at 32 rows (1.26 vs 1.33
 #: ms), loses narrowly at 64 (1.71 vs 1.68 ms) and clearly beyond (2-7x slower at 256 rows).
 TC_MAX_ROWS = int(os.environ.get("VAPI_TC_MAX_ROWS", "32"))
+#: steps with a prompt portion run the stream form of their blocks (norms, SwiGLU and residual adds inside the products)
+#: up to this many rows.  They are launched one by one, and what bounds them is the launches, of which this form has 81 where
+#: the other has 145 (57 tokens of LFM2-700M: 2.03 -> 1.77 ms, while the kernels themselves take 1.0 instead of 0.82 ms).
+#: From 129 rows on a product's tokens no longer fit beside a share of K (200 tokens of LFM2-700M: 1.98 -> 4.37 ms), and
+#: captured decode steps, which cost no launches, stay with TC_MAX_ROWS (LFM2-2.6B, 64 requests: 1.93 ms a step on the
+#: library, 2.08 ms in this form).
+STREAM_PROMPT_MAX_ROWS = 128
 #: set False to keep products of 17..TC_MAX_ROWS rows on the library
 use_tc = os.environ.get("VAPI_TC", "1") != "0"
 
@@ -464,10 +478,11 @@ def skinny_shortconv(w_in: torch.Tensor, *, xw: torch.Tensor, ss_in: torch.Tenso
     return out
 
 
-def tc_applies(rows: int, weight: torch.Tensor) -> bool:
-    """Whether the tcgen05 kernel takes this product: bfloat16 weight, 17..TC_MAX_ROWS rows, inner size
+def tc_applies(rows: int, weight: torch.Tensor, most: Optional[int] = None) -> bool:
+    """Whether the tcgen05 kernel takes this product: bfloat16 weight, 17..``most`` rows (TC_MAX_ROWS), inner size
     a multiple of 8 (16-byte rows for TMA)."""
-    return (use_tc and weight.is_cuda and weight.dtype == torch.bfloat16 and SKINNY_MAX_ROWS < rows <= TC_MAX_ROWS
+    return (use_tc and weight.is_cuda and weight.dtype == torch.bfloat16
+            and SKINNY_MAX_ROWS < rows <= (TC_MAX_ROWS if most is None else most)
             and weight.dim() == 2 and weight.shape[1] % 8 == 0 and weight.is_contiguous())
 
 
@@ -503,10 +518,10 @@ def _fused_product(which: str, weight: torch.Tensor, act, xw, ss_in, eps: float,
         raise KernelError(f"unknown epilogue {epilogue}")
     lib = _lib(which)
     if which == "linear_tc":
-        parts = _tc_plan(N, K, M, _EPI[epilogue])[0]
+        parts = _tc_plan(N, K, M, _EPI[epilogue])[0] if epilogue == "resid" else 0      # (only the sums of squares ask)
         fn = lib.vapi_linear_tc
     else:
-        parts = _prompt_plan(N, K, M, _EPI[epilogue])[2]
+        parts = _prompt_plan(N, K, M, _EPI[epilogue])[2] if epilogue == "resid" else 0
         fn = lib.vapi_prompt_linear
     out_bf16 = out_f32 = sso = xwo = None
     out_stride = N
@@ -633,15 +648,18 @@ def prompt_linear(weight: torch.Tensor, *, act: Optional[torch.Tensor] = None, x
 def few_rows_applies(rows: int, weight: torch.Tensor) -> bool:
     """Whether one of this package's own products (with their fused prologues and epilogues)
     takes a step of ``rows`` rows against ``weight``."""
-    return skinny_applies(rows, weight) or tc_applies(rows, weight) or prompt_applies(rows, weight)
+    return (skinny_applies(rows, weight) or tc_applies(rows, weight, max(TC_MAX_ROWS, STREAM_PROMPT_MAX_ROWS))
+            or prompt_applies(rows, weight))
 
 
 def few_rows_linear(weight: torch.Tensor, **kw):
-    """:func:`skinny_linear` up to 16 rows, :func:`linear_tc` up to TC_MAX_ROWS, :func:`prompt_linear` above."""
-    src = kw.get("act") if kw.get("act") is not None else kw.get("xw")
-    if src.shape[0] <= SKINNY_MAX_ROWS:
+    """:func:`skinny_linear` up to 16 rows, :func:`linear_tc` up to TC_MAX_ROWS (STREAM_PROMPT_MAX_ROWS, where the prompt
+    product is not in use), :func:`prompt_linear` above."""
+    act = kw.get("act")
+    rows = (act if act is not None else kw["xw"]).shape[0]
+    if rows <= SKINNY_MAX_ROWS:
         return skinny_linear(weight, **kw)
-    if src.shape[0] <= TC_MAX_ROWS:
+    if rows <= TC_MAX_ROWS or (rows <= STREAM_PROMPT_MAX_ROWS and not prompt_applies(rows, weight)):
         return linear_tc(weight, **kw)
     return prompt_linear(weight, **kw)
 
@@ -1638,7 +1656,6 @@ def gated_delta(qkv: torch.Tensor, ab: torch.Tensor, A_log: torch.Tensor, dt_bia
             dk, dv, state.shape[0], ctypes.c_float(norm_eps), int(min(max_q, 1 << 30)), chunks, _p(status), _stream()))
     if chunks:
         lib = _lib("recurrent_chunks")
-        lib.vapi_delta_chunks_scratch.restype = ctypes.c_longlong
         scratch = torch.empty(lib.vapi_delta_chunks_scratch(n, seqs, nh), dtype=torch.uint8, device=qkv.device)
         _check(lib, lib.vapi_gated_delta_chunks(
             _p(qkv), ctypes.c_longlong(qkv.stride(0)), 0, nkv * dk, 2 * nkv * dk, _p(ab), ctypes.c_longlong(ab.stride(0)),
@@ -2112,7 +2129,6 @@ def fixed_decay_memory(qkv: torch.Tensor, powers: torch.Tensor, state: torch.Ten
     if (0 < least <= max_q and qkv.dtype == torch.bfloat16 and dk % 8 == 0 and dv % 8 == 0 and qkv.stride(0) % 8 == 0
             and qkv.data_ptr() % 16 == 0 and state.stride(0) % 2 == 0 and state.data_ptr() % 8 == 0):
         chunks = n // FIXED_DECAY_CHUNK + min(S, n // least)
-        lib.vapi_fixed_decay_chunk_words.restype = ctypes.c_longlong
         words = lib.vapi_fixed_decay_chunk_words(nh, dk, dv)
         scratch = torch.empty((chunks * words * 4,), dtype=torch.int32, device=qkv.device)
     launches = 1 if scratch is None else (2 if S == 1 else 3)
