@@ -71,10 +71,10 @@ flash_f32_kernel(const float* q, long long q_row_stride, const float* cache, con
     unsigned char *sK = sQ + 3 * FF_PLANE, *sV = sK + 3 * FF_PLANE;
     float *fK = reinterpret_cast<float*>(sV + 3 * FF_PLANE), *fV = fK + FF_BK * FF_HD;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g4 = lane >> 2, p4 = (lane & 3) * 2, mat = lane >> 3, r8 = lane & 7;
-    const int g = blockIdx.y, sp = blockIdx.z, n_rep = nh / nkv;
+    const int g = (int)blockIdx.x % nkv, sp = blockIdx.y, n_rep = nh / nkv;      // (heads side by side: the longest tiles of all start first)
     pdl_trigger();
     int s = 0, tile = 0;
-    const bool mine = ft_tile(cu_q, num_seqs, 1, n_rep, FF_ROWS, (int)blockIdx.x, s, tile);
+    const bool mine = ft_tile(cu_q, num_seqs, 1, n_rep, FF_ROWS, (int)blockIdx.x / nkv, s, tile);
     pdl_wait();
     if (!mine) return;
     const int q0 = cu_q[s], qlen = cu_q[s + 1] - q0, klen = seqlens_k[s];
@@ -284,7 +284,7 @@ static int launch_flash_f32(const void* q, long long q_row_stride, const void* c
     const int n_rep = nh / nkv;
     const long long longest = ((long long)max_q * n_rep + FF_ROWS - 1) / FF_ROWS, whole = (long long)n * n_rep / FF_ROWS + num_seqs;
     const long long tiles = longest * num_seqs < whole ? longest * num_seqs : whole;
-    if (tiles > 0x7fffffffLL || nkv > 65535 || (long long)num_seqs * splits > 65535)
+    if (tiles * nkv > 0x7fffffffLL || nkv > 65535 || (long long)num_seqs * splits > 65535)
         return fail(-1, "paged_attention: %d kv heads or %d sequences x %d splits exceed the grid", nkv, num_seqs, splits);
     static bool attr_set = false;
     if (!attr_set) {
@@ -292,7 +292,7 @@ static int launch_flash_f32(const void* q, long long q_row_stride, const void* c
         if (e != cudaSuccess) return fail(-101, "paged_attention: cannot reserve %zu bytes of shared memory: %s", FF_SMEM, cudaGetErrorString(e));
         attr_set = true;
     }
-    return check_launch("paged_attention (float)", launch(flash_f32_kernel, dim3((unsigned)tiles, nkv, splits), dim3(FF_THREADS), FF_SMEM, stream,
+    return check_launch("paged_attention (float)", launch(flash_f32_kernel, dim3((unsigned)(tiles * nkv), splits), dim3(FF_THREADS), FF_SMEM, stream,
         (const float*)q, q_row_stride, (const float*)cache, block_table, table_stride, cu_q, seqlens_k, (float*)out, part_o, part_ml,
         num_seqs, nh, nkv, page_size, num_pages, scale, window, splits, status));
 }

@@ -124,11 +124,13 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const FaTcParams p) {
     int* flags = reinterpret_cast<int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = blockIdx.y, n_rep = p.nh / p.nkv;
+    // (heads side by side, so that the longest tiles of all heads start first: head by head, the last head's longest tile started
+    // when half of the kernel was over: 2,048 tokens, 32 / 8 heads 68 us, so 54)
+    const int g = (int)blockIdx.x % p.nkv, n_rep = p.nh / p.nkv;
     pdl_trigger();
     // index data was copied from the host before the step's first kernel: safe before the wait
     int s = 0, tile = 0;
-    if (!ft_tile(p.cu_q, p.num_seqs, p.min_q, n_rep, FT_ROWS, (int)blockIdx.x, s, tile)) {
+    if (!ft_tile(p.cu_q, p.num_seqs, p.min_q, n_rep, FT_ROWS, (int)blockIdx.x / p.nkv, s, tile)) {
         pdl_wait();
         return;
     }
@@ -447,7 +449,7 @@ static int launch_flash_tc(const void* q, long long q_row_stride, const void* ca
     // tiles of all sequences together: at most those of n tokens in one piece and a ragged one a sequence
     const long long longest = ((long long)max_q * n_rep + FT_ROWS - 1) / FT_ROWS, whole = (long long)n * n_rep / FT_ROWS + num_seqs;
     const long long tiles = longest * num_seqs < whole ? longest * num_seqs : whole;
-    if (tiles > 0x7fffffffLL || nkv > 65535 || num_seqs > 65535)
+    if (tiles * nkv > 0x7fffffffLL || nkv > 65535 || num_seqs > 65535)
         return fail(-1, "paged_attention: the step exceeds the grid (%lld row tiles, %d kv heads, %d sequences)", tiles, nkv, num_seqs);
     if (!(scale > 0.f)) return fail(-1, "paged_attention: the tcgen05 kernel needs a positive scale");
     if (q_row_stride % 8 != 0 || ((uintptr_t)q & 15) != 0 || ((uintptr_t)out & 15) != 0 || form.out_stride % 8 != 0)
@@ -468,7 +470,7 @@ static int launch_flash_tc(const void* q, long long q_row_stride, const void* ca
     p.mask_chunk = mask_chunk; p.keep = keep; p.sinks = sinks; p.gate = (const __nv_bfloat16*)gate; p.gate_stride = gate_stride;
     p.sig = sigmoid_form(scale, form.softcap); p.score_bias = form.bias; p.out_scale = form.out_scale;
     p.out_stride = form.out_stride > 0 ? form.out_stride : (long long)nh * FT_HD;
-    dim3 grid((unsigned)tiles, nkv);
+    dim3 grid((unsigned)(tiles * nkv));
     return check_launch("paged_attention (tcgen05)", launch(flash_tc_kernel<SIG>, grid, FT_THREADS, FT_SMEM, stream, map, p));
 }
 
