@@ -22,11 +22,10 @@
 // independent of each other: a block owns a head and 32 (state space) or 16 (delta rule) of them, which gives 128 blocks for
 // one sequence of either recurrence at the widths this is for.  T = (I + A)^-1 and the scores do not depend on the state: a
 // kernel before the walk works them out for all chunks at once (its own substitution, in float) and leaves them as
-// bfloat16 planes in scratch memory.  One sequence of 2,000 tokens: state space (64 heads of 64) 704 -> 161 us, delta rule (16
-// heads of 128) 624 -> 142 us with the kernel before it; of 300 tokens 110 -> 29 and 97 -> 31 us.  Against float64 neither is
+// bfloat16 planes in scratch memory.  One sequence of 2,000 tokens: state space (64 heads of 64) 701 -> 167 us, delta rule (16
+// heads of 128) 624 -> 152 us with the kernel before it; of 300 tokens 110 -> 30 and 97 -> 33 us.  Against float64 neither is
 // further off than the walk (1.0e-7 to 1.7e-7 of the outputs' 2-norm against 1.1e-7 to 1.9e-7).  What bounds it now is the chain
-// of a chunk's dependent instructions and barriers, 3.5 to 5 us a chunk with two warps a scheduler (issue slots used 0.3, tensor
-// pipe 0.21 to 0.26; 12 and 16 warps with half of the products each took 172 and 135 us where these take 161 and 112).
+// of a chunk's matrix products and barriers, ~5 us a chunk.
 //
 // Every sequence of a step takes the walk of recurrent.cu or the chunks by its own number of tokens alone.
 #include "common.cuh"
@@ -46,15 +45,19 @@ constexpr int RC_SS_COLS = 32, RC_SS_XLD = RC_SS_COLS + 8;
 constexpr int RC_GD_COLS = 16, RC_GD_CLD = RC_GD_COLS + 8, RC_TLD = RC_T + 8;
 
 __device__ __forceinline__ float rc_softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
-// two floats as three pairs of bfloat16 that add up to them (an infinity leaves a NaN behind it: a chunk that holds one has no
-// finite outputs from there on, nor before it, where the walk has infinities or NaN from that token on)
+// what is left of x beside its bfloat16 part; nothing where that part is not finite
+__device__ __forceinline__ float rc_rest(float x, unsigned bits) {
+    const float p = __uint_as_float(bits);
+    return (bits & 0x7f800000u) == 0x7f800000u ? 0.f : x - p;
+}
+// two floats as three pairs of bfloat16 that add up to them
 __device__ __forceinline__ void rc_split(float a, float b, unsigned& p1, unsigned& p2, unsigned& p3) {
     p1 = pack_bf16(a, b);
-    a -= __uint_as_float(p1 << 16);
-    b -= __uint_as_float(p1 & 0xffff0000u);
+    a = rc_rest(a, p1 << 16);
+    b = rc_rest(b, p1 & 0xffff0000u);
     p2 = pack_bf16(a, b);
-    a -= __uint_as_float(p2 << 16);
-    b -= __uint_as_float(p2 & 0xffff0000u);
+    a = rc_rest(a, p2 << 16);
+    b = rc_rest(b, p2 & 0xffff0000u);
     p3 = pack_bf16(a, b);
 }
 template <int N> __device__ __forceinline__ void rc_zero(float (&t)[N][4]) {
@@ -218,8 +221,7 @@ state_space_chunks_kernel(const __nv_bfloat16* __restrict__ xbc, long long xbc_s
             const int m0 = warp * 16;
             float cb[2][8][4], y[2][4][4], low[4][4];       // [k even | odd], first plane; the other planes
             rc_zero(cb[0]); rc_zero(cb[1]); rc_zero(y[0]); rc_zero(y[1]); rc_zero(low);
-            // (unrolled no further than the accumulators ask for: a chunk's straight code does not fit the instruction caches)
-#pragma unroll 2
+#pragma unroll
             for (int k = 0; k < RC_ROWS / 16; ++k) {
                 unsigned a[4], b[4];
                 rc_a(a, &sm.C[buf][0][0], RC_LD, m0, k * 16);
@@ -295,7 +297,7 @@ state_space_chunks_kernel(const __nv_bfloat16* __restrict__ xbc, long long xbc_s
             const float last = sm.last[buf];
             float add[2][4][4], low[2][4][4];
             rc_zero(add[0]); rc_zero(add[1]); rc_zero(low[0]); rc_zero(low[1]);
-#pragma unroll 1
+#pragma unroll
             for (int kt = 0; kt < 4; ++kt) {
                 unsigned b[2][4];
 #pragma unroll
@@ -547,15 +549,14 @@ struct RcGdSmem {
     float scal[2][5][RC_T];
 };
 
-// The six products of weight 2^-16 and above of two operands in planes: the first planes' into acc, the others into two more
-// accumulators (one chain of five a step would be what a chunk waits for)
-__device__ __forceinline__ void rc_mma6(float (&acc)[4], float (&low)[2][4], const unsigned (&a)[3][4], const unsigned (&b)[3][4], int half) {
-    mma_bf16_16816(low[0], a[2], b[0][2 * half], b[0][2 * half + 1]);
-    mma_bf16_16816(low[1], a[0], b[2][2 * half], b[2][2 * half + 1]);
+// The six products of weight 2^-16 and above of two operands in planes: the first planes' into acc, the others into low
+__device__ __forceinline__ void rc_mma6(float (&acc)[4], float (&low)[4], const unsigned (&a)[3][4], const unsigned (&b)[3][4], int half) {
+    mma_bf16_16816(low, a[2], b[0][2 * half], b[0][2 * half + 1]);
+    mma_bf16_16816(low, a[0], b[2][2 * half], b[2][2 * half + 1]);
+    mma_bf16_16816(low, a[1], b[1][2 * half], b[1][2 * half + 1]);
+    mma_bf16_16816(low, a[1], b[0][2 * half], b[0][2 * half + 1]);
+    mma_bf16_16816(low, a[0], b[1][2 * half], b[1][2 * half + 1]);
     mma_bf16_16816(acc, a[0], b[0][2 * half], b[0][2 * half + 1]);
-    mma_bf16_16816(low[0], a[1], b[1][2 * half], b[1][2 * half + 1]);
-    mma_bf16_16816(low[1], a[1], b[0][2 * half], b[0][2 * half + 1]);
-    mma_bf16_16816(low[0], a[0], b[1][2 * half], b[1][2 * half + 1]);
 }
 
 // A chunk has three parts with a barrier behind each: k.S (warps 0..3, 16 tokens each: R) and q.S (warps 4..7, kept in
@@ -635,10 +636,10 @@ delta_chunks_kernel(const __nv_bfloat16* __restrict__ qkv, long long qkv_stride,
         else cp_async_commit();
         const int ta = quad * 16 + g4, tb = ta + 8;
         // ---- k.S and q.S ----
-        float ks[2][4];
+        float ks[2][4], low[2][4];
         {
-            float odd[2][4], low[2][2][4];
-            rc_zero(ks); rc_zero(odd); rc_zero(low[0]); rc_zero(low[1]);
+            float odd[2][4];
+            rc_zero(ks); rc_zero(odd); rc_zero(low);
             const __nv_bfloat16* rows = warp < 4 ? &sm.K[buf][0][0] : &sm.Q[buf][0][0];
 #pragma unroll
             for (int k = 0; k < RC_ROWS / 16; ++k) {
@@ -647,14 +648,14 @@ delta_chunks_kernel(const __nv_bfloat16* __restrict__ qkv, long long qkv_stride,
 #pragma unroll
                 for (int pl = 2; pl >= 0; --pl) {
                     rc_b(b, &sm.S[pl][0][0], RC_LD, 0, k * 16);
-                    mma_bf16_16816(pl ? low[pl - 1][0] : (k & 1 ? odd[0] : ks[0]), a, b[0], b[1]);
-                    mma_bf16_16816(pl ? low[pl - 1][1] : (k & 1 ? odd[1] : ks[1]), a, b[2], b[3]);
+                    mma_bf16_16816(pl ? low[0] : (k & 1 ? odd[0] : ks[0]), a, b[0], b[1]);
+                    mma_bf16_16816(pl ? low[1] : (k & 1 ? odd[1] : ks[1]), a, b[2], b[3]);
                 }
             }
 #pragma unroll
             for (int n = 0; n < 2; ++n)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) ks[n][i] = (ks[n][i] + odd[n][i]) + (low[0][n][i] + low[1][n][i]);
+                for (int i = 0; i < 4; ++i) ks[n][i] = (ks[n][i] + odd[n][i]) + low[n][i];
         }
         if (warp < 4) {
             const float ba = sm.scal[buf][0][ta], bb = sm.scal[buf][0][tb], ra = sm.scal[buf][1][ta], rb = sm.scal[buf][1][tb];
@@ -676,8 +677,7 @@ delta_chunks_kernel(const __nv_bfloat16* __restrict__ qkv, long long qkv_stride,
         __syncthreads();
         // ---- U = T R: 16 tokens x 8 columns a warp ----
         {
-            float u[4] = {0.f, 0.f, 0.f, 0.f}, ul[2][4];
-            rc_zero(ul);
+            float u[4] = {0.f, 0.f, 0.f, 0.f}, ul[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int kt = 0; kt < 4; ++kt)
                 if (kt <= quad) {
@@ -691,7 +691,7 @@ delta_chunks_kernel(const __nv_bfloat16* __restrict__ qkv, long long qkv_stride,
                     else rc_mma6(u, ul, a, b, 1);
                 }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) u[i] += ul[0][i] + ul[1][i];
+            for (int i = 0; i < 4; ++i) u[i] += ul[i];
             const float wa = sm.scal[buf][3][ta], wb = sm.scal[buf][3][tb];
             const int col = (warp >> 2) * 8 + p4;
 #pragma unroll
@@ -716,8 +716,8 @@ delta_chunks_kernel(const __nv_bfloat16* __restrict__ qkv, long long qkv_stride,
             const float ea = sm.scal[buf][2][ta], eb = sm.scal[buf][2][tb];
 #pragma unroll
             for (int n = 0; n < 2; ++n) { ks[n][0] *= ea; ks[n][1] *= ea; ks[n][2] *= eb; ks[n][3] *= eb; }
-            float o[2][4], low[2][2][4];
-            rc_zero(o); rc_zero(low[0]); rc_zero(low[1]);
+            float o[2][4];
+            rc_zero(o); rc_zero(low);
 #pragma unroll
             for (int kt = 0; kt < 4; ++kt)
                 if (kt <= quad) {
@@ -737,8 +737,7 @@ delta_chunks_kernel(const __nv_bfloat16* __restrict__ qkv, long long qkv_stride,
                     const int at = c * RC_T + (q ? tb : ta);
                     if (at < qlen)
                         *reinterpret_cast<float2*>(out + ((size_t)(t0 + at) * nh + h) * cols + col0 + n * 8 + p4) = 
-                            make_float2((o[n][2 * q] + (low[n][0][2 * q] + low[n][1][2 * q])) + ks[n][2 * q],
-                                        (o[n][2 * q + 1] + (low[n][0][2 * q + 1] + low[n][1][2 * q + 1])) + ks[n][2 * q + 1]);
+                            make_float2((o[n][2 * q] + low[n][2 * q]) + ks[n][2 * q], (o[n][2 * q + 1] + low[n][2 * q + 1]) + ks[n][2 * q + 1]);
                 }
         } else {
             // ---- the state ----
