@@ -322,7 +322,7 @@ gated_delta_kernel(const T* __restrict__ qkv, long long qkv_stride, int q_off, i
                    const float* __restrict__ dt_bias, float* __restrict__ state, long long slot_stride,
                    const int* __restrict__ state_slots, const int* __restrict__ cu_q,
                    const int* __restrict__ positions, float* __restrict__ out, int nh, int nkv, int rows, int cols,
-                   int num_slots, float norm_eps, int walk_below, int* __restrict__ status) {
+                   int num_slots, float norm_eps, int* __restrict__ status) {
     using Stage = RecStage<T, RT, LPC>;
     constexpr int CPB = Stage::CPB, RPP = Stage::RPP;
     __shared__ __align__(16) float sk[REC_TC * RPP], sq[REC_TC * RPP];
@@ -336,10 +336,7 @@ gated_delta_kernel(const T* __restrict__ qkv, long long qkv_stride, int q_off, i
     const bool col_ok = col < cols;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = cu_q[s], qlen = cu_q[s + 1] - t0;
-    if (qlen <= 0 || (walk_below > 0 && qlen >= walk_below)) {       // (nothing to do, or another kernel's sequence)
-        pdl_wait();
-        return;
-    }
+    if (qlen <= 0) return;
     const int slot = state_slots[s];
     if (slot < 0 || slot >= num_slots) {
         if (threadIdx.x == 0 && status) atomicExch(status, 3);
@@ -453,7 +450,7 @@ state_space_kernel(const T* __restrict__ xbc, long long xbc_stride, const T* __r
                    const float* __restrict__ A_log, const float* __restrict__ dt_bias, const float* __restrict__ D,
                    float* __restrict__ state, long long slot_stride, const int* __restrict__ state_slots,
                    const int* __restrict__ cu_q, const int* __restrict__ positions, float* __restrict__ out, int nh,
-                   int groups, int rows, int cols, int num_slots, int walk_below, int* __restrict__ status) {
+                   int groups, int rows, int cols, int num_slots, int* __restrict__ status) {
     using Stage = RecStage<T, RT, LPC>;
     constexpr int CPB = Stage::CPB, RPP = Stage::RPP;
     __shared__ __align__(16) float sB[REC_TC * RPP], sC[REC_TC * RPP];
@@ -467,10 +464,7 @@ state_space_kernel(const T* __restrict__ xbc, long long xbc_stride, const T* __r
     const bool col_ok = col < cols;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = cu_q[s], qlen = cu_q[s + 1] - t0;
-    if (qlen <= 0 || (walk_below > 0 && qlen >= walk_below)) {       // (nothing to do, or another kernel's sequence)
-        pdl_wait();
-        return;
-    }
+    if (qlen <= 0) return;
     const int slot = state_slots[s];
     if (slot < 0 || slot >= num_slots) {
         if (threadIdx.x == 0 && status) atomicExch(status, 3);
@@ -562,14 +556,13 @@ state_space_kernel(const T* __restrict__ xbc, long long xbc_stride, const T* __r
         else { CALL(16, 16); }                                      \
     } while (0)
 
-// walk_below > 0: sequences that bring at least that many tokens are left alone (recurrent_chunks.cu takes them)
 static inline int rec_lpc(int rows) { return rows <= 32 ? 4 : (rows <= 128 ? 8 : 16); }
 
 VAPI_EXPORT int vapi_gated_delta(const void* qkv, long long qkv_stride, int q_off, int k_off, int v_off, const void* ab,
                                  long long ab_stride, int dtype, const float* A_log, const float* dt_bias, float* state,
                                  long long slot_stride, const int* state_slots, const int* cu_q, const int* positions,
                                  float* out, int num_seqs, int nh, int nkv, int rows, int cols, int num_slots,
-                                 float norm_eps, int max_q, int walk_below, int* status, cudaStream_t stream) {
+                                 float norm_eps, int max_q, int* status, cudaStream_t stream) {
     if (num_seqs <= 0) return 0;
     if (nh <= 0 || nkv <= 0 || nh % nkv || rows <= 0 || rows > 256 || cols <= 0)
         return fail(-1, "gated_delta: %d heads over %d, state %d x %d (rows up to 256)", nh, nkv, rows, cols);
@@ -581,11 +574,11 @@ VAPI_EXPORT int vapi_gated_delta(const void* qkv, long long qkv_stride, int q_of
     if (dtype == VAPI_F32)                                                                                                 \
         e = launch_if(early, gated_delta_kernel<float, RT, LPC>, grid, REC_THREADS, 0, stream, (const float*)qkv, qkv_stride, q_off, \
                    k_off, v_off, (const float*)ab, ab_stride, A_log, dt_bias, state, slot_stride, state_slots, cu_q,       \
-                   positions, out, nh, nkv, rows, cols, num_slots, norm_eps, walk_below, status);                                      \
+                   positions, out, nh, nkv, rows, cols, num_slots, norm_eps, status);                                      \
     else                                                                                                                   \
         e = launch_if(early, gated_delta_kernel<__nv_bfloat16, RT, LPC>, grid, REC_THREADS, 0, stream, (const __nv_bfloat16*)qkv,    \
                    qkv_stride, q_off, k_off, v_off, (const __nv_bfloat16*)ab, ab_stride, A_log, dt_bias, state,            \
-                   slot_stride, state_slots, cu_q, positions, out, nh, nkv, rows, cols, num_slots, norm_eps, walk_below, status)
+                   slot_stride, state_slots, cu_q, positions, out, nh, nkv, rows, cols, num_slots, norm_eps, status)
     if (dtype != VAPI_F32 && dtype != VAPI_BF16) return fail(-2, "gated_delta: unsupported dtype %d", dtype);
     REC_DISPATCH(rows, GD_CALL);
 #undef GD_CALL
@@ -596,7 +589,7 @@ VAPI_EXPORT int vapi_state_space(const void* xbc, long long xbc_stride, const vo
                                  const float* A_log, const float* dt_bias, const float* D, float* state,
                                  long long slot_stride, const int* state_slots, const int* cu_q, const int* positions,
                                  float* out, int num_seqs, int nh, int groups, int rows, int cols, int num_slots,
-                                 int max_q, int walk_below, int* status, cudaStream_t stream) {
+                                 int max_q, int* status, cudaStream_t stream) {
     if (num_seqs <= 0) return 0;
     if (nh <= 0 || groups <= 0 || nh % groups || rows <= 0 || rows > 256 || cols <= 0)
         return fail(-1, "state_space: %d heads over %d groups, state %d x %d (rows up to 256)", nh, groups, rows, cols);
@@ -608,11 +601,11 @@ VAPI_EXPORT int vapi_state_space(const void* xbc, long long xbc_stride, const vo
     if (dtype == VAPI_F32)                                                                                                \
         e = launch_if(early, state_space_kernel<float, RT, LPC>, grid, REC_THREADS, 0, stream, (const float*)xbc, xbc_stride,       \
                    (const float*)dt, dt_stride, A_log, dt_bias, D, state, slot_stride, state_slots, cu_q, positions, out, \
-                   nh, groups, rows, cols, num_slots, walk_below, status);                                                            \
+                   nh, groups, rows, cols, num_slots, status);                                                            \
     else                                                                                                                  \
         e = launch_if(early, state_space_kernel<__nv_bfloat16, RT, LPC>, grid, REC_THREADS, 0, stream, (const __nv_bfloat16*)xbc,   \
                    xbc_stride, (const __nv_bfloat16*)dt, dt_stride, A_log, dt_bias, D, state, slot_stride, state_slots,   \
-                   cu_q, positions, out, nh, groups, rows, cols, num_slots, walk_below, status)
+                   cu_q, positions, out, nh, groups, rows, cols, num_slots, status)
     if (dtype != VAPI_F32 && dtype != VAPI_BF16) return fail(-2, "state_space: unsupported dtype %d", dtype);
     REC_DISPATCH(rows, SS_CALL);
 #undef SS_CALL

@@ -1607,16 +1607,6 @@ def causal_conv(x: torch.Tensor, taps: torch.Tensor, bias: Optional[torch.Tensor
     return out
 
 
-def _recurrent_chunk_rule(delta: bool, rows: torch.Tensor, state_rows: int, cols_fit: bool, n: int, max_q: int) -> int:
-    """From how many tokens on a sequence of this step is taken in chunks (csrc/recurrent_chunks.cu); 0: none is.  bfloat16
-    rows on 16-byte boundaries, states of 128 rows, and a step that can hold such a sequence."""
-    if (rows.dtype != torch.bfloat16 or state_rows != 128 or not cols_fit or rows.stride(0) % 8 or rows.data_ptr() % 16
-            or rows.shape[1] % 8):
-        return 0
-    least = int(_lib("recurrent_chunks").vapi_recurrent_chunks_min(1 if delta else 0))
-    return least if min(n, max_q) >= least else 0
-
-
 def gated_delta(qkv: torch.Tensor, ab: torch.Tensor, A_log: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor,
                 state_offset: int, state_slots: torch.Tensor, cu_q: torch.Tensor, positions: torch.Tensor, nh: int,
                 nkv: int, dk: int, dv: int, norm_eps: float = 1e-6, status: Optional[torch.Tensor] = None,
@@ -1645,24 +1635,11 @@ def gated_delta(qkv: torch.Tensor, ab: torch.Tensor, A_log: torch.Tensor, dt_bia
         raise KernelError("the state must be float32 [slots, >= offset + heads*dk*dv] with unit inner stride")
     out = torch.empty((n, nh * dv), dtype=torch.float32, device=qkv.device)
     lib = _lib("recurrent")
-    seqs = cu_q.numel() - 1
-    # the step's long sequences in chunks, the others token by token (one that is alone and long enough needs no walk)
-    chunks = _recurrent_chunk_rule(True, qkv, dk, dv % 16 == 0, n, max_q)
-    if chunks == 0 or seqs > 1:
-        _check(lib, lib.vapi_gated_delta(
-            _p(qkv), ctypes.c_longlong(qkv.stride(0)), 0, nkv * dk, 2 * nkv * dk, _p(ab), ctypes.c_longlong(ab.stride(0)),
-            _dt(qkv), _p(A_log), _p(dt_bias), ctypes.c_void_p(state.data_ptr() + 4 * int(state_offset)),
-            ctypes.c_longlong(state.stride(0)), _p(state_slots), _p(cu_q), _p(positions), _p(out), seqs, nh, nkv,
-            dk, dv, state.shape[0], ctypes.c_float(norm_eps), int(min(max_q, 1 << 30)), chunks, _p(status), _stream()))
-    if chunks:
-        lib = _lib("recurrent_chunks")
-        scratch = torch.empty(lib.vapi_delta_chunks_scratch(n, seqs, nh), dtype=torch.uint8, device=qkv.device)
-        _check(lib, lib.vapi_gated_delta_chunks(
-            _p(qkv), ctypes.c_longlong(qkv.stride(0)), 0, nkv * dk, 2 * nkv * dk, _p(ab), ctypes.c_longlong(ab.stride(0)),
-            _p(A_log), _p(dt_bias), ctypes.c_void_p(state.data_ptr() + 4 * int(state_offset)),
-            ctypes.c_longlong(state.stride(0)), _p(state_slots), _p(cu_q), _p(positions), _p(out), n, seqs, nh, nkv,
-            dk, dv, state.shape[0], ctypes.c_float(norm_eps), _p(scratch), chunks if seqs > 1 else 1, _p(status), _stream()),
-            launches=2)
+    _check(lib, lib.vapi_gated_delta(
+        _p(qkv), ctypes.c_longlong(qkv.stride(0)), 0, nkv * dk, 2 * nkv * dk, _p(ab), ctypes.c_longlong(ab.stride(0)),
+        _dt(qkv), _p(A_log), _p(dt_bias), ctypes.c_void_p(state.data_ptr() + 4 * int(state_offset)),
+        ctypes.c_longlong(state.stride(0)), _p(state_slots), _p(cu_q), _p(positions), _p(out), cu_q.numel() - 1, nh, nkv,
+        dk, dv, state.shape[0], ctypes.c_float(norm_eps), int(min(max_q, 1 << 30)), _p(status), _stream()))
     return out
 
 
@@ -1692,22 +1669,11 @@ def state_space(xbc: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, dt_bia
         raise KernelError("the state must be float32 [slots, >= offset + heads*state*head] with unit inner stride")
     out = torch.empty((n, nh * head), dtype=torch.float32, device=xbc.device)
     lib = _lib("recurrent")
-    seqs = cu_q.numel() - 1
-    # the step's long sequences in chunks, the others token by token (one that is alone and long enough needs no walk)
-    chunks = _recurrent_chunk_rule(False, xbc, n_state, head % 32 == 0, n, max_q)
-    if chunks == 0 or seqs > 1:
-        _check(lib, lib.vapi_state_space(
-            _p(xbc), ctypes.c_longlong(xbc.stride(0)), _p(dt), ctypes.c_longlong(dt.stride(0)), _dt(xbc), _p(A_log),
-            _p(dt_bias), _p(D), ctypes.c_void_p(state.data_ptr() + 4 * int(state_offset)), ctypes.c_longlong(state.stride(0)),
-            _p(state_slots), _p(cu_q), _p(positions), _p(out), seqs, nh, groups, n_state, head, state.shape[0],
-            int(min(max_q, 1 << 30)), chunks, _p(status), _stream()))
-    if chunks:
-        lib = _lib("recurrent_chunks")
-        _check(lib, lib.vapi_state_space_chunks(
-            _p(xbc), ctypes.c_longlong(xbc.stride(0)), _p(dt), ctypes.c_longlong(dt.stride(0)), _p(A_log),
-            _p(dt_bias), _p(D), ctypes.c_void_p(state.data_ptr() + 4 * int(state_offset)), ctypes.c_longlong(state.stride(0)),
-            _p(state_slots), _p(cu_q), _p(positions), _p(out), seqs, nh, groups, n_state, head, state.shape[0],
-            chunks if seqs > 1 else 1, _p(status), _stream()))
+    _check(lib, lib.vapi_state_space(
+        _p(xbc), ctypes.c_longlong(xbc.stride(0)), _p(dt), ctypes.c_longlong(dt.stride(0)), _dt(xbc), _p(A_log),
+        _p(dt_bias), _p(D), ctypes.c_void_p(state.data_ptr() + 4 * int(state_offset)), ctypes.c_longlong(state.stride(0)),
+        _p(state_slots), _p(cu_q), _p(positions), _p(out), cu_q.numel() - 1, nh, groups, n_state, head, state.shape[0],
+        int(min(max_q, 1 << 30)), _p(status), _stream()))
     return out
 
 
