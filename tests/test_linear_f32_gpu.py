@@ -38,6 +38,14 @@ def test_float32_product_is_no_further_from_the_exact_one_than_its_bound(ops, M,
     assert M <= 16 or N * K < 1 << 20 or (ops.launch_count == before + 2 and torch.equal(via, got))
 
 
+def test_float32_product_of_more_rows_than_its_scratch_holds(ops, monkeypatch):
+    g = torch.Generator(device="cuda").manual_seed(8)
+    a, w, b = (torch.randn(*s, generator=g, device="cuda") for s in ((301, 260), (140, 260), (140,)))
+    monkeypatch.setattr(ops, "LINEAR_F32_ROWS", 128)
+    got = ops.linear_f32(a, w, b)
+    assert ((got.double() - a.double() @ w.double().t() - b.double()).abs() <= _bound(a, w) + 2.0 ** -23 * b.double().abs()).all()
+
+
 @pytest.mark.parametrize("M,N,K", [(70, 300, 256), (40, 130, 2048), (300, 20000, 68)])
 def test_float32_product_of_what_cannot_be_split(ops, M, N, K):
     """Infinities, NaN and magnitudes next to the largest float, in tokens and in weights, in the first and the last row, in tiles of one

@@ -690,6 +690,8 @@ def skinny_linear_f32(weight: torch.Tensor, act: torch.Tensor, bias: Optional[to
 
 #: numbers in a float32 weight from which on products of more than 16 rows go to csrc/linear_f32.cu
 LINEAR_F32_LEAST = 1 << 20
+#: rows that go through that kernel at a time: its scratch (three bfloat16 planes of them) stays at 6 bytes x this x the inner size
+LINEAR_F32_ROWS = 4096
 
 
 def linear_f32_applies(x: torch.Tensor, weight: torch.Tensor) -> bool:
@@ -719,11 +721,14 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     _i32(status, "status")
     out = torch.empty((M, N), dtype=torch.float32, device=weight.device)
     kp = -(-K // 8) * 8
-    planes = torch.empty(3 * M * kp, dtype=torch.bfloat16, device=weight.device)
-    bad = torch.empty(M, dtype=torch.int32, device=weight.device)
+    most = min(M, LINEAR_F32_ROWS)
+    planes = torch.empty(3 * most * kp, dtype=torch.bfloat16, device=weight.device)
+    bad = torch.empty(most, dtype=torch.int32, device=weight.device)
     lib = _lib("linear_f32")
-    _check(lib, lib.vapi_linear_f32(_p(weight), N, K, M, _p(x), _p(planes), _p(bad), _p(bias), _p(out), ctypes.c_longlong(N),
-                                    _p(status), _stream()), launches=2)
+    for at in range(0, M, LINEAR_F32_ROWS):
+        rows = min(most, M - at)
+        _check(lib, lib.vapi_linear_f32(_p(weight), N, K, rows, x.data_ptr() + 4 * at * K, _p(planes), _p(bad), _p(bias),
+                                        out.data_ptr() + 4 * at * N, N, _p(status), _stream()), launches=2)
     return out
 
 
