@@ -870,9 +870,13 @@ def attention_splits(num_seqs: int, max_q: int, max_k: int, nh: int, nkv: int, d
     The decode kernel (measured at head size 64, 8 kv heads, context 4096 and 32768): while the
     (sequence, kv head) pairs are fewer than two blocks per SM, slices up to that many blocks, and
     no more than the kernel combines itself unless a slice would then be longer than 32 tiles and
-    there would be fewer blocks than SMs;
-    a step with more pairs than the device holds blocks is cut for about four rounds of blocks, so
-    that the last ones do not run alone."""
+    there would be fewer blocks than SMs.
+    A step with more pairs than half of what the device holds is only cut where its longest sequences could be long: to
+    slices of about 32 tiles, or of 24 where the pairs alone are more than the device holds, and into no more
+    than four rounds of blocks.  Slices cost a block's start each and a combine kernel (8 kv heads, both kernels): 64 sequences of
+    128 to 2,048 keys 28.8 us whole, 35.2 / 38.5 / 39.9 in 2 / 3 / 4 slices; of 20 to 300 10.4 and 22.6 in 4; 32 of 33 to 700
+    11.5 and 13.6 in 2, but 32 of 500 to 4,000 48.5 whole and 32.5 in 2, where the longest sequence's block runs alone, and 64
+    of 4,096 114 whole, 96 in 3 and 95 in 4."""
     n_rep = nh // nkv
     rows = max_q * n_rep
     tiles = -(-rows // (16 if rows <= 16 else 64))
@@ -881,8 +885,9 @@ def attention_splits(num_seqs: int, max_q: int, max_k: int, nh: int, nkv: int, d
         key_tiles = max(1, -(-max_k // 64))
         slots, cluster = decode_attention_limits()
         by_len = max(1, key_tiles // 2)
-        if blocks > slots:
-            return max(1, min(-(-4 * slots // blocks), by_len, 32))
+        if 2 * blocks > slots:
+            tiles = 24 if blocks > slots else 32
+            return max(1, min((key_tiles + tiles // 2) // tiles, -(-4 * slots // blocks), by_len, 32))
         want = max(1, int(round(2 * slots / 3 / blocks)))
         if want > cluster and (key_tiles <= 32 * cluster or 3 * blocks * cluster >= slots):
             want = cluster
