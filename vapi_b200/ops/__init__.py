@@ -167,6 +167,13 @@ def _f32(t: Optional[torch.Tensor], what: str) -> None:
         raise KernelError(f"{what} must be contiguous float32")
 
 
+def _bias(t: Optional[torch.Tensor], n: int, what: str = "bias") -> None:
+    """A vector that a kernel reads ``n`` numbers of."""
+    _f32(t, what)
+    if t is not None and t.numel() != n:
+        raise KernelError(f"{what} of {tuple(t.shape)} does not fit {n} features")
+
+
 _sm_counts: Dict[int, int] = {}
 
 
@@ -381,7 +388,7 @@ def skinny_linear(weight: torch.Tensor, *, act: Optional[torch.Tensor] = None,
         _f32(ss_in, "partial sums")
         if ss_in is None or ss_in.dim() != 2 or ss_in.shape[1] != M:
             raise KernelError("partial sums must be [parts, M]")
-    _f32(bias, "bias")
+    _bias(bias, N)
     _f32(next_weight, "norm weight")
     rpb = rows_per_block or 16
     out_bf16 = out_f32 = sso = xwo = None
@@ -454,8 +461,9 @@ def skinny_shortconv(w_in: torch.Tensor, *, xw: torch.Tensor, ss_in: torch.Tenso
     _f32(ss_in, "partial sums")
     if ss_in.dim() != 2 or ss_in.shape[1] != M:
         raise KernelError("partial sums must be [parts, M]")
-    for t, w in ((in_bias, "in_proj bias"), (taps, "conv taps"), (conv_bias, "conv bias")):
-        _f32(t, w)
+    _f32(taps, "conv taps")
+    _bias(in_bias, H3, "in_proj bias")
+    _bias(conv_bias, H, "conv bias")
     if tuple(taps.shape) != (L, H):
         raise KernelError("taps must be [L, H]")
     _i32(state_slots, "state slots")
@@ -512,7 +520,7 @@ def _fused_product(which: str, weight: torch.Tensor, act, xw, ss_in, eps: float,
         _f32(ss_in, "partial sums")
         if ss_in is None or ss_in.dim() != 2 or ss_in.shape[1] != M:
             raise KernelError("partial sums must be [parts, M]")
-    _f32(bias, "bias")
+    _bias(bias, N)
     _f32(next_weight, "norm weight")
     if epilogue not in _EPI:
         raise KernelError(f"unknown epilogue {epilogue}")
@@ -681,7 +689,7 @@ def skinny_linear_f32(weight: torch.Tensor, act: torch.Tensor, bias: Optional[to
         raise KernelError("skinny_linear_f32 needs a contiguous float32 weight")
     if act.dtype != torch.float32 or tuple(act.shape) != (M, K) or not act.is_contiguous():
         raise KernelError(f"skinny_linear_f32: token operand {tuple(act.shape)} / {act.dtype} does not fit a weight of {N}x{K}")
-    _f32(bias, "bias")
+    _bias(bias, N)
     out = torch.empty((M, N), dtype=torch.float32, device=weight.device)
     lib = _lib("gemv")
     _check(lib, lib.vapi_skinny_linear_f32(_p(weight), N, K, M, _p(act), _p(bias), _p(out), ctypes.c_longlong(N), _stream()))
@@ -717,7 +725,7 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
         raise KernelError("linear_f32 needs a contiguous float32 weight")
     if x.dtype != torch.float32 or tuple(x.shape) != (M, K) or not x.is_contiguous():
         raise KernelError(f"linear_f32: token operand {tuple(x.shape)} / {x.dtype} does not fit a weight of {N}x{K}")
-    _f32(bias, "bias")
+    _bias(bias, N)
     _i32(status, "status")
     out = torch.empty((M, N), dtype=torch.float32, device=weight.device)
     kp = -(-K // 8) * 8
@@ -732,30 +740,50 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     return out
 
 
+def _bias_vector(bias: torch.Tensor, n: int) -> Optional[torch.Tensor]:
+    """A product's bias as the kernels of this package read it, ``n`` contiguous float32 numbers; None for one that is not the
+    same for every token or does not fit, which is left to the library (to add, or to refuse)."""
+    if bias.dtype == torch.float32 and bias.dim() == 1 and bias.shape[0] == n and bias.is_contiguous():
+        return bias
+    if bias.dim() > 2 or (bias.dim() == 2 and bias.shape[0] != 1) or (bias.dim() > 0 and bias.shape[-1] not in (1, n)):
+        return None
+    return bias.reshape(-1).to(torch.float32).expand(n).contiguous()
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """``x @ weight.T (+ bias)``.  The library matrix product, except for decode-sized
-    bfloat16 products (at most 16 rows), which go to the weight-streaming kernel.
+    """``x @ weight.T (+ bias)``: decode-sized products (at most 16 rows, bfloat16 up to TC_MAX_ROWS) and large float32 ones on
+    this package's kernels, the others on the library.
 
     float32 runs without any reduced-precision mode (see :func:`strict_fp32`).  A weight kept
     in float32 beside bfloat16 activations is multiplied in float32.
     """
     _cuda(x, weight)
+    if bias is not None:
+        vector = _bias_vector(bias, weight.shape[0])
+        if vector is None:
+            return _library_linear(x, weight, bias, out_dtype)
+    else:
+        vector = None
     if x.dtype == torch.bfloat16 and skinny_applies(x.shape[0], weight) and x.is_contiguous():
         if out_dtype in (None, torch.bfloat16):
-            return skinny_linear(weight, act=x, epilogue="bf16", bias=bias)
+            return skinny_linear(weight, act=x, epilogue="bf16", bias=vector)
         if out_dtype == torch.float32:
-            return skinny_linear(weight, act=x, epilogue="f32", bias=bias)
+            return skinny_linear(weight, act=x, epilogue="f32", bias=vector)
     if x.dtype == torch.bfloat16 and tc_applies(x.shape[0], weight) and x.is_contiguous():
         if out_dtype in (None, torch.bfloat16):
-            return linear_tc(weight, act=x, epilogue="bf16", bias=bias)
+            return linear_tc(weight, act=x, epilogue="bf16", bias=vector)
         if out_dtype == torch.float32:
-            return linear_tc(weight, act=x, epilogue="f32", bias=bias)
+            return linear_tc(weight, act=x, epilogue="f32", bias=vector)
     if (x.dtype == torch.float32 and out_dtype in (None, torch.float32) and skinny_f32_applies(x.shape[0], weight)
             and x.is_contiguous() and x.data_ptr() % 16 == 0):
-        return skinny_linear_f32(weight, x, bias)
+        return skinny_linear_f32(weight, x, vector)
     if out_dtype in (None, torch.float32) and linear_f32_applies(x, weight):
-        return linear_f32(x, weight, bias)
+        return linear_f32(x, weight, vector)
+    return _library_linear(x, weight, bias, out_dtype)
+
+
+def _library_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], out_dtype: Optional[torch.dtype]) -> torch.Tensor:
     if weight.dtype != x.dtype:
         y = torch.mm(x.to(torch.float32), weight.to(torch.float32).t())
         if bias is not None:
