@@ -49,6 +49,53 @@ def test_a_bias_has_one_number_a_feature(calls, which):
     assert [name for name, _ in calls.got] == ["vapi_" + which]
 
 
+@pytest.mark.parametrize("which", ["linear_tc", "prompt_linear", "linear_f32"])
+def test_a_product_of_a_step_records_into_the_steps_status_word(calls, which):
+    """Those with bounded waits: the word that the step holds, unless the call brings its own; none outside of a step."""
+    dtype, product = PRODUCTS[which]
+    w, x = torch.zeros(48, 32, dtype=dtype), torch.zeros(20, 32, dtype=dtype)
+    word, own = torch.zeros(1, dtype=torch.int32), torch.zeros(1, dtype=torch.int32)
+    with ops.one_stream(word):
+        product(w, x, None)
+        ops.linear_f32(x.float(), w.float(), status=own)
+        with ops.one_stream():
+            product(w, x, None)
+        product(w, x, None)
+    product(w, x, None)
+    held = [word.data_ptr() in args for _, args in calls.got]
+    assert held == [True, False, False, True, False] and own.data_ptr() in calls.got[1][1]
+
+
+@pytest.mark.gpu
+def test_a_step_hands_its_status_word_to_every_product_with_a_bounded_wait(monkeypatch, tmp_path):
+    """A prompt of 33 rows in float32 and in bfloat16: whatever product runs, ordinary or in the stream form of its block."""
+    from vapi_b200 import LLM, SamplingParams
+    from vapi_b200.weights import write_random_model
+    cfg = {"architectures": ["Lfm2ForCausalLM"], "model_type": "lfm2", "vocab_size": 4096, "conv_L_cache": 3, "conv_bias": False,
+           "rope_theta": 1e6, "norm_eps": 1e-5, "tie_word_embeddings": True, "max_position_embeddings": 256, "num_hidden_layers": 2,
+           "layer_types": ["conv", "full_attention"], "hidden_size": 512, "intermediate_size": 3072, "num_attention_heads": 8,
+           "num_key_value_heads": 2, "head_dim": 64}
+    write_random_model(str(tmp_path), cfg, seed=0, std=0.02, dtype=BF16)
+    for dtype, names in (("f32", {"vapi_linear_f32"}), ("bf16", {"vapi_linear_tc"})):
+        llm = LLM(str(tmp_path), dtype=dtype, num_blocks=16, max_concurrent_seqs=4, max_batched_tokens=256, max_context=256)
+        seen, real = [], ops._lib
+
+        class Watched:
+            def __init__(self, lib):
+                self.lib = lib
+
+            def __getattr__(self, name):
+                f = getattr(self.lib, name)
+                if name not in ("vapi_linear_f32", "vapi_linear_tc", "vapi_prompt_linear"):
+                    return f
+                return lambda *args: (seen.append((name, llm.runner.status.data_ptr() in args)), f(*args))[1]
+
+        monkeypatch.setattr(ops, "_lib", lambda name: Watched(real(name)))
+        llm.generate([list(range(33))], SamplingParams(temperature=0.0, max_tokens=1, ignore_eos=True))
+        monkeypatch.setattr(ops, "_lib", real)
+        assert {n for n, _ in seen} == names and all(held for _, held in seen), seen
+
+
 # rows on both sides of 16 (the weight-streaming kernel, the split product) and a weight on both sides of the split product's least size
 @pytest.mark.gpu
 @pytest.mark.parametrize("M", [5, 33])

@@ -182,7 +182,7 @@ class ModelRunner:
         """Device work of a step for a prepared context; returns float32 logits [rows, vocab]
         or None when no logits are wanted (the caches are written either way)."""
         if self.device.type == "cuda":
-            with ops.one_stream():
+            with ops.one_stream(self.status):
                 return self._forward(ctx)
         return self._forward(ctx)
 

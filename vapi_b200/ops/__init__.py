@@ -129,26 +129,36 @@ def _p(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
-_held_stream = threading.local()
+_held = threading.local()
 
 
 def _stream() -> int:
-    h = getattr(_held_stream, "handle", None)
+    h = getattr(_held, "stream", None)
     return torch.cuda.current_stream().cuda_stream if h is None else h
+
+
+def _status(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """The status word of a call: its own, or the running step's (:class:`one_stream`)."""
+    return getattr(_held, "status", None) if t is None else t
 
 
 class one_stream:
     """Within the block every kernel of this module launches on the stream that is current at its
     entry, looked up once instead of once per kernel (a step launches a few hundred).  The caller
-    must not switch streams inside the block."""
+    must not switch streams inside the block.  ``status``: the step's status word, into which the
+    products record a bounded wait that ran out (their callers, the parts of a model, do not carry it)."""
+
+    def __init__(self, status: Optional[torch.Tensor] = None):
+        self.status = status
 
     def __enter__(self):
-        self.before = getattr(_held_stream, "handle", None)
-        _held_stream.handle = torch.cuda.current_stream().cuda_stream if torch.cuda.is_available() else None
+        self.before = getattr(_held, "stream", None), getattr(_held, "status", None)
+        _held.stream = torch.cuda.current_stream().cuda_stream if torch.cuda.is_available() else None
+        _held.status = self.status
         return self
 
     def __exit__(self, *exc):
-        _held_stream.handle = self.before
+        _held.stream, _held.status = self.before
         return False
 
 
@@ -550,7 +560,7 @@ def _fused_product(which: str, weight: torch.Tensor, act, xw, ss_in, eps: float,
     _check(lib, fn(
         _p(weight), N, K, M, _PRO[pro], _p(src), _p(ss_in), 0 if ss_in is None else ss_in.shape[0], ctypes.c_float(eps),
         _EPI[epilogue], _p(out_bf16), _p(out_f32), ctypes.c_longlong(out_stride), _p(bias), _p(resid), _p(sso),
-        _p(next_weight), _p(xwo), _p(status), _stream(), _p(xielu), _glu(glu)))
+        _p(next_weight), _p(xwo), _p(_status(status)), _stream(), _p(xielu), _glu(glu)))
     if epilogue == "resid":
         return sso, xwo
     return out_bf16 if out_bf16 is not None else out_f32
@@ -726,6 +736,7 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     if x.dtype != torch.float32 or tuple(x.shape) != (M, K) or not x.is_contiguous():
         raise KernelError(f"linear_f32: token operand {tuple(x.shape)} / {x.dtype} does not fit a weight of {N}x{K}")
     _bias(bias, N)
+    status = _status(status)
     _i32(status, "status")
     out = torch.empty((M, N), dtype=torch.float32, device=weight.device)
     kp = -(-K // 8) * 8
