@@ -82,3 +82,23 @@ def test_float32_product_of_tiny_and_exact_numbers(ops):
     w = torch.randint(-9, 10, (150, 200), generator=g, device="cuda").float()
     assert torch.equal(ops.linear_f32(a, w).double(), a.double() @ w.double().t())
     assert torch.equal(ops.linear_f32(a * 2.0 ** -60, w).double(), (a.double() @ w.double().t()) * 2.0 ** -60)
+
+
+# one tile a block, tiles in turn, a tile shared by two to eight blocks
+@pytest.mark.parametrize("M,N,K", [(70, 300, 60), (300, 20000, 132), (64, 2048, 520), (40, 130, 4160)])
+def test_a_float32_product_that_gives_up_a_wait_writes_nothing_and_says_so(ops, M, N, K):
+    """Waits that give up without a poll, or after one (what then is complete is written, the rest is not); the next call is unaffected."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    a, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    want = ops.linear_f32(a, w)
+    lib, kp = ops._lib("linear_f32"), -(-K // 8) * 8
+    planes, bad = torch.empty(3 * M * kp, dtype=torch.bfloat16, device="cuda"), torch.empty(M, dtype=torch.int32, device="cuda")
+    for polls in (0, 1):
+        out, status = torch.full((M, N), float("nan"), device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        rc = lib.vapi_linear_f32(w.data_ptr(), N, K, M, a.data_ptr(), planes.data_ptr(), bad.data_ptr(), None, out.data_ptr(), N, polls,
+                                 status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        left = torch.isnan(out)
+        assert int(status) == (16 if bool(left.any()) else 0) and torch.equal(out[~left], want[~left])
+        assert polls > 0 or bool(left.all())
+        assert torch.equal(ops.linear_f32(a, w, status=status.zero_()), want) and int(status) == 0

@@ -33,8 +33,9 @@
 // Few tiles.  Where the tiles would leave most multiprocessors idle, a cluster of S blocks shares a tile: each takes a part of
 // K, and the partial sums are added in the order of the ranks through distributed shared memory.
 //
-// Every wait on an mbarrier is bounded: after the limit a role records that it gave up, the block drains and status 16 is
-// recorded; the cluster barriers are reached by every thread on every path.
+// Every wait on an mbarrier is bounded: after the limit a role gives up and the others follow; the block records status 16, waits
+// (with a limit) for the copies and products that are under way, and leaves its tile unwritten, as do the blocks that share it.  The
+// cluster barriers are reached by every thread on every path.
 #include "tcgen05.cuh"
 
 #include <unordered_map>
@@ -62,11 +63,12 @@ template <int NT> struct LfCfg {
 struct LfParams {
     const float* W; const float* act; const float* bias; const int* tok_bad; float* out; int* status;
     int N, K, M, num_kb, num_m, num_tiles, split;
+    unsigned polls;                       // of an mbarrier before a role gives up
     long long out_stride;
 };
 
-__device__ __forceinline__ bool lf_wait(unsigned bar, unsigned parity, volatile int* abort_flag) {
-    for (unsigned i = 0; i < TC5_WAIT_LIMIT; ++i) {
+__device__ __forceinline__ bool lf_wait(unsigned bar, unsigned parity, volatile int* abort_flag, unsigned polls) {
+    for (unsigned i = 0; i < polls; ++i) {
         unsigned done;
         asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}"
                      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
@@ -154,7 +156,7 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(lf_smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* tok_mem = base + (size_t)LF_W_STAGES * LF_W_BYTES;
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(tok_mem + (size_t)LF_STAGES * Cfg::STAGE_BYTES);
-    unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * LF_STAGES + 4 + 2 * LF_W_STAGES);
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 3 * LF_STAGES + 4 + 2 * LF_W_STAGES + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     unsigned char* w_bad = reinterpret_cast<unsigned char*>(bars) + 256;            // [LF_BAD_TILES][128]
 
@@ -167,11 +169,13 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     const unsigned full0 = smem_u32(bars), empty0 = smem_u32(bars + LF_STAGES);
     const unsigned accfull0 = smem_u32(bars + 2 * LF_STAGES), accempty0 = smem_u32(bars + 2 * LF_STAGES + 2);
     const unsigned wfull0 = smem_u32(bars + 2 * LF_STAGES + 4), wempty0 = smem_u32(bars + 2 * LF_STAGES + 4 + LF_W_STAGES);
+    const unsigned tokfull0 = smem_u32(bars + 2 * LF_STAGES + 4 + 2 * LF_W_STAGES), drained = tokfull0 + 8 * LF_STAGES;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < LF_STAGES; ++i) { mbar_init(full0 + 8 * i, 1 + 4); mbar_init(empty0 + 8 * i, 1); }
+        for (int i = 0; i < LF_STAGES; ++i) { mbar_init(full0 + 8 * i, 4); mbar_init(tokfull0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(accfull0 + 8 * i, 1); mbar_init(accempty0 + 8 * i, 4); }
         for (int i = 0; i < LF_W_STAGES; ++i) { mbar_init(wfull0 + 8 * i, 1); mbar_init(wempty0 + 8 * i, 4); }
+        mbar_init(drained, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -186,19 +190,20 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     pdl_trigger();
 
     float* part = reinterpret_cast<float*>(base);        // [NT][128]: a shared tile's partial sums, over the weights' stages
+    int it = 0;                                          // stages that this thread's role has finished
 
     if (warp >= 4 && warp < 8) {
         // ---- split of the weights: a row a thread ----
         const int row = (int)threadIdx.x - 128;
         const unsigned a0 = tmem_base + ((unsigned)((warp - 4) * 32) << 16) + LF_A_COL0;
-        int it = 0, tl = 0;
+        int tl = 0;
         bool ok = true;
         for (int t = first; t < p.num_tiles && ok; t += step, ++tl) {
             float top = 0.f;
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
                 const int s = it % LF_STAGES, ws = it % LF_W_STAGES;
-                if (!lf_wait(wfull0 + 8 * ws, (it / LF_W_STAGES) & 1, abort_flag)) ok = false;
-                if (!lf_wait(empty0 + 8 * s, ((it / LF_STAGES) & 1) ^ 1, abort_flag)) ok = false;
+                if (!lf_wait(wfull0 + 8 * ws, (it / LF_W_STAGES) & 1, abort_flag, p.polls)) ok = false;
+                if (!lf_wait(empty0 + 8 * s, ((it / LF_STAGES) & 1) ^ 1, abort_flag, p.polls)) ok = false;
                 if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
                 tc5_fence_after();
                 const unsigned char* w = base + (size_t)ws * LF_W_BYTES + row * 128;
@@ -227,13 +232,12 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     } else if (warp == 10) {
         if (lane == 0) {
             // ---- TMA of the weights (they do not depend on the kernel before this one) ----
-            int it = 0;
             bool ok = true;
             for (int t = first; t < p.num_tiles && ok; t += step) {
                 const int n0 = (t / p.num_m) * LF_BM;
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int ws = it % LF_W_STAGES;
-                    if (!lf_wait(wempty0 + 8 * ws, ((it / LF_W_STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+                    if (!lf_wait(wempty0 + 8 * ws, ((it / LF_W_STAGES) & 1) ^ 1, abort_flag, p.polls)) { ok = false; break; }
                     const unsigned w = smem_u32(base + (size_t)ws * LF_W_BYTES);
                     mbar_expect_tx(wfull0 + 8 * ws, LF_W_BYTES);
                     tma_load_2d(w, &tm_w, wfull0 + 8 * ws, kb * LF_BK, n0);
@@ -245,18 +249,17 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         if (lane == 0) {
             // ---- TMA of the tokens' planes ----
             pdl_wait();
-            int it = 0;
             bool ok = true;
             for (int t = first; t < p.num_tiles && ok; t += step) {
                 const int m0 = (t % p.num_m) * NT;
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % LF_STAGES;
-                    if (!lf_wait(empty0 + 8 * s, ((it / LF_STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+                    if (!lf_wait(empty0 + 8 * s, ((it / LF_STAGES) & 1) ^ 1, abort_flag, p.polls)) { ok = false; break; }
                     const unsigned b = smem_u32(tok_mem + (size_t)s * Cfg::STAGE_BYTES);
-                    mbar_expect_tx(full0 + 8 * s, 3 * Cfg::B_PLANE);
+                    mbar_expect_tx(tokfull0 + 8 * s, 3 * Cfg::B_PLANE);
 #pragma unroll
                     for (int i = 0; i < 3; ++i)          // (rows behind the last token are the next plane's, or zeros: never stored)
-                        tma_load_2d(b + i * Cfg::B_PLANE, &tm_tok, full0 + 8 * s, kb * LF_BK, i * p.M + m0);
+                        tma_load_2d(b + i * Cfg::B_PLANE, &tm_tok, tokfull0 + 8 * s, kb * LF_BK, i * p.M + m0);
                 }
             }
         }
@@ -264,13 +267,13 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         if (lane == 0) {
             // ---- MMA issue ----
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(NT >> 3) << 17) | ((unsigned)(LF_BM >> 4) << 24);
-            int it = 0;
             bool ok = true;
             for (int t = first; t < p.num_tiles && ok; t += step) {
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % LF_STAGES, buf = it & 1;
-                    if (!lf_wait(accempty0 + 8 * buf, ((it >> 1) & 1) ^ 1, abort_flag) ||
-                        !lf_wait(full0 + 8 * s, (it / LF_STAGES) & 1, abort_flag)) { ok = false; break; }
+                    if (!lf_wait(accempty0 + 8 * buf, ((it >> 1) & 1) ^ 1, abort_flag, p.polls) ||
+                        !lf_wait(tokfull0 + 8 * s, (it / LF_STAGES) & 1, abort_flag, p.polls) ||
+                        !lf_wait(full0 + 8 * s, (it / LF_STAGES) & 1, abort_flag, p.polls)) { ok = false; break; }
                     tc5_fence_after();
                     const unsigned a = tmem_base + LF_A_COL0 + (unsigned)(s * 3 * LF_A_COLS), b = smem_u32(tok_mem + (size_t)s * Cfg::STAGE_BYTES);
                     const unsigned d = tmem_base + (unsigned)(buf * NT);
@@ -293,12 +296,12 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         float acc[NT];
 #pragma unroll
         for (int j = 0; j < NT; ++j) acc[j] = 0.f;
-        int it = 0, tl = 0;
+        int tl = 0;
         bool ok = true;
         for (int t = first; t < p.num_tiles && ok; t += step, ++tl) {
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
                 const int buf = it & 1;
-                if (!lf_wait(accfull0 + 8 * buf, (it >> 1) & 1, abort_flag)) ok = false;
+                if (!lf_wait(accfull0 + 8 * buf, (it >> 1) & 1, abort_flag, p.polls)) ok = false;
                 if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
                 tc5_fence_after();
 #pragma unroll
@@ -342,7 +345,13 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         __syncthreads();
         __syncwarp();
         lf_cluster_sync();
-        if (warp < 4 && first < p.num_tiles) {
+        bool whole = true;                               // (a block that gave up has left no partial sums)
+        for (int r = 0; r < split; ++r) {
+            unsigned gone;
+            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(gone) : "r"(lf_map_rank(smem_u32(const_cast<int*>(abort_flag)), (unsigned)r)));
+            whole &= gone == 0u;
+        }
+        if (warp < 4 && first < p.num_tiles && whole) {
             const int m0 = (first % p.num_m) * NT;
             const long long n = (long long)(first / p.num_m) * LF_BM + threadIdx.x;
             bool wb = false;
@@ -373,7 +382,20 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     }
     tc5_fence_before();
     __syncthreads();
-    if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 16);
+    if (*abort_flag) {                                   // (the same for all: every role is through)
+        if (threadIdx.x == 0 && p.status) atomicExch(p.status, 16);
+        if (lane == 0) {                                 // what is under way ends before its memory is given back
+            if (warp == 8)
+                for (int i = max(it - LF_STAGES, 0); i < it; ++i) mbar_wait(tokfull0 + 8 * (i % LF_STAGES), (i / LF_STAGES) & 1);
+            if (warp == 10)
+                for (int i = max(it - LF_W_STAGES, 0); i < it; ++i) mbar_wait(wfull0 + 8 * (i % LF_W_STAGES), (i / LF_W_STAGES) & 1);
+            if (warp == 9 && it > 0) {
+                umma_commit(drained);
+                mbar_wait(drained, 0);
+            }
+        }
+        __syncthreads();
+    }
     if (warp == 9) {
         __syncwarp();
         tc5_fence_after();
@@ -442,8 +464,9 @@ VAPI_EXPORT int vapi_linear_f32_plan(int N, int K, int M, int* nt, int* split) {
 }
 
 // y = act W^T (+ bias).  ``planes``: scratch of 3 * M * (K rounded up to 8) bfloat16; ``bad``: scratch of M ints.
+// ``polls``: of an mbarrier before a role gives up, below zero for the usual limit (about a second).
 VAPI_EXPORT int vapi_linear_f32(const float* W, int N, int K, int M, const float* act, void* planes, int* bad, const float* bias,
-                                float* out, long long out_stride, int* status, cudaStream_t stream) {
+                                float* out, long long out_stride, int polls, int* status, cudaStream_t stream) {
     if (M <= 0) return 0;
     if (N <= 0 || K <= 0 || K % 4 != 0) return fail(-1, "linear_f32: K=%d must be a positive multiple of 4 (N=%d)", K, N);
     if (!W || !act || !planes || !bad || !out) return fail(-1, "linear_f32: missing array");
@@ -455,7 +478,7 @@ VAPI_EXPORT int vapi_linear_f32(const float* W, int N, int K, int M, const float
     int nt;
     vapi_linear_f32_plan(N, K, M, &nt, &p.split);
     p.W = W; p.act = act; p.bias = bias; p.tok_bad = bad; p.out = out; p.status = status;
-    p.N = N; p.K = K; p.M = M; p.out_stride = out_stride;
+    p.N = N; p.K = K; p.M = M; p.out_stride = out_stride; p.polls = polls < 0 ? TC5_WAIT_LIMIT : (unsigned)polls;
     p.num_kb = (K + LF_BK - 1) / LF_BK;
     p.num_m = (M + nt - 1) / nt;
     p.num_tiles = p.num_m * ((N + LF_BM - 1) / LF_BM);

@@ -747,7 +747,7 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     for at in range(0, M, LINEAR_F32_ROWS):
         rows = min(most, M - at)
         _check(lib, lib.vapi_linear_f32(_p(weight), N, K, rows, x.data_ptr() + 4 * at * K, _p(planes), _p(bad), _p(bias),
-                                        out.data_ptr() + 4 * at * N, N, _p(status), _stream()), launches=2)
+                                        out.data_ptr() + 4 * at * N, N, -1, _p(status), _stream()), launches=2)
     return out
 
 
