@@ -910,12 +910,13 @@ def attention_splits(num_seqs: int, max_q: int, max_k: int, nh: int, nkv: int, d
     (sequence, kv head) pairs are fewer than two blocks per SM, slices up to that many blocks, and
     no more than the kernel combines itself unless a slice would then be longer than 32 tiles and
     there would be fewer blocks than SMs.
-    A step with more pairs than half of what the device holds is only cut where its longest sequences could be long: to
-    slices of about 32 tiles, or of 24 where the pairs alone are more than the device holds, and into no more
-    than four rounds of blocks.  Slices cost a block's start each and a combine kernel (8 kv heads, both kernels): 64 sequences of
-    128 to 2,048 keys 28.8 us whole, 35.2 / 38.5 / 39.9 in 2 / 3 / 4 slices; of 20 to 300 10.4 and 22.6 in 4; 32 of 33 to 700
-    11.5 and 13.6 in 2, but 32 of 500 to 4,000 48.5 whole and 32.5 in 2, where the longest sequence's block runs alone, and 64
-    of 4,096 114 whole, 96 in 3 and 95 in 4."""
+    Half of the device's places and more are filled by the pairs alone: whole sequences up to all of them, then about four rounds of blocks,
+    so that the last ones do not run alone.  ``max_k`` bounds the lengths but does not tell them (a captured step is given the
+    configured context), so only what loses at no length is cut less: a step of more pairs than the device holds stays whole where
+    no sequence can be longer than 20 tiles and is cut in two up to 36.  8 kv heads, 444 places, us in 1 / 2 / 4 slices: 64 sequences of 20 to 300
+    keys 11.4 / 17.1 / 23.2, of 1,216 43.3 / 45.2 / 47.6, of 1,600 53.3 / 53.8 / 54.2 (56: 49.5 / 48.3 / 48.4), of 2,300
+    70.0 / 68.4 / 68.4, of 4,096 119.5 / 105.1 / 100.2.  Fewer pairs: 32 of 33 to 700 10.9 / 15.1 / 16.3, of 2,000 31.2 / 42.0 / 40.1, but
+    of 500 to 4,000, where the longest sequence's block runs alone, 49.7 / 45.6 / 41.6."""
     n_rep = nh // nkv
     rows = max_q * n_rep
     tiles = -(-rows // (16 if rows <= 16 else 64))
@@ -924,9 +925,9 @@ def attention_splits(num_seqs: int, max_q: int, max_k: int, nh: int, nkv: int, d
         key_tiles = max(1, -(-max_k // 64))
         slots, cluster = decode_attention_limits()
         by_len = max(1, key_tiles // 2)
-        if 2 * blocks > slots:
-            tiles = 24 if blocks > slots else 32
-            return max(1, min((key_tiles + tiles // 2) // tiles, -(-4 * slots // blocks), by_len, 32))
+        if blocks > slots:
+            most = 1 if key_tiles <= 20 else 2 if key_tiles <= 36 else 32
+            return max(1, min(-(-4 * slots // blocks), by_len, most))
         want = max(1, int(round(2 * slots / 3 / blocks)))
         if want > cluster and (key_tiles <= 32 * cluster or 3 * blocks * cluster >= slots):
             want = cluster
