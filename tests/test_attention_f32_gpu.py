@@ -64,3 +64,22 @@ def test_float_attention_of_what_cannot_be_split(ops):
     assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
     fin = torch.isfinite(want)
     torch.testing.assert_close(got[fin], want[fin], atol=2e-5, rtol=2e-5)
+
+
+# planted at the first, a middle and the last token of a group of 32, of a tile of 64 rows and of the portion; with and without a window
+@pytest.mark.parametrize("impl", ["auto", "general"])
+@pytest.mark.parametrize("window", [0, 40])
+@pytest.mark.parametrize("token", [0, 15, 31, 32, 44, 63, 64, 99])
+def test_a_value_that_a_row_may_not_see_does_not_come_into_it(ops, impl, window, token):
+    """An infinity and a NaN in one key's value: only rows that see the key, and only those two elements of them."""
+    q, cache, args = _random_case(3, 100, 260, 4, 2)
+    clean = ops.paged_attention(q, 256, cache, *args, window, 1, None, impl).view(100, 4, 64)
+    at = 160 + token
+    cache[at // 64, 1, :, at % 64, 3], cache[at // 64, 1, :, at % 64, 60] = float("inf"), float("nan")
+    got = ops.paged_attention(q, 256, cache, *args, window, 1, None, impl).view(100, 4, 64)
+    rows = torch.arange(100, device="cuda")
+    sees = (rows >= token) & ((rows < token + window) if window else torch.ones_like(rows, dtype=torch.bool))
+    hit = torch.zeros(100, 4, 64, dtype=torch.bool, device="cuda")
+    hit[sees] = torch.zeros(64, dtype=torch.bool, device="cuda").index_fill_(0, torch.tensor([3, 60], device="cuda"), True)
+    assert torch.equal(~torch.isfinite(got), hit)
+    torch.testing.assert_close(got[~hit], clean[~hit], atol=2e-5, rtol=2e-5)
