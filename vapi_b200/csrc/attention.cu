@@ -24,8 +24,6 @@
 #include "attention_f32.cuh"
 #include "attention_decode.cuh"
 
-#include <type_traits>
-
 using namespace vapi;
 
 constexpr int ATT_ROWS = 16;
@@ -156,9 +154,6 @@ paged_attention_kernel(const T* __restrict__ q, long long q_row_stride,
         }
         const int j = kt * ATT_BK + lane;
         float* pw = Ps + (warp * ATT_RPW) * ATT_BK;
-        // whether a row may have to leave out a key that another row of the tile sees: its weight is then -1, and its value (an
-        // infinity, a NaN) does not come into the row
-        const bool edge = p_min < p_max && ((kt + 1) * ATT_BK - 1 > p_min || (window > 0 && kt * ATT_BK <= p_max - window));
 #pragma unroll
         for (int a = 0; a < ATT_RPW; ++a) {
             if (!row_ok[a]) continue;  // uniform across the warp
@@ -174,28 +169,24 @@ paged_attention_kernel(const T* __restrict__ q, long long q_row_stride,
             m[a] = m_new;
 #pragma unroll
             for (int c = 0; c < DPL; ++c) acc[a][c] *= alpha;
-            pw[a * ATT_BK + lane] = edge && !vis ? -1.f : p;
+            pw[a * ATT_BK + lane] = p;
         }
         __syncwarp();
-        auto add_values = [&](auto some_left_out) {
-            for (int jj = 0; jj < ATT_BK; ++jj) {
-                float vcol[DPL];
+        for (int jj = 0; jj < ATT_BK; ++jj) {
+            float vcol[DPL];
 #pragma unroll
-                for (int c = 0; c < DPL; ++c) {
-                    const int col = lane + 32 * c;
-                    vcol[c] = col < d ? Vs[jj * ld + col] : 0.f;
-                }
-#pragma unroll
-                for (int a = 0; a < ATT_RPW; ++a) {
-                    if (!row_ok[a]) continue;
-                    const float p = pw[a * ATT_BK + jj];
-                    if (decltype(some_left_out)::value && p < 0.f) continue;
-#pragma unroll
-                    for (int c = 0; c < DPL; ++c) acc[a][c] = fmaf(p, vcol[c], acc[a][c]);
-                }
+            for (int c = 0; c < DPL; ++c) {
+                const int col = lane + 32 * c;
+                vcol[c] = col < d ? Vs[jj * ld + col] : 0.f;
             }
-        };
-        if (edge) add_values(std::true_type()); else add_values(std::false_type());
+#pragma unroll
+            for (int a = 0; a < ATT_RPW; ++a) {
+                if (!row_ok[a]) continue;
+                const float p = pw[a * ATT_BK + jj];
+#pragma unroll
+                for (int c = 0; c < DPL; ++c) acc[a][c] = fmaf(p, vcol[c], acc[a][c]);
+            }
+        }
         __syncwarp();
     }
 

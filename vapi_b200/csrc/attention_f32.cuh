@@ -100,7 +100,6 @@ flash_f32_kernel(const float* q, long long q_row_stride, const float* cache, con
         qrow[i] = q + (size_t)(q0 + tok) * q_row_stride + (size_t)h * FF_HD;
         grow[i] = (long long)(q0 + tok) * nh + h;
     }
-    auto visible = [&](int i, int j) { return j <= pos[i] && j < klen && (window <= 0 || j > pos[i] - window); };
     const bool busy = tile_start + warp * 16 < rows_total;          // (a warp without rows helps to split and multiplies nothing)
     const int* bt = block_table + (size_t)s * table_stride;
     auto load = [&](int kt) {
@@ -192,7 +191,8 @@ flash_f32_kernel(const float* q, long long q_row_stride, const float* cache, con
             for (int n = 0; n < 8; ++n)
 #pragma unroll
                 for (int x = 2 * i; x < 2 * i + 2; ++x) {
-                    const bool vis = visible(i, kt * FF_BK + n * 8 + p4 + (x & 1));
+                    const int j = kt * FF_BK + n * 8 + p4 + (x & 1);
+                    const bool vis = j <= pos[i] && j < klen && (window <= 0 || j > pos[i] - window);
                     sc[n][x] = vis ? sc[n][x] + low[n][x] : -INFINITY;
                     mx = fmaxf(mx, sc[n][x]);
                 }
@@ -204,7 +204,8 @@ flash_f32_kernel(const float* q, long long q_row_stride, const float* cache, con
             for (int n = 0; n < 8; ++n)
 #pragma unroll
                 for (int x = 2 * i; x < 2 * i + 2; ++x) {
-                    const bool vis = visible(i, kt * FF_BK + n * 8 + p4 + (x & 1));
+                    const int j = kt * FF_BK + n * 8 + p4 + (x & 1);
+                    const bool vis = j <= pos[i] && j < klen && (window <= 0 || j > pos[i] - window);
                     const float p = vis && mx != -INFINITY ? expf(sc[n][x] - mx) : 0.f;
                     sc[n][x] = p;
                     sum += p;
@@ -236,13 +237,11 @@ flash_f32_kernel(const float* q, long long q_row_stride, const float* cache, con
                 }
             }
         } else {
-            // [64][64], over the keys' planes; -1 where the row may not see the key, whose value, infinity or NaN, is no concern of it
-            float* P = reinterpret_cast<float*>(sK);
+            float* P = reinterpret_cast<float*>(sK);                // [64][64], over the keys' planes
 #pragma unroll
             for (int n = 0; n < 8; ++n)
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    P[(warp * 16 + (i >> 1) * 8 + g4) * FF_BK + n * 8 + p4 + (i & 1)] = visible(i >> 1, kt * FF_BK + n * 8 + p4 + (i & 1)) ? sc[n][i] : -1.f;
+                for (int i = 0; i < 4; ++i) P[(warp * 16 + (i >> 1) * 8 + g4) * FF_BK + n * 8 + p4 + (i & 1)] = sc[n][i];
             __syncthreads();
 #pragma unroll
             for (int n = 0; n < 8; ++n)
@@ -252,8 +251,8 @@ flash_f32_kernel(const float* q, long long q_row_stride, const float* cache, con
                     float d = 0.f;
 #pragma unroll 1
                     for (int k = 0; k < FF_BK; ++k) {
-                        const float w = pr[k];
-                        if (!(w < 0.f)) d = fmaf(w, fV[k * FF_HD + n * 8 + p4 + (i & 1)], d);
+                        const int j = kt * FF_BK + k, at = pos[i >> 1];
+                        if (j <= at && j < klen && (window <= 0 || j > at - window)) d = fmaf(pr[k], fV[k * FF_HD + n * 8 + p4 + (i & 1)], d);
                     }
                     pv[n][i] = d;
                 }
