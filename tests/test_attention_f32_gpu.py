@@ -87,3 +87,33 @@ def test_a_value_that_a_row_may_not_see_does_not_come_into_it(ops, window, token
     hit[sees] = torch.zeros(64, dtype=torch.bool, device="cuda").index_fill_(0, torch.tensor([3, 60], device="cuda"), True)
     assert torch.equal(~torch.isfinite(got), hit)
     torch.testing.assert_close(got[~hit], clean[~hit], atol=2e-5, rtol=2e-5)
+
+
+# signs and mantissas just above and below one of eight bits: the partial products of a score overflow together or against each other
+@pytest.mark.parametrize("impl", ["auto", "general"])
+@pytest.mark.parametrize("mq", [1.0 + 2.0 ** -9, 1.0 - 2.0 ** -10, 1.5 + 2.0 ** -9, 1.5 - 2.0 ** -9])
+@pytest.mark.parametrize("mk", [1.0 + 2.0 ** -9, 1.5 - 2.0 ** -9])
+def test_a_score_beyond_the_largest_float_is_what_float_products_make_of_it(ops, impl, mq, mk):
+    """Queries and keys of 1e28 to 1e32: a score of minus infinity has no weight, one of infinity makes the row NaN; other rows stay."""
+    q, cache, args = _random_case(6, 100, 260, 4, 2)
+    q.view(100, 4, 64)[:, :, 9] = 0.0
+    cache[:, 0, :, :, 9] = 0.0
+    clean = ops.paged_attention(q, 256, cache, *args, splits=1, impl=impl).view(100, 4, 64)
+    q.view(100, 4, 64)[[20, 70], :, 9] = mq * 2.0 ** 95
+    cache[1, 0, 0, 30, 9] = -mk * 2.0 ** 104               # key 94, seen by all
+    cache[3, 0, 1, 40, 9] = mk * 2.0 ** 104                # key 232, seen by the tokens from 72 on: by neither of the two
+    got = ops.paged_attention(q, 256, cache, *args, splits=1, impl=impl).view(100, 4, 64)
+    assert torch.isfinite(got).all()
+    k, v = (cache.double()[:, i].transpose(0, 1).reshape(2, -1, 64)[:, :260] for i in (0, 1))
+    for t in (20, 70):
+        keep = [j for j in range(161 + t) if j != 94]
+        for h in (0, 1):                                   # the heads of the first kv head: as if the key were not there
+            s = (q.double().view(100, 4, 64)[t, h] * (torch.arange(64, device="cuda") != 9)) @ k[0, keep].t() * 0.125
+            torch.testing.assert_close(got[t, h].double(), s.softmax(-1) @ v[0, keep], atol=2e-5, rtol=2e-5)
+    rows = [t for t in range(100) if t not in (20, 70)]
+    torch.testing.assert_close(got[rows], clean[rows], atol=2e-5, rtol=2e-5)
+    cache[1, 0, 0, 30, 9] = mk * 2.0 ** 104                # now infinity
+    got = ops.paged_attention(q, 256, cache, *args, splits=1, impl=impl).view(100, 4, 64)
+    nan = torch.zeros_like(got, dtype=torch.bool)
+    nan[[20, 70], :2] = True
+    assert torch.equal(torch.isnan(got), nan)

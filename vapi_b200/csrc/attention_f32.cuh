@@ -12,7 +12,7 @@
 // A block of four warps owns 64 rows and walks the 64-key tiles any of them can see: the tile's floats come by asynchronous copies
 // while the tile before is multiplied, all threads split them into planes (128-byte rows, 16-byte pieces swizzled), a warp
 // takes 16 rows.  106 KB of shared memory and two blocks a multiprocessor, so that one block splits while the other
-// multiplies.  A tile with an infinity, a NaN or a magnitude of 2^127 and more, which have no such planes, is computed by FMAs.
+// multiplies.  A tile with an infinity or a NaN, which have no such planes, or with magnitudes whose products could overflow is computed by FMAs.
 #pragma once
 #include "attention_mma.cuh"
 #include "attention_tc.cuh"        // ft_tile
@@ -22,7 +22,9 @@ namespace vapi {
 constexpr int FF_ROWS = 64, FF_BK = 64, FF_HD = 64, FF_THREADS = 128;
 constexpr int FF_PLANE = FF_BK * FF_HD * 2;
 constexpr size_t FF_SMEM = 9 * FF_PLANE + 2 * FF_BK * FF_HD * 4 + 128;     // planes of Q, K, V; floats of K, V
-constexpr float FF_LIMIT = 1.7014118346046923e38f;                         // 2^127
+// From here on a tile is computed by FMAs: below 2^60 a score, and below 2^120 a sum of 64 values, stays finite in every partial
+// sum (one that overflows takes the others with it: plus infinity of x1 y1 and minus infinity of x1 y2 are NaN, a float product infinity).
+constexpr float FF_LIMIT_QK = 1.152921504606846976e18f, FF_LIMIT_V = 1.329227995784915873e36f;
 
 __device__ __forceinline__ void ff_split2(float a, float b, unsigned& p1, unsigned& p2, unsigned& p3) {
     p1 = pack_bf16(a, b);
@@ -138,13 +140,13 @@ flash_f32_kernel(const float* q, long long q_row_stride, const float* cache, con
     for (int kt = kt_begin; kt < kt_end; ++kt) {
         cp_async_wait<0>();
         __syncthreads();                                            // the tile's floats are here, the planes of the last tile have been read
-        float top = qtop;
+        float top = qtop, vtop = 0.f;
 #pragma unroll 4
         for (int i = tid; i < FF_BK * FF_HD / 4; i += FF_THREADS) {
             top = ff_store(sK, i >> 4, i & 15, *reinterpret_cast<const float4*>(fK + i * 4), top);
-            top = ff_store(sV, i >> 4, i & 15, *reinterpret_cast<const float4*>(fV + i * 4), top);
+            vtop = ff_store(sV, i >> 4, i & 15, *reinterpret_cast<const float4*>(fV + i * 4), vtop);
         }
-        const bool plain = __syncthreads_or(!(top < FF_LIMIT)) != 0;
+        const bool plain = __syncthreads_or(!(top < FF_LIMIT_QK && vtop < FF_LIMIT_V)) != 0;
         if (!plain && kt + 1 < kt_end) load(kt + 1);
 
         if (!busy && !plain) continue;
