@@ -361,19 +361,31 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                 wb |= f != 0;
             }
             const float b = (p.bias && n < p.N) ? p.bias[n] : 0.f;
-            const int cols = NT / split;
-            for (int j = rank * cols; j < (rank + 1) * cols; ++j) {
-                const int m = m0 + j;
-                if (m >= p.M) break;
-                float y = 0.f;
+            // (a load from another block's memory takes about as long as one from L2: eight tokens' at a time, of two ranks before they are
+            // added.  One by one, with the sum between them, they were 13 to 26 us of a call: 65 x 2,048 x 512 34 us, so 19, 300 x 1,536 x 1,536
+            // 53 and 39, 129 x 1,024 x 1,024 24 and 17)
+            const int cols = NT / split;                 // (at least eight)
+            for (int j = rank * cols; j < (rank + 1) * cols && m0 + j < p.M; j += 8) {
+                float y[8];
+                int tb[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { y[i] = 0.f; tb[i] = m0 + j + i < p.M ? p.tok_bad[m0 + j + i] : 0; }
+#pragma unroll 2
                 for (int r = 0; r < split; ++r) {
-                    float f;
-                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f) : "r"(lf_map_rank(smem_u32(part + j * LF_BM + threadIdx.x), (unsigned)r)));
-                    y += f;
+                    const unsigned src = lf_map_rank(smem_u32(part + j * LF_BM + threadIdx.x), (unsigned)r);
+                    float f[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f[i]) : "r"(src + i * LF_BM * 4));
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) y[i] += f[i];
                 }
-                if (n < p.N) {
-                    if (wb || p.tok_bad[m] != 0) y = lf_plain(p.act + (size_t)m * p.K, p.W + (size_t)n * p.K, p.K);
-                    p.out[(size_t)m * p.out_stride + n] = y + b;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int m = m0 + j + i;
+                    if (n < p.N && m < p.M) {
+                        if (wb || tb[i] != 0) y[i] = lf_plain(p.act + (size_t)m * p.K, p.W + (size_t)n * p.K, p.K);
+                        p.out[(size_t)m * p.out_stride + n] = y[i] + b;
+                    }
                 }
             }
         }
