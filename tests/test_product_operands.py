@@ -96,6 +96,15 @@ def test_a_step_hands_its_status_word_to_every_product_with_a_bounded_wait(monke
         assert {n for n, _ in seen} == names and all(held for _, held in seen), seen
 
 
+# products that had become slower than the library's (short K, a few features), and the edges of the rule; what a model's prompt has stays
+@pytest.mark.parametrize("rows,n,k,pays", [(65, 2048, 512, False), (300, 4096, 256, True), (129, 4096, 256, False), (64, 8192, 128, False), (4000, 8192, 128, False),
+                                           (1024, 262144, 4, False), (17, 1024, 1024, True), (17, 1024, 1023, False), (64, 64, 16384, True),
+                                           (64, 63, 20000, False), (1024, 16, 65536, False), (17, 2048, 2048, True), (57, 2048, 1536, True),
+                                           (1024, 16384, 2048, True), (1000, 2052, 512, True), (500, 2200, 512, True), (499, 2200, 512, False)])
+def test_the_split_product_takes_what_it_is_faster_at(rows, n, k, pays):
+    assert ops.linear_f32_pays(rows, n, k) == pays
+
+
 # rows on both sides of 16 (the weight-streaming kernel, the split product) and a weight on both sides of the split product's least size
 @pytest.mark.gpu
 @pytest.mark.parametrize("M", [5, 33])

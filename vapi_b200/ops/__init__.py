@@ -712,14 +712,21 @@ LINEAR_F32_LEAST = 1 << 20
 LINEAR_F32_ROWS = 4096
 
 
+def linear_f32_pays(rows: int, n: int, k: int) -> bool:
+    """Whether the split product is at least as fast as the library's for ``rows`` x ``n`` x ``k``.  Its two launches, and the sum over
+    the blocks that share a tile, want a large weight, a long K and more than half a tile of features.  In a captured chain of products,
+    us against the library's: 17 x 1,024 x 1,024 13 and 14, 33 x 1,536 x 1,536 16 and 32; 65 x 2,048 x 512 19 and 12, 300 x 2,048 x 512 20 and
+    26; 129 x 4,096 x 256 16 and 15, 300 x 4,096 x 256 16 and 23; 64 x 8,192 x 128 10 and 7, 129 x 8,192 x 128 14.5 and 14; 64 x 64 x 16,384
+    54 and 58, 64 x 16 x 65,536 191 and 114."""
+    return n * k >= LINEAR_F32_LEAST and n >= 64 and (k >= 1024 or (k >= 256 and rows * n >= 1100000))
+
+
 def linear_f32_applies(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether the split product on the tensor cores takes this float32 product: 16-byte rows of the weight and the
-    tokens (inner size a multiple of 4, both contiguous and aligned), and a weight large enough that its two launches
-    pay: 17 x 100 x 36 takes 12 us against the library's 8, 129 tokens x 1536 x 1024 30 against 31 to 33, and from there
-    on it is ahead (33 tokens x 1536 x 1536 26 against 45)."""
+    tokens (inner size a multiple of 4, both contiguous and aligned), and a size at which it pays (:func:`linear_f32_pays`)."""
     return (use_tc and weight.is_cuda and weight.dtype == torch.float32 and x.dtype == torch.float32 and weight.dim() == 2
             and x.dim() == 2 and x.shape[0] > 0 and weight.shape[0] > 0 and x.shape[1] == weight.shape[1] > 0
-            and weight.shape[1] % 4 == 0 and weight.numel() >= LINEAR_F32_LEAST and weight.is_contiguous() and x.is_contiguous()
+            and weight.shape[1] % 4 == 0 and linear_f32_pays(x.shape[0], *weight.shape) and weight.is_contiguous() and x.is_contiguous()
             and weight.data_ptr() % 16 == 0 and x.data_ptr() % 16 == 0)
 
 
