@@ -102,3 +102,20 @@ def test_a_float32_product_that_gives_up_a_wait_writes_nothing_and_says_so(ops, 
         assert int(status) == (16 if bool(left.any()) else 0) and torch.equal(out[~left], want[~left])
         assert polls > 0 or bool(left.all())
         assert torch.equal(ops.linear_f32(a, w, status=status.zero_()), want) and int(status) == 0
+
+
+# both sides of every line of the dispatch: shared K or whole rows at 3,072, 6,144 and 8,192 rows and a K of 1,024, 1,536 and 2,048; whole rows
+# with and without the staged tokens (K of 128 and 256; more than eight tokens in rounds of blocks that are filled and that are not)
+@pytest.mark.parametrize("N,K", [(3071, 1024), (3073, 1024), (3072, 1028), (8191, 2048), (8193, 2048), (6143, 1536), (6145, 1536),
+                                 (6147, 1540), (6150, 2052), (3075, 4), (4099, 128), (4099, 132), (3077, 256),
+                                 (3077, 260), (12289, 512), (12287, 512), (12290, 2048), (12290, 2052), (8200, 4100)])
+def test_decode_product_of_wide_weights(ops, N, K):
+    """Against float64 within the bound of K float FMAs, and a token's result is the same bits whatever the batch."""
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    a, w, b = (torch.randn(*s, generator=g, device="cuda") for s in ((16, K), (N, K), (N,)))
+    want = a.double() @ w.double().t() + b.double()
+    bound = (K + 2) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t() + b.double().abs())
+    whole = ops.skinny_linear_f32(w, a, b)
+    assert ((whole.double() - want).abs() <= bound).all()
+    for M in (1, 2, 4, 5, 8, 9, 13):
+        assert torch.equal(ops.skinny_linear_f32(w, a[16 - M:].contiguous(), b), whole[16 - M:]), M

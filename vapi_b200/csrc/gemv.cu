@@ -887,8 +887,8 @@ VAPI_EXPORT int vapi_skinny_linear_conv(const void* W, int H, int K, int M, cons
 // The same product on the true 32-bit path: float weights, float tokens, float FMA and nothing
 // else (no tensor cores, no reduced-precision mode), for the decode steps of that path.
 //
-// Bound by reading the weights once, and by what is in flight: a block of four warps owns four weight rows and shares their
-// K, warp w takes the pieces w, w + 4, ... of 128 k, a lane 16 bytes of a piece of each row.  So even the narrowest product
+// Bound by reading the weights once, and by what is in flight.  Narrow weights (SHARE = 4): a block of four warps owns four weight rows and
+// shares their K, warp w takes the pieces w, w + 4, ... of 128 k, a lane 16 bytes of a piece of each row.  So even the narrowest product
 // of a model (2,048 rows) is 2,048 warps, the grid of many short blocks leaves no long last wave, and four blocks a
 // multiprocessor with f32_depth pieces of four rows a lane in flight keep about 100 KB on their way (before: eight warps of four
 // rows each, one round of loads between two barriers: 64 blocks for 2,048 rows).  The tokens' pieces come from L1, which
@@ -896,7 +896,9 @@ VAPI_EXPORT int vapi_skinny_linear_conv(const void* W, int H, int K, int M, cons
 // 2,048 x 2,048 6.3 us, 16,384 x 2,048 33, 2,048 x 8,192 17.6, 65,536 x 2,048 120 (4.5 TB/s); 3 tokens: 65,536 x 2,048 80 us
 // (6.7 TB/s).  One or two warps a row group instead of four (one launch, L2 flushed): 25 or 18 against 14 us at 2,048 x 2,048,
 // 84 or 48 against 29 at 2,048 x 8,192, and 143 against 125 at 65,536.
-// A lane's partial sums, the exchange over the lanes and the sum over the four warps add in an order that depends on K
+// Wide weights fill the device without sharing K, and the short blocks' starts and ends cost more than they give: there a warp owns its
+// four rows alone (SHARE = 1), or the form behind this one takes over, which adds in the same order.
+// A lane's partial sums, the exchange over the lanes and the sum over the four warps add in an order that depends on N and K
 // alone, so a token's result does not depend on what else is in the batch.
 constexpr int F32_WARPS = 4, F32_ROWS = 4;
 // pieces of the four rows that a lane has in flight.  The sums of many tokens take the registers, and what they leave is worth
@@ -910,22 +912,23 @@ __device__ __forceinline__ float4 f32_stream(const float4* p) {
     return v;
 }
 
-template <int MT>
+template <int MT, int SHARE>
 __global__ void __launch_bounds__(F32_WARPS * 32, MT <= 8 ? 4 : 3)
 skinny_linear_f32_kernel(const float* __restrict__ W, const float* act /*(the kernel before this one writes it)*/,
                          const float* __restrict__ bias, float* out, int N, int K, int M, long long out_stride) {
     constexpr int D = f32_depth(MT), C = F32_ROWS * MT, MG = MT < 8 ? MT : 8;    // (MG tokens at a time: registers)
     __shared__ float part[F32_WARPS][C];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long n0 = (long long)blockIdx.x * F32_ROWS;
+    constexpr int GROUPS = F32_WARPS / SHARE;                           // groups of rows in a block
+    const long long b0 = (long long)blockIdx.x * (GROUPS * F32_ROWS), n0 = b0 + warp / SHARE * F32_ROWS;
     pdl_trigger();
     const int k4 = K >> 2;
-    const int first = warp * 32 + lane;                                 // this lane's 16-byte pieces of a row: first, first + step, ...
-    constexpr int step = F32_WARPS * 32;
-    const int steps = (k4 - warp * 32 + step - 1) / step;               // (the same for the whole warp; <= 0: none)
+    const int first = warp % SHARE * 32 + lane;                         // this lane's 16-byte pieces of a row: first, first + step, ...
+    constexpr int step = SHARE * 32;
+    const int steps = n0 < N ? (k4 - warp % SHARE * 32 + step - 1) / step : 0;      // (the same for the whole warp; <= 0: none)
     const float4* wrow[F32_ROWS];
 #pragma unroll
-    for (int r = 0; r < F32_ROWS; ++r) wrow[r] = reinterpret_cast<const float4*>(W + (size_t)(n0 + r < N ? n0 + r : n0) * K);
+    for (int r = 0; r < F32_ROWS; ++r) wrow[r] = reinterpret_cast<const float4*>(W + (size_t)(n0 + r < N ? n0 + r : b0) * K);
     float acc[C];
 #pragma unroll
     for (int i = 0; i < C; ++i) acc[i] = 0.f;
@@ -989,11 +992,106 @@ skinny_linear_f32_kernel(const float* __restrict__ W, const float* act /*(the ke
         part[warp][lane / (32 / (C < 32 ? C : 32))] = acc[0];
     }
     __syncthreads();
-    // the four warps in order; neighbouring threads write neighbouring features of a token
-    if (threadIdx.x < C) {
-        const int r = threadIdx.x % F32_ROWS, m = threadIdx.x / F32_ROWS, i = r * MT + m;
-        if (n0 + r < N && m < M)
-            out[(size_t)m * out_stride + n0 + r] = part[0][i] + part[1][i] + part[2][i] + part[3][i] + (bias ? bias[n0 + r] : 0.f);
+    // the warps that share K in order; neighbouring threads write neighbouring features of a token
+    constexpr int ROWS = GROUPS * F32_ROWS;
+    for (int j = threadIdx.x; j < ROWS * MT; j += F32_WARPS * 32) {
+        const int r = j % ROWS, m = j / ROWS, i = r % F32_ROWS * MT + m, w0 = r / F32_ROWS * SHARE;
+        if (b0 + r < N && m < M) {
+            float y = part[w0][i];
+#pragma unroll
+            for (int w = 1; w < SHARE; ++w) y += part[w0 + w][i];
+            out[(size_t)m * out_stride + b0 + r] = y + (bias ? bias[b0 + r] : 0.f);
+        }
+    }
+}
+
+// Wide weights, up to eight tokens: eight warps a block, each with whole weight rows of its own, the tokens staged through shared
+// memory a chunk of K at a time (two buffers, filled by asynchronous copies one chunk ahead), so that they are read from L2 once a
+// block and serve eight warps.  65,536 x 2,048, 8 tokens 106 us against 120 with shared K, 16,384 x 2,048 34 against 36, 8,192 x
+// 2,048 17.7 against 19.6, 3,072 x 512 3.5 against 4.0, 16,384 x 256 9.4 against 11.4; 2,048 x 2,048 10.4 against 6.6.
+constexpr int F32_STAGED_WARPS = 8;
+// rows of the weight a warp owns, and 16-byte pieces of each row that a lane asks for together
+// (fewer of both for nine to sixteen tokens, whose sums take the registers)
+__host__ __device__ constexpr int f32_staged_rows(int mt) { return mt <= 8 ? 4 : 2; }
+__host__ __device__ constexpr int f32_staged_depth(int mt) { return mt <= 8 ? 4 : 2; }
+
+template <int MT>
+__global__ void __launch_bounds__(F32_STAGED_WARPS * 32)
+skinny_linear_f32_staged_kernel(const float* __restrict__ W, const float* __restrict__ act, const float* __restrict__ bias,
+                         float* __restrict__ out, int N, int K, int M, long long out_stride) {
+    constexpr int ROWS = f32_staged_rows(MT), DEPTH = f32_staged_depth(MT);
+    constexpr int CHUNK = 32 * DEPTH;             // pieces of K in a chunk
+    __shared__ float4 abuf[2][MT][CHUNK];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long n0 = ((long long)blockIdx.x * F32_STAGED_WARPS + warp) * ROWS;
+    pdl_trigger();
+    float acc[ROWS][MT];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) acc[r][m] = 0.f;
+    const int k4 = K >> 2;
+    const int chunks = (k4 + CHUNK - 1) / CHUNK;
+    const float4* wrow[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) wrow[r] = reinterpret_cast<const float4*>(W + (size_t)(n0 + r < N ? n0 + r : 0) * K);
+    float4 w[DEPTH][ROWS];
+    auto fetch = [&](int c0) {          // this lane's pieces of a chunk of its rows
+#pragma unroll
+        for (int u = 0; u < DEPTH; ++u)
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+                w[u][r] = (c0 + 32 * u < k4 && n0 < N) ? __ldcs(wrow[r] + c0 + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto stage = [&](int chunk, int buf) {     // the tokens' pieces of a chunk, by the whole block
+        for (int idx = threadIdx.x; idx < MT * CHUNK; idx += F32_STAGED_WARPS * 32) {
+            const int m = idx / CHUNK, c = idx - m * CHUNK, cg = chunk * CHUNK + c;
+            const bool ok = m < M && cg < k4;
+            gv_cp16(&abuf[buf][m][c], reinterpret_cast<const float4*>(act + (size_t)(ok ? m : 0) * K) + (ok ? cg : 0), ok ? 16 : 0);
+        }
+        gv_commit();
+    };
+    fetch(lane);                         // the weights do not depend on the kernel before this one
+    pdl_wait();
+    stage(0, 0);
+    for (int ch = 0; ch < chunks; ++ch) {
+        if (ch + 1 < chunks) stage(ch + 1, (ch + 1) & 1);
+        else gv_commit();
+        gv_wait<1>();
+        __syncthreads();                 // chunk ch of the tokens is in place for every warp
+        if (ch > 0) fetch(ch * CHUNK + lane);
+#pragma unroll
+        for (int u = 0; u < DEPTH; ++u) {
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const float4 a = abuf[ch & 1][m][lane + 32 * u];
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r) {
+                    acc[r][m] = fmaf(w[u][r].x, a.x, acc[r][m]);
+                    acc[r][m] = fmaf(w[u][r].y, a.y, acc[r][m]);
+                    acc[r][m] = fmaf(w[u][r].z, a.z, acc[r][m]);
+                    acc[r][m] = fmaf(w[u][r].w, a.w, acc[r][m]);
+                }
+            }
+        }
+        __syncthreads();                 // everyone is done with this buffer before it is filled again
+    }
+    gv_wait<0>();
+    if (n0 >= N) return;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) acc[r][m] = warp_sum(acc[r][m]);
+    if (lane == 0) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            if (n0 + r < N) {
+                const float b = bias ? bias[n0 + r] : 0.f;
+#pragma unroll
+                for (int m = 0; m < MT; ++m)
+                    if (m < M) out[(size_t)m * out_stride + n0 + r] = acc[r][m] + b;
+            }
+        }
     }
 }
 
@@ -1005,12 +1103,31 @@ VAPI_EXPORT int vapi_skinny_linear_f32(const float* W, int N, int K, int M, cons
     if (N <= 0 || K <= 0 || K % 4 != 0) return fail(-1, "skinny_linear_f32: K=%d must be a positive multiple of 4 (N=%d)", K, N);
     if (!W || !act || !out) return fail(-1, "skinny_linear_f32: missing array");
     if ((((uintptr_t)W | (uintptr_t)act) & 15) != 0) return fail(-1, "skinny_linear_f32: operands must be 16-byte aligned");
-    const int blocks = (N + F32_ROWS - 1) / F32_ROWS;
+    // Which order of addition (SHARE 4, or a warp for whole rows) is a matter of N and K alone, see above; where the lines lie, in us in a
+    // captured chain of products at 1 / 8 tokens, shared K against whole rows: 2,048 x 1,024 2.7 / 3.8 against 2.8 / 5.1, 3,072 x 1,024 4.0 /
+    // 6.0 against 3.7 / 6.5; 4,608 x 1,536 6.7 / 9.7 against 6.6 / 10.8, 6,144 x 1,536 8.1 / 12.4 against 7.5 / 12.1, x 2,048 10.1 / 15.2 against
+    // 10.2 / 16.2, x 4,096 21.1 / 27.1 against 19.1 / 30.6; 8,192 x 2,048 13.0 / 19.6 against 12.6 / 17.7, x 4,096 24.1 / 36.6 against 21.7 / 34.0.
+    const bool whole = N >= 8192 || (K <= 1024 && N >= 3072) || (N >= 6144 && (K <= 1536 || K > 2048));
+    // Of the two forms for whole rows the unstaged one is ahead where K is a piece or two (65,536 x 128 at 1 / 8 tokens 10.9 / 14.2 against
+    // 12.2 / 29.6; 8,192 x 512 4.7 / 6.7 against 3.5 / 5.8; 16 tokens x 256 7.8 against 8.4) and, above eight tokens, where its blocks, three a
+    // multiprocessor, fill their rounds: 16 tokens 6,144 x 4,096 57 against 70 (a round, filled to 0.86), 16,384 x 2,048 69 against 74,
+    // 65,536 x 2,048 194 against 245, but 8,192 x 2,048 53 against 38 (two, to 0.58) and 16,384 x 4,096 159 against 139.
+    const long long own = (N + F32_WARPS * F32_ROWS - 1) / (F32_WARPS * F32_ROWS), places = 3LL * sm_count(), rounds = (own + places - 1) / places;
+    const bool filled = 4 * own >= 3 * places * rounds && (rounds == 1 || K <= 2048);
+    const bool staged = whole && K > 128 && (M <= 8 || (K > 256 && !filled));
     cudaError_t e;
-    if (M <= 1) e = launch(skinny_linear_f32_kernel<1>, blocks, F32_WARPS * 32, 0, stream, W, act, bias, out, N, K, M, out_stride);
-    else if (M <= 4) e = launch(skinny_linear_f32_kernel<4>, blocks, F32_WARPS * 32, 0, stream, W, act, bias, out, N, K, M, out_stride);
-    else if (M <= 8) e = launch(skinny_linear_f32_kernel<8>, blocks, F32_WARPS * 32, 0, stream, W, act, bias, out, N, K, M, out_stride);
-    else e = launch(skinny_linear_f32_kernel<16>, blocks, F32_WARPS * 32, 0, stream, W, act, bias, out, N, K, M, out_stride);
+#define VAPI_F32(KERNEL, WARPS, ROWS)                                                                                                     \
+    e = launch(KERNEL, (N + (ROWS) - 1) / (ROWS), (WARPS) * 32, 0, stream, W, act, bias, out, N, K, M, out_stride)
+#define VAPI_F32_MT(MT)                                                                                                                   \
+    if (staged) VAPI_F32(skinny_linear_f32_staged_kernel<MT>, F32_STAGED_WARPS, F32_STAGED_WARPS * f32_staged_rows(MT));                   \
+    else if (whole) VAPI_F32((skinny_linear_f32_kernel<MT, 1>), F32_WARPS, F32_WARPS * F32_ROWS);                                          \
+    else VAPI_F32((skinny_linear_f32_kernel<MT, F32_WARPS>), F32_WARPS, F32_ROWS)
+    if (M <= 1) { VAPI_F32_MT(1); }
+    else if (M <= 4) { VAPI_F32_MT(4); }
+    else if (M <= 8) { VAPI_F32_MT(8); }
+    else { VAPI_F32_MT(16); }
+#undef VAPI_F32_MT
+#undef VAPI_F32
     return check_launch("skinny_linear_f32", e);
 }
 
