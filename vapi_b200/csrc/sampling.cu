@@ -183,22 +183,26 @@ __device__ __forceinline__ float tr_unkey(unsigned k) {
 constexpr int TR_LIST = 4096;
 
 // f(scaled logit, id, whether there is one) for every logit of a row, the same number of times in every thread of the
-// block; 16 bytes at a time where the row's start allows (`vec`: how many such pieces, the rest one by one).
+// block: 16 bytes at a time, one by one only the `head` before the first 16-byte boundary (at most three) and what is left at the end, or
+// all of a row that would not give every thread a piece.  (Every row of an odd vocabulary but the first begins off the boundary: 5 rows
+// of 65,537 logits at top-p 0.95 210 us one by one, 166 so.)
 template <typename F>
-__device__ __forceinline__ void tr_row(const float* __restrict__ l, int vocab, int vec, float it, F f) {
-    const float4* l4 = reinterpret_cast<const float4*>(l);
+__device__ __forceinline__ void tr_row(const float* __restrict__ l, int vocab, int head, float it, F f) {
+    const int vec = vocab > 4 * TR_THREADS ? (vocab - head) / 4 : 0;
+    const float4* l4 = reinterpret_cast<const float4*>(l + head);
 #pragma unroll 4
     for (int base = 0; base < vec; base += TR_THREADS) {
         const int i = base + (int)threadIdx.x;
         const bool ok = i < vec;
         const float4 v = ok ? l4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        f(v.x * it, 4 * i, ok);
-        f(v.y * it, 4 * i + 1, ok);
-        f(v.z * it, 4 * i + 2, ok);
-        f(v.w * it, 4 * i + 3, ok);
+        const int id = head + 4 * i;
+        f(v.x * it, id, ok);
+        f(v.y * it, id + 1, ok);
+        f(v.z * it, id + 2, ok);
+        f(v.w * it, id + 3, ok);
     }
-    for (int base = 4 * vec; base < vocab; base += TR_THREADS) {
-        const int i = base + (int)threadIdx.x;
+    for (int base = 0; base < vocab - 4 * vec; base += TR_THREADS) {
+        const int t = base + (int)threadIdx.x, i = t < head ? t : t + 4 * vec;
         const bool ok = i < vocab;
         f(ok ? l[i] * it : 0.f, i, ok);
     }
@@ -293,8 +297,8 @@ sample_truncated_kernel(const float* __restrict__ logits, int vocab, long long r
     if (k < 0) return;                                  // not a row of this kernel (uniform over the block)
     const float* l = logits + (size_t)row * row_stride;
     const float it = inv_t[row];
-    const int vec = (reinterpret_cast<uintptr_t>(l) & 15) == 0 ? vocab / 4 : 0;
-    auto whole = [&](auto f) { tr_row(l, vocab, vec, it, f); };
+    const int head = min(vocab, (int)((16u - (unsigned)(reinterpret_cast<uintptr_t>(l) & 15)) & 15) / 4);
+    auto whole = [&](auto f) { tr_row(l, vocab, head, it, f); };
 
     // the maximum of the scaled logits
     float m = -INFINITY;
@@ -306,38 +310,45 @@ sample_truncated_kernel(const float* __restrict__ logits, int vocab, long long r
     m = sv[0];
     for (int w = 1; w < TR_WARPS; ++w) m = fmaxf(m, sv[w]);
     __syncthreads();
-    float tau = m - TR_WINDOW;
+    const float window = m - TR_WINDOW;
+    float tau = window;
 
-    // top-k: the upper half of the k-th largest key; nothing below it survives
+    // top-k: the upper half of the k-th largest key; nothing below it, or below min-p's threshold, survives
     unsigned long long target = (unsigned long long)k;
     unsigned prefix = 0u;
-    bool cut = k > 0 && k < vocab && tr_descend<false>(whole, 0, 2, m, tau, target, prefix, hist, bins, sh_u);
-    const float least = cut ? fmaxf(tau, tr_unkey(prefix << 16)) : tau;
-    const float tp = top_p ? top_p[row] : 1.f;
+    const bool cut = k > 0 && k < vocab && tr_descend<false>(whole, 0, 2, m, tau, target, prefix, hist, bins, sh_u);
+    const float mp = min_p ? min_p[row] : 0.f, tp = top_p ? top_p[row] : 1.f;
+    const float floor_p = mp > 0.f ? m + logf(mp) : -INFINITY;
+    const float least = fmaxf(cut ? fmaxf(tau, tr_unkey(prefix << 16)) : tau, floor_p);
 
-    // the mass of the whole 30-nat window, in fixed point (integer sums: any order), and the list
+    // the mass of the whole 30-nat window, in fixed point (integer sums: any order), and the list.  Without top-k and top-p all that is
+    // left is the draw, which may as well walk the row (65,536 logits, min-p alone: 9.5 us, 24.5 with a list).
+    const bool mass = tp < 1.f;
     unsigned long long z = 0ull;
-    whole([&](float sc, int i, bool ok) {
-        if (tp < 1.f && ok && sc >= tau) z += (unsigned long long)(expf(sc - m) * TR_FIX);
-        const bool in = ok && sc >= least;
-        const unsigned who = __ballot_sync(0xffffffffu, in);
-        if (who == 0u) return;
-        unsigned at = 0u;
-        // (a count beyond the list's room stays beyond it)
-        if (lane == 0) at = *reinterpret_cast<volatile unsigned*>(&sh_u[1]) > TR_LIST ? TR_LIST + 1u : atomicAdd(&sh_u[1], (unsigned)__popc(who));
-        at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)__popc(who & ((1u << lane) - 1u));
-        if (in && at < TR_LIST) {
-            list_s[at] = sc;
-            list_i[at] = i;
-        }
-    });
-    for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-    if (lane == 0) bins[warp] = z;
-    __syncthreads();
-    z = 0ull;
-    for (int w = 0; w < TR_WARPS; ++w) z += bins[w];
-    const unsigned listed = sh_u[1];
-    __syncthreads();
+    unsigned listed = TR_LIST + 1u;
+    if (mass || cut) {
+        whole([&](float sc, int i, bool ok) {
+            if (mass && ok && sc >= window) z += (unsigned long long)(expf(sc - m) * TR_FIX);
+            const bool in = ok && sc >= least;
+            const unsigned who = __ballot_sync(0xffffffffu, in);
+            if (who == 0u) return;
+            unsigned at = 0u;
+            // (a count beyond the list's room stays beyond it)
+            if (lane == 0) at = *reinterpret_cast<volatile unsigned*>(&sh_u[1]) > TR_LIST ? TR_LIST + 1u : atomicAdd(&sh_u[1], (unsigned)__popc(who));
+            at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)__popc(who & ((1u << lane) - 1u));
+            if (in && at < TR_LIST) {
+                list_s[at] = sc;
+                list_i[at] = i;
+            }
+        });
+        for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+        if (lane == 0) bins[warp] = z;
+        __syncthreads();
+        z = 0ull;
+        for (int w = 0; w < TR_WARPS; ++w) z += bins[w];
+        listed = sh_u[1];
+        __syncthreads();
+    }
     auto candidates = [&](auto f) {
         if (listed > TR_LIST) {
             whole(f);
@@ -349,10 +360,10 @@ sample_truncated_kernel(const float* __restrict__ logits, int vocab, long long r
             f(ok ? list_s[i] : 0.f, ok ? list_i[i] : 0, ok);
         }
     };
+    // (where the k-th largest lies below min-p's threshold, which the list ends at, the lower half finds too few and cuts nothing)
     if (cut && tr_descend<false>(candidates, 2, 4, m, tau, target, prefix, hist, bins, sh_u)) tau = fmaxf(tau, tr_unkey(prefix));
-    const float mp = min_p ? min_p[row] : 0.f;
-    if (mp > 0.f) tau = fmaxf(tau, m + logf(mp));
-    if (tp < 1.f) {
+    tau = fmaxf(tau, floor_p);
+    if (mass) {
         target = (unsigned long long)((double)z * (double)tp);
         prefix = 0u;
         if (target > 0ull && tr_descend<true>(candidates, 0, 4, m, tau, target, prefix, hist, bins, sh_u)) tau = fmaxf(tau, tr_unkey(prefix));
