@@ -63,7 +63,7 @@ template <int NT> struct LfCfg {
 struct LfParams {
     const float* W; const float* act; const float* bias; const int* tok_bad; float* out; int* status;
     int N, K, M, num_kb, num_m, num_tiles, split;
-    unsigned polls;                       // of an mbarrier before a role gives up
+    unsigned polls;                       // of an mbarrier before a role gives up, where that is not the usual limit
     long long out_stride;
 };
 
@@ -148,15 +148,18 @@ __device__ __forceinline__ float lf_plain(const float* __restrict__ a, const flo
     return s;
 }
 
-template <int NT>
+// TRIAL: the number of polls before a role gives up comes with the call (a limit that is not a constant costs the thread that issues
+// the products 3 %, a second barrier to wait for before a stage's products 4 %)
+template <int NT, bool TRIAL>
 __global__ void __launch_bounds__(LF_THREADS, 1)
 linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_tok, const LfParams p) {
     using Cfg = LfCfg<NT>;
+    const unsigned polls = TRIAL ? p.polls : TC5_WAIT_LIMIT;
     extern __shared__ unsigned char lf_smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(lf_smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* tok_mem = base + (size_t)LF_W_STAGES * LF_W_BYTES;
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(tok_mem + (size_t)LF_STAGES * Cfg::STAGE_BYTES);
-    unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 3 * LF_STAGES + 4 + 2 * LF_W_STAGES + 1);
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * LF_STAGES + 4 + 2 * LF_W_STAGES + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     unsigned char* w_bad = reinterpret_cast<unsigned char*>(bars) + 256;            // [LF_BAD_TILES][128]
 
@@ -169,10 +172,10 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     const unsigned full0 = smem_u32(bars), empty0 = smem_u32(bars + LF_STAGES);
     const unsigned accfull0 = smem_u32(bars + 2 * LF_STAGES), accempty0 = smem_u32(bars + 2 * LF_STAGES + 2);
     const unsigned wfull0 = smem_u32(bars + 2 * LF_STAGES + 4), wempty0 = smem_u32(bars + 2 * LF_STAGES + 4 + LF_W_STAGES);
-    const unsigned tokfull0 = smem_u32(bars + 2 * LF_STAGES + 4 + 2 * LF_W_STAGES), drained = tokfull0 + 8 * LF_STAGES;
+    const unsigned drained = smem_u32(bars + 2 * LF_STAGES + 4 + 2 * LF_W_STAGES);
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < LF_STAGES; ++i) { mbar_init(full0 + 8 * i, 4); mbar_init(tokfull0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
+        for (int i = 0; i < LF_STAGES; ++i) { mbar_init(full0 + 8 * i, 1 + 4); mbar_init(empty0 + 8 * i, 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(accfull0 + 8 * i, 1); mbar_init(accempty0 + 8 * i, 4); }
         for (int i = 0; i < LF_W_STAGES; ++i) { mbar_init(wfull0 + 8 * i, 1); mbar_init(wempty0 + 8 * i, 4); }
         mbar_init(drained, 1);
@@ -202,8 +205,8 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
             float top = 0.f;
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
                 const int s = it % LF_STAGES, ws = it % LF_W_STAGES;
-                if (!lf_wait(wfull0 + 8 * ws, (it / LF_W_STAGES) & 1, abort_flag, p.polls)) ok = false;
-                if (!lf_wait(empty0 + 8 * s, ((it / LF_STAGES) & 1) ^ 1, abort_flag, p.polls)) ok = false;
+                if (!lf_wait(wfull0 + 8 * ws, (it / LF_W_STAGES) & 1, abort_flag, polls)) ok = false;
+                if (!lf_wait(empty0 + 8 * s, ((it / LF_STAGES) & 1) ^ 1, abort_flag, polls)) ok = false;
                 if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
                 tc5_fence_after();
                 const unsigned char* w = base + (size_t)ws * LF_W_BYTES + row * 128;
@@ -237,7 +240,7 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                 const int n0 = (t / p.num_m) * LF_BM;
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int ws = it % LF_W_STAGES;
-                    if (!lf_wait(wempty0 + 8 * ws, ((it / LF_W_STAGES) & 1) ^ 1, abort_flag, p.polls)) { ok = false; break; }
+                    if (!lf_wait(wempty0 + 8 * ws, ((it / LF_W_STAGES) & 1) ^ 1, abort_flag, polls)) { ok = false; break; }
                     const unsigned w = smem_u32(base + (size_t)ws * LF_W_BYTES);
                     mbar_expect_tx(wfull0 + 8 * ws, LF_W_BYTES);
                     tma_load_2d(w, &tm_w, wfull0 + 8 * ws, kb * LF_BK, n0);
@@ -254,12 +257,12 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                 const int m0 = (t % p.num_m) * NT;
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % LF_STAGES;
-                    if (!lf_wait(empty0 + 8 * s, ((it / LF_STAGES) & 1) ^ 1, abort_flag, p.polls)) { ok = false; break; }
+                    if (!lf_wait(empty0 + 8 * s, ((it / LF_STAGES) & 1) ^ 1, abort_flag, polls)) { ok = false; break; }
                     const unsigned b = smem_u32(tok_mem + (size_t)s * Cfg::STAGE_BYTES);
-                    mbar_expect_tx(tokfull0 + 8 * s, 3 * Cfg::B_PLANE);
+                    mbar_expect_tx(full0 + 8 * s, 3 * Cfg::B_PLANE);
 #pragma unroll
                     for (int i = 0; i < 3; ++i)          // (rows behind the last token are the next plane's, or zeros: never stored)
-                        tma_load_2d(b + i * Cfg::B_PLANE, &tm_tok, tokfull0 + 8 * s, kb * LF_BK, i * p.M + m0);
+                        tma_load_2d(b + i * Cfg::B_PLANE, &tm_tok, full0 + 8 * s, kb * LF_BK, i * p.M + m0);
                 }
             }
         }
@@ -271,9 +274,8 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
             for (int t = first; t < p.num_tiles && ok; t += step) {
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % LF_STAGES, buf = it & 1;
-                    if (!lf_wait(accempty0 + 8 * buf, ((it >> 1) & 1) ^ 1, abort_flag, p.polls) ||
-                        !lf_wait(tokfull0 + 8 * s, (it / LF_STAGES) & 1, abort_flag, p.polls) ||
-                        !lf_wait(full0 + 8 * s, (it / LF_STAGES) & 1, abort_flag, p.polls)) { ok = false; break; }
+                    if (!lf_wait(accempty0 + 8 * buf, ((it >> 1) & 1) ^ 1, abort_flag, polls) ||
+                        !lf_wait(full0 + 8 * s, (it / LF_STAGES) & 1, abort_flag, polls)) { ok = false; break; }
                     tc5_fence_after();
                     const unsigned a = tmem_base + LF_A_COL0 + (unsigned)(s * 3 * LF_A_COLS), b = smem_u32(tok_mem + (size_t)s * Cfg::STAGE_BYTES);
                     const unsigned d = tmem_base + (unsigned)(buf * NT);
@@ -301,7 +303,7 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         for (int t = first; t < p.num_tiles && ok; t += step, ++tl) {
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
                 const int buf = it & 1;
-                if (!lf_wait(accfull0 + 8 * buf, (it >> 1) & 1, abort_flag, p.polls)) ok = false;
+                if (!lf_wait(accfull0 + 8 * buf, (it >> 1) & 1, abort_flag, polls)) ok = false;
                 if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
                 tc5_fence_after();
 #pragma unroll
@@ -396,9 +398,13 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     __syncthreads();
     if (*abort_flag) {                                   // (the same for all: every role is through)
         if (threadIdx.x == 0 && p.status) atomicExch(p.status, 16);
+        if (threadIdx.x == 8 * 32) abort_flag[1] = it;
+        __syncthreads();
         if (lane == 0) {                                 // what is under way ends before its memory is given back
+            if (warp >= 4 && warp < 8)                   // (a tokens' stage is full when these warps have arrived too)
+                for (int i = it; i < abort_flag[1]; ++i) mbar_arrive(full0 + 8 * (i % LF_STAGES));
             if (warp == 8)
-                for (int i = max(it - LF_STAGES, 0); i < it; ++i) mbar_wait(tokfull0 + 8 * (i % LF_STAGES), (i / LF_STAGES) & 1);
+                for (int i = max(it - LF_STAGES, 0); i < it; ++i) mbar_wait(full0 + 8 * (i % LF_STAGES), (i / LF_STAGES) & 1);
             if (warp == 10)
                 for (int i = max(it - LF_W_STAGES, 0); i < it; ++i) mbar_wait(wfull0 + 8 * (i % LF_W_STAGES), (i / LF_W_STAGES) & 1);
             if (warp == 9 && it > 0) {
@@ -429,10 +435,10 @@ static int lf_encode(CUtensorMap* map, CUtensorMapDataType type, int size, const
     return r == CUDA_SUCCESS ? 0 : fail(-103, "linear_f32: cuTensorMapEncodeTiled failed with %d", (int)r);
 }
 
-template <int NT>
+template <int NT, bool TRIAL>
 static int launch_lf(const CUtensorMap& tw, const CUtensorMap& tm, const LfParams& p, cudaStream_t stream) {
     using Cfg = LfCfg<NT>;
-    auto kern = linear_f32_kernel<NT>;
+    auto kern = linear_f32_kernel<NT, TRIAL>;
     static bool attr_done = false;
     if (!attr_done) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
@@ -490,7 +496,7 @@ VAPI_EXPORT int vapi_linear_f32(const float* W, int N, int K, int M, const float
     int nt;
     vapi_linear_f32_plan(N, K, M, &nt, &p.split);
     p.W = W; p.act = act; p.bias = bias; p.tok_bad = bad; p.out = out; p.status = status;
-    p.N = N; p.K = K; p.M = M; p.out_stride = out_stride; p.polls = polls < 0 ? TC5_WAIT_LIMIT : (unsigned)polls;
+    p.N = N; p.K = K; p.M = M; p.out_stride = out_stride; p.polls = polls < 0 ? 0u : (unsigned)polls;
     p.num_kb = (K + LF_BK - 1) / LF_BK;
     p.num_m = (M + nt - 1) / nt;
     p.num_tiles = p.num_m * ((N + LF_BM - 1) / LF_BM);
@@ -498,7 +504,8 @@ VAPI_EXPORT int vapi_linear_f32(const float* W, int N, int K, int M, const float
     rc = lf_encode(&tw, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, W, N, K, LF_BM);
     if (rc == 0) rc = lf_encode(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, planes, 3LL * M, Kp, nt);
     if (rc) return rc;
-    return nt == 64 ? launch_lf<64>(tw, tm, p, stream) : launch_lf<128>(tw, tm, p, stream);
+    if (polls >= 0) return nt == 64 ? launch_lf<64, true>(tw, tm, p, stream) : launch_lf<128, true>(tw, tm, p, stream);
+    return nt == 64 ? launch_lf<64, false>(tw, tm, p, stream) : launch_lf<128, false>(tw, tm, p, stream);
 }
 
 VAPI_EXPORT const char* vapi_last_error() { return error_buffer(); }
