@@ -75,6 +75,28 @@ def test_float32_product_of_what_cannot_be_split(ops, M, N, K):
     assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
 
 
+# a tile of one block, and one shared by several
+@pytest.mark.parametrize("M,N,K", [(70, 300, 256), (40, 130, 2048)])
+def test_float32_product_whose_terms_overflow_though_no_operand_is_huge(ops, M, N, K):
+    """Products beyond the largest float from operands of 1e25 to 1e35, with every combination of signs of the second planes (a mantissa just above
+    or below one of eight bits): infinities of the product's sign, as float FMAs give, and no NaN; nothing else changes."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    clean = ops.linear_f32(a, w)
+    a2, w2 = a.clone(), w.clone()
+    mantissas = torch.tensor([1.0 + 2.0 ** -9, 1.0 - 2.0 ** -10, -1.5 - 2.0 ** -9, -1.5 + 2.0 ** -9], device="cuda")
+    a2[:4, K - 3], w2[:4, K - 3] = mantissas * 2.0 ** 83, mantissas * 2.0 ** 117
+    a2[M - 1, 5], w2[N - 1, 5] = 1.1e35, -1.1e25
+    a2[4:M - 1, [5, K - 3]], w2[4:N - 1, [5, K - 3]] = 0.0, 0.0      # (one huge term a sum: what more give depends on their order)
+    a2[:4, 5], w2[:4, 5], a2[M - 1, K - 3], w2[N - 1, K - 3] = 0.0, 0.0, 0.0, 0.0
+    got, want = ops.linear_f32(a2, w2), (a2.double() @ w2.double().t()).float()
+    assert int(torch.isinf(want).sum()) == 17 and torch.equal(torch.isinf(got), torch.isinf(want)) and not torch.isnan(got).any()
+    assert torch.equal(got[torch.isinf(got)], want[torch.isinf(want)])
+    fin = torch.isfinite(want)
+    assert ((got.double() - a2.double() @ w2.double().t()).abs() <= _bound(a2, w2))[fin].all()
+    assert torch.equal(ops.linear_f32(a, w), clean)
+
+
 def test_float32_product_of_tiny_and_exact_numbers(ops):
     """Numbers of eight bits have empty lower planes; small whole numbers come out exactly; small magnitudes keep their bits."""
     g = torch.Generator(device="cuda").manual_seed(4)

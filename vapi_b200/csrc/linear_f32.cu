@@ -14,7 +14,8 @@
 // 1,225 us (203 TFLOP/s, 1,220 on the tensor cores), 1,024 x 2,048 x 8,192 in 197 against 616 us, 57 x 2,048 x 1,536 in 26
 // against 45 us (events, L2 flushed).
 // Elements below 2^-109 in magnitude lose what lies below 2^-134.  A row with an element of 2^127 or more, an
-// infinity or a NaN cannot be split; its results are computed by plain FMAs, so they are what they always were.
+// infinity or a NaN cannot be split, and where a product overflows the partial ones do so in different directions (x1 y1 to infinity, x1 y2 to
+// minus infinity); such results are computed by plain FMAs, so they are what they always were.
 //
 // Orientation.  The weight rows are the 128-row operand, the tokens the columns (NT = 64 or 128 a tile): an epilogue
 // thread owns a weight row, and the 32 threads of a warp store 32 neighbouring features of a token, a whole line.
@@ -140,13 +141,17 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* x, __nv_bf
     if (threadIdx.x == 0) bad[m] = any;
 }
 
-// a result whose row or token cannot be split
+// a result whose row or token cannot be split, or that came out as no finite number
 __device__ __forceinline__ float lf_plain(const float* __restrict__ a, const float* __restrict__ w, int K) {
     float s = 0.f;
 #pragma unroll 1
-    for (int k = 0; k < K; ++k) s = fmaf(a[k], w[k], s);
+    for (int k = 0; k < K; k += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
+        s = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, s))));
+    }
     return s;
 }
+__device__ __forceinline__ bool lf_finite(float x) { return fabsf(x) <= 3.402823466e38f; }
 
 // TRIAL: the number of polls before a role gives up comes with the call (a limit that is not a constant costs the thread that issues
 // the products 3 %, a second barrier to wait for before a stage's products 4 %)
@@ -327,16 +332,23 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
             const long long n = (long long)(t / p.num_m) * LF_BM + warp * 32 + lane;
             const bool wb = w_bad[(tl % LF_BAD_TILES) * LF_BM + warp * 32 + lane] != 0;
             const float b = (p.bias && n < p.N) ? p.bias[n] : 0.f;
+            unsigned odd[NT / 32];
+#pragma unroll
+            for (int c = 0; c < NT / 32; ++c) odd[c] = 0u;
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
                 if (n < p.N && m0 + j < p.M) p.out[(size_t)(m0 + j) * p.out_stride + n] = acc[j] + b;
+                if (!lf_finite(acc[j])) odd[j / 32] |= 1u << (j % 32);
                 acc[j] = 0.f;
             }
+#pragma unroll
             for (int c = 0; c < NT; c += 32) {           // (rare) what could not be split, over what was just written
                 const unsigned tb = __ballot_sync(0xffffffffu, m0 + c + lane < p.M && p.tok_bad[m0 + c + lane] != 0);
-                if (n >= p.N || !(wb || tb)) continue;
+                const unsigned again = wb ? 0xffffffffu : (tb | odd[c / 32]);
+                if (n >= p.N || again == 0u) continue;
+#pragma unroll 1
                 for (int j = 0; j < 32 && m0 + c + j < p.M; ++j)
-                    if (wb || (tb >> j & 1))
+                    if (again >> j & 1)
                         p.out[(size_t)(m0 + c + j) * p.out_stride + n] = lf_plain(p.act + (size_t)(m0 + c + j) * p.K, p.W + (size_t)n * p.K, p.K) + b;
             }
         }
@@ -385,7 +397,7 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                 for (int i = 0; i < 8; ++i) {
                     const int m = m0 + j + i;
                     if (n < p.N && m < p.M) {
-                        if (wb || tb[i] != 0) y[i] = lf_plain(p.act + (size_t)m * p.K, p.W + (size_t)n * p.K, p.K);
+                        if (wb || tb[i] != 0 || !lf_finite(y[i])) y[i] = lf_plain(p.act + (size_t)m * p.K, p.W + (size_t)n * p.K, p.K);
                         p.out[(size_t)m * p.out_stride + n] = y[i] + b;
                     }
                 }
