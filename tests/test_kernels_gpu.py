@@ -1004,7 +1004,7 @@ def test_linear_tc_plain_products(ops, M, N, K):
     torch.testing.assert_close(got.cpu(), want, atol=3e-3 * math.sqrt(K / 96), rtol=1e-3)
 
 
-@pytest.mark.parametrize("M", [24, 64, 130])
+@pytest.mark.parametrize("M", [24, 64, 100, 128, 130])
 def test_linear_tc_fusions(ops, M):
     torch.manual_seed(31)
     H, F, eps = 256, 328, 1e-6
