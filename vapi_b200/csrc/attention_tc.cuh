@@ -446,9 +446,13 @@ static int launch_flash_tc(const void* q, long long q_row_stride, const void* ca
                            const void* gate = nullptr, long long gate_stride = 0, int keep = 0,
                            const ScoreForm& form = ScoreForm()) {
     const int n_rep = nh / nkv;
-    // tiles of all sequences together: at most those of n tokens in one piece and a ragged one a sequence
-    const long long longest = ((long long)max_q * n_rep + FT_ROWS - 1) / FT_ROWS, whole = (long long)n * n_rep / FT_ROWS + num_seqs;
-    const long long tiles = longest * num_seqs < whole ? longest * num_seqs : whole;
+    // tiles of all sequences together: at most those of n tokens in one piece and a ragged one a sequence of at least min_q tokens, of which
+    // there are no more than n / min_q.  (With one for every sequence, 255 decode tokens beside a portion of 70 were 2,120 blocks for 24
+    // tiles, each of which read the whole list before it ended: 24 / 8 heads 101 us, so REPLACE_ME)
+    const long long longest = ((long long)max_q * n_rep + FT_ROWS - 1) / FT_ROWS, most = n / min_q < num_seqs ? n / min_q : num_seqs;
+    const long long whole = (long long)n * n_rep / FT_ROWS + most;
+    const long long tiles = longest * most < whole ? longest * most : whole;
+    if (tiles == 0) return 0;                            // (fewer tokens than min_q: no sequence is this kernel's)
     if (tiles * nkv > 0x7fffffffLL || nkv > 65535 || num_seqs > 65535)
         return fail(-1, "paged_attention: the step exceeds the grid (%lld row tiles, %d kv heads, %d sequences)", tiles, nkv, num_seqs);
     if (!(scale > 0.f)) return fail(-1, "paged_attention: the tcgen05 kernel needs a positive scale");
