@@ -124,3 +124,28 @@ def test_linear_takes_every_bias_that_the_library_takes(M, N, K):
     for wrong in (N - 1, N + 1, 2):
         with pytest.raises(RuntimeError):
             ops.linear(x, w, torch.zeros(wrong, device="cuda"))
+
+
+@pytest.mark.gpu
+def test_large_float32_products_can_be_differentiated_and_mapped():
+    """33 rows against a weight of 2^20 numbers: gradients, forward mode and vmap see the product as they see the library's."""
+    ops.strict_fp32()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, w, b = (torch.randn(*s, generator=g, device="cuda") for s in ((33, 1024), (1024, 1024), (1024,)))
+    assert ops.linear_f32_pays(33, 1024, 1024)
+    tol = dict(atol=1e-3, rtol=1e-4)
+    xs, ws, bs = (t.clone().requires_grad_() for t in (x, w, b))
+    ops.linear(xs, ws, bs).square().sum().backward()
+    up = 2 * (x.double() @ w.double().t() + b.double())
+    torch.testing.assert_close(xs.grad.double(), up @ w.double(), atol=0.1, rtol=1e-4)
+    torch.testing.assert_close(ws.grad.double(), up.t() @ x.double(), atol=0.1, rtol=1e-4)
+    torch.testing.assert_close(bs.grad.double(), up.sum(0), atol=0.1, rtol=1e-4)
+    with torch.no_grad():
+        assert not ops.linear(xs, ws, bs).requires_grad
+    value, tangent = torch.func.jvp(lambda t: ops.linear(t, w, b), (x,), (x,))
+    torch.testing.assert_close(tangent.double(), x.double() @ w.double().t(), **tol)
+    torch.testing.assert_close(torch.vmap(lambda t: ops.linear(t, w))(x.view(1, 33, 1024).repeat(3, 1, 1)).double(),
+                               (x.double() @ w.double().t()).repeat(3, 1, 1), **tol)
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(x, x)
+        assert torch.autograd.forward_ad.unpack_dual(ops.linear(dual, w)).tangent is not None

@@ -17,6 +17,7 @@ import threading
 from typing import Dict, Optional, Tuple
 
 import torch
+from torch.autograd import forward_ad
 
 from ..csrc import build as _build
 
@@ -768,6 +769,14 @@ def _bias_vector(bias: torch.Tensor, n: int) -> Optional[torch.Tensor]:
     return bias.reshape(-1).to(torch.float32).expand(n).contiguous()
 
 
+def _followed(*ts: Optional[torch.Tensor]) -> bool:
+    """Whether autograd, forward mode or a transform of torch.func looks at what is done with these tensors (a kernel called by address
+    leaves no trace of itself)."""
+    ts = tuple(t for t in ts if t is not None)
+    return (forward_ad._current_level >= 0 or (torch.is_grad_enabled() and any(t.requires_grad for t in ts))
+            or any(torch._C._functorch.is_functorch_wrapped_tensor(t) for t in ts))
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """``x @ weight.T (+ bias)``: decode-sized products (at most 16 rows, bfloat16 up to TC_MAX_ROWS) and large float32 ones on
@@ -796,7 +805,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if (x.dtype == torch.float32 and out_dtype in (None, torch.float32) and skinny_f32_applies(x.shape[0], weight)
             and x.is_contiguous() and x.data_ptr() % 16 == 0):
         return skinny_linear_f32(weight, x, vector)
-    if out_dtype in (None, torch.float32) and linear_f32_applies(x, weight):
+    if out_dtype in (None, torch.float32) and x.dtype == torch.float32 and not _followed(x, weight, bias) and linear_f32_applies(x, weight):
         return linear_f32(x, weight, vector)
     return _library_linear(x, weight, bias, out_dtype)
 
