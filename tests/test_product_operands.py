@@ -1,4 +1,6 @@
 """What the products' wrappers accept beside a weight: the bias' shape and type, the step's status word, autograd."""
+import math
+
 import pytest
 import torch
 
@@ -103,6 +105,26 @@ def test_a_step_hands_its_status_word_to_every_product_with_a_bounded_wait(monke
                                            (1024, 16384, 2048, True), (1000, 2052, 512, True), (500, 2200, 512, True), (499, 2200, 512, False)])
 def test_the_split_product_takes_what_it_is_faster_at(rows, n, k, pays):
     assert ops.linear_f32_pays(rows, n, k) == pays
+
+
+def test_the_stream_form_of_prompt_steps_ends_where_it_was_not_measured_to_pay(monkeypatch):
+    """More rows than a decode step only with a prompt portion, in models of the measured sizes (LFM2's, of which the average layer is
+    counted), and not where the product it rests on is switched off."""
+    from conftest import serving_width_config
+    from vapi_b200.config.model import resolve_architecture
+    for size in ("700m", "1.2b"):
+        cfg = serving_width_config(size)
+        arch = resolve_architecture(cfg)
+        plan = arch.plan(arch.parse(cfg))
+        layer = sum(math.prod(s.shape) for b in plan.layers for s in b.tensor_specs("") if s.role == "matrix") // len(plan.layers)
+        assert 30_000_000 < layer < 70_000_000 and ops.stream_max_rows(57, layer) == ops.STREAM_PROMPT_MAX_ROWS == 128
+    assert ops.stream_max_rows(1, layer) == ops.TC_MAX_ROWS and ops.stream_max_rows(57, 4 * layer) == ops.TC_MAX_ROWS
+    monkeypatch.setattr(ops, "TC_MAX_ROWS", 16)
+    assert ops.stream_max_rows(57, layer) == 16
+    monkeypatch.setattr(ops, "TC_MAX_ROWS", 200)
+    assert ops.stream_max_rows(1, layer) == ops.stream_max_rows(57, layer) == 200
+    monkeypatch.setattr(ops, "use_tc", False)
+    assert ops.stream_max_rows(1, layer) == ops.stream_max_rows(57, layer) == 16
 
 
 # rows on both sides of 16 (the weight-streaming kernel, the split product) and a weight on both sides of the split product's least size

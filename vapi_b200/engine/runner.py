@@ -12,6 +12,7 @@ It corresponds to the reference's ``ExecutionBackend::forward`` over
 """
 from __future__ import annotations
 
+import math
 import os
 from typing import Any, Dict, List, Optional, Sequence
 
@@ -100,6 +101,8 @@ class ModelRunner:
         #: whether every block has the stream form that steps of few rows run (blocks without it hand
         #: their output on in another shape than a plain delta, so such a model takes the ordinary path)
         self._stream_form = all(hasattr(b, "forward_stream") for b in plan.layers) and not plan.stream_parts
+        #: numbers in the matrices of a layer, on average
+        self._layer_numbers = sum(math.prod(s.shape) for b in plan.layers for s in b.tensor_specs("") if s.role == "matrix") // max(1, len(plan.layers))
         self._keep_embedding = any(getattr(p, "needs_embedding_output", False) for p in plan.stream_parts.values())
         self.steps_run = 0
         self.graph_max_batch = min(64, max_requests)
@@ -194,9 +197,7 @@ class ModelRunner:
             ctx.pos[pe.name] = pe.prepare(ctx)
         views = self.views(ctx)
         ctx.fused = (self._stream_form and self.device.type == "cuda" and self.dtype == torch.bfloat16 and ops.use_skinny
-                     and (ctx.n <= (ops.SKINNY_MAX_ROWS if not ops.use_tc else ops.TC_MAX_ROWS if ctx.max_q <= 1
-                                    else max(ops.TC_MAX_ROWS, ops.STREAM_PROMPT_MAX_ROWS))
-                          or 0 < ops.PROMPT_MIN_ROWS <= ctx.n))
+                     and (ctx.n <= ops.stream_max_rows(ctx.max_q, self._layer_numbers) or 0 < ops.PROMPT_MIN_ROWS <= ctx.n))
         if ctx.fused:
             return self._forward_few_rows(ctx, views)
         x = self._embed(ctx)

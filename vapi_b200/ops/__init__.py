@@ -436,13 +436,19 @@ def skinny_linear(weight: torch.Tensor, *, act: Optional[torch.Tensor] = None,
 #: beats the library's product plus separate norm / SwiGLU / add kernels at 32 rows (1.26 vs 1.33
 #: ms), loses narrowly at 64 (1.71 vs 1.68 ms) and clearly beyond (2-7x slower at 256 rows).
 TC_MAX_ROWS = int(os.environ.get("VAPI_TC_MAX_ROWS", "32"))
-#: steps with a prompt portion run the stream form of their blocks (norms, SwiGLU and residual adds inside the products)
-#: up to this many rows.  They are launched one by one, and what bounds them is the launches, of which this form has 81 where
-#: the other has 145 (57 tokens of LFM2-700M: 2.03 -> 1.77 ms, while the kernels themselves take 1.0 instead of 0.82 ms).
-#: From 129 rows on a product's tokens no longer fit beside a share of K (200 tokens of LFM2-700M: 1.98 -> 4.37 ms), and
-#: captured decode steps, which cost no launches, stay with TC_MAX_ROWS (LFM2-2.6B, 64 requests: 1.93 ms a step on the
-#: library, 2.08 ms in this form).
+#: steps with a prompt portion run the stream form of their blocks (norms, SwiGLU and residual adds inside the products; LFM2's blocks have
+#: one) up to this many rows.  They are launched one by one, and what bounds them is the launches, of which this form has 81 where the other
+#: has 145 at 16 layers.  Steps one after the other, without a wait between them / the device's share, ms in this form against the other:
+#: 33 tokens of the 700M, 1.2B and 2.6B sizes 1.70 / 0.88, 1.71 / 1.03, 2.90 / 1.81 against 1.94 / 0.94, 1.96 / 1.05, 3.37 / 1.84; 64 1.67 / 0.99,
+#: 1.69 / 1.15, 2.90 / 2.02 against 1.94 / 0.96, 1.95 / 1.09, 3.38 / 1.86; 128 1.68 / 1.43, 1.69 / 1.61, 2.92 / 2.91 against 1.93 / 1.03, 1.95 / 1.14,
+#: 3.40 / 2.00; 60 decoding requests beside a portion of 60 1.92 / 1.61, 1.94 / 1.83, 3.20 / 3.15 against 2.16 / 1.21, 2.14 / 1.38, 3.62 / 2.28.  So
+#: it pays as far as the host is what a step waits for, and from about 50 rows on only that far: with weights much wider than these the
+#: device's share is what counts, and the other form is ahead.  From 129 rows on a product's tokens no longer fit beside a share of K (200
+#: tokens of the 700M size: 1.98 -> 4.37 ms), and captured decode steps, which cost no launches, stay with TC_MAX_ROWS (2.6B, 64
+#: requests: 1.93 ms a step on the library, 2.08 ms in this form).
 STREAM_PROMPT_MAX_ROWS = 128
+#: and this many numbers in a layer's matrices (40, 65 and 59 million in the sizes above)
+STREAM_PROMPT_MAX_LAYER = 80_000_000
 #: set False to keep products of 17..TC_MAX_ROWS rows on the library
 use_tc = os.environ.get("VAPI_TC", "1") != "0"
 
@@ -495,6 +501,15 @@ def skinny_shortconv(w_in: torch.Tensor, *, xw: torch.Tensor, ss_in: torch.Tenso
         L, _p(state_layer if L > 1 else None), ctypes.c_longlong(slot_stride), num_slots, _p(state_slots),
         _p(positions), _p(out), _p(status), _stream()))
     return out
+
+
+def stream_max_rows(max_q: int, layer: int) -> int:
+    """The most rows of a step that runs the stream form of its blocks: a decode step (``max_q`` 1), or one with a prompt portion, of a
+    model with ``layer`` numbers in the matrices of a layer."""
+    if not use_tc:
+        return SKINNY_MAX_ROWS
+    decode_only = max_q <= 1 or layer > STREAM_PROMPT_MAX_LAYER or TC_MAX_ROWS <= SKINNY_MAX_ROWS
+    return TC_MAX_ROWS if decode_only else max(TC_MAX_ROWS, STREAM_PROMPT_MAX_ROWS)
 
 
 def tc_applies(rows: int, weight: torch.Tensor, most: Optional[int] = None) -> bool:
