@@ -44,22 +44,6 @@ def _random_case(seed, n, klen, nh, nkv):
     return q, cache, (torch.arange(pages, device="cuda").int()[None], i32([0, n]), i32([klen]), n, 1, n, klen, nh, nkv, 64, 0.125)
 
 
-@pytest.mark.parametrize("lens,general", [([(36, 36), (5, 20)], True), ([(37, 37), (5, 20)], False), ([(9, 36)], True), ([(9, 37)], False),
-                                          ([(1, 30), (1, 5)], False)])
-def test_short_float_portions_stay_on_the_general_kernel(ops, monkeypatch, lens, general):
-    """Where no sequence is longer than 36 tokens, but for decode tokens, which have a kernel of their own."""
-    seen, real = [], ops._lib("attention")
-
-    class Watched:
-        def __getattr__(self, name):
-            f = getattr(real, name)
-            return (lambda *args: (seen.append(args[-3]), f(*args))[1]) if name == "vapi_paged_attention" else f
-
-    monkeypatch.setattr(ops, "_lib", lambda name: Watched())
-    _attention_case(ops, torch.float32, 8, 2, 64, 64, lens)
-    assert seen == [1 if general else 0]
-
-
 def test_float_attention_is_no_further_from_the_exact_one(ops):
     q, cache, args = _random_case(1, 200, 700, 4, 2)
     got, general = (ops.paged_attention(q, 256, cache, *args, splits=1, impl=impl).double() for impl in ("auto", "general"))

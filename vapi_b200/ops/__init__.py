@@ -971,12 +971,6 @@ def attention_splits(num_seqs: int, max_q: int, max_k: int, nh: int, nkv: int, d
     return max(1, min(want, by_len, 32))
 
 
-#: float32 portions of sequences no longer than this stay on the general attention kernel: one tile of 64 keys is mostly empty, and
-#: splitting it for the tensor cores takes longer than its float FMAs (us against the general kernel's, 32 / 8 heads: 17 tokens 11.4 and
-#: 7.6, 33 11.5 and 9.3, 40 11.4 and 12.0; 16 portions of 33 23.3 and 21.9, of 40 23.4 and 27.0)
-SHORT_PROMPT_F32 = 36
-
-
 def paged_attention(q: torch.Tensor, q_row_stride: int, cache_layer: torch.Tensor,
                     block_table: torch.Tensor, cu_q: torch.Tensor, seqlens_k: torch.Tensor,
                     n: int, num_seqs: int, max_q: int, max_k: int, nh: int, nkv: int, d: int,
@@ -1027,8 +1021,6 @@ def paged_attention(q: torch.Tensor, q_row_stride: int, cache_layer: torch.Tenso
             and decode_attention_applies(q.dtype, d, page_size, nh // nkv)):
         launches += 1                     # short portions on the flash kernel, decode tokens on the decode kernel
     code = {"auto": 0, "general": 1, "tensor_core": 2, "tcgen05": 3, "decode": 4}[impl]
-    if code == 0 and q.dtype == torch.float32 and max_q > 1 and max_k <= SHORT_PROMPT_F32:
-        code = 1
     _check(lib, lib.vapi_paged_attention(
         _p(q), ctypes.c_longlong(q_row_stride), _p(cache_layer), _dt(q), _p(block_table),
         block_table.stride(0), _p(cu_q), _p(seqlens_k), _p(out), _p(part_o), _p(part_ml), n, num_seqs,
