@@ -14,7 +14,7 @@ def ops():
 
 def _bound(a, w):
     """Elementwise: a piece of 64 k is 6 x 4 tensor-core additions of 16 products, each of which may drop what lies below the
-    last of 24 bits (2^-23 of the sum so far), the pieces are K / 64 float additions, the split leaves out 2^-25, and
+    last of 24 bits (2^-23 of the sum so far), the pieces are K / 64 float additions, the split leaves out 2^-24, and
     the bias is one more rounding; all against the sum of the magnitudes."""
     K = a.shape[1]
     return (2 * 24 + -(-K // 64) + 8 + 2) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t()) + 1e-30

@@ -4,10 +4,13 @@
 // float FMAs fed from shared memory.
 //
 // Both products run on the tensor cores without giving up float: a float is the exact sum of three bfloat16 (24 bits), and of
-// the nine products the six of weight 2^-16 and above are taken (the rest is below 2^-25 of the term; see linear_f32.cu).
+// the nine products the six of weight 2^-16 and above are taken (the rest is at most 2^-24 of the term; see linear_f32.cu).
 // The leading products and the five small ones have accumulators of their own, and a tile's P.V is added to the output by
-// float FMAs: a tensor core cuts off what it adds to an accumulator, so chains are kept to four instructions.  Maximum,
-// exponentials and sums are float as before.
+// float FMAs: a tensor core cuts off what it adds to an accumulator, so the leading products' chains are kept to four instructions (the
+// small ones, of 2^-8 and less, come to twenty).  Maximum, exponentials and sums are float as before.
+//
+// Portions of sequences of up to 36 tokens would be a little faster on the general kernel (17 tokens, 32 / 8 heads: 7.6 us against 11.4), but its
+// results are further from exact (1.3e-7 against 7.6e-8 of their 2-norm), so they stay here.
 //
 // A block of four warps owns 64 rows and walks the 64-key tiles any of them can see: the tile's floats come by asynchronous copies
 // while the tile before is multiplied, all threads split them into planes (128-byte rows, 16-byte pieces swizzled), a warp
@@ -26,30 +29,16 @@ constexpr size_t FF_SMEM = 9 * FF_PLANE + 2 * FF_BK * FF_HD * 4 + 128;     // pl
 // sum (one that overflows takes the others with it: plus infinity of x1 y1 and minus infinity of x1 y2 are NaN, a float product infinity).
 constexpr float FF_LIMIT_QK = 1.152921504606846976e18f, FF_LIMIT_V = 1.329227995784915873e36f;
 
-__device__ __forceinline__ void ff_split2(float a, float b, unsigned& p1, unsigned& p2, unsigned& p3) {
-    p1 = pack_bf16(a, b);
-    a -= __uint_as_float(p1 << 16);
-    b -= __uint_as_float(p1 & 0xffff0000u);
-    p2 = pack_bf16(a, b);
-    a -= __uint_as_float(p2 << 16);
-    b -= __uint_as_float(p2 & 0xffff0000u);
-    p3 = pack_bf16(a, b);
-}
-__device__ __forceinline__ float ff_absmax(float m, float x) {
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(m), "f"(fabsf(x)));
-    return r;
-}
 // four floats of a row (piece c4 of 16 bytes of float) into the three planes; the largest magnitude so far
 __device__ __forceinline__ float ff_store(unsigned char* planes, int row, int c4, float4 v, float top) {
     uint2 p1, p2, p3;
-    ff_split2(v.x, v.y, p1.x, p2.x, p3.x);
-    ff_split2(v.z, v.w, p1.y, p2.y, p3.y);
+    split_f32x2(v.x, v.y, p1.x, p2.x, p3.x);
+    split_f32x2(v.z, v.w, p1.y, p2.y, p3.y);
     unsigned char* at = planes + row * 128 + ((((c4 >> 1) ^ (row & 7)) << 4) | ((c4 & 1) << 3));
     *reinterpret_cast<uint2*>(at) = p1;
     *reinterpret_cast<uint2*>(at + FF_PLANE) = p2;
     *reinterpret_cast<uint2*>(at + 2 * FF_PLANE) = p3;
-    return ff_absmax(ff_absmax(ff_absmax(ff_absmax(top, v.x), v.y), v.z), v.w);
+    return absmax_nan(absmax_nan(absmax_nan(absmax_nan(top, v.x), v.y), v.z), v.w);
 }
 __device__ __forceinline__ const unsigned char* ff_at(const unsigned char* plane, int row, int piece) {
     return plane + row * 128 + ((piece ^ (row & 7)) << 4);
@@ -225,10 +214,10 @@ flash_f32_kernel(const float* q, long long q_row_stride, const float* cache, con
 #pragma unroll
             for (int k = 0; k < FF_BK / 16; ++k) {
                 unsigned a[3][4], b[3][4];
-                ff_split2(sc[2 * k][0], sc[2 * k][1], a[0][0], a[1][0], a[2][0]);
-                ff_split2(sc[2 * k][2], sc[2 * k][3], a[0][1], a[1][1], a[2][1]);
-                ff_split2(sc[2 * k + 1][0], sc[2 * k + 1][1], a[0][2], a[1][2], a[2][2]);
-                ff_split2(sc[2 * k + 1][2], sc[2 * k + 1][3], a[0][3], a[1][3], a[2][3]);
+                split_f32x2(sc[2 * k][0], sc[2 * k][1], a[0][0], a[1][0], a[2][0]);
+                split_f32x2(sc[2 * k][2], sc[2 * k][3], a[0][1], a[1][1], a[2][1]);
+                split_f32x2(sc[2 * k + 1][0], sc[2 * k + 1][1], a[0][2], a[1][2], a[2][2]);
+                split_f32x2(sc[2 * k + 1][2], sc[2 * k + 1][3], a[0][3], a[1][3], a[2][3]);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
 #pragma unroll

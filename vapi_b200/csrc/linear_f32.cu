@@ -1,18 +1,20 @@
 // Matrix product of the true 32-bit path for more rows than a decode step has:
-//   y[m][n] = sum_k a[m][k] * W[n][k] (+ bias[n]),  float in, float out, no loss against float FMAs,
+//   y[m][n] = sum_k a[m][k] * W[n][k] (+ bias[n]),  float in, float out, dense sums no further from exact than by float FMAs,
 // on the fifth-generation tensor cores.
 //
-// How a float product gets onto bfloat16 tensor cores.  A float has 24 significant bits, a bfloat16 eight, so
+// How a float product gets onto bfloat16 tensor cores (the split of Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence
+// datatype for higher-precision computations", 2019).  A float has 24 significant bits, a bfloat16 eight, so
 // x = x1 + x2 + x3 exactly with x1 = bf16(x), x2 = bf16(x - x1), x3 = x - x1 - x2 (the differences are exact, and the last
 // one has at most seven bits left).  Products of two bfloat16 are exact in float.  Of the nine partial products
-// the six of weight 2^-16 and above are computed (1.1, 1.2, 2.1, 2.2, 1.3, 3.1); the three that are left out are below
-// 2^-25 of |x||y| together, less than what one float FMA rounds away.  The tensor core adds up 64 k at a time, the
-// smallest products first, and every such piece is then added to a float accumulator in registers, rounded to
-// nearest: a sum over K is K / 64 float additions long instead of K.  Against float64 the result is closer than that of the
+// the six of weight 2^-16 and above are computed (1.1, 1.2, 2.1, 2.2, 1.3, 3.1); the three that are left out come to at most
+// 2^-24 of |x||y| together, as much as a float rounding.  The tensor core adds up 64 k at a time, the
+// smallest products first, and cuts off what does not fit; every such piece is then added to a float accumulator in registers, rounded to
+// nearest: a sum over K is K / 64 float additions long instead of K.  For a sum of one term, or a few, that is more than a float FMA
+// loses (which rounds once); for dense ones it is less, and against float64 the result is closer than that of the
 // library's FMA product, which this replaces: 1.3e-7 against 8.1e-7 of its 2-norm at K = 2,048, 2.2e-7 against 1.6e-6 at
-// K = 8,192.  Six tensor-core products in place of one still leave it far ahead: 1,024 tokens x 16,384 x 2,048 in 339 us against
-// 1,225 us (203 TFLOP/s, 1,220 on the tensor cores), 1,024 x 2,048 x 8,192 in 197 against 616 us, 57 x 2,048 x 1,536 in 26
-// against 45 us (events, L2 flushed).
+// K = 8,192.  Six tensor-core products in place of one still leave it far ahead: 1,024 tokens x 16,384 x 2,048 in 336 us against
+// 1,225 us (204 TFLOP/s, 1,227 on the tensor cores), 1,024 x 2,048 x 8,192 in 182 against 616 us, 64 x 2,048 x 2,048 in 28
+// against 51 us (in a captured chain of products).
 // Elements below 2^-109 in magnitude lose what lies below 2^-134.  A row with an element of 2^127 or more, an
 // infinity or a NaN cannot be split, and where a product overflows the partial ones do so in different directions (x1 y1 to infinity, x1 y2 to
 // minus infinity); such results are computed by plain FMAs, so they are what they always were.
@@ -38,8 +40,6 @@
 // (with a limit) for the copies and products that are under way, and leaves its tile unwritten, as do the blocks that share it.  The
 // cluster barriers are reached by every thread on every path.
 #include "tcgen05.cuh"
-
-#include <unordered_map>
 
 using namespace vapi;
 
@@ -68,17 +68,6 @@ struct LfParams {
     long long out_stride;
 };
 
-__device__ __forceinline__ bool lf_wait(unsigned bar, unsigned parity, volatile int* abort_flag, unsigned polls) {
-    for (unsigned i = 0; i < polls; ++i) {
-        unsigned done;
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}"
-                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-        if (done) return true;
-        if ((i & 0xFFF) == 0xFFF && *abort_flag) break;
-    }
-    *abort_flag = 1;
-    return false;
-}
 // the same MMA as umma_f16 with A (two bfloat16 a column, a row a lane) in tensor memory
 __device__ __forceinline__ void lf_umma_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long db, unsigned idesc, unsigned accumulate) {
     asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
@@ -89,25 +78,6 @@ __device__ __forceinline__ void lf_tmem_st16(unsigned taddr, const unsigned (&v)
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
                  ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
                    "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
-}
-// the larger magnitude; a NaN stays one
-__device__ __forceinline__ float lf_absmax(float m, float x) {
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(m), "f"(fabsf(x)));
-    return r;
-}
-// two floats as three pairs of bfloat16 that add up to them
-__device__ __forceinline__ void lf_split2(float a, float b, unsigned& p1, unsigned& p2, unsigned& p3) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    p1 = *reinterpret_cast<unsigned*>(&v);
-    a -= __uint_as_float(p1 << 16);
-    b -= __uint_as_float(p1 & 0xffff0000u);
-    v = __floats2bfloat162_rn(a, b);
-    p2 = *reinterpret_cast<unsigned*>(&v);
-    a -= __uint_as_float(p2 << 16);
-    b -= __uint_as_float(p2 & 0xffff0000u);
-    v = __floats2bfloat162_rn(a, b);
-    p3 = *reinterpret_cast<unsigned*>(&v);
 }
 __device__ __forceinline__ unsigned lf_map_rank(unsigned addr, unsigned rank) {
     unsigned r;
@@ -129,10 +99,10 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* x, __nv_bf
     float top = 0.f;
     for (int k = threadIdx.x * 4; k < Kp; k += blockDim.x * 4) {
         const float4 v = k < K ? *reinterpret_cast<const float4*>(x + (size_t)m * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-        top = lf_absmax(lf_absmax(lf_absmax(lf_absmax(top, v.x), v.y), v.z), v.w);
+        top = absmax_nan(absmax_nan(absmax_nan(absmax_nan(top, v.x), v.y), v.z), v.w);
         uint2 p1, p2, p3;
-        lf_split2(v.x, v.y, p1.x, p2.x, p3.x);
-        lf_split2(v.z, v.w, p1.y, p2.y, p3.y);
+        split_f32x2(v.x, v.y, p1.x, p2.x, p3.x);
+        split_f32x2(v.z, v.w, p1.y, p2.y, p3.y);
         *reinterpret_cast<uint2*>(row + k) = p1;
         *reinterpret_cast<uint2*>(row + plane + k) = p2;
         *reinterpret_cast<uint2*>(row + 2 * plane + k) = p3;
@@ -210,8 +180,8 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
             float top = 0.f;
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
                 const int s = it % LF_STAGES, ws = it % LF_W_STAGES;
-                if (!lf_wait(wfull0 + 8 * ws, (it / LF_W_STAGES) & 1, abort_flag, polls)) ok = false;
-                if (!lf_wait(empty0 + 8 * s, ((it / LF_STAGES) & 1) ^ 1, abort_flag, polls)) ok = false;
+                if (!mbar_wait_role(wfull0 + 8 * ws, (it / LF_W_STAGES) & 1, abort_flag, polls)) ok = false;
+                if (!mbar_wait_role(empty0 + 8 * s, ((it / LF_STAGES) & 1) ^ 1, abort_flag, polls)) ok = false;
                 if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
                 tc5_fence_after();
                 const unsigned char* w = base + (size_t)ws * LF_W_BYTES + row * 128;
@@ -221,9 +191,9 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
                         const float4 v = *reinterpret_cast<const float4*>(w + h * (LF_W_BYTES / 2) + ((c ^ (row & 7)) << 4));
-                        top = lf_absmax(lf_absmax(lf_absmax(lf_absmax(top, v.x), v.y), v.z), v.w);
-                        lf_split2(v.x, v.y, p1[2 * c], p2[2 * c], p3[2 * c]);
-                        lf_split2(v.z, v.w, p1[2 * c + 1], p2[2 * c + 1], p3[2 * c + 1]);
+                        top = absmax_nan(absmax_nan(absmax_nan(absmax_nan(top, v.x), v.y), v.z), v.w);
+                        split_f32x2(v.x, v.y, p1[2 * c], p2[2 * c], p3[2 * c]);
+                        split_f32x2(v.z, v.w, p1[2 * c + 1], p2[2 * c + 1], p3[2 * c + 1]);
                     }
                     const unsigned a = a0 + (unsigned)(s * 3 * LF_A_COLS + h * 16);
                     lf_tmem_st16(a, p1);
@@ -245,7 +215,7 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                 const int n0 = (t / p.num_m) * LF_BM;
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int ws = it % LF_W_STAGES;
-                    if (!lf_wait(wempty0 + 8 * ws, ((it / LF_W_STAGES) & 1) ^ 1, abort_flag, polls)) { ok = false; break; }
+                    if (!mbar_wait_role(wempty0 + 8 * ws, ((it / LF_W_STAGES) & 1) ^ 1, abort_flag, polls)) { ok = false; break; }
                     const unsigned w = smem_u32(base + (size_t)ws * LF_W_BYTES);
                     mbar_expect_tx(wfull0 + 8 * ws, LF_W_BYTES);
                     tma_load_2d(w, &tm_w, wfull0 + 8 * ws, kb * LF_BK, n0);
@@ -262,7 +232,7 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                 const int m0 = (t % p.num_m) * NT;
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % LF_STAGES;
-                    if (!lf_wait(empty0 + 8 * s, ((it / LF_STAGES) & 1) ^ 1, abort_flag, polls)) { ok = false; break; }
+                    if (!mbar_wait_role(empty0 + 8 * s, ((it / LF_STAGES) & 1) ^ 1, abort_flag, polls)) { ok = false; break; }
                     const unsigned b = smem_u32(tok_mem + (size_t)s * Cfg::STAGE_BYTES);
                     mbar_expect_tx(full0 + 8 * s, 3 * Cfg::B_PLANE);
 #pragma unroll
@@ -279,8 +249,8 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
             for (int t = first; t < p.num_tiles && ok; t += step) {
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % LF_STAGES, buf = it & 1;
-                    if (!lf_wait(accempty0 + 8 * buf, ((it >> 1) & 1) ^ 1, abort_flag, polls) ||
-                        !lf_wait(full0 + 8 * s, (it / LF_STAGES) & 1, abort_flag, polls)) { ok = false; break; }
+                    if (!mbar_wait_role(accempty0 + 8 * buf, ((it >> 1) & 1) ^ 1, abort_flag, polls) ||
+                        !mbar_wait_role(full0 + 8 * s, (it / LF_STAGES) & 1, abort_flag, polls)) { ok = false; break; }
                     tc5_fence_after();
                     const unsigned a = tmem_base + LF_A_COL0 + (unsigned)(s * 3 * LF_A_COLS), b = smem_u32(tok_mem + (size_t)s * Cfg::STAGE_BYTES);
                     const unsigned d = tmem_base + (unsigned)(buf * NT);
@@ -308,7 +278,7 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         for (int t = first; t < p.num_tiles && ok; t += step, ++tl) {
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
                 const int buf = it & 1;
-                if (!lf_wait(accfull0 + 8 * buf, (it >> 1) & 1, abort_flag, polls)) ok = false;
+                if (!mbar_wait_role(accfull0 + 8 * buf, (it >> 1) & 1, abort_flag, polls)) ok = false;
                 if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
                 tc5_fence_after();
 #pragma unroll

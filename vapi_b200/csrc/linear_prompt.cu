@@ -117,18 +117,6 @@ __device__ __forceinline__ void pl_tmem_ld32(unsigned taddr, unsigned (&r)[32]) 
                    "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
                  : "r"(taddr));
 }
-// bounded wait that also ends when another role of the block has given up
-__device__ __forceinline__ bool pl_wait(unsigned bar, unsigned parity, volatile int* abort_flag) {
-    for (unsigned i = 0; i < TC5_WAIT_LIMIT; ++i) {
-        unsigned done;
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}"
-                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-        if (done) return true;
-        if ((i & 0xFFF) == 0xFFF && *abort_flag) break;
-    }
-    *abort_flag = 1;
-    return false;
-}
 // barrier of the four epilogue warps that also tells whether every thread brought `ok`
 __device__ __forceinline__ bool pl_epi_all(bool ok) {
     unsigned r;
@@ -198,7 +186,7 @@ prompt_linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                 const int m0 = (m_blk * PAIR + (int)rank) * PL_BM;
                 for (int kb = 0; kb < p.num_kb; ++kb, ++it) {
                     const int s = it % STAGES;
-                    if (!pl_wait(empty0 + 8 * s, ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_role(empty0 + 8 * s, ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
                     const unsigned a = smem_u32(stage_mem + (size_t)s * Cfg::STAGE_BYTES), b = a + PL_A_BYTES;
                     if (PAIR == 2) {
                         if (leader) mbar_expect_tx(full0 + 8 * s, 2 * Cfg::STAGE_BYTES);
@@ -230,12 +218,12 @@ prompt_linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
             bool ok = true;
             for (int t = cluster_id; t < p.num_tiles && ok; t += num_clusters, ++tl) {
                 const int buf = tl & 1;
-                if (!pl_wait(accempty0 + 8 * buf, ((tl >> 1) & 1) ^ 1, abort_flag)) break;     // the epilogues have read this buffer
+                if (!mbar_wait_role(accempty0 + 8 * buf, ((tl >> 1) & 1) ^ 1, abort_flag)) break;     // the epilogues have read this buffer
                 tc5_fence_after();
                 const unsigned d = tmem_base + (unsigned)(buf * BN);
                 for (int kb = 0; kb < p.num_kb; ++kb, ++it) {
                     const int s = it % STAGES;
-                    if (!pl_wait(full0 + 8 * s, (it / STAGES) & 1, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_role(full0 + 8 * s, (it / STAGES) & 1, abort_flag)) { ok = false; break; }
                     tc5_fence_after();
                     const unsigned a = smem_u32(stage_mem + (size_t)s * Cfg::STAGE_BYTES), b = a + PL_A_BYTES;
 #pragma unroll
@@ -297,7 +285,7 @@ prompt_linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                 colv[256 + j] = (p.next_w && n < p.N) ? p.next_w[n] : 0.f;
             }
             // (the warps leave together or not at all: they meet at barriers in every tile)
-            if (!pl_epi_all(pl_wait(accfull0 + 8 * buf, (tl >> 1) & 1, abort_flag))) break;
+            if (!pl_epi_all(mbar_wait_role(accfull0 + 8 * buf, (tl >> 1) & 1, abort_flag))) break;
             tc5_fence_after();
             const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * BN);
             // 32 finished columns of bfloat16 output, from the patch, as rows of 64 bytes

@@ -29,6 +29,18 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
     }
     return false;
 }
+// the same for a role of a block, which also ends when another role has given up
+__device__ __forceinline__ bool mbar_wait_role(unsigned bar, unsigned parity, volatile int* abort_flag, unsigned polls = TC5_WAIT_LIMIT) {
+    for (unsigned i = 0; i < polls; ++i) {
+        unsigned done;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}"
+                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        if (done) return true;
+        if ((i & 0xFFF) == 0xFFF && *abort_flag) break;
+    }
+    *abort_flag = 1;
+    return false;
+}
 __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map, unsigned bar, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
@@ -99,6 +111,27 @@ __device__ __forceinline__ unsigned long long umma_desc_mn(unsigned smem_addr) {
     d |= (unsigned long long)1 << 46;
     d |= (unsigned long long)2 << 61;
     return d;
+}
+
+// Two floats as three pairs of bfloat16 that add up to them, high plane first (a in the low half of a pair).  A float has 24 significant bits, a
+// bfloat16 eight: the differences are exact, and the last one has at most seven bits left.
+__device__ __forceinline__ void split_f32x2(float a, float b, unsigned& p1, unsigned& p2, unsigned& p3) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    p1 = *reinterpret_cast<unsigned*>(&v);
+    a -= __uint_as_float(p1 << 16);
+    b -= __uint_as_float(p1 & 0xffff0000u);
+    v = __floats2bfloat162_rn(a, b);
+    p2 = *reinterpret_cast<unsigned*>(&v);
+    a -= __uint_as_float(p2 << 16);
+    b -= __uint_as_float(p2 & 0xffff0000u);
+    v = __floats2bfloat162_rn(a, b);
+    p3 = *reinterpret_cast<unsigned*>(&v);
+}
+// the larger magnitude; a NaN stays one
+__device__ __forceinline__ float absmax_nan(float m, float x) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(m), "f"(fabsf(x)));
+    return r;
 }
 
 // ---- host side -------------------------------------------------------------------------------

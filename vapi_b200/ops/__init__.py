@@ -941,8 +941,8 @@ def attention_splits(num_seqs: int, max_q: int, max_k: int, nh: int, nkv: int, d
     (sequence, kv head) pairs are fewer than two blocks per SM, slices up to that many blocks, and
     no more than the kernel combines itself unless a slice would then be longer than 32 tiles and
     there would be fewer blocks than SMs.
-    Half of the device's places and more are filled by the pairs alone: whole sequences up to all of them, then about four rounds of blocks,
-    so that the last ones do not run alone.  ``max_k`` bounds the lengths but does not tell them (a captured step is given the
+    A step whose pairs alone fill half of the device's places, up to all of them, is left whole; one with more is cut for about four rounds
+    of blocks, so that the last ones do not run alone.  ``max_k`` bounds the lengths but does not tell them (a captured step is given the
     configured context), so only what loses at no length is cut less: a step of more pairs than the device holds stays whole where
     no sequence can be longer than 20 tiles and is cut in two up to 36.  8 kv heads, 444 places, us in 1 / 2 / 4 slices: 64 sequences of 20 to 300
     keys 11.4 / 17.1 / 23.2, of 1,216 43.3 / 45.2 / 47.6, of 1,600 53.3 / 53.8 / 54.2 (56: 49.5 / 48.3 / 48.4), of 2,300
