@@ -127,7 +127,7 @@ def test_a_float32_product_that_gives_up_a_wait_writes_nothing_and_says_so(ops, 
 
 
 # both sides of every line of the dispatch: shared K or whole rows at 3,072, 6,144 and 8,192 rows and a K of 1,024, 1,536 and 2,048; whole rows
-# with and without the staged tokens (K of 128 and 256; more than eight tokens in rounds of blocks that are filled and that are not)
+# with and without the staged tokens (K of 128; up to eight tokens, and above twelve where rounds of blocks are not filled)
 @pytest.mark.parametrize("N,K", [(3071, 1024), (3073, 1024), (3072, 1028), (8191, 2048), (8193, 2048), (6143, 1536), (6145, 1536),
                                  (6147, 1540), (6150, 2052), (3075, 4), (4099, 128), (4099, 132), (3077, 256),
                                  (3077, 260), (12289, 512), (12287, 512), (12290, 2048), (12290, 2052), (8200, 4100)])

@@ -904,7 +904,7 @@ constexpr int F32_WARPS = 4, F32_ROWS = 4;
 // pieces of the four rows that a lane has in flight.  The sums of many tokens take the registers, and what they leave is worth
 // more as room between the tokens' loads and their use: 2,048 x 8,192, 8 tokens 18.8 us with three pieces, 17.6 with two; 16
 // tokens 43.6 with two, 37.5 with one.
-__host__ __device__ constexpr int f32_depth(int mt) { return mt <= 4 ? 4 : (mt <= 8 ? 2 : 1); }
+__host__ __device__ constexpr int f32_depth(int mt, int share) { return mt <= 4 ? 4 : (mt <= 8 || share == 1 ? 2 : 1); }
 
 __device__ __forceinline__ float4 f32_stream(const float4* p) {
     float4 v;
@@ -912,11 +912,19 @@ __device__ __forceinline__ float4 f32_stream(const float4* p) {
     return v;
 }
 
+// Eight products of one lane, two pieces.  Where a warp has whole rows a lane's sum runs over four times as many pieces as where four share
+// them: it takes two pieces at a time, so that it is no longer a chain of roundings than theirs.
+__device__ __forceinline__ float f32_pieces(const float4& w0, const float4& a0, const float4& w1, const float4& a1) {
+    const float t = fmaf(w0.w, a0.w, fmaf(w0.z, a0.z, fmaf(w0.y, a0.y, w0.x * a0.x)));
+    return fmaf(w1.w, a1.w, fmaf(w1.z, a1.z, fmaf(w1.y, a1.y, fmaf(w1.x, a1.x, t))));
+}
+
 template <int MT, int SHARE>
 __global__ void __launch_bounds__(F32_WARPS * 32, MT <= 8 ? 4 : 3)
 skinny_linear_f32_kernel(const float* __restrict__ W, const float* act /*(the kernel before this one writes it)*/,
                          const float* __restrict__ bias, float* out, int N, int K, int M, long long out_stride) {
-    constexpr int D = f32_depth(MT), C = F32_ROWS * MT, MG = MT < 8 ? MT : 8;    // (MG tokens at a time: registers)
+    constexpr int D = f32_depth(MT, SHARE), C = F32_ROWS * MT;
+    constexpr int MG = SHARE == 1 ? (MT < 4 ? MT : 4) : (MT < 8 ? MT : 8);       // (tokens at a time: registers)
     __shared__ float part[F32_WARPS][C];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int GROUPS = F32_WARPS / SHARE;                           // groups of rows in a block
@@ -940,29 +948,52 @@ skinny_linear_f32_kernel(const float* __restrict__ W, const float* act /*(the ke
 #pragma unroll
     for (int d = 0; d < D; ++d) fetch(w[d], first + d * step);          // the weights do not depend on the kernel before this one
     pdl_wait();
+    auto token = [&](int m, int c) {
+        return c < k4 ? *(reinterpret_cast<const float4*>(act + (size_t)(m < M ? m : 0) * K) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
     for (int i = 0; i < steps; i += D) {
+        if constexpr (SHARE == 1) {
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
-            const int c = first + (i + d) * step;
-            if (i + d < steps) {
+            for (int d = 0; d < D; d += 2) {
+                const int c = first + (i + d) * step;
+                if (i + d < steps) {                                    // (what lies behind K is zero)
 #pragma unroll
-                for (int g = 0; g < MT; g += MG) {
-                    float4 a[MG];
+                    for (int g = 0; g < MT; g += MG) {
+                        float4 a0[MG], a1[MG];
 #pragma unroll
-                    for (int m = 0; m < MG; ++m)
-                        a[m] = c < k4 ? *(reinterpret_cast<const float4*>(act + (size_t)(g + m < M ? g + m : 0) * K) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        for (int m = 0; m < MG; ++m) { a0[m] = token(g + m, c); a1[m] = token(g + m, c + step); }
 #pragma unroll
-                    for (int r = 0; r < F32_ROWS; ++r)
+                        for (int r = 0; r < F32_ROWS; ++r)
 #pragma unroll
-                        for (int m = 0; m < MG; ++m) {
-                            float s = acc[r * MT + g + m];
-                            s = fmaf(w[d][r].x, a[m].x, s);
-                            s = fmaf(w[d][r].y, a[m].y, s);
-                            s = fmaf(w[d][r].z, a[m].z, s);
-                            acc[r * MT + g + m] = fmaf(w[d][r].w, a[m].w, s);
-                        }
+                            for (int m = 0; m < MG; ++m) acc[r * MT + g + m] += f32_pieces(w[d][r], a0[m], w[d + 1][r], a1[m]);
+                    }
+                    fetch(w[d], c + D * step);
+                    fetch(w[d + 1], c + (D + 1) * step);
                 }
-                fetch(w[d], c + D * step);
+            }
+        } else {
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                const int c = first + (i + d) * step;
+                if (i + d < steps) {
+#pragma unroll
+                    for (int g = 0; g < MT; g += MG) {
+                        float4 a[MG];
+#pragma unroll
+                        for (int m = 0; m < MG; ++m) a[m] = token(g + m, c);
+#pragma unroll
+                        for (int r = 0; r < F32_ROWS; ++r)
+#pragma unroll
+                            for (int m = 0; m < MG; ++m) {
+                                float s = acc[r * MT + g + m];
+                                s = fmaf(w[d][r].x, a[m].x, s);
+                                s = fmaf(w[d][r].y, a[m].y, s);
+                                s = fmaf(w[d][r].z, a[m].z, s);
+                                acc[r * MT + g + m] = fmaf(w[d][r].w, a[m].w, s);
+                            }
+                    }
+                    fetch(w[d], c + D * step);
+                }
             }
         }
     }
@@ -1005,10 +1036,10 @@ skinny_linear_f32_kernel(const float* __restrict__ W, const float* act /*(the ke
     }
 }
 
-// Wide weights, up to eight tokens: eight warps a block, each with whole weight rows of its own, the tokens staged through shared
+// Wide weights, a few tokens: eight warps a block, each with whole weight rows of its own, the tokens staged through shared
 // memory a chunk of K at a time (two buffers, filled by asynchronous copies one chunk ahead), so that they are read from L2 once a
-// block and serve eight warps.  65,536 x 2,048, 8 tokens 106 us against 120 with shared K, 16,384 x 2,048 34 against 36, 8,192 x
-// 2,048 17.7 against 19.6, 3,072 x 512 3.5 against 4.0, 16,384 x 256 9.4 against 11.4; 2,048 x 2,048 10.4 against 6.6.
+// block and serve eight warps.  65,536 x 2,048, 8 tokens 103 us against 120 with shared K, 16,384 x 2,048 32 against 36, 8,192 x
+// 2,048 17 against 19.6, 3,072 x 512 3.7 against 4.0, 16,384 x 256 9.4 against 11.4; 2,048 x 2,048 10.4 against 6.6.
 constexpr int F32_STAGED_WARPS = 8;
 // rows of the weight a warp owns, and 16-byte pieces of each row that a lane asks for together
 // (fewer of both for nine to sixteen tokens, whose sums take the registers)
@@ -1061,17 +1092,12 @@ skinny_linear_f32_staged_kernel(const float* __restrict__ W, const float* __rest
         __syncthreads();                 // chunk ch of the tokens is in place for every warp
         if (ch > 0) fetch(ch * CHUNK + lane);
 #pragma unroll
-        for (int u = 0; u < DEPTH; ++u) {
+        for (int u = 0; u < DEPTH; u += 2) {
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-                const float4 a = abuf[ch & 1][m][lane + 32 * u];
+                const float4 a0 = abuf[ch & 1][m][lane + 32 * u], a1 = abuf[ch & 1][m][lane + 32 * (u + 1)];
 #pragma unroll
-                for (int r = 0; r < ROWS; ++r) {
-                    acc[r][m] = fmaf(w[u][r].x, a.x, acc[r][m]);
-                    acc[r][m] = fmaf(w[u][r].y, a.y, acc[r][m]);
-                    acc[r][m] = fmaf(w[u][r].z, a.z, acc[r][m]);
-                    acc[r][m] = fmaf(w[u][r].w, a.w, acc[r][m]);
-                }
+                for (int r = 0; r < ROWS; ++r) acc[r][m] += f32_pieces(w[u][r], a0, w[u + 1][r], a1);
             }
         }
         __syncthreads();                 // everyone is done with this buffer before it is filled again
@@ -1109,12 +1135,11 @@ VAPI_EXPORT int vapi_skinny_linear_f32(const float* W, int N, int K, int M, cons
     // 10.2 / 16.2, x 4,096 21.1 / 27.1 against 19.1 / 30.6; 8,192 x 2,048 13.0 / 19.6 against 12.6 / 17.7, x 4,096 24.1 / 36.6 against 21.7 / 34.0.
     const bool whole = N >= 8192 || (K <= 1024 && N >= 3072) || (N >= 6144 && (K <= 1536 || K > 2048));
     // Of the two forms for whole rows the unstaged one is ahead where K is a piece or two (65,536 x 128 at 1 / 8 tokens 10.9 / 14.2 against
-    // 12.2 / 29.6; 8,192 x 512 4.7 / 6.7 against 3.5 / 5.8; 16 tokens x 256 7.8 against 8.4) and, above eight tokens, where its blocks, three a
-    // multiprocessor, fill their rounds: 16 tokens 6,144 x 4,096 57 against 70 (a round, filled to 0.86), 16,384 x 2,048 69 against 74,
-    // 65,536 x 2,048 194 against 245, but 8,192 x 2,048 53 against 38 (two, to 0.58) and 16,384 x 4,096 159 against 139.
+    // 12.2 / 29.6; 8,192 x 512 4.7 / 6.7 against 3.5 / 5.8) and above eight tokens (9 / 16 tokens: 4,096 x 512 5.7 / 6.6 against 8.2 / 8.3,
+    // 6,144 x 1,536 16 / 19 against 27 / 27, 13,824 x 4,096 73 / 91 against 91 / 91, 65,536 x 1,536 126 / 128 against 187 / 187), but for more than
+    // twelve whose blocks, three a multiprocessor, do not fill their rounds (8,192 x 4,096, two rounds to 0.58, 68 / 86 against 78 / 78).
     const long long own = (N + F32_WARPS * F32_ROWS - 1) / (F32_WARPS * F32_ROWS), places = 3LL * sm_count(), rounds = (own + places - 1) / places;
-    const bool filled = 4 * own >= 3 * places * rounds && (rounds == 1 || K <= 2048);
-    const bool staged = whole && K > 128 && (M <= 8 || (K > 256 && !filled));
+    const bool staged = whole && K > 128 && (M <= 8 || (M > 12 && N >= 8192 && 4 * own < 3 * places * rounds));
     cudaError_t e;
 #define VAPI_F32(KERNEL, WARPS, ROWS)                                                                                                     \
     e = launch(KERNEL, (N + (ROWS) - 1) / (ROWS), (WARPS) * 32, 0, stream, W, act, bias, out, N, K, M, out_stride)
