@@ -171,3 +171,36 @@ def test_large_float32_products_can_be_differentiated_and_mapped():
     with torch.autograd.forward_ad.dual_level():
         dual = torch.autograd.forward_ad.make_dual(x, x)
         assert torch.autograd.forward_ad.unpack_dual(ops.linear(dual, w)).tangent is not None
+
+
+def test_traces_dispatch_modes_and_tensor_classes_see_large_float32_products(monkeypatch):
+    """What records or replaces the operations of a program finds the library's product, not the empty tensor that a kernel fills."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Own(torch.Tensor):
+        pass
+
+    class Seen(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            names.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    took = []
+    monkeypatch.setattr(ops, "_cuda", lambda *t: None)
+    monkeypatch.setattr(ops, "skinny_f32_applies", lambda *a: False)
+    monkeypatch.setattr(ops, "linear_f32_applies", lambda *a: True)
+    monkeypatch.setattr(ops, "linear_f32", lambda x, w, b=None: took.append(1) or x.new_zeros(x.shape[0], w.shape[0]))
+    x, y, w = torch.randn(33, 64), torch.randn(33, 64), torch.randn(48, 64)
+    want = torch.mm(y, w.t())
+    f = lambda t: ops.linear(t, w)
+    torch.testing.assert_close(torch.jit.trace(f, (x,), check_trace=False)(y), want)
+    torch.testing.assert_close(make_fx(f)(x)(y), want)
+    names = []
+    with Seen():
+        f(x)
+    assert any("mm" in n for n in names), names
+    assert isinstance(f(x.as_subclass(Own)), Own)
+    assert not took
+    f(x)
+    assert took

@@ -785,10 +785,12 @@ def _bias_vector(bias: torch.Tensor, n: int) -> Optional[torch.Tensor]:
 
 
 def _followed(*ts: Optional[torch.Tensor]) -> bool:
-    """Whether autograd, forward mode or a transform of torch.func looks at what is done with these tensors (a kernel called by address
-    leaves no trace of itself)."""
+    """Whether autograd, forward mode, a transform of torch.func, a trace, a dispatch mode or a tensor's own class looks at what is done
+    with these tensors (a kernel called by address leaves no trace of itself)."""
     ts = tuple(t for t in ts if t is not None)
-    return (forward_ad._current_level >= 0 or (torch.is_grad_enabled() and any(t.requires_grad for t in ts))
+    return (forward_ad._current_level >= 0 or torch._C._get_tracing_state() is not None or torch._C._len_torch_dispatch_stack() > 0
+            or any(type(t) not in (torch.Tensor, torch.nn.Parameter) for t in ts)
+            or (torch.is_grad_enabled() and any(t.requires_grad for t in ts))
             or any(torch._C._functorch.is_functorch_wrapped_tensor(t) for t in ts))
 
 
