@@ -485,6 +485,14 @@ def test_attention_picks_its_kernels_for_a_mixed_step(ops):
         _attention_case(ops, nh=4, nkv=2, d=128, page=64, lens=[(70, 70)], **T5)
 
 
+# as many sequences of the shortest portion as the tokens allow, one token fewer, ragged tiles of each, and many tokens of other kernels beside them
+@pytest.mark.parametrize("lens", [[(64, 64)] + [(32, 90)] * 12, [(65, 65)] + [(33, 33)] * 9 + [(1, 70)], [(64, 200)] + [(31, 31)] * 12 + [(32, 32)],
+                                  [(1, 30 + i) for i in range(120)] + [(70, 70)], [(64, 64)] + [(1, 3)] * 3])
+def test_the_tcgen05_kernel_has_blocks_for_every_portion_that_is_its_own(ops, lens):
+    for nh, nkv in ((6, 2), (8, 2), (5, 1)):
+        _attention_case(ops, dtype=torch.bfloat16, nh=nh, nkv=nkv, d=64, page=64, lens=lens, splits=1, planted=True)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("L,bias,hidden", [(3, False, 72), (4, True, 96), (2, True, 40), (1, False, 64), (8, False, 130), (3, True, 2048)])
 def test_shortconv_portions_and_state(ops, dtype, L, bias, hidden):
