@@ -130,17 +130,23 @@ def _p(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
-_held = threading.local()
+class _Held(threading.local):
+    """What the running step of a thread holds for its kernels (class attributes: a lookup with a default costs every launch)."""
+    stream: Optional[int] = None
+    status: Optional[int] = None
+
+
+_held = _Held()
 
 
 def _stream() -> int:
-    h = getattr(_held, "stream", None)
+    h = _held.stream
     return torch.cuda.current_stream().cuda_stream if h is None else h
 
 
-def _status(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
-    """The status word of a call: its own, or the running step's (:class:`one_stream`)."""
-    return getattr(_held, "status", None) if t is None else t
+def _status(t: Optional[torch.Tensor]) -> Optional[int]:
+    """The address of a call's status word: its own, or the running step's (:class:`one_stream`)."""
+    return _held.status if t is None else t.data_ptr()
 
 
 class one_stream:
@@ -153,9 +159,9 @@ class one_stream:
         self.status = status
 
     def __enter__(self):
-        self.before = getattr(_held, "stream", None), getattr(_held, "status", None)
+        self.before = _held.stream, _held.status
         _held.stream = torch.cuda.current_stream().cuda_stream if torch.cuda.is_available() else None
-        _held.status = self.status
+        _held.status = _p(self.status)
         return self
 
     def __exit__(self, *exc):
@@ -180,8 +186,10 @@ def _f32(t: Optional[torch.Tensor], what: str) -> None:
 
 def _bias(t: Optional[torch.Tensor], n: int, what: str = "bias") -> None:
     """A vector that a kernel reads ``n`` numbers of."""
+    if t is None:
+        return
     _f32(t, what)
-    if t is not None and t.numel() != n:
+    if t.numel() != n:
         raise KernelError(f"{what} of {tuple(t.shape)} does not fit {n} features")
 
 
@@ -574,9 +582,9 @@ def _fused_product(which: str, weight: torch.Tensor, act, xw, ss_in, eps: float,
             sso = torch.empty((parts, M), dtype=torch.float32, device=weight.device)
             xwo = torch.empty((M, N), dtype=torch.bfloat16, device=weight.device)
     _check(lib, fn(
-        _p(weight), N, K, M, _PRO[pro], _p(src), _p(ss_in), 0 if ss_in is None else ss_in.shape[0], ctypes.c_float(eps),
-        _EPI[epilogue], _p(out_bf16), _p(out_f32), ctypes.c_longlong(out_stride), _p(bias), _p(resid), _p(sso),
-        _p(next_weight), _p(xwo), _p(_status(status)), _stream(), _p(xielu), _glu(glu)))
+        _p(weight), N, K, M, _PRO[pro], _p(src), _p(ss_in), 0 if ss_in is None else ss_in.shape[0], eps,
+        _EPI[epilogue], _p(out_bf16), _p(out_f32), out_stride, _p(bias), _p(resid), _p(sso),
+        _p(next_weight), _p(xwo), _status(status), _stream(), _p(xielu), _glu(glu)))
     if epilogue == "resid":
         return sso, xwo
     return out_bf16 if out_bf16 is not None else out_f32
@@ -759,8 +767,8 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     if x.dtype != torch.float32 or tuple(x.shape) != (M, K) or not x.is_contiguous():
         raise KernelError(f"linear_f32: token operand {tuple(x.shape)} / {x.dtype} does not fit a weight of {N}x{K}")
     _bias(bias, N)
-    status = _status(status)
     _i32(status, "status")
+    word = _status(status)
     out = torch.empty((M, N), dtype=torch.float32, device=weight.device)
     kp = -(-K // 8) * 8
     most = min(M, LINEAR_F32_ROWS)
@@ -770,7 +778,7 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     for at in range(0, M, LINEAR_F32_ROWS):
         rows = min(most, M - at)
         _check(lib, lib.vapi_linear_f32(_p(weight), N, K, rows, x.data_ptr() + 4 * at * K, _p(planes), _p(bad), _p(bias),
-                                        out.data_ptr() + 4 * at * N, N, -1, _p(status), _stream()), launches=2)
+                                        out.data_ptr() + 4 * at * N, N, -1, word, _stream()), launches=2)
     return out
 
 
