@@ -4,12 +4,12 @@ import torch
 
 
 # (sequences, longest, slices) of 8 kv heads where the device holds 444 blocks: more than half of it and all of it stay whole at any configured
-# context (short sequences lose by every slice, and a captured step does not know their lengths); more than all is cut for four rounds of
-# blocks, but not where no sequence can be long; the edges at 20 and 36 tiles of 64 keys
-@pytest.mark.parametrize("seqs,longest,slices", [(27, 4096, 1), (28, 3072, 1), (28, 8192, 1), (32, 8192, 1), (32, 128000, 1), (55, 8192, 1), (55, 32768, 1),
-                                                 (56, 1280, 1), (56, 1281, 2), (64, 2304, 2), (64, 2305, 4), (64, 8192, 4), (64, 1, 1),
-                                                 (64, 128000, 4), (128, 2000, 2), (128, 8192, 2), (300, 32768, 1)])
-def test_a_full_step_is_only_cut_where_that_loses_at_no_length(monkeypatch, seqs, longest, slices):
+# context (short sequences lose by every slice, and a captured step does not know their lengths); more than all: the edge at one and a half
+# times 24 tiles of 64 keys, and the cap of four rounds of blocks
+@pytest.mark.parametrize("seqs,longest,slices", [(27, 4096, 1), (28, 3008, 1), (28, 3072, 1), (28, 8192, 1), (32, 8192, 1), (32, 128000, 1), (55, 3072, 1),
+                                                 (55, 32768, 1), (56, 2240, 1), (56, 2304, 2), (64, 2049, 1), (64, 4096, 3), (64, 8192, 4), (64, 1, 1),
+                                                 (64, 32768, 4), (128, 8192, 2), (300, 32768, 1)])
+def test_a_full_step_is_only_cut_where_a_sequence_could_be_long(monkeypatch, seqs, longest, slices):
     from vapi_b200 import ops
     monkeypatch.setattr(ops, "_decode_limits", (444, 8))
     assert ops.attention_splits(seqs, 1, longest, 32, 8, True) == slices

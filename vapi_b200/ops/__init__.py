@@ -951,13 +951,14 @@ def attention_splits(num_seqs: int, max_q: int, max_k: int, nh: int, nkv: int, d
     (sequence, kv head) pairs are fewer than two blocks per SM, slices up to that many blocks, and
     no more than the kernel combines itself unless a slice would then be longer than 32 tiles and
     there would be fewer blocks than SMs.
-    A step whose pairs alone fill half of the device's places, up to all of them, is left whole; one with more is cut for about four rounds
-    of blocks, so that the last ones do not run alone.  ``max_k`` bounds the lengths but does not tell them (a captured step is given the
-    configured context), so only what loses at no length is cut less: a step of more pairs than the device holds stays whole where
-    no sequence can be longer than 20 tiles and is cut in two up to 36.  8 kv heads, 444 places, us in 1 / 2 / 4 slices: 64 sequences of 20 to 300
-    keys 11.4 / 17.1 / 23.2, of 1,216 43.3 / 45.2 / 47.6, of 1,600 53.3 / 53.8 / 54.2 (56: 49.5 / 48.3 / 48.4), of 2,300
-    70.0 / 68.4 / 68.4, of 4,096 119.5 / 105.1 / 100.2.  Fewer pairs: 32 of 33 to 700 10.9 / 15.1 / 16.3, of 2,000 31.2 / 42.0 / 40.1, but
-    of 500 to 4,000, where the longest sequence's block runs alone, 49.7 / 45.6 / 41.6."""
+    A step whose pairs alone fill half of the device's places, up to all of them, is left whole: ``max_k`` bounds the lengths but does not
+    tell them (a captured step is given the configured context), and short sequences lose by every slice.  One with more pairs than
+    the device holds is cut to slices of about 24 tiles, and into no more than four rounds of blocks, so that the last ones do not run
+    alone.  8 kv heads, 444 places, us in 1 / 2 / 4 slices: 64 sequences of 20 to 300 keys 11.4 / 17.1 / 23.2, of 128 to 2,048 28.8 / 35.2 / 39.9,
+    all of 1,216 43.3 / 45.2 / 47.6, of 1,600 53.3 / 53.8 / 54.2 (56: 49.5 / 48.3 / 48.4), of 2,300 70.0 / 68.4 / 68.4, of 4,096 119.5 / 105.1 /
+    100.2: where none is longer than 36 tiles slices give 5 % at the most and cost up to a third.  Fewer pairs: 32 of 33 to 700
+    10.9 / 15.1 / 16.3, of 2,000 31.2 / 42.0 / 40.1, but of 500 to 4,000, where the longest sequence's block runs alone, 49.7 / 45.6 /
+    41.6."""
     n_rep = nh // nkv
     rows = max_q * n_rep
     tiles = -(-rows // (16 if rows <= 16 else 64))
@@ -967,8 +968,7 @@ def attention_splits(num_seqs: int, max_q: int, max_k: int, nh: int, nkv: int, d
         slots, cluster = decode_attention_limits()
         by_len = max(1, key_tiles // 2)
         if blocks > slots:
-            most = 1 if key_tiles <= 20 else 2 if key_tiles <= 36 else 32
-            return max(1, min(-(-4 * slots // blocks), by_len, most))
+            return max(1, min((key_tiles + 12) // 24, -(-4 * slots // blocks), by_len, 32))
         want = max(1, int(round(2 * slots / 3 / blocks)))
         if want > cluster and (key_tiles <= 32 * cluster or 3 * blocks * cluster >= slots):
             want = cluster
