@@ -323,6 +323,33 @@ def test_recurrent_kernels_continue_from_their_state_and_start_fresh_at_position
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", [(64, 32), (128, 96), (128, 48), (64, 40)])
+def test_long_walks_give_the_bits_of_the_short_ones(dtype, rows, cols):
+    """Portions of 16 tokens and more have kernels of their own (128 x 48 only the delta rule, 64 x 40 neither): ``max_q`` is what
+    tells them apart, and the sums are the same ones.  Portions that end on and beside the 8 and 16 tokens that are taken at once,
+    an empty one, fresh and continued states, rows that do not start on 16 bytes."""
+    from vapi_b200 import ops
+    g = torch.Generator().manual_seed(11)
+    qlens, starts, slots = [33, 1, 16, 0, 47, 8], [0, 5, 3, 0, 0, 1], [3, 0, 5, 4, 2, 1]
+    cu, pos, _, sl = _step_meta(qlens, starts, slots, "cuda")
+    n, nh = sum(qlens), 4
+    A, dtb, D = torch.rand(nh, generator=g).cuda() * 2 - 1, torch.randn(nh, generator=g).cuda(), torch.randn(nh, generator=g).cuda()
+    ab = torch.randn((n, 2 * nh + 3), generator=g).to(dtype).cuda()
+    state = torch.randn((7, 9 + nh * rows * cols), generator=g).cuda()
+
+    def same(fn, width):
+        whole = torch.randn(n * width + 1, generator=g).to(dtype).cuda()
+        for x in (whole[:n * width].view(n, width), whole[1:].view(n, width)):
+            s0, s1 = state.clone(), state.clone()
+            a, b = fn(x, s0, 1), fn(x, s1, max(qlens))
+            assert torch.equal(a, b) and torch.equal(s0, s1)
+
+    same(lambda x, s, m: ops.gated_delta(x, ab[:, :2 * nh], A, dtb, s, 9, sl, cu, pos, nh, 2, rows, cols, max_q=m), 4 * rows + nh * cols)
+    same(lambda x, s, m: ops.state_space(x, ab[:, 1:1 + nh], A, dtb, D, s, 9, sl, cu, pos, nh, 2, rows, cols, max_q=m), nh * cols + 4 * rows)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_norm_kernels_of_the_blocks_and_the_gated_group_norm(dtype):
     from vapi_b200 import ops
     g = torch.Generator().manual_seed(9)

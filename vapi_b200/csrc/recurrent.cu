@@ -7,6 +7,7 @@
 // unit norms, the state itself) is float; the projections and convolutions that feed it may be
 // bfloat16.
 #include "common.cuh"
+#include "recurrent_prompt.cuh"
 
 using namespace vapi;
 
@@ -566,10 +567,25 @@ VAPI_EXPORT int vapi_gated_delta(const void* qkv, long long qkv_stride, int q_of
     if (num_seqs <= 0) return 0;
     if (nh <= 0 || nkv <= 0 || nh % nkv || rows <= 0 || rows > 256 || cols <= 0)
         return fail(-1, "gated_delta: %d heads over %d, state %d x %d (rows up to 256)", nh, nkv, rows, cols);
+    if (dtype != VAPI_F32 && dtype != VAPI_BF16) return fail(-2, "gated_delta: unsupported dtype %d", dtype);
     const int cpb = REC_THREADS / rec_lpc(rows);
     dim3 grid((cols + cpb - 1) / cpb, nh, num_seqs);
     const bool early = max_q < REC_TC;                     // decode steps may start beside the kernel before; long walks may not
     cudaError_t e = cudaSuccess;
+    // Portions of at least a buffer's half, full rows and whole blocks of columns, 16-byte pieces: the walk of recurrent_prompt.cuh
+    // (same bits).
+    constexpr int NC = 1, WW = 4;
+    if (!early && (rows == 64 || rows == 128) && cols % (4 * WW * NC) == 0 && walk_aligned(qkv, qkv_stride, dtype, q_off, k_off)) {
+        grid.x = cols / (4 * WW * NC);
+#define GD_WALK(T, RT)                                                                                                     \
+    launch_if(false, gated_delta_prompt_kernel<T, RT, NC, WW>, grid, WalkShape<T, RT, NC, WW>::THREADS, 0, stream,         \
+              (const T*)qkv, qkv_stride, q_off, k_off, v_off, (const T*)ab, ab_stride, A_log, dt_bias, state, slot_stride, \
+              state_slots, cu_q, positions, out, nh, nkv, rows, cols, num_slots, norm_eps, status)
+        e = dtype == VAPI_F32 ? (rows == 64 ? GD_WALK(float, 8) : GD_WALK(float, 16))
+                              : (rows == 64 ? GD_WALK(__nv_bfloat16, 8) : GD_WALK(__nv_bfloat16, 16));
+#undef GD_WALK
+        return check_launch("gated_delta", e);
+    }
 #define GD_CALL(RT, LPC)                                                                                                   \
     if (dtype == VAPI_F32)                                                                                                 \
         e = launch_if(early, gated_delta_kernel<float, RT, LPC>, grid, REC_THREADS, 0, stream, (const float*)qkv, qkv_stride, q_off, \
@@ -579,7 +595,6 @@ VAPI_EXPORT int vapi_gated_delta(const void* qkv, long long qkv_stride, int q_of
         e = launch_if(early, gated_delta_kernel<__nv_bfloat16, RT, LPC>, grid, REC_THREADS, 0, stream, (const __nv_bfloat16*)qkv,    \
                    qkv_stride, q_off, k_off, v_off, (const __nv_bfloat16*)ab, ab_stride, A_log, dt_bias, state,            \
                    slot_stride, state_slots, cu_q, positions, out, nh, nkv, rows, cols, num_slots, norm_eps, status)
-    if (dtype != VAPI_F32 && dtype != VAPI_BF16) return fail(-2, "gated_delta: unsupported dtype %d", dtype);
     REC_DISPATCH(rows, GD_CALL);
 #undef GD_CALL
     return check_launch("gated_delta", e);
@@ -593,10 +608,23 @@ VAPI_EXPORT int vapi_state_space(const void* xbc, long long xbc_stride, const vo
     if (num_seqs <= 0) return 0;
     if (nh <= 0 || groups <= 0 || nh % groups || rows <= 0 || rows > 256 || cols <= 0)
         return fail(-1, "state_space: %d heads over %d groups, state %d x %d (rows up to 256)", nh, groups, rows, cols);
+    if (dtype != VAPI_F32 && dtype != VAPI_BF16) return fail(-2, "state_space: unsupported dtype %d", dtype);
     const int cpb = REC_THREADS / rec_lpc(rows);
     dim3 grid((cols + cpb - 1) / cpb, nh, num_seqs);
     const bool early = max_q < REC_TC;
     cudaError_t e = cudaSuccess;
+    constexpr int NC = 2, WW = 4;                           // (as in vapi_gated_delta)
+    if (!early && (rows == 64 || rows == 128) && cols % (4 * WW * NC) == 0 && walk_aligned(xbc, xbc_stride, dtype, nh * cols, rows)) {
+        grid.x = cols / (4 * WW * NC);
+#define SS_WALK(T, RT)                                                                                                     \
+    launch_if(false, state_space_prompt_kernel<T, RT, NC, WW>, grid, WalkShape<T, RT, NC, WW>::THREADS, 0, stream,         \
+              (const T*)xbc, xbc_stride, (const T*)dt, dt_stride, A_log, dt_bias, D, state, slot_stride, state_slots, cu_q, \
+              positions, out, nh, groups, cols, num_slots, status)
+        e = dtype == VAPI_F32 ? (rows == 64 ? SS_WALK(float, 8) : SS_WALK(float, 16))
+                              : (rows == 64 ? SS_WALK(__nv_bfloat16, 8) : SS_WALK(__nv_bfloat16, 16));
+#undef SS_WALK
+        return check_launch("state_space", e);
+    }
 #define SS_CALL(RT, LPC)                                                                                                  \
     if (dtype == VAPI_F32)                                                                                                \
         e = launch_if(early, state_space_kernel<float, RT, LPC>, grid, REC_THREADS, 0, stream, (const float*)xbc, xbc_stride,       \
@@ -606,7 +634,6 @@ VAPI_EXPORT int vapi_state_space(const void* xbc, long long xbc_stride, const vo
         e = launch_if(early, state_space_kernel<__nv_bfloat16, RT, LPC>, grid, REC_THREADS, 0, stream, (const __nv_bfloat16*)xbc,   \
                    xbc_stride, (const __nv_bfloat16*)dt, dt_stride, A_log, dt_bias, D, state, slot_stride, state_slots,   \
                    cu_q, positions, out, nh, groups, rows, cols, num_slots, status)
-    if (dtype != VAPI_F32 && dtype != VAPI_BF16) return fail(-2, "state_space: unsupported dtype %d", dtype);
     REC_DISPATCH(rows, SS_CALL);
 #undef SS_CALL
     return check_launch("state_space", e);
