@@ -61,11 +61,19 @@ __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: 
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ float ld_cluster_f32(unsigned local_smem_addr, unsigned rank) {
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// four floats at the same place of the shared memory of the block of `rank`: 16 bytes, or two pieces of 8 bytes `second` bytes apart
+__device__ __forceinline__ float4 ld_cluster_f4(unsigned local_smem_addr, unsigned rank, bool two, unsigned second) {
     unsigned remote;
-    float v;
+    float4 v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_smem_addr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+    if (!two) {
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+    } else {
+        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(remote) : "memory");
+        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.z), "=f"(v.w) : "r"(remote + second) : "memory");
+    }
     return v;
 }
 
@@ -182,13 +190,19 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         if (!glu && p.bias && row_ok) v += p.bias[n];
         fin[slot * TC_BM + row] = v;
     };
-    auto store_token = [&](int slot, int m) {                      // phase B for token m, whole warp
-        const float* f = fin + slot * TC_BM;
+    // what a lane takes of a token: four features, or (SwiGLU) two gate features from rows 0..63 and the two up features from
+    // rows 64..127
+    const unsigned lane_off = glu ? 2 * lane : 4 * lane;
+    // the stream's old values of a token, this lane's four features (full, aligned rows only)
+    auto old_values = [&](int m) {
+        const long long f0 = (long long)n0 + 4 * lane;
+        return p.epi == TC_EPI_RESID && m < p.M && f0 + 3 < p.N && (p.N & 3) == 0
+                   ? *reinterpret_cast<const float4*>(p.resid + (size_t)m * p.N + f0) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto store_token = [&](const float4& v, const float4& old, int m) {          // phase B for token m, whole warp
         if (glu) {
-            // 64 features: gate in rows 0..63, up in rows 64..127; two features per lane
             const long long f0 = (long long)n0 + 2 * lane;
-            const float g0 = f[2 * lane], g1 = f[2 * lane + 1], u0 = f[64 + 2 * lane], u1 = f[64 + 2 * lane + 1];
-            const float s0 = glu_gate_16(g0, p.glu) * u0, s1 = glu_gate_16(g1, p.glu) * u1;
+            const float s0 = glu_gate_16(v.x, p.glu) * v.z, s1 = glu_gate_16(v.y, p.glu) * v.w;
             __nv_bfloat16* o = p.out_bf16 + (size_t)m * p.out_stride + f0;
             if (f0 + 1 < p.ff && (p.out_stride & 1) == 0) *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(s0, s1);
             else {
@@ -198,7 +212,6 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             return;
         }
         const long long f0 = (long long)n0 + 4 * lane;             // four features per lane
-        const float4 v = *reinterpret_cast<const float4*>(f + 4 * lane);
         float vv[4] = {v.x, v.y, v.z, v.w};
         const bool full = f0 + 3 < p.N;
         if (p.epi == TC_EPI_BF16) {
@@ -228,7 +241,6 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             float* x = p.resid + (size_t)m * p.N + f0;
             float nv[4] = {0.f, 0.f, 0.f, 0.f};
             if (full && (p.N & 3) == 0) {
-                const float4 old = *reinterpret_cast<const float4*>(x);
                 nv[0] = old.x + vv[0]; nv[1] = old.y + vv[1]; nv[2] = old.z + vv[2]; nv[3] = old.w + vv[3];
                 *reinterpret_cast<float4*>(x) = make_float4(nv[0], nv[1], nv[2], nv[3]);
             } else {
@@ -247,8 +259,13 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         }
     };
 
+    float4 old[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
     if (epi_warp) {
         pdl_wait();
+        if (p.splits > 1) {                                          // (on their way while the tile accumulates)
+            old[0] = old_values(sp + (warp - 2) * p.splits);
+            old[1] = old_values(sp + (warp + 2) * p.splits);
+        }
         if (p.pro == TC_PRO_NORM) {
             for (int m = et; m < p.M; m += 128) {
                 float s = 0.f;
@@ -279,45 +296,69 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             if (p.splits == 1) {
                 epi_bar();
 #pragma unroll 4
-                for (int m = g0 + warp - 2; m < min(p.M, g0 + GROUP); m += 4) store_token(m - g0, m);
+                for (int m = g0 + warp - 2; m < min(p.M, g0 + GROUP); m += 4) {
+                    const float* f = fin + (m - g0) * TC_BM;
+                    const float2 lo = *reinterpret_cast<const float2*>(f + lane_off), hi = *reinterpret_cast<const float2*>(f + lane_off + (glu ? 64 : 2));
+                    store_token(make_float4(lo.x, lo.y, hi.x, hi.y), old_values(m), m);
+                }
                 epi_bar();
             }
         }
     }
     if (p.splits > 1) {
+        __syncwarp();
         cluster_sync_all();                                          // every block's partial tile is in place
+        // Token m belongs to the block of rank m % splits, there to one warp, whose lanes take their features' partials from
+        // every rank, 16 bytes at a time, add them in rank order and go on to phase B in registers.  Remote shared memory is far
+        // away: everything of two tokens is asked for before the first sum.  A block says that it needs nobody's memory any more
+        // as soon as its last partials have arrived, and waits for the others only after it has stored its tokens.
+        // (A product of this size is mostly this way from the last MMA to the stores, so it is kept short.  Four products of a layer in
+        // a captured chain, 32 / 64 / 128 tokens: 41.0 / 49.7 / 76.1 us at 1,536 / 6,912 features, so 36.2 / 43.5 / 65.2; 49.4 / 57.7 / 88.2 us
+        // at 2,048 / 7,168, so 43.3 / 49.7 / 73.0.  Before: one float at a time, a row a thread, the sums through shared memory
+        // and another barrier, the stream's old values asked for behind them.)
+        bool told = false;
         if (epi_warp) {
-            // token m belongs to the block of rank m % splits; partials are added in rank order.
-            // Remote shared memory is far away: fetch the partials of eight tokens from every
-            // rank first, then add them.  The sums replace this block's own partials of its tokens
-            // (which no other block reads).
-            for (int m0 = sp; m0 < p.M; m0 += 8 * p.splits) {
-                float part[8][8];
+            const unsigned a0 = smem_u32(part_s + lane_off), second = 64 * 4;
+            const long long f0 = (long long)n0 + 4 * lane;
+            for (int i = warp - 2; sp + i * p.splits < p.M; i += 8) {
+                const int m[2] = {sp + i * p.splits, sp + (i + 4) * p.splits};
+                float4 part[2][8];
 #pragma unroll
-                for (int t8 = 0; t8 < 8; ++t8) {
-                    const int m = m0 + t8 * p.splits;
-                    const unsigned a = smem_u32(part_s + (m < p.M ? m : 0) * TC_BM + row);
+                for (int t = 0; t < 2; ++t)
 #pragma unroll
-                    for (int r = 0; r < 8; ++r) part[t8][r] = (m < p.M && r < p.splits) ? ld_cluster_f32(a, (unsigned)r) : 0.f;
+                    for (int r = 0; r < 8; ++r)
+                        part[t][r] = m[t] < p.M && r < p.splits ? ld_cluster_f4(a0 + (unsigned)m[t] * (TC_BM * 4), (unsigned)r, glu, second)
+                                                                : make_float4(0.f, 0.f, 0.f, 0.f);
+                if (i != warp - 2) {
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) old[t] = old_values(m[t]);
                 }
+                float4 v[2];
 #pragma unroll
-                for (int t8 = 0; t8 < 8; ++t8) {
-                    const int m = m0 + t8 * p.splits;
-                    if (m < p.M) {
-                        float v = 0.f;
+                for (int t = 0; t < 2; ++t) {
+                    v[t] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                        for (int r = 0; r < 8; ++r) v += part[t8][r];
-                        finish(m, v, m);
+                    for (int r = 0; r < 8; ++r) { v[t].x += part[t][r].x; v[t].y += part[t][r].y; v[t].z += part[t][r].z; v[t].w += part[t][r].w; }
+                }
+                if (sp + (i + 8) * p.splits >= p.M) { cluster_arrive(); told = true; }
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    if (m[t] >= p.M) break;
+                    float4 w = v[t];
+                    if (p.pro == TC_PRO_NORM) { const float f = inv_s[m[t]]; w.x *= f; w.y *= f; w.z *= f; w.w *= f; }
+                    if (!glu && p.bias) {
+                        if (f0 < p.N) w.x += p.bias[f0];
+                        if (f0 + 1 < p.N) w.y += p.bias[f0 + 1];
+                        if (f0 + 2 < p.N) w.z += p.bias[f0 + 2];
+                        if (f0 + 3 < p.N) w.w += p.bias[f0 + 3];
                     }
+                    store_token(w, old[t], m[t]);
                 }
             }
         }
+        if (!told) cluster_arrive();
+        cluster_wait();                                              // nobody reads this block's memory any more
     }
-    if (epi_warp && p.splits > 1) {
-        epi_bar();                                                   // phase A is complete for this block's tokens
-        for (int i = warp - 2; sp + i * p.splits < p.M; i += 4) store_token(sp + i * p.splits, sp + i * p.splits);
-    }
-    if (p.splits > 1) cluster_sync_all();                            // nobody reads this block's memory any more
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
