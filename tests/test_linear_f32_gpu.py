@@ -141,3 +141,16 @@ def test_decode_product_of_wide_weights(ops, N, K):
     assert ((whole.double() - want).abs() <= bound).all()
     for M in (1, 2, 4, 5, 8, 9, 13):
         assert torch.equal(ops.skinny_linear_f32(w, a[16 - M:].contiguous(), b), whole[16 - M:]), M
+
+
+# each form of the gated product (staged, whole rows, shared K), odd features, one and many pieces of K
+@pytest.mark.parametrize("N,K", [(16384, 512), (8198, 1540), (8194, 128), (3074, 1024), (1034, 2048), (6, 4)])
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
+def test_gated_decode_product_is_the_product_and_its_gate(ops, N, K, act):
+    """The gate in the product's epilogue gives the bits of the two launches it stands for."""
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    a, w = (torch.randn(*s, generator=g, device="cuda") for s in ((16, K), (N, K)))
+    for M in (1, 3, 8, 9, 16):
+        x = a[:M].contiguous()
+        want = ops.swiglu(ops.skinny_linear_f32(w, x), act)
+        assert torch.equal(ops.linear_swiglu(x, w, act), want), M

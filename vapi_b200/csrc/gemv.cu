@@ -919,24 +919,53 @@ __device__ __forceinline__ float f32_pieces(const float4& w0, const float4& a0, 
     return fmaf(w1.w, a1.w, fmaf(w1.z, a1.z, fmaf(w1.y, a1.y, fmaf(w1.x, a1.x, t))));
 }
 
-template <int MT, int SHARE>
+// C sums over the 32 lanes: halves are exchanged while there is more than one left, so the lanes end with C / 32 of them (lane l: l * C / 32
+// and on) or, where C is less, with one (lane l: l * C / 32)
+template <int C>
+__device__ __forceinline__ void f32_lanes_sum(float (&acc)[C], int lane) {
+    int n = C;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int j = 0; j < C / 2; ++j) {
+                if (j < n) {
+                    const float keep = up ? acc[j + n] : acc[j], give = up ? acc[j] : acc[j + n];
+                    acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+            }
+        } else {
+            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+        }
+    }
+}
+
+// GLU: the weight is a stack of gate and up rows, N = 2 ff; a warp's rows are then half gate rows and half the up rows that belong to
+// them, and what it writes is gate(y_gate) * y_up of ff features: the sums, and the values, of the product and the elementwise
+// kernel behind it, one launch (about 3 us of a decode step) less.
+template <int MT, int SHARE, bool GLU = false>
 __global__ void __launch_bounds__(F32_WARPS * 32, MT <= 8 ? 4 : 3)
 skinny_linear_f32_kernel(const float* __restrict__ W, const float* act /*(the kernel before this one writes it)*/,
-                         const float* __restrict__ bias, float* out, int N, int K, int M, long long out_stride) {
+                         const float* __restrict__ bias, float* out, int N, int K, int M, long long out_stride, int glu) {
     constexpr int D = f32_depth(MT, SHARE), C = F32_ROWS * MT;
     constexpr int MG = SHARE == 1 ? (MT < 4 ? MT : 4) : (MT < 8 ? MT : 8);       // (tokens at a time: registers)
     __shared__ float part[F32_WARPS][C];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int GROUPS = F32_WARPS / SHARE;                           // groups of rows in a block
-    const long long b0 = (long long)blockIdx.x * (GROUPS * F32_ROWS), n0 = b0 + warp / SHARE * F32_ROWS;
+    constexpr int OWN = GLU ? F32_ROWS / 2 : F32_ROWS;                  // features of a group of rows
+    const int features = GLU ? N / 2 : N;
+    const long long b0 = (long long)blockIdx.x * (GROUPS * OWN), n0 = b0 + warp / SHARE * OWN;
     pdl_trigger();
     const int k4 = K >> 2;
     const int first = warp % SHARE * 32 + lane;                         // this lane's 16-byte pieces of a row: first, first + step, ...
     constexpr int step = SHARE * 32;
-    const int steps = n0 < N ? (k4 - warp % SHARE * 32 + step - 1) / step : 0;      // (the same for the whole warp; <= 0: none)
+    const int steps = n0 < features ? (k4 - warp % SHARE * 32 + step - 1) / step : 0;      // (the same for the whole warp; <= 0: none)
     const float4* wrow[F32_ROWS];
 #pragma unroll
-    for (int r = 0; r < F32_ROWS; ++r) wrow[r] = reinterpret_cast<const float4*>(W + (size_t)(n0 + r < N ? n0 + r : b0) * K);
+    for (int r = 0; r < F32_ROWS; ++r)
+        wrow[r] = reinterpret_cast<const float4*>(W + (size_t)((n0 + r % OWN < features ? n0 + r % OWN : b0) + (r < OWN ? 0 : features)) * K);
     float acc[C];
 #pragma unroll
     for (int i = 0; i < C; ++i) acc[i] = 0.f;
@@ -997,25 +1026,7 @@ skinny_linear_f32_kernel(const float* __restrict__ W, const float* act /*(the ke
             }
         }
     }
-    // the C sums over the 32 lanes: halves are exchanged while there is more than one left, so the lanes end with C / 32 (or one
-    // of C, in 32 / C lanes) each
-    int n = C;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        if (n > 1) {
-            n >>= 1;
-            const bool up = (lane & o) != 0;
-#pragma unroll
-            for (int j = 0; j < C / 2; ++j) {
-                if (j < n) {
-                    const float keep = up ? acc[j + n] : acc[j], give = up ? acc[j] : acc[j + n];
-                    acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-                }
-            }
-        } else {
-            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
-        }
-    }
+    f32_lanes_sum(acc, lane);
     if (C >= 32) {
 #pragma unroll
         for (int j = 0; j < (C >= 32 ? C / 32 : 1); ++j) part[warp][lane * (C / 32) + j] = acc[j];
@@ -1024,55 +1035,64 @@ skinny_linear_f32_kernel(const float* __restrict__ W, const float* act /*(the ke
     }
     __syncthreads();
     // the warps that share K in order; neighbouring threads write neighbouring features of a token
-    constexpr int ROWS = GROUPS * F32_ROWS;
+    constexpr int ROWS = GROUPS * OWN;
     for (int j = threadIdx.x; j < ROWS * MT; j += F32_WARPS * 32) {
-        const int r = j % ROWS, m = j / ROWS, i = r % F32_ROWS * MT + m, w0 = r / F32_ROWS * SHARE;
-        if (b0 + r < N && m < M) {
+        const int r = j % ROWS, m = j / ROWS, i = r % OWN * MT + m, w0 = r / OWN * SHARE;
+        if (b0 + r < features && m < M) {
             float y = part[w0][i];
 #pragma unroll
             for (int w = 1; w < SHARE; ++w) y += part[w0 + w][i];
-            out[(size_t)m * out_stride + b0 + r] = y + (bias ? bias[b0 + r] : 0.f);
+            if (GLU) {
+                float u = part[w0][i + C / 2];
+#pragma unroll
+                for (int w = 1; w < SHARE; ++w) u += part[w0 + w][i + C / 2];
+                out[(size_t)m * out_stride + b0 + r] = glu_gate(y, glu) * u;
+            } else {
+                out[(size_t)m * out_stride + b0 + r] = y + (bias ? bias[b0 + r] : 0.f);
+            }
         }
     }
 }
 
 // Wide weights, a few tokens: eight warps a block, each with whole weight rows of its own, the tokens staged through shared
 // memory a chunk of K at a time (two buffers, filled by asynchronous copies one chunk ahead), so that they are read from L2 once a
-// block and serve eight warps.  65,536 x 2,048, 8 tokens 103 us against 120 with shared K, 16,384 x 2,048 32 against 36, 8,192 x
-// 2,048 17 against 19.6, 3,072 x 512 3.7 against 4.0, 16,384 x 256 9.4 against 11.4; 2,048 x 2,048 10.4 against 6.6.
+// block and serve eight warps.  A lane's weights of the next chunk are asked for as soon as those of this one are used up: asked for
+// at the chunk's start instead, every chunk waited for memory (8 tokens: 65,536 x 2,048 104 us, so 99.8; 16,384 x 2,048 31.4, so 29.7;
+// 8,192 x 2,048 16.7, so 14.9; 1 token 22.4, 11.5, so 21.3 and 10.5 at the latter two).  With shared K 65,536 x 2,048 takes 120 us, 16,384 x 2,048
+// 36, 8,192 x 2,048 19.6, 3,072 x 512 4.0 against 3.7, 16,384 x 256 11.4 against 9.4; but 2,048 x 2,048 6.6 against 10.4.
 constexpr int F32_STAGED_WARPS = 8;
 // rows of the weight a warp owns, and 16-byte pieces of each row that a lane asks for together
 // (fewer of both for nine to sixteen tokens, whose sums take the registers)
 __host__ __device__ constexpr int f32_staged_rows(int mt) { return mt <= 8 ? 4 : 2; }
 __host__ __device__ constexpr int f32_staged_depth(int mt) { return mt <= 8 ? 4 : 2; }
 
-template <int MT>
-__global__ void __launch_bounds__(F32_STAGED_WARPS * 32)
+template <int MT, bool GLU = false>
+__global__ void __launch_bounds__(F32_STAGED_WARPS * 32, MT > 8 ? 3 : 2)
 skinny_linear_f32_staged_kernel(const float* __restrict__ W, const float* __restrict__ act, const float* __restrict__ bias,
-                         float* __restrict__ out, int N, int K, int M, long long out_stride) {
-    constexpr int ROWS = f32_staged_rows(MT), DEPTH = f32_staged_depth(MT);
+                         float* __restrict__ out, int N, int K, int M, long long out_stride, int glu) {
+    constexpr int ROWS = f32_staged_rows(MT), OWN = GLU ? ROWS / 2 : ROWS, C = ROWS * MT, DEPTH = f32_staged_depth(MT);
     constexpr int CHUNK = 32 * DEPTH;             // pieces of K in a chunk
     __shared__ float4 abuf[2][MT][CHUNK];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long n0 = ((long long)blockIdx.x * F32_STAGED_WARPS + warp) * ROWS;
+    const int features = GLU ? N / 2 : N;
+    const long long n0 = ((long long)blockIdx.x * F32_STAGED_WARPS + warp) * OWN;
     pdl_trigger();
-    float acc[ROWS][MT];
+    float acc[C];
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-        for (int m = 0; m < MT; ++m) acc[r][m] = 0.f;
+    for (int i = 0; i < C; ++i) acc[i] = 0.f;
     const int k4 = K >> 2;
     const int chunks = (k4 + CHUNK - 1) / CHUNK;
     const float4* wrow[ROWS];
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) wrow[r] = reinterpret_cast<const float4*>(W + (size_t)(n0 + r < N ? n0 + r : 0) * K);
+    for (int r = 0; r < ROWS; ++r)
+        wrow[r] = reinterpret_cast<const float4*>(W + (size_t)((n0 + r % OWN < features ? n0 + r % OWN : 0) + (r < OWN ? 0 : features)) * K);
     float4 w[DEPTH][ROWS];
-    auto fetch = [&](int c0) {          // this lane's pieces of a chunk of its rows
+    auto fetch = [&](int u, int c0) {   // this lane's pieces u and u + 1 of a chunk of its rows
 #pragma unroll
-        for (int u = 0; u < DEPTH; ++u)
+        for (int v = u; v < u + 2; ++v)
 #pragma unroll
             for (int r = 0; r < ROWS; ++r)
-                w[u][r] = (c0 + 32 * u < k4 && n0 < N) ? __ldcs(wrow[r] + c0 + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+                w[v][r] = (c0 + 32 * v < k4 && n0 < features) ? __ldcs(wrow[r] + c0 + 32 * v) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     auto stage = [&](int chunk, int buf) {     // the tokens' pieces of a chunk, by the whole block
         for (int idx = threadIdx.x; idx < MT * CHUNK; idx += F32_STAGED_WARPS * 32) {
@@ -1082,7 +1102,8 @@ skinny_linear_f32_staged_kernel(const float* __restrict__ W, const float* __rest
         }
         gv_commit();
     };
-    fetch(lane);                         // the weights do not depend on the kernel before this one
+#pragma unroll
+    for (int u = 0; u < DEPTH; u += 2) fetch(u, lane);      // the weights do not depend on the kernel before this one
     pdl_wait();
     stage(0, 0);
     for (int ch = 0; ch < chunks; ++ch) {
@@ -1090,40 +1111,33 @@ skinny_linear_f32_staged_kernel(const float* __restrict__ W, const float* __rest
         else gv_commit();
         gv_wait<1>();
         __syncthreads();                 // chunk ch of the tokens is in place for every warp
-        if (ch > 0) fetch(ch * CHUNK + lane);
 #pragma unroll
         for (int u = 0; u < DEPTH; u += 2) {
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
                 const float4 a0 = abuf[ch & 1][m][lane + 32 * u], a1 = abuf[ch & 1][m][lane + 32 * (u + 1)];
 #pragma unroll
-                for (int r = 0; r < ROWS; ++r) acc[r][m] += f32_pieces(w[u][r], a0, w[u + 1][r], a1);
+                for (int r = 0; r < ROWS; ++r) acc[r * MT + m] += f32_pieces(w[u][r], a0, w[u + 1][r], a1);
             }
+            fetch(u, (ch + 1) * CHUNK + lane);               // (the next chunk's, a whole chunk of arithmetic ahead of their use)
         }
         __syncthreads();                 // everyone is done with this buffer before it is filled again
     }
     gv_wait<0>();
-    if (n0 >= N) return;
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-        for (int m = 0; m < MT; ++m) acc[r][m] = warp_sum(acc[r][m]);
-    if (lane == 0) {
-#pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            if (n0 + r < N) {
-                const float b = bias ? bias[n0 + r] : 0.f;
-#pragma unroll
-                for (int m = 0; m < MT; ++m)
-                    if (m < M) out[(size_t)m * out_stride + n0 + r] = acc[r][m] + b;
-            }
-        }
-    }
+    if (n0 >= features) return;
+    f32_lanes_sum(acc, lane);
+    constexpr int LANES = 32 / C;                // lanes that hold the same sum
+    static_assert(32 % C == 0, "a lane holds one sum");
+    const int i = lane / LANES, r = i / MT, m = i % MT;
+    // (a gate's sum and its up row's are C / 2 apart, 16 lanes)
+    const float up = GLU ? __shfl_xor_sync(0xffffffffu, acc[0], 16) : 0.f;
+    if (lane % LANES == 0 && r < OWN && n0 + r < features && m < M)
+        out[(size_t)m * out_stride + n0 + r] = GLU ? glu_gate(acc[0], glu) * up : acc[0] + (bias ? bias[n0 + r] : 0.f);
 }
 
 // y[m][n] = sum_k act[m][k] * W[n][k] (+ bias[n]) in float, M <= 16, K a multiple of 4.
-VAPI_EXPORT int vapi_skinny_linear_f32(const float* W, int N, int K, int M, const float* act, const float* bias,
-                                       float* out, long long out_stride, cudaStream_t stream) {
+static int skinny_linear_f32(const float* W, int N, int K, int M, const float* act, const float* bias, float* out, long long out_stride,
+                             bool gated, int glu, cudaStream_t stream) {
     if (M <= 0) return 0;
     if (M > 16) return fail(-1, "skinny_linear_f32: %d rows are more than 16", M);
     if (N <= 0 || K <= 0 || K % 4 != 0) return fail(-1, "skinny_linear_f32: K=%d must be a positive multiple of 4 (N=%d)", K, N);
@@ -1142,18 +1156,33 @@ VAPI_EXPORT int vapi_skinny_linear_f32(const float* W, int N, int K, int M, cons
     const bool staged = whole && K > 128 && (M <= 8 || (M > 12 && N >= 8192 && 4 * own < 3 * places * rounds));
     cudaError_t e;
 #define VAPI_F32(KERNEL, WARPS, ROWS)                                                                                                     \
-    e = launch(KERNEL, (N + (ROWS) - 1) / (ROWS), (WARPS) * 32, 0, stream, W, act, bias, out, N, K, M, out_stride)
-#define VAPI_F32_MT(MT)                                                                                                                   \
-    if (staged) VAPI_F32(skinny_linear_f32_staged_kernel<MT>, F32_STAGED_WARPS, F32_STAGED_WARPS * f32_staged_rows(MT));                   \
-    else if (whole) VAPI_F32((skinny_linear_f32_kernel<MT, 1>), F32_WARPS, F32_WARPS * F32_ROWS);                                          \
-    else VAPI_F32((skinny_linear_f32_kernel<MT, F32_WARPS>), F32_WARPS, F32_ROWS)
-    if (M <= 1) { VAPI_F32_MT(1); }
-    else if (M <= 4) { VAPI_F32_MT(4); }
-    else if (M <= 8) { VAPI_F32_MT(8); }
-    else { VAPI_F32_MT(16); }
+    e = launch(KERNEL, (N + (ROWS) - 1) / (ROWS), (WARPS) * 32, 0, stream, W, act, bias, out, N, K, M, out_stride, glu)
+#define VAPI_F32_MT(MT, GLU)                                                                                                              \
+    if (staged) VAPI_F32((skinny_linear_f32_staged_kernel<MT, GLU>), F32_STAGED_WARPS, F32_STAGED_WARPS * f32_staged_rows(MT));            \
+    else if (whole) VAPI_F32((skinny_linear_f32_kernel<MT, 1, GLU>), F32_WARPS, F32_WARPS * F32_ROWS);                                     \
+    else VAPI_F32((skinny_linear_f32_kernel<MT, F32_WARPS, GLU>), F32_WARPS, F32_ROWS)
+#define VAPI_F32_ROWS(GLU)                                                                                                                \
+    if (M <= 1) { VAPI_F32_MT(1, GLU); }                                                                                                  \
+    else if (M <= 4) { VAPI_F32_MT(4, GLU); }                                                                                             \
+    else if (M <= 8) { VAPI_F32_MT(8, GLU); }                                                                                             \
+    else { VAPI_F32_MT(16, GLU); }
+    if (gated) { VAPI_F32_ROWS(true) } else { VAPI_F32_ROWS(false) }
+#undef VAPI_F32_ROWS
 #undef VAPI_F32_MT
 #undef VAPI_F32
     return check_launch("skinny_linear_f32", e);
+}
+
+VAPI_EXPORT int vapi_skinny_linear_f32(const float* W, int N, int K, int M, const float* act, const float* bias,
+                                       float* out, long long out_stride, cudaStream_t stream) {
+    return skinny_linear_f32(W, N, K, M, act, bias, out, out_stride, false, 0, stream);
+}
+
+// The same for a stack of gate and up rows, out[m][f] = gate(y[m][f]) * y[m][N / 2 + f] (`glu`: glu_gate's kind).
+VAPI_EXPORT int vapi_skinny_linear_f32_glu(const float* W, int N, int K, int M, const float* act, float* out, long long out_stride,
+                                           int glu, cudaStream_t stream) {
+    if (N % 2 != 0) return fail(-1, "skinny_linear_f32: a gated product needs an even N (%d)", N);
+    return skinny_linear_f32(W, N, K, M, act, nullptr, out, out_stride, true, glu, stream);
 }
 
 VAPI_EXPORT const char* vapi_last_error() { return error_buffer(); }

@@ -637,6 +637,9 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, act: str = "silu") -> t
     if (x.dtype == torch.bfloat16 and x.is_contiguous() and weight.shape[0] % 16 == 0 and rows <= TC_MAX_ROWS
             and few_rows_applies(rows, weight)):
         return few_rows_linear(weight, act=x, epilogue="swiglu", glu=act)      # a decode step: the gate rides on the product
+    if (x.dtype == torch.float32 and weight.shape[0] % 2 == 0 and skinny_f32_applies(rows, weight) and x.is_contiguous()
+            and x.data_ptr() % 16 == 0):
+        return skinny_linear_f32(weight, x, glu=act)
     return swiglu(linear(x, weight), act)
 
 
@@ -713,9 +716,11 @@ def skinny_f32_applies(rows: int, weight: torch.Tensor) -> bool:
             and weight.dim() == 2 and weight.shape[1] % 4 == 0 and weight.is_contiguous() and weight.data_ptr() % 16 == 0)
 
 
-def skinny_linear_f32(weight: torch.Tensor, act: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+def skinny_linear_f32(weight: torch.Tensor, act: torch.Tensor, bias: Optional[torch.Tensor] = None,
+                      glu: Optional[str] = None) -> torch.Tensor:
     """``act @ weight.T (+ bias)`` for at most 16 rows in true float32 (FMA only): the decode
-    product of the 32-bit path, bound by reading the weight once."""
+    product of the 32-bit path, bound by reading the weight once.  ``glu``: ``weight`` is [Wg; Wu] and the result
+    ``glu(act @ Wg.T) * (act @ Wu.T)``, the values of this product and :func:`swiglu` in one launch (without a bias)."""
     _cuda(weight, act, bias)
     N, K = weight.shape
     M = act.shape[0]
@@ -724,8 +729,14 @@ def skinny_linear_f32(weight: torch.Tensor, act: torch.Tensor, bias: Optional[to
     if act.dtype != torch.float32 or tuple(act.shape) != (M, K) or not act.is_contiguous():
         raise KernelError(f"skinny_linear_f32: token operand {tuple(act.shape)} / {act.dtype} does not fit a weight of {N}x{K}")
     _bias(bias, N)
-    out = torch.empty((M, N), dtype=torch.float32, device=weight.device)
     lib = _lib("gemv")
+    if glu is not None:
+        if bias is not None or N % 2:
+            raise KernelError("a gated product needs an even number of features and takes no bias")
+        out = torch.empty((M, N // 2), dtype=torch.float32, device=weight.device)
+        _check(lib, lib.vapi_skinny_linear_f32_glu(_p(weight), N, K, M, _p(act), _p(out), N // 2, _glu(glu), _stream()))
+        return out
+    out = torch.empty((M, N), dtype=torch.float32, device=weight.device)
     _check(lib, lib.vapi_skinny_linear_f32(_p(weight), N, K, M, _p(act), _p(bias), _p(out), ctypes.c_longlong(N), _stream()))
     return out
 
