@@ -33,8 +33,6 @@
 // that every thread reaches on every path).
 #include "tcgen05.cuh"
 
-#include <unordered_map>
-
 using namespace vapi;
 
 constexpr int PL_BM = 128;
@@ -455,40 +453,6 @@ prompt_linear_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 }
 
 // ---- host side -------------------------------------------------------------------------------
-// a [rows][K] bfloat16 matrix, K contiguous, tiled in boxes of 64 k x box_rows rows, 128-byte swizzle;
-// encoded once per (address, shape, box) and thread
-static int pl_map(const CUtensorMap** out, const void* ptr, long long rows, long long K, int box_rows) {
-    struct Key {
-        const void* p; long long r, k; int b;
-        bool operator==(const Key& o) const { return p == o.p && r == o.r && k == o.k && b == o.b; }
-    };
-    struct Hash {
-        size_t operator()(const Key& k) const {
-            return std::hash<const void*>()(k.p) ^ (std::hash<long long>()(k.r) * 31) ^ (std::hash<long long>()(k.k) * 131) ^ (size_t)k.b;
-        }
-    };
-    static thread_local std::unordered_map<Key, CUtensorMap, Hash> cache;
-    const Key key{ptr, rows, K, box_rows};
-    auto it = cache.find(key);
-    if (it != cache.end()) { *out = &it->second; return 0; }
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail(-102, "prompt_linear: cuTensorMapEncodeTiled is not available from the driver");
-    if (((uintptr_t)ptr & 15) != 0 || (K * 2) % 16 != 0)
-        return fail(-1, "prompt_linear: operand address or row pitch is not 16-byte aligned (K=%lld)", K);
-    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    cuuint32_t box[2] = {(cuuint32_t)PL_BK, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUtensorMap map;
-    CUresult r = fn(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(-103, "prompt_linear: cuTensorMapEncodeTiled failed with %d", (int)r);
-    if (cache.size() > 4096) cache.clear();
-    *out = &cache.emplace(key, map).first->second;
-    return 0;
-}
-
 template <int BN, int PAIR>
 static int launch_pl(const CUtensorMap& ta, const CUtensorMap& tw, const PlParams& p, cudaStream_t stream) {
     using Cfg = PlCfg<BN, PAIR>;
@@ -586,14 +550,15 @@ VAPI_EXPORT int vapi_prompt_linear(const void* W, int N, int K, int M, int pro, 
     p.status = status; p.xielu = xielu_consts; p.glu = glu;
     const bool half_rows = epi == PL_EPI_SWIGLU || pair == 2;      // boxes of BN/2 weight rows
     const CUtensorMap *ta, *tw;
-    int rc = pl_map(&ta, tokens, M, K, PL_BM);
+    int rc = kmajor_map(&tw, "prompt_linear", W, N, K, half_rows ? bn / 2 : bn, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     if (rc) return rc;
-    rc = pl_map(&tw, W, N, K, half_rows ? bn / 2 : bn);
+    const CUtensorMap weights = *tw;                               // (the second call may empty the store)
+    rc = kmajor_map(&ta, "prompt_linear", tokens, M, K, PL_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     if (rc) return rc;
-    if (bn == 256 && pair == 2) return launch_pl<256, 2>(*ta, *tw, p, stream);
-    if (bn == 128 && pair == 2) return launch_pl<128, 2>(*ta, *tw, p, stream);
-    if (bn == 256 && pair == 1) return launch_pl<256, 1>(*ta, *tw, p, stream);
-    if (bn == 128 && pair == 1) return launch_pl<128, 1>(*ta, *tw, p, stream);
+    if (bn == 256 && pair == 2) return launch_pl<256, 2>(*ta, weights, p, stream);
+    if (bn == 128 && pair == 2) return launch_pl<128, 2>(*ta, weights, p, stream);
+    if (bn == 256 && pair == 1) return launch_pl<256, 1>(*ta, weights, p, stream);
+    if (bn == 128 && pair == 1) return launch_pl<128, 1>(*ta, weights, p, stream);
     return fail(-2, "prompt_linear: no kernel for tiles of %d features and %d blocks", bn, pair);
 }
 

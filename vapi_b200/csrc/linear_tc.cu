@@ -467,23 +467,6 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 }
 
 // ---- host side -------------------------------------------------------------------------------
-// a [rows][K] bfloat16 matrix, K contiguous, tiled in boxes of 64 k x box_rows rows, 128-byte swizzle
-static int make_map(CUtensorMap* map, const void* ptr, long long rows, long long K, int box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail(-102, "linear_tc: cuTensorMapEncodeTiled is not available from the driver");
-    if (((uintptr_t)ptr & 15) != 0 || (K * 2) % 16 != 0)
-        return fail(-1, "linear_tc: operand address or row pitch is not 16-byte aligned (K=%lld)", K);
-    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(-103, "linear_tc: cuTensorMapEncodeTiled failed with %d", (int)r);
-    return 0;
-}
-
 template <int BN>
 static int launch_tc(const CUtensorMap& tw, const CUtensorMap& ta, const TcParams& p, int tiles, cudaStream_t stream) {
     using Cfg = TcCfg<BN>;
@@ -546,16 +529,17 @@ static int run_tc(TcParams& p, const void* W, int N, int K, int M, int epi, cons
     vapi_linear_tc_plan(N, K, M, epi, &tiles, &splits, &bn);
     p.N = N; p.K = K; p.M = M; p.epi = epi;
     p.num_kb = (K + TC_BK - 1) / TC_BK; p.splits = splits; p.kb_per_split = (p.num_kb + splits - 1) / splits;
-    CUtensorMap tw, ta;
-    int rc = make_map(&tw, W, N, K, epi == TC_EPI_SWIGLU ? 64 : (epi == TC_EPI_CONV ? TC_CONV_CH : TC_BM));
+    const CUtensorMap *tw, *ta;
+    int rc = kmajor_map(&tw, "linear_tc", W, N, K, epi == TC_EPI_SWIGLU ? 64 : (epi == TC_EPI_CONV ? TC_CONV_CH : TC_BM), CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     if (rc) return rc;
-    rc = make_map(&ta, tokens, M, K, bn);
+    const CUtensorMap weights = *tw;                               // (the second call may empty the store)
+    rc = kmajor_map(&ta, "linear_tc", tokens, M, K, bn, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     if (rc) return rc;
     switch (bn) {
-        case 32: return launch_tc<32>(tw, ta, p, tiles, stream);
-        case 64: return launch_tc<64>(tw, ta, p, tiles, stream);
-        case 128: return launch_tc<128>(tw, ta, p, tiles, stream);
-        case 256: return launch_tc<256>(tw, ta, p, tiles, stream);
+        case 32: return launch_tc<32>(weights, *ta, p, tiles, stream);
+        case 64: return launch_tc<64>(weights, *ta, p, tiles, stream);
+        case 128: return launch_tc<128>(weights, *ta, p, tiles, stream);
+        case 256: return launch_tc<256>(weights, *ta, p, tiles, stream);
     }
     return fail(-2, "linear_tc: no kernel for %d tokens", bn);
 }

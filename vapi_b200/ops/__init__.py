@@ -12,6 +12,7 @@ taps) are always float32.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import threading
 from typing import Dict, Optional, Tuple
@@ -535,6 +536,7 @@ def tc_applies(rows: int, weight: torch.Tensor, most: Optional[int] = None) -> b
             and weight.dim() == 2 and weight.shape[1] % 8 == 0 and weight.is_contiguous())
 
 
+@functools.lru_cache(maxsize=4096)
 def _tc_plan(N: int, K: int, M: int, epi: int):
     lib = _lib("linear_tc")
     t, s, b = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
