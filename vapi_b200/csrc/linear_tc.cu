@@ -92,7 +92,7 @@ __device__ __forceinline__ float4 ld_cluster_f4(unsigned local_smem_addr, unsign
     return v;
 }
 
-template <int BN>
+template <int BN, bool CONV = false>
 __global__ void __launch_bounds__(TC_THREADS, 2)
 linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a, const TcParams p) {
     using Cfg = TcCfg<BN>;
@@ -112,7 +112,8 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     const unsigned full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES), accbar = smem_u32(bars + 2 * STAGES);
     const int kb0 = sp * p.kb_per_split;
     const int nkb = max(0, min(p.num_kb, kb0 + p.kb_per_split) - kb0);
-    const bool glu = p.epi == TC_EPI_SWIGLU, conv = p.epi == TC_EPI_CONV;
+    constexpr bool conv = CONV;                                    // p.epi == TC_EPI_CONV
+    const bool glu = !conv && p.epi == TC_EPI_SWIGLU;
     // rows of the tile: 128 weight rows, or 64 gate rows (MMA rows 0..63) + the 64 up rows (64..127), or the B, C and x rows of 32
     // channels (0..31, 32..63, 64..95; the tensor core's other rows are whatever lies there, and their sums are not read)
     const int n0 = glu ? tile * 64 : tile * (conv ? TC_CONV_CH : TC_BM);
@@ -320,14 +321,16 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     };
 
     float4 old[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-    Past past[2] = {};
+    Past past[4] = {};                                             // (of the first four tokens of a warp: none of this step's kernels writes them)
+    if (conv && epi_warp) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) past[t] = conv_past(sp + (warp - 2 + 4 * t) * p.splits);
+    }
     if (epi_warp) {
         pdl_wait();
         if (p.splits > 1) {                                          // (on their way while the tile accumulates)
             old[0] = old_values(sp + (warp - 2) * p.splits);
             old[1] = old_values(sp + (warp + 2) * p.splits);
-            past[0] = conv_past(sp + (warp - 2) * p.splits);
-            past[1] = conv_past(sp + (warp + 2) * p.splits);
         }
         if (p.pro == TC_PRO_NORM) {
             for (int m = et; m < p.M; m += 128) {
@@ -403,15 +406,16 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
                         for (int r = 0; r < 8; ++r) v[t][j] += part[t][r][j];
                     }
                 if (sp + (i + 8) * p.splits >= p.M) { cluster_arrive(); told = true; }
-                if (i != warp - 2) {
-#pragma unroll
-                    for (int t = 0; t < 2; ++t) past[t] = conv_past(m[t]);
-                }
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {
                     if (m[t] >= p.M) break;
                     const float f = p.pro == TC_PRO_NORM ? inv_s[m[t]] : 1.f;
                     conv_token(v[t][0] * f, v[t][1] * f, v[t][2] * f, past[t], m[t]);
+                }
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    past[t] = past[t + 2];
+                    past[t + 2] = conv_past(sp + (i + 16 + 4 * t) * p.splits);
                 }
             }
         } else if (epi_warp) {
@@ -467,10 +471,10 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 }
 
 // ---- host side -------------------------------------------------------------------------------
-template <int BN>
+template <int BN, bool CONV = false>
 static int launch_tc(const CUtensorMap& tw, const CUtensorMap& ta, const TcParams& p, int tiles, cudaStream_t stream) {
     using Cfg = TcCfg<BN>;
-    auto kern = linear_tc_kernel<BN>;
+    auto kern = linear_tc_kernel<BN, CONV>;
     static bool attr_done = false;
     if (!attr_done) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
@@ -535,6 +539,14 @@ static int run_tc(TcParams& p, const void* W, int N, int K, int M, int epi, cons
     const CUtensorMap weights = *tw;                               // (the second call may empty the store)
     rc = kmajor_map(&ta, "linear_tc", tokens, M, K, bn, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     if (rc) return rc;
+    if (epi == TC_EPI_CONV) {
+        switch (bn) {
+            case 32: return launch_tc<32, true>(weights, *ta, p, tiles, stream);
+            case 64: return launch_tc<64, true>(weights, *ta, p, tiles, stream);
+            case 128: return launch_tc<128, true>(weights, *ta, p, tiles, stream);
+            case 256: return launch_tc<256, true>(weights, *ta, p, tiles, stream);
+        }
+    }
     switch (bn) {
         case 32: return launch_tc<32>(weights, *ta, p, tiles, stream);
         case 64: return launch_tc<64>(weights, *ta, p, tiles, stream);
