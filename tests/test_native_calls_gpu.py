@@ -1,0 +1,100 @@
+"""The native calls of a few-row step (csrc/calls.cpp) against the same steps in Python, which take what those do not."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF, F32 = torch.bfloat16, torch.float32
+
+
+@pytest.fixture
+def ops():
+    from vapi_b200 import ops
+    return ops
+
+
+def _both(ops, monkeypatch, fn):
+    """``fn`` by the native call and without it; what the native call answered goes along."""
+    answers = []
+    native = ops._calls()
+
+    def counted(name):
+        def call(*a):
+            answers.append(getattr(native, name)(*a))
+            return answers[-1]
+        return call
+
+    monkeypatch.setattr(ops, "_calls", lambda: types.SimpleNamespace(product=counted("product"), shortconv=counted("shortconv")))
+    a = fn()
+    monkeypatch.setattr(ops, "_calls", lambda: types.SimpleNamespace(product=lambda *a: NotImplemented, shortconv=lambda *a: NotImplemented))
+    b = fn()
+    monkeypatch.setattr(ops, "_calls", lambda: native)
+    return a, b, [x is not NotImplemented for x in answers]
+
+
+def _same(a, b):
+    a, b = (x if isinstance(x, tuple) else (x,) for x in (a, b))
+    return len(a) == len(b) and all((x is None and y is None) or (x.dtype == y.dtype and torch.equal(x, y)) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("which,M", [("linear_tc", 17), ("linear_tc", 57), ("prompt_linear", 300)])
+@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("epilogue", ["bf16", "f32", "swiglu", "resid", "resid alone"])
+def test_native_product_is_the_product(ops, monkeypatch, which, M, norm, epilogue):
+    g = torch.Generator(device="cuda").manual_seed(M)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    N, K = 384, 136
+    w, x, bias, nw, x0 = torch.nn.Parameter(r(N, K).to(BF), requires_grad=False), r(M, K).to(BF), r(N), r(N), r(M, N)
+    kw = dict(xw=x, ss_in=r(3, M).square() * K, eps=1e-5) if norm else dict(act=x)
+    kw["epilogue"] = epilogue.split()[0]
+    if epilogue != "swiglu":
+        kw["bias"] = bias
+    streams = []
+
+    def run():
+        if kw["epilogue"] == "resid":
+            streams.append(x0.clone())
+            return getattr(ops, which)(w, resid=streams[-1], next_weight=None if "alone" in epilogue else nw, **kw)
+        return getattr(ops, which)(w, **kw)
+
+    before = ops.launch_count
+    a, b, native = _both(ops, monkeypatch, run)
+    assert native == [True] and ops.launch_count == before + 2
+    assert _same(a, b) and (not streams or torch.equal(*streams))
+
+
+@pytest.mark.parametrize("dtype,L,native", [(BF, 3, True), (BF, 1, True), (F32, 3, False)])
+def test_native_shortconv_is_the_shortconv(ops, monkeypatch, dtype, L, native):
+    g = torch.Generator(device="cuda").manual_seed(L)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    i = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    H, qlens = 40, [1, 5, 2]
+    n = sum(qlens)
+    h3, state = r(n, 3 * H).to(dtype), r(4, max(L - 1, 1) + 1, H).to(dtype)[:, :L - 1]
+    states = []
+
+    def run():
+        states.append(state.clone(memory_format=torch.preserve_format))
+        return ops.shortconv(h3, r(3 * H) * 0, r(L, H) * 0 + 0.5, None, states[-1] if L > 1 else None, i([2, 0, 3]),
+                             i([0, 1, 1, 1, 1, 1, 2, 2]), i([0, 1, 6, 8]), i([4, 0, 1, 2, 3, 4, 1, 2]))
+
+    a, b, taken = _both(ops, monkeypatch, run)
+    assert taken == [native] and _same(a, b) and torch.equal(*states)
+
+
+def test_what_the_native_product_does_not_take_is_refused_or_done_as_before(ops):
+    w, x = torch.randn(64, 32, device="cuda").to(BF), torch.randn(20, 32, device="cuda").to(BF)
+    for bad in (dict(act=x[:, :16]), dict(act=x.float()), dict(xw=x), dict(act=x, bias=torch.ones(63, device="cuda")), dict(act=x, epilogue="none"),
+                dict(act=x, epilogue="resid", resid=torch.zeros(20, 63, device="cuda")), dict(act=x, glu="none"), dict(act=x.cpu())):
+        with pytest.raises(ops.KernelError):
+            ops.linear_tc(w, **bad)
+    with pytest.raises(ops.KernelError):
+        ops.linear_tc(w.t(), act=x)
+    with pytest.raises(ops.KernelError, match="more than 256"):          # (the C function's own refusal)
+        ops.linear_tc(w, act=torch.zeros(257, 32, device="cuda", dtype=BF))
+
+    class Other(torch.Tensor):
+        pass
+
+    assert torch.equal(ops.linear_tc(w, act=x.as_subclass(Other)).as_subclass(torch.Tensor), ops.linear_tc(w, act=x))

@@ -40,6 +40,23 @@ class BuildError(RuntimeError):
 HOST_FLAGS = ["-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden"]
 
 
+def _torch_flags() -> List[str]:
+    """What ``calls.cpp``, which speaks torch's C++ interface, is compiled and linked with."""
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(os.path.abspath(torch.__file__))
+    lib = os.path.join(root, "lib")
+    abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
+    return ["-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+            "-isystem", sysconfig.get_paths()["include"], f"-D_GLIBCXX_USE_CXX11_ABI={abi}", f"-DVAPI_TORCH=\"{torch.__version__}\"",
+            "-L", lib, f"-Wl,-rpath,{lib}", "-ltorch_python", "-ltorch_cpu", "-lc10"]
+
+
+def _extra(name: str) -> List[str]:
+    return EXTRA.get(name, []) + (_torch_flags() if name == "calls" else [])
+
+
 def sources() -> List[str]:
     """Names (without extension) of every native source of the package."""
     return sorted(os.path.splitext(f)[0] for f in os.listdir(CSRC_DIR) if f.endswith((".cu", ".cpp")))
@@ -102,7 +119,7 @@ def _digest(name: str) -> str:
             h.update(f.read())
         h.update(b"\0")
     flags = HOST_FLAGS if _is_host(name) else ARCH_FLAGS + COMMON_FLAGS + _ENV_FLAGS
-    h.update(" ".join(flags + EXTRA.get(name, [])).encode())
+    h.update(" ".join(flags + _extra(name)).encode())
     return h.hexdigest()[:12]
 
 
@@ -174,7 +191,7 @@ def build(name: str, verbose: bool = True) -> str:
     out = os.path.join(out_dir, f"lib{name}-{_digest(name)}.so")
     tmp = out + f".tmp{os.getpid()}"
     if _is_host(name):
-        cmd = [find_cxx()] + HOST_FLAGS + ["-I", CSRC_DIR] + EXTRA.get(name, []) + ["-o", tmp, src]
+        cmd = [find_cxx()] + HOST_FLAGS + ["-I", CSRC_DIR, "-o", tmp, src] + _extra(name)
     else:
         cmd = [find_nvcc()] + ARCH_FLAGS + COMMON_FLAGS + ["-I", CSRC_DIR] + EXTRA.get(name, []) + _ENV_FLAGS + ["-o", tmp, src]
     env = dict(os.environ)
