@@ -907,41 +907,6 @@ def test_skinny_shortconv_is_in_proj_then_the_conv_kernel(ops, M, H, K, L, bias)
             torch.testing.assert_close(state_gpu.cpu().float(), state_ref.float(), atol=6e-2, rtol=4e-2)
 
 
-@pytest.mark.parametrize("M,H,K,L,bias", [(17, 1536, 1536, 3, False), (32, 72, 104, 4, True), (19, 40, 640, 2, True),
-                                          (32, 3200, 64, 3, False), (23, 33 * 8, 128, 1, True), (20, 200, 2048, 8, False)])
-def test_tc_shortconv_is_in_proj_then_the_conv_kernel(ops, M, H, K, L, bias):
-    """Decode steps of 17 to 32 sequences: the convolution as the tcgen05 product's epilogue against that product and the
-    convolution kernel (the tolerance of the two-launch test above: they cut K differently), over steps that share their slots, one
-    request starting over and one whose slot is outside the pool, which is reported and left alone."""
-    torch.manual_seed(37)
-    bf = torch.bfloat16
-    w_in, taps = dev((torch.randn(3 * H, K) / math.sqrt(K)).to(bf)), dev(torch.randn(L, H))
-    in_b, cv_b = (dev(torch.randn(3 * H)), dev(torch.randn(H))) if bias else (None, None)
-    state = dev(torch.randn(M + 2, max(L - 1, 1), H).to(bf)[:, :L - 1].contiguous())
-    state_ref = state.clone()
-    slots, pos = dev(torch.randperm(M + 2)[:M].to(torch.int32)), dev(torch.randint(0, 4, (M,), dtype=torch.int32))
-    ar = dev(torch.arange(M + 1, dtype=torch.int32))
-    for step in range(3):
-        if step == 2:
-            pos[0] = 0
-        st = torch.zeros(1, dtype=torch.int32).cuda()
-        if step == 1 and L > 1:
-            slots[3] = M + 2
-        xw, ss = dev(torch.randn(M, K).to(bf)), dev(torch.rand(3, M) * K)
-        kw = dict(xw=xw, ss_in=ss, eps=1e-5)
-        h3 = ops.linear_tc(w_in, epilogue="bf16", **kw)
-        want = ops.shortconv(h3, in_b, taps, cv_b, state_ref if L > 1 else None, slots, ar[:M], ar, pos, st.clone())
-        got = ops.skinny_shortconv(w_in, in_bias=in_b, taps=taps, conv_bias=cv_b, state_layer=state if L > 1 else None,
-                                   state_slots=slots, positions=pos, status=st, **kw)
-        keep = [m for m in range(M) if not (L > 1 and step == 1 and m == 3)]
-        torch.testing.assert_close(got[keep].float(), want[keep].float(), atol=6e-2, rtol=4e-2)
-        torch.testing.assert_close(state.float(), state_ref.float(), atol=6e-2, rtol=4e-2)
-        assert int(st.item()) == (3 if len(keep) < M else 0)
-        if step == 1 and L > 1:
-            slots[3] = int(next(s for s in range(M + 2) if s not in slots.tolist()))
-        pos += 1
-
-
 @pytest.mark.parametrize("vocab", [1000, 65536, 70001])
 def test_sample_truncated_cuts_where_the_host_sampler_cuts(ops, vocab):
     """top-k, min-p and top-p on the device: the survivors are exactly the host sampler's (random

@@ -79,29 +79,6 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return y;
 }
 
-#ifndef FT_V
-#define FT_V 2
-#endif
-#ifndef FT_POLY
-#define FT_POLY 2
-#endif
-// 2^t of two finite t below 120, on the FMA pipe: t = n + f with |f| <= 1/2, a polynomial in f (relative error of the minimax fit 9.2e-8,
-// with the roundings 1.7e-7; ex2.approx 2.4e-7) and the exponent n put together by a shift.  Below -126 it is 2^-126; a NaN stays one.
-__device__ __forceinline__ float2 ex2_poly2(float2 t) {
-    asm("max.NaN.f32 %0, %0, %1;" : "+f"(t.x) : "f"(-126.f));
-    asm("max.NaN.f32 %0, %0, %1;" : "+f"(t.y) : "f"(-126.f));
-    const float2 magic = make_float2(12583039.f, 12583039.f), nmagic = make_float2(-12583039.f, -12583039.f);      // 1.5 * 2^23 + 127
-    const float2 r = __fadd2_rn(t, magic), n = __fadd2_rn(r, nmagic);
-    const float2 f = __ffma2_rn(n, make_float2(-1.f, -1.f), t);
-    float2 p = make_float2(0.0013264726899090153f, 0.0013264726899090153f);
-    p = __ffma2_rn(p, f, make_float2(0.009671512660564766f, 0.009671512660564766f));
-    p = __ffma2_rn(p, f, make_float2(0.055507337442444876f, 0.055507337442444876f));
-    p = __ffma2_rn(p, f, make_float2(0.24022242084919257f, 0.24022242084919257f));
-    p = __ffma2_rn(p, f, make_float2(0.6931469775984712f, 0.6931469775984712f));
-    p = __ffma2_rn(p, f, make_float2(1.f, 1.f));
-    return __fmul2_rn(p, make_float2(__uint_as_float(__float_as_uint(r.x) << 23), __uint_as_float(__float_as_uint(r.y) << 23)));
-}
-
 // The row tiles (of `rows` rows) of all sequences that a kernel takes stand in one list, sequence after sequence, longest tiles (the last
 // rows) of a sequence first: entry `want` of it as (sequence, row tile); false behind its end.  For whole warps.  A grid of
 // (longest sequence's tiles) x sequences instead is mostly blocks with nothing to do when one portion stands beside many
@@ -133,9 +110,6 @@ __device__ __forceinline__ bool ft_tile(const int* cu_q, int num_seqs, int min_q
     }
     return false;
 }
-
-struct FtTrue { static constexpr bool value = true; };
-struct FtFalse { static constexpr bool value = false; };
 
 template <bool SIG>
 __global__ void __launch_bounds__(FT_THREADS, 2)
@@ -380,29 +354,24 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const FaTcParams p) {
             // this tile's P buffer was last read by P.V of the tile two before
             if (i >= 2 && !__all_sync(0xffffffffu, mbar_wait(pv_done + 8 * sb, ((i >> 1) - 1) & 1))) { ok = false; break; }
             const float2 sc2 = make_float2(p.scale_log2e, p.scale_log2e), mu2 = make_float2(-m_use, -m_use);
-            // one or two of every eight pairs on the FMA pipe (see ex2_poly2), where no score is hidden
-            auto weights = [&](auto poly) {
+            // (two scores an instruction: fma.rn.f32x2; 8,000 tokens, 32 / 8 heads 492 us one by one, so 481.  A polynomial on the FMA pipe for
+            // an eighth to a half of the exponentials takes 500 to 566 us: what the warps wait for is not the special function units)
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    unsigned w[4];
-                    float2 t[4];
+            for (int c = 0; c < 8; ++c) {
+                unsigned w[4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        t[e] = make_float2(sv[c * 8 + 2 * e], sv[c * 8 + 2 * e + 1]);
-                        if (!SIG) {
-                            t[e] = __ffma2_rn(t[e], sc2, mu2);
-                            if (decltype(poly)::value && e >= 4 - (c & 1 ? FT_POLY / 2 : (FT_POLY + 1) / 2)) t[e] = ex2_poly2(t[e]);
-                            else t[e] = make_float2(ex2_approx(t[e].x), ex2_approx(t[e].y));
-                            rs4[e] += t[e].x + t[e].y;
-                        }
-                        __nv_bfloat162 h2 = __floats2bfloat162_rn(t[e].x, t[e].y);
-                        w[e] = *reinterpret_cast<unsigned*>(&h2);
+                for (int e = 0; e < 4; ++e) {
+                    float2 t = make_float2(sv[c * 8 + 2 * e], sv[c * 8 + 2 * e + 1]);
+                    if (!SIG) {
+                        t = __ffma2_rn(t, sc2, mu2);
+                        t = make_float2(ex2_approx(t.x), ex2_approx(t.y));
+                        rs4[e] += t.x + t.y;
                     }
-                    *reinterpret_cast<uint4*>(sP + sb * FT_ROWS * FT_BK * 2 + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                    __nv_bfloat162 h2 = __floats2bfloat162_rn(t.x, t.y);
+                    w[e] = *reinterpret_cast<unsigned*>(&h2);
                 }
-            };
-            if (!SIG && FT_POLY > 0 && !need_mask) weights(FtTrue{});
-            else weights(FtFalse{});
+                *reinterpret_cast<uint4*>(sP + sb * FT_ROWS * FT_BK * 2 + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
             l_run += (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
             if (k0 + FT_BK > klen) {
                 // V rows of keys beyond the sequence: zero them (a row is 128 bytes whatever the swizzle)

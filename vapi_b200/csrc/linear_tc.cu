@@ -19,8 +19,7 @@
 // memory allocation, and (one lane) the MMA issue loop; tcgen05.commit hands a stage back to
 // the producer and, at the end, the accumulator to the epilogue.  Warps 2-5: epilogue, one
 // weight row per thread: bfloat16 out | float out | SwiGLU | add into the float residual stream
-// with what the next norm needs (partial sums of squares, bfloat16(stream * next norm weight)) | the
-// gated short convolution of a decode step (a tile's rows are the B, C and x rows of 32 channels).
+// with what the next norm needs (partial sums of squares, bfloat16(stream * next norm weight)).
 // The token operand may be the residual stream seen through a deferred RMSNorm (see gemv.cu):
 // then the epilogue scales every token's column by rsqrt(mean x^2 + eps).
 //
@@ -37,9 +36,7 @@ constexpr int TC_THREADS = 192;
 constexpr int TC_A_BYTES = TC_BM * TC_BK * 2;
 
 enum { TC_PRO_ACT = 0, TC_PRO_NORM = 1 };
-enum { TC_EPI_BF16 = 0, TC_EPI_SWIGLU = 1, TC_EPI_RESID = 2, TC_EPI_F32 = 3, TC_EPI_CONV = 4 };
-constexpr int TC_CONV_CH = 32;            // EPI_CONV: channels a tile, one a lane
-constexpr int TC_CONV_LMAX = 8;
+enum { TC_EPI_BF16 = 0, TC_EPI_SWIGLU = 1, TC_EPI_RESID = 2, TC_EPI_F32 = 3 };
 
 struct TcParams {
     int N, K, M, epi, pro, ff;
@@ -50,11 +47,6 @@ struct TcParams {
     int* status;
     const float* xielu;                                            // EPI_BF16: null, or {up, down}: the output passes xIELU
     int glu;                                                       // EPI_SWIGLU: the gate's activation (glu_gate)
-    // EPI_CONV (W is a short-conv in_proj [3 ff][K], rows B | C | x; every token is a sequence of its own)
-    const float* taps; const float* conv_bias;                     // [L][ff] oldest tap first, [ff] or null
-    __nv_bfloat16* state; long long slot_stride;                   // [slots][L-1][ff]
-    const int* state_slots; const int* positions;                  // [M]
-    int L, num_slots;
 };
 
 template <int BN> struct TcCfg {
@@ -71,13 +63,6 @@ __device__ __forceinline__ void cluster_sync_all() {
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ float ld_cluster_f32(unsigned local_smem_addr, unsigned rank) {
-    unsigned remote;
-    float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_smem_addr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
-    return v;
-}
 // four floats at the same place of the shared memory of the block of `rank`: 16 bytes, or two pieces of 8 bytes `second` bytes apart
 __device__ __forceinline__ float4 ld_cluster_f4(unsigned local_smem_addr, unsigned rank, bool two, unsigned second) {
     unsigned remote;
@@ -92,7 +77,7 @@ __device__ __forceinline__ float4 ld_cluster_f4(unsigned local_smem_addr, unsign
     return v;
 }
 
-template <int BN, bool CONV = false>
+template <int BN>
 __global__ void __launch_bounds__(TC_THREADS, 2)
 linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a, const TcParams p) {
     using Cfg = TcCfg<BN>;
@@ -112,19 +97,14 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     const unsigned full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES), accbar = smem_u32(bars + 2 * STAGES);
     const int kb0 = sp * p.kb_per_split;
     const int nkb = max(0, min(p.num_kb, kb0 + p.kb_per_split) - kb0);
-    constexpr bool conv = CONV;                                    // p.epi == TC_EPI_CONV
-    const bool glu = !conv && p.epi == TC_EPI_SWIGLU;
-    // rows of the tile: 128 weight rows, or 64 gate rows (MMA rows 0..63) + the 64 up rows (64..127), or the B, C and x rows of 32
-    // channels (0..31, 32..63, 64..95; the tensor core's other rows are whatever lies there, and their sums are not read)
-    const int n0 = glu ? tile * 64 : tile * (conv ? TC_CONV_CH : TC_BM);
-    const unsigned stage_tx = Cfg::STAGE_BYTES - (conv ? (TC_BM - 3 * TC_CONV_CH) * TC_BK * 2 : 0);
+    const bool glu = p.epi == TC_EPI_SWIGLU;
+    // rows of the tile: 128 weight rows, or 64 gate rows (MMA rows 0..63) + the 64 up rows (64..127)
+    const int n0 = glu ? tile * 64 : tile * TC_BM;
 
     auto load_weights = [&](unsigned a, unsigned bar, int kb) {
         if (glu) {      // tm_w has boxes of 64 rows here
             tma_load_2d(a, &tm_w, bar, kb * TC_BK, n0);
             tma_load_2d(a + TC_A_BYTES / 2, &tm_w, bar, kb * TC_BK, p.ff + n0);
-        } else if (conv) {                                          // boxes of 32 rows
-            for (int j = 0; j < 3; ++j) tma_load_2d(a + j * TC_CONV_CH * TC_BK * 2, &tm_w, bar, kb * TC_BK, j * p.ff + n0);
         } else {
             tma_load_2d(a, &tm_w, bar, kb * TC_BK, n0);
         }
@@ -140,7 +120,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         // The weights depend on nothing that runs before this kernel: request the first stages
         // right away, before tensor memory is even allocated (this thread is the producer).
         for (int i = 0; i < pre; ++i) {
-            mbar_expect_tx(full0 + 8 * i, stage_tx);
+            mbar_expect_tx(full0 + 8 * i, Cfg::STAGE_BYTES);
             load_weights(smem_u32(stage_mem + (size_t)i * Cfg::STAGE_BYTES), full0 + 8 * i, kb0 + i);
         }
     }
@@ -163,7 +143,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
                 const int s = i % STAGES;
                 if (!mbar_wait(empty0 + 8 * s, ((i / STAGES) & 1) ^ 1)) { flags[0] = 1; break; }
                 const unsigned a = smem_u32(stage_mem + (size_t)s * Cfg::STAGE_BYTES);
-                mbar_expect_tx(full0 + 8 * s, stage_tx);
+                mbar_expect_tx(full0 + 8 * s, Cfg::STAGE_BYTES);
                 load_weights(a, full0 + 8 * s, kb0 + i);
                 tma_load_2d(a + TC_A_BYTES, &tm_a, full0 + 8 * s, (kb0 + i) * TC_BK, 0);
             }
@@ -197,7 +177,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     // the output feature of this row: for SwiGLU rows 0..63 are gate rows of feature n0 + row,
     // rows 64..127 the up rows of feature n0 + row - 64
     const long long n = glu ? (long long)n0 + (row & 63) : (long long)n0 + row;
-    const bool row_ok = glu ? n < p.ff : (!conv && n < p.N);
+    const bool row_ok = glu ? n < p.ff : n < p.N;
     bool ok = true;
 
     // Phase A (one weight row per thread): the finished sums over K, scaled for a deferred norm
@@ -218,47 +198,6 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         const long long f0 = (long long)n0 + 4 * lane;
         return p.epi == TC_EPI_RESID && m < p.M && f0 + 3 < p.N && (p.N & 3) == 0
                    ? *reinterpret_cast<const float4*>(p.resid + (size_t)m * p.N + f0) : make_float4(0.f, 0.f, 0.f, 0.f);
-    };
-    // EPI_CONV, a lane's channel: the request's past, asked for before the sums are there (nothing of this step writes it before this kernel)
-    const int ch = n0 + lane;
-    float taps[TC_CONV_LMAX];
-#pragma unroll
-    for (int k = 0; k < TC_CONV_LMAX; ++k) taps[k] = conv && warp >= 2 && k < p.L && ch < p.ff ? p.taps[(size_t)k * p.ff + ch] : 0.f;
-    struct Past { int slot; float row[TC_CONV_LMAX - 1]; };
-    auto conv_past = [&](int m) {
-        Past h;
-        h.slot = conv && m < p.M ? p.state_slots[m] : -1;
-        const bool there = h.slot >= 0 && h.slot < p.num_slots && p.L > 1 && ch < p.ff;
-        const int pos = there ? p.positions[m] : 0;
-#pragma unroll
-        for (int k = 0; k < TC_CONV_LMAX - 1; ++k)                  // (rows for positions before 0 count as zero)
-            h.row[k] = there && k < p.L - 1 && pos - (p.L - 1) + k >= 0
-                           ? __bfloat162float(p.state[(size_t)h.slot * p.slot_stride + (size_t)k * p.ff + ch]) : 0.f;
-        return h;
-    };
-    // The values of the product stored as bfloat16 and the convolution kernel behind it: B, C and x are rounded first, g = B x is too.
-    auto conv_token = [&](float b, float c, float x, const Past& h, int m) {       // token m, whole warp, a lane's channel
-        if (p.L > 1 && (h.slot < 0 || h.slot >= p.num_slots)) {
-            if (lane == 0 && p.status) atomicExch(p.status, 3);
-            return;
-        }
-        if (ch >= p.ff) return;
-        b = round_to<__nv_bfloat16>(b); c = round_to<__nv_bfloat16>(c); x = round_to<__nv_bfloat16>(x);
-        if (p.bias) { b += p.bias[ch]; c += p.bias[p.ff + ch]; x += p.bias[2 * p.ff + ch]; }
-        const float g = round_to<__nv_bfloat16>(b * x);
-        float acc = 0.f;
-#pragma unroll
-        for (int k = 0; k < TC_CONV_LMAX; ++k) {
-            if (k < p.L - 1) acc += taps[k] * h.row[k < TC_CONV_LMAX - 1 ? k : 0];
-            if (k == p.L - 1) acc += taps[k] * g;
-        }
-        p.out_bf16[(size_t)m * p.out_stride + ch] = __float2bfloat16_rn(c * (acc + (p.conv_bias ? p.conv_bias[ch] : 0.f)));
-        __nv_bfloat16* st = p.L > 1 ? p.state + (size_t)h.slot * p.slot_stride + ch : nullptr;
-#pragma unroll
-        for (int k = 0; k < TC_CONV_LMAX - 1; ++k) {
-            if (k < p.L - 2) st[(size_t)k * p.ff] = __float2bfloat16_rn(h.row[k + 1 < TC_CONV_LMAX - 1 ? k + 1 : 0]);
-            if (k == p.L - 2) st[(size_t)k * p.ff] = __float2bfloat16_rn(g);
-        }
     };
     auto store_token = [&](const float4& v, const float4& old, int m) {          // phase B for token m, whole warp
         if (glu) {
@@ -321,11 +260,6 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     };
 
     float4 old[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-    Past past[4] = {};                                             // (of the first four tokens of a warp: none of this step's kernels writes them)
-    if (conv && epi_warp) {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) past[t] = conv_past(sp + (warp - 2 + 4 * t) * p.splits);
-    }
     if (epi_warp) {
         pdl_wait();
         if (p.splits > 1) {                                          // (on their way while the tile accumulates)
@@ -364,7 +298,6 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 #pragma unroll 4
                 for (int m = g0 + warp - 2; m < min(p.M, g0 + GROUP); m += 4) {
                     const float* f = fin + (m - g0) * TC_BM;
-                    if (conv) { conv_token(f[lane], f[TC_CONV_CH + lane], f[2 * TC_CONV_CH + lane], conv_past(m), m); continue; }
                     const float2 lo = *reinterpret_cast<const float2*>(f + lane_off), hi = *reinterpret_cast<const float2*>(f + lane_off + (glu ? 64 : 2));
                     store_token(make_float4(lo.x, lo.y, hi.x, hi.y), old_values(m), m);
                 }
@@ -384,41 +317,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         // at 2,048 / 7,168, so 43.3 / 49.7 / 73.0.  Before: one float at a time, a row a thread, the sums through shared memory
         // and another barrier, the stream's old values asked for behind them.)
         bool told = false;
-        if (epi_warp && conv) {                                      // the same, a lane's channel
-            const unsigned a0 = smem_u32(part_s + lane);
-            for (int i = warp - 2; sp + i * p.splits < p.M; i += 8) {
-                const int m[2] = {sp + i * p.splits, sp + (i + 4) * p.splits};
-                float part[2][8][3], v[2][3];
-#pragma unroll
-                for (int t = 0; t < 2; ++t)
-#pragma unroll
-                    for (int r = 0; r < 8; ++r)
-#pragma unroll
-                        for (int j = 0; j < 3; ++j)
-                            part[t][r][j] = m[t] < p.M && r < p.splits
-                                ? ld_cluster_f32(a0 + (unsigned)(m[t] * TC_BM + j * TC_CONV_CH) * 4, (unsigned)r) : 0.f;
-#pragma unroll
-                for (int t = 0; t < 2; ++t)
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        v[t][j] = 0.f;
-#pragma unroll
-                        for (int r = 0; r < 8; ++r) v[t][j] += part[t][r][j];
-                    }
-                if (sp + (i + 8) * p.splits >= p.M) { cluster_arrive(); told = true; }
-#pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    if (m[t] >= p.M) break;
-                    const float f = p.pro == TC_PRO_NORM ? inv_s[m[t]] : 1.f;
-                    conv_token(v[t][0] * f, v[t][1] * f, v[t][2] * f, past[t], m[t]);
-                }
-#pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    past[t] = past[t + 2];
-                    past[t + 2] = conv_past(sp + (i + 16 + 4 * t) * p.splits);
-                }
-            }
-        } else if (epi_warp) {
+        if (epi_warp) {
             const unsigned a0 = smem_u32(part_s + lane_off), second = 64 * 4;
             const long long f0 = (long long)n0 + 4 * lane;
             for (int i = warp - 2; sp + i * p.splits < p.M; i += 8) {
@@ -471,10 +370,10 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 }
 
 // ---- host side -------------------------------------------------------------------------------
-template <int BN, bool CONV = false>
+template <int BN>
 static int launch_tc(const CUtensorMap& tw, const CUtensorMap& ta, const TcParams& p, int tiles, cudaStream_t stream) {
     using Cfg = TcCfg<BN>;
-    auto kern = linear_tc_kernel<BN, CONV>;
+    auto kern = linear_tc_kernel<BN>;
     static bool attr_done = false;
     if (!attr_done) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
@@ -507,15 +406,17 @@ static int launch_tc(const CUtensorMap& tw, const CUtensorMap& ta, const TcParam
 
 // How a call is cut: tiles of weight rows, slices of K (= cluster size), tokens per tile.
 VAPI_EXPORT int vapi_linear_tc_plan(int N, int K, int M, int epi, int* tiles, int* splits, int* bn) {
-    const int t = epi == TC_EPI_SWIGLU ? (N / 2 + 63) / 64
-                  : (epi == TC_EPI_CONV ? (N / 3 + TC_CONV_CH - 1) / TC_CONV_CH : (N + TC_BM - 1) / TC_BM);
+    const int t = epi == TC_EPI_SWIGLU ? (N / 2 + 63) / 64 : (N + TC_BM - 1) / TC_BM;
     int b = 32;
     while (b < M) b *= 2;
     const int num_kb = (K + TC_BK - 1) / TC_BK;
     int s = 1;
     const int sms = sm_count();
-    if (3 * t <= 2 * sms && b <= 128) {               // too few tiles for the multiprocessors: cut K (partials must fit the stages)
-        s = sms / t;
+#ifndef TC_SLOTS
+#define TC_SLOTS 1
+#endif
+    if (3 * t <= 2 * TC_SLOTS * sms && b <= 128) {               // too few tiles for the multiprocessors: cut K (partials must fit the stages)
+        s = TC_SLOTS * sms / t;
         if (s > 8) s = 8;                            // portable cluster size
         const int max_s = num_kb / 2 > 0 ? num_kb / 2 : 1;      // at least 2 k-blocks a slice
         if (s > max_s) s = max_s;
@@ -525,35 +426,6 @@ VAPI_EXPORT int vapi_linear_tc_plan(int N, int K, int M, int epi, int* tiles, in
     }
     *tiles = t; *splits = s; *bn = b;
     return 0;
-}
-
-// (what the call's form decides is in `p` already)
-static int run_tc(TcParams& p, const void* W, int N, int K, int M, int epi, const void* tokens, cudaStream_t stream) {
-    int tiles, splits, bn;
-    vapi_linear_tc_plan(N, K, M, epi, &tiles, &splits, &bn);
-    p.N = N; p.K = K; p.M = M; p.epi = epi;
-    p.num_kb = (K + TC_BK - 1) / TC_BK; p.splits = splits; p.kb_per_split = (p.num_kb + splits - 1) / splits;
-    const CUtensorMap *tw, *ta;
-    int rc = kmajor_map(&tw, "linear_tc", W, N, K, epi == TC_EPI_SWIGLU ? 64 : (epi == TC_EPI_CONV ? TC_CONV_CH : TC_BM), CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-    if (rc) return rc;
-    const CUtensorMap weights = *tw;                               // (the second call may empty the store)
-    rc = kmajor_map(&ta, "linear_tc", tokens, M, K, bn, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-    if (rc) return rc;
-    if (epi == TC_EPI_CONV) {
-        switch (bn) {
-            case 32: return launch_tc<32, true>(weights, *ta, p, tiles, stream);
-            case 64: return launch_tc<64, true>(weights, *ta, p, tiles, stream);
-            case 128: return launch_tc<128, true>(weights, *ta, p, tiles, stream);
-            case 256: return launch_tc<256, true>(weights, *ta, p, tiles, stream);
-        }
-    }
-    switch (bn) {
-        case 32: return launch_tc<32>(weights, *ta, p, tiles, stream);
-        case 64: return launch_tc<64>(weights, *ta, p, tiles, stream);
-        case 128: return launch_tc<128>(weights, *ta, p, tiles, stream);
-        case 256: return launch_tc<256>(weights, *ta, p, tiles, stream);
-    }
-    return fail(-2, "linear_tc: no kernel for %d tokens", bn);
 }
 
 VAPI_EXPORT int vapi_linear_tc(const void* W, int N, int K, int M, int pro, const void* tokens,
@@ -572,32 +444,28 @@ VAPI_EXPORT int vapi_linear_tc(const void* W, int N, int K, int M, int pro, cons
     if (epi == TC_EPI_F32 && !out_f32) return fail(-1, "linear_tc: no output");
     if (epi == TC_EPI_RESID && !resid) return fail(-1, "linear_tc: no residual stream");
     if (xw_out && !next_w) return fail(-1, "linear_tc: a weighted copy of the stream needs the next norm's weight");
-    TcParams p = {};
-    p.pro = pro; p.ff = N / 2; p.ss_in = ss_in; p.ss_parts = ss_parts; p.eps = eps;
+    int tiles, splits, bn;
+    vapi_linear_tc_plan(N, K, M, epi, &tiles, &splits, &bn);
+    TcParams p;
+    p.N = N; p.K = K; p.M = M; p.epi = epi; p.pro = pro; p.ff = N / 2;
+    p.num_kb = (K + TC_BK - 1) / TC_BK; p.splits = splits; p.kb_per_split = (p.num_kb + splits - 1) / splits;
+    p.ss_in = ss_in; p.ss_parts = ss_parts; p.eps = eps;
     p.out_bf16 = (__nv_bfloat16*)out_bf16; p.out_f32 = out_f32; p.out_stride = out_stride; p.bias = bias;
     p.resid = resid; p.ss_out = ss_out; p.next_w = next_w; p.xw_out = (__nv_bfloat16*)xw_out;
     p.status = status; p.xielu = xielu_consts; p.glu = glu;
-    return run_tc(p, W, N, K, M, epi, tokens, stream);
-}
-
-// The short-conv mixer up to its out_proj for a decode step, in one launch: in_proj [3 H][K] on the stream seen through a deferred norm,
-// gate, taps over each request's state, C * conv, state update (see vapi_skinny_linear_conv).
-VAPI_EXPORT int vapi_linear_tc_conv(const void* W, int H, int K, int M, const void* tokens, const float* ss_in, int ss_parts, float eps,
-                                    const float* in_bias, const float* taps, const float* conv_bias, int L, void* state,
-                                    long long slot_stride, int num_slots, const int* state_slots, const int* positions,
-                                    void* out_bf16, int* status, cudaStream_t stream) {
-    if (M <= 0) return 0;
-    if (M > 256) return fail(-1, "linear_tc: %d rows are more than 256", M);
-    if (H <= 0 || K <= 0 || K % 8 != 0) return fail(-1, "linear_tc: K=%d must be a positive multiple of 8 (H=%d)", K, H);
-    if (L < 1 || L > TC_CONV_LMAX) return fail(-1, "linear_tc: a convolution of %d taps is outside 1..%d", L, TC_CONV_LMAX);
-    if (L > 1 && (!state || num_slots <= 0)) return fail(-1, "linear_tc: no state buffer");
-    if (!tokens || !ss_in || ss_parts <= 0 || !taps || !state_slots || !positions || !out_bf16) return fail(-1, "linear_tc: missing array");
-    TcParams p = {};
-    p.pro = TC_PRO_NORM; p.ff = H; p.ss_in = ss_in; p.ss_parts = ss_parts; p.eps = eps;
-    p.out_bf16 = (__nv_bfloat16*)out_bf16; p.out_stride = H; p.bias = in_bias; p.status = status;
-    p.taps = taps; p.conv_bias = conv_bias; p.state = (__nv_bfloat16*)state; p.slot_stride = slot_stride;
-    p.state_slots = state_slots; p.positions = positions; p.L = L; p.num_slots = num_slots;
-    return run_tc(p, W, 3 * H, K, M, TC_EPI_CONV, tokens, stream);
+    const CUtensorMap *tw, *ta;
+    int rc = kmajor_map(&tw, "linear_tc", W, N, K, epi == TC_EPI_SWIGLU ? 64 : TC_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    if (rc) return rc;
+    const CUtensorMap weights = *tw;                               // (the second call may empty the store)
+    rc = kmajor_map(&ta, "linear_tc", tokens, M, K, bn, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    if (rc) return rc;
+    switch (bn) {
+        case 32: return launch_tc<32>(weights, *ta, p, tiles, stream);
+        case 64: return launch_tc<64>(weights, *ta, p, tiles, stream);
+        case 128: return launch_tc<128>(weights, *ta, p, tiles, stream);
+        case 256: return launch_tc<256>(weights, *ta, p, tiles, stream);
+    }
+    return fail(-2, "linear_tc: no kernel for %d tokens", bn);
 }
 
 VAPI_EXPORT const char* vapi_last_error() { return error_buffer(); }

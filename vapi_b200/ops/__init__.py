@@ -494,7 +494,7 @@ use_tc = os.environ.get("VAPI_TC", "1") != "0"
 
 def skinny_shortconv_applies(rows: int, w_in: torch.Tensor, kernel: int, state_layer: Optional[torch.Tensor]) -> bool:
     """Whether :func:`skinny_shortconv` takes a decode step of ``rows`` single-token sequences."""
-    return ((skinny_applies(rows, w_in) or (tc_applies(rows, w_in) and not prompt_applies(rows, w_in))) and 1 <= kernel <= 8 and w_in.shape[0] % 3 == 0
+    return (skinny_applies(rows, w_in) and 1 <= kernel <= 8 and w_in.shape[0] % 3 == 0
             and (kernel == 1 or (state_layer is not None and state_layer.dtype == torch.bfloat16)))
 
 
@@ -504,8 +504,7 @@ def skinny_shortconv(w_in: torch.Tensor, *, xw: torch.Tensor, ss_in: torch.Tenso
                      status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The short-conv mixer up to its out_proj for a decode step, in one launch: in_proj on the
     stream seen through a deferred norm (``xw``, ``ss_in``, ``eps`` as for :func:`skinny_linear`),
-    gate, taps over each request's state, ``C * conv``, state update (above 16 tokens as the tcgen05 product's epilogue: the
-    values of :func:`linear_tc` and :func:`shortconv`).  Every one of the M
+    gate, taps over each request's state, ``C * conv``, state update.  Every one of the M <= 16
     tokens must be a sequence of its own: token m uses ``state_slots[m]`` and ``positions[m]``.
     Returns y [M, H] bfloat16."""
     _cuda(w_in, xw, ss_in, in_bias, taps, conv_bias, state_layer, state_slots, positions)
@@ -535,12 +534,6 @@ def skinny_shortconv(w_in: torch.Tensor, *, xw: torch.Tensor, ss_in: torch.Tenso
             raise KernelError("state rows must be contiguous")
         slot_stride, num_slots = state_layer.stride(0), state_layer.shape[0]
     out = torch.empty((M, H), dtype=torch.bfloat16, device=w_in.device)
-    if M > SKINNY_MAX_ROWS:
-        lib = _lib("linear_tc")
-        _check(lib, lib.vapi_linear_tc_conv(
-            _p(w_in), H, K, M, _p(xw), _p(ss_in), ss_in.shape[0], eps, _p(in_bias), _p(taps), _p(conv_bias), L,
-            _p(state_layer if L > 1 else None), slot_stride, num_slots, _p(state_slots), _p(positions), _p(out), _status(status), _stream()))
-        return out
     lib = _lib("gemv")
     _check(lib, lib.vapi_skinny_linear_conv(
         _p(w_in), H, K, M, _p(xw), _p(ss_in), ss_in.shape[0], ctypes.c_float(eps), _p(in_bias), _p(taps), _p(conv_bias),
