@@ -106,11 +106,11 @@ def trace_read() -> list:
 _addresses: Dict[str, int] = {}
 
 
-def _address(name: str, fn: str) -> int:
+def _address(lib: ctypes.CDLL, fn: str) -> int:
     """Where a library's C function is."""
     at = _addresses.get(fn)
     if at is None:
-        at = _addresses[fn] = ctypes.cast(getattr(_lib(name), fn), ctypes.c_void_p).value
+        at = _addresses[fn] = ctypes.cast(getattr(lib, fn), ctypes.c_void_p).value
     return at
 
 
@@ -570,15 +570,16 @@ def _tc_plan(N: int, K: int, M: int, epi: int):
 def _fused_product(which: str, weight: torch.Tensor, act, xw, ss_in, eps: float, epilogue: str, bias, resid,
                    next_weight, status, xielu=None, glu: str = "silu"):
     """Operand checks, outputs and the call shared by :func:`linear_tc` and :func:`prompt_linear`: in one native piece
-    (csrc/calls.cpp; 57 tokens of 1,536 features, a residual product 13.7 us of the host's time, so XXX), or, for whatever that does not take as it is, here,
-    which is what says what is wrong with it."""
-    if weight.is_cuda and epilogue in _EPI and glu in _GLU:
+    (csrc/calls.cpp: 57 tokens of 1,536 features take 6.4 us of the host's time with a residual epilogue and 5.4 without, where the
+    steps below take 13.7 and 9.8), or here, for whatever that does not take as it is (and to say what is wrong with it)."""
+    lib = _lib(which)
+    if weight.is_cuda and epilogue in _EPI and glu in _GLU and type(lib) is ctypes.CDLL:
         tc = which == "linear_tc"
         fn = "vapi_linear_tc" if tc else "vapi_prompt_linear"
-        got = _calls().product(_address(which, fn), _address(which, fn + "_plan"), 0 if tc else 2, weight, act, xw, ss_in, eps,
+        got = _calls().product(_address(lib, fn), _address(lib, fn + "_plan"), 0 if tc else 2, weight, act, xw, ss_in, eps,
                                _EPI[epilogue], bias, resid, next_weight, _status(status), xielu, _GLU[glu], _stream())
         if got is not NotImplemented:
-            _check(_lib(which), got if type(got) is int else 0)
+            _check(lib, got if type(got) is int else 0)
             return got
     _cuda(weight, act, xw, ss_in, bias, resid, next_weight, xielu)
     _f32(xielu, "the activation's numbers")
@@ -600,7 +601,6 @@ def _fused_product(which: str, weight: torch.Tensor, act, xw, ss_in, eps: float,
     _f32(next_weight, "norm weight")
     if epilogue not in _EPI:
         raise KernelError(f"unknown epilogue {epilogue}")
-    lib = _lib(which)
     if which == "linear_tc":
         parts = _tc_plan(N, K, M, _EPI[epilogue])[0] if epilogue == "resid" else 0      # (only the sums of squares ask)
         fn = lib.vapi_linear_tc
@@ -1170,11 +1170,12 @@ def shortconv(h3: torch.Tensor, in_bias: Optional[torch.Tensor], taps: torch.Ten
     ``h3`` [n, 3H] = B | C | x; ``taps`` [L, H] oldest first; ``state_layer`` is a view
     [slots, L-1, H] of the per-request state (any slot stride).  Returns y [n, H].
     """
-    if h3.is_cuda:
-        got = _calls().shortconv(_address("shortconv", "vapi_shortconv"), h3, in_bias, taps, conv_bias, state_layer, state_slots, tok_seq,
-                                 cu_q, positions, _p(status), _stream())
+    lib = _lib("shortconv") if h3.is_cuda else None
+    if type(lib) is ctypes.CDLL:
+        got = _calls().shortconv(_address(lib, "vapi_shortconv"), h3, in_bias, taps, conv_bias, state_layer, state_slots, tok_seq, cu_q,
+                                 positions, _p(status), _stream())
         if got is not NotImplemented:
-            _check(_lib("shortconv"), got if type(got) is int else 0)
+            _check(lib, got if type(got) is int else 0)
             return got
     _cuda(h3, in_bias, taps, conv_bias, state_layer, state_slots, tok_seq, cu_q, positions)
     _contig(h3, "h3")
