@@ -414,7 +414,10 @@ VAPI_EXPORT int vapi_linear_tc_plan(int N, int K, int M, int epi, int* tiles, in
     const int sms = sm_count();
     if (b <= 128) {                                  // (partials must fit the stages)
         if (3 * t <= 2 * sms) {                      // too few tiles for the multiprocessors: cut K
-            s = sms / t;
+#ifndef TC_SX
+#define TC_SX 2
+#endif
+            s = TC_SX * sms / 2 / t;
             if (s > 8) s = 8;                        // portable cluster size
         } else if (t <= sms) {
             // one tile a multiprocessor and some without: two slices, both on their way at once where two blocks fit (108 tiles of 1,536 k, 32 /

@@ -488,6 +488,8 @@ TC_MAX_ROWS = int(os.environ.get("VAPI_TC_MAX_ROWS", "32"))
 STREAM_PROMPT_MAX_ROWS = 128
 #: and this many numbers in a layer's matrices (40, 65 and 59 million in the sizes above)
 STREAM_PROMPT_MAX_LAYER = 80_000_000
+#: and decode steps, captured or not, up to this many
+STREAM_DECODE_MAX_ROWS = int(os.environ.get("VAPI_STREAM_DECODE_MAX_ROWS", "64"))
 #: set False to keep products of 17..TC_MAX_ROWS rows on the library
 use_tc = os.environ.get("VAPI_TC", "1") != "0"
 
@@ -547,8 +549,9 @@ def stream_max_rows(max_q: int, layer: int) -> int:
     model with ``layer`` numbers in the matrices of a layer."""
     if not use_tc:
         return SKINNY_MAX_ROWS
-    decode_only = max_q <= 1 or layer > STREAM_PROMPT_MAX_LAYER or TC_MAX_ROWS <= SKINNY_MAX_ROWS
-    return TC_MAX_ROWS if decode_only else max(TC_MAX_ROWS, STREAM_PROMPT_MAX_ROWS)
+    if layer > STREAM_PROMPT_MAX_LAYER or TC_MAX_ROWS <= SKINNY_MAX_ROWS:
+        return TC_MAX_ROWS
+    return max(TC_MAX_ROWS, STREAM_DECODE_MAX_ROWS if max_q <= 1 else STREAM_PROMPT_MAX_ROWS)
 
 
 def tc_applies(rows: int, weight: torch.Tensor, most: Optional[int] = None) -> bool:
