@@ -293,44 +293,13 @@ static int launch_attention(const void* q, long long q_row_stride, const void* c
 static int g_decode_kernel = 1;
 VAPI_EXPORT void vapi_attention_use_decode_kernel(int on) { g_decode_kernel = on != 0; }
 
-// A stream beside the caller's, for the decode tokens of a step with a large portion, and the events that fork it and join it again: one set
-// a thread and device, made at its first use and given back when the thread ends.
-struct SidePath {
-    cudaStream_t stream = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-    bool tried = false;
-    ~SidePath() {
-        if (join) cudaEventDestroy(join);
-        if (fork) cudaEventDestroy(fork);
-        if (stream) cudaStreamDestroy(stream);
-    }
-};
-static SidePath* side_path() {
-    static thread_local SidePath paths[16];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return nullptr;
-    SidePath& s = paths[dev];
-    if (!s.tried) {
-        s.tried = true;
-        if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess) s.stream = nullptr;
-        if (cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) != cudaSuccess) s.fork = nullptr;
-        if (cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) != cudaSuccess) s.join = nullptr;
-        cudaGetLastError();
-    }
-    return s.stream && s.fork && s.join ? &s : nullptr;
-}
-#ifndef SIDE_MIN_ROWS
-#define SIDE_MIN_ROWS 512
-#endif
-
-// beside: the kernels for the short sequences of a step with a portion may run on a stream of the library's own beside the portion's.
-static int paged_attention(const void* q, long long q_row_stride, const void* cache,
-                           int dtype, const int* block_table, int table_stride,
-                           const int* cu_q, const int* seqlens_k, void* out,
-                           float* part_o, float* part_ml, int n, int num_seqs,
-                           int max_q, int nh, int nkv, int d, int page_size,
-                           int num_pages, float scale, int window, int splits,
-                           int impl, int* status, cudaStream_t stream, bool beside) {
+VAPI_EXPORT int vapi_paged_attention(const void* q, long long q_row_stride, const void* cache,
+                                     int dtype, const int* block_table, int table_stride,
+                                     const int* cu_q, const int* seqlens_k, void* out,
+                                     float* part_o, float* part_ml, int n, int num_seqs,
+                                     int max_q, int nh, int nkv, int d, int page_size,
+                                     int num_pages, float scale, int window, int splits,
+                                     int impl, int* status, cudaStream_t stream) {
     if (n <= 0 || num_seqs <= 0 || max_q <= 0) return 0;
     if (d < 16 || d > 256 || d % 16 != 0)
         return fail(-1, "paged_attention: head_dim %d is not a multiple of 16 in 16..256", d);
@@ -358,34 +327,18 @@ static int paged_attention(const void* q, long long q_row_stride, const void* ca
         // prompt portions on tcgen05; in a mixed step the short sequences (decode tokens) go to the
         // flash kernel, whose small blocks suit them: each kernel skips the other's sequences
         const int min_q = (impl == 3 || num_seqs == 1) ? 1 : FT_MIN_Q;
+        rc = launch_flash_tc(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, n, num_seqs, max_q,
+                             nh, nkv, page_size, num_pages, scale, window, min_q, status, stream);
+        if (rc != 0 || min_q == 1) return rc;
         // (of the shorter ones, those of at most 16 rows - decode tokens, whose contexts can be long -
         // go to the decode kernel, which puts four warps on their keys where the flash kernel has one)
-        const bool dec_too = min_q > 1 && g_decode_kernel && nh / nkv <= FD_MAX_ROWS && ((uintptr_t)out & 15) == 0;
-        // The portion's kernel computes and the decode tokens' kernel reads memory, and neither fills the device: they run beside each
-        // other where the step is large enough to be bound by its kernels and not by the host, which pays some 4 us for the events.
-        SidePath* side = dec_too && beside && n >= SIDE_MIN_ROWS ? side_path() : nullptr;
-        if (side && (cudaEventRecord(side->fork, stream) != cudaSuccess || cudaStreamWaitEvent(side->stream, side->fork, 0) != cudaSuccess))
-            return check_launch("paged_attention: fork", cudaGetLastError());
-        const cudaStream_t other = side ? side->stream : stream;
-        auto portions = [&]() {
-            return launch_flash_tc(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, n, num_seqs, max_q,
-                                   nh, nkv, page_size, num_pages, scale, window, min_q, status, stream);
-        };
-        auto shorter = [&]() {
-            const int r = launch_flash<64, 4, 3>(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, part_o,
-                                                 part_ml, num_seqs, FT_MIN_Q - 1, nh, nkv, page_size, num_pages, scale, window, 1,
-                                                 status, other, FT_MIN_Q, dec_too ? FD_MAX_ROWS : 0);
-            if (r != 0 || !dec_too) return r;
-            return launch_flash_decode(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, part_o, part_ml,
-                                       num_seqs, nh, nkv, page_size, num_pages, scale, window, 1, status, other);
-        };
-        rc = portions();
-        if (rc == 0 && min_q > 1) rc = shorter();
-        if (side) {                                   // (joined whatever came of it)
-            const cudaError_t a = cudaEventRecord(side->join, side->stream), b = cudaStreamWaitEvent(stream, side->join, 0);
-            if (rc == 0 && (a != cudaSuccess || b != cudaSuccess)) rc = check_launch("paged_attention: join", a != cudaSuccess ? a : b);
-        }
-        return rc;
+        const bool dec_too = g_decode_kernel && nh / nkv <= FD_MAX_ROWS && ((uintptr_t)out & 15) == 0;
+        rc = launch_flash<64, 4, 3>(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, part_o,
+                                    part_ml, num_seqs, FT_MIN_Q - 1, nh, nkv, page_size, num_pages, scale, window, 1,
+                                    status, stream, FT_MIN_Q, dec_too ? FD_MAX_ROWS : 0);
+        if (rc != 0 || !dec_too) return rc;
+        return launch_flash_decode(q, q_row_stride, cache, block_table, table_stride, cu_q, seqlens_k, out, part_o, part_ml,
+                                   num_seqs, nh, nkv, page_size, num_pages, scale, window, 1, status, stream);
     }
 #define VAPI_FLASH(HD, NW, ST)                                                                   \
     rc = launch_flash<HD, NW, ST>(q, q_row_stride, cache, block_table, table_stride, cu_q,       \
@@ -450,17 +403,6 @@ static int paged_attention(const void* q, long long q_row_stride, const void* ca
         return check_launch("attention_combine", e);
     }
     return 0;
-}
-
-VAPI_EXPORT int vapi_paged_attention(const void* q, long long q_row_stride, const void* cache,
-                                     int dtype, const int* block_table, int table_stride,
-                                     const int* cu_q, const int* seqlens_k, void* out,
-                                     float* part_o, float* part_ml, int n, int num_seqs,
-                                     int max_q, int nh, int nkv, int d, int page_size,
-                                     int num_pages, float scale, int window, int splits,
-                                     int impl, int* status, cudaStream_t stream) {
-    return paged_attention(q, q_row_stride, cache, dtype, block_table, table_stride, cu_q, seqlens_k, out, part_o, part_ml, n, num_seqs,
-                           max_q, nh, nkv, d, page_size, num_pages, scale, window, splits, impl, status, stream, true);
 }
 
 // How many blocks of the decode kernel the device holds at once (0: unknown), and the largest
@@ -551,9 +493,9 @@ VAPI_EXPORT int vapi_paged_attention_noalloc(const void* q, long long q_row_stri
         part_o = noalloc_scratch_addr[dev];
         part_ml = part_o + rows * d;                       // rows * d is a multiple of 16 floats: stays aligned
     }
-    return paged_attention(q, q_row_stride, cache, dtype, block_table, table_stride, cu_q, seqlens_k, out,
+    return vapi_paged_attention(q, q_row_stride, cache, dtype, block_table, table_stride, cu_q, seqlens_k, out,
                                 part_o, part_ml, n, num_seqs, max_q, nh, nkv, d, page_size, num_pages, scale,
-                                window, splits, impl, status, stream, false);
+                                window, splits, impl, status, stream);
 }
 
 VAPI_EXPORT const char* vapi_last_error() { return error_buffer(); }

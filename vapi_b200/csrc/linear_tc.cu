@@ -412,19 +412,13 @@ VAPI_EXPORT int vapi_linear_tc_plan(int N, int K, int M, int epi, int* tiles, in
     const int num_kb = (K + TC_BK - 1) / TC_BK;
     int s = 1;
     const int sms = sm_count();
-    if (b <= 128) {                                  // (partials must fit the stages)
-        if (3 * t <= 2 * sms) {                      // too few tiles for the multiprocessors: cut K
-#ifndef TC_SX
-#define TC_SX 2
+#ifndef TC_RULE
+#define TC_RULE 1
 #endif
-            s = TC_SX * sms / 2 / t;
-            if (s > 8) s = 8;                        // portable cluster size
-        } else if (t <= sms) {
-            // one tile a multiprocessor and some without: two slices, both on their way at once where two blocks fit (108 tiles of 1,536 k, 32 /
-            // 64 tokens 14.1 / 16.5 us, so 12.4 / 14.5; 112 of 2,048 17.2 / 19.6, so 15.6 / 17.7.  Two slices a multiprocessor for fewer tiles
-            // too, six where three fill the device: 48 tiles of 2,048 k 10.4 / 11.6 us, so 13.9 / 17.0)
-            s = 2;
-        }
+    if (b <= 128 && (TC_RULE ? t <= sms : 3 * t <= 2 * sms)) {       // (partials must fit the stages)
+        s = sms / t;
+        if (TC_RULE) { const int two = 2 * sms / t < 4 ? 2 * sms / t : 4; s = s > two ? s : two; }
+        if (s > 8) s = 8;                            // portable cluster size
         const int max_s = num_kb / 2 > 0 ? num_kb / 2 : 1;      // at least 2 k-blocks a slice
         if (s > max_s) s = max_s;
         if (s < 1) s = 1;
