@@ -1070,6 +1070,22 @@ def test_prompt_linear_plain_products(ops, prompt_tiles, M, N, K):
     assert int(st.item()) == 0
 
 
+# slices of K by the number of tiles: four and fewer up to two blocks a multiprocessor (64 and 65 tiles), two (98 to 148), one (149); a K of
+# few pieces, which cannot be cut so often
+@pytest.mark.parametrize("tiles,K", [(37, 512), (49, 512), (64, 520), (65, 512), (87, 384), (98, 512), (148, 512), (149, 512), (64, 128), (100, 192)])
+def test_linear_tc_cuts_k_for_any_number_of_tiles(ops, tiles, K):
+    g = torch.Generator(device="cuda").manual_seed(tiles)
+    N = tiles * 128 - 5
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    w, b = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16), torch.randn(N, generator=g, device="cuda")
+    for M in (17, 64, 128, 129):
+        x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+        got = ops.linear_tc(w, act=x, epilogue="f32", bias=b, status=st)
+        # (products of bfloat16 are exact in float32: what is left are K roundings of partial sums below sqrt(K) * 6)
+        torch.testing.assert_close(got.double(), x.double() @ w.double().t() + b.double(), atol=K * 2.0 ** -24 * 6 * K ** 0.5, rtol=0)
+    assert int(st.item()) == 0
+
+
 @pytest.mark.parametrize("M", [35, 260])
 def test_prompt_linear_rows_that_are_not_16_byte_aligned(ops, prompt_tiles, M):
     """Output rows whose pitch is no multiple of 8 elements take the value-by-value ends of the

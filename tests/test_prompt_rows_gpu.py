@@ -95,3 +95,32 @@ def test_captured_float32_decode_on_the_split_product(tmp_path):
     span = float(want.max() - want.min())
     # (bound: three layers and the head of float32 sums of at most 6,912 terms, some 1e-6 of what they add up)
     assert float((rows[True] - want).abs().max()) < 3e-5 * span and float((rows[False] - want).abs().max()) < 3e-5 * span
+
+
+@pytest.mark.parametrize("S", [33, 47, 64])
+def test_decode_steps_of_33_to_64_requests_in_the_stream_form(tmp_path, S):
+    """The bucket of 64 rows, captured, and the step as it is, eager (33 and 47 rows of a tile of 64 tokens): both run the blocks' stream
+    form, and the logits are the plain model's within bfloat16 rounding."""
+    from vapi_b200.engine.runner import ModelRunner
+    from vapi_b200.engine.step import StepEntry
+    d, plain, cfg = _model(tmp_path, "700m", 7, torch.bfloat16)
+    prompts = [_tokens(3 + (5 * i) % 23, 400 + i, cfg["vocab_size"]) for i in range(S)]
+    for graphs in (True, False):
+        r = ModelRunner.from_dir(d, dtype="bfloat16", num_pages=160, max_requests=64, max_batched_tokens=1024, max_context=128)
+        r._graphs_off = not graphs
+        seen, real = [], r._forward_few_rows
+        r._forward_few_rows = lambda ctx, views: (seen.append((ctx.n, ctx.max_q)), real(ctx, views))[1]
+        rcs = [r.cache.open(i) for i in range(S)]
+        for rc, p in zip(rcs, prompts):
+            assert r.cache.reserve(rc, len(p) + 2)
+        for i in range(0, S, 16):
+            r.step([StepEntry(rc, p, []) for rc, p in zip(rcs[i:i + 16], prompts[i:i + 16])])
+        del seen[:]
+        for at in range(2):
+            entries = [StepEntry(rc, [200 + at], [0]) for rc in rcs]
+            logits = r.step_decode_graph(entries) if graphs else r.step(entries)
+        assert seen and set(seen) == {(64 if graphs else S, 1)}
+        for i in (0, S // 2, S - 1):
+            want = plain.logits(prompts[i] + [200, 201])[-1]
+            assert float((logits[i].float().cpu() - want).abs().max()) < 0.02 * float(want.max() - want.min())
+        r.check_status()

@@ -412,12 +412,16 @@ VAPI_EXPORT int vapi_linear_tc_plan(int N, int K, int M, int epi, int* tiles, in
     const int num_kb = (K + TC_BK - 1) / TC_BK;
     int s = 1;
     const int sms = sm_count();
-#ifndef TC_RULE
-#define TC_RULE 1
-#endif
-    if (b <= 128 && (TC_RULE ? t <= sms : 3 * t <= 2 * sms)) {       // (partials must fit the stages)
+    if (b <= 128 && t <= sms) {                      // (partials must fit the stages)
+        // Too few tiles for the multiprocessors: K is cut until they are one block each, or up to four slices as far as two blocks a
+        // multiprocessor go, and both stream at once.  19 / 64 / 128 tokens, K = 2,048, one slice or as many as make one block, and then two:
+        // 48 tiles 9.0 / 11.4 / 15.7 us, so 8.7 / 10.5 / 13.9; 64 tiles 11.6 / 13.9 / 19.4, so 9.6 / 11.6 / 14.7; 80 tiles 15.3 / 19.0 / 27.0, so
+        // 10.9 / 13.5 / 17.4; 128 tiles 17.7 / 21.3 / 29.7, so 16.6 / 19.3 / 24.5.  Not more than that: six slices of 48 tiles 13.0 / 17.0 us at
+        // 19 / 64 (clusters that do not all find room at once), and three of 98 tiles 17.9 / 22.8, where two fill seven eighths of the places.
         s = sms / t;
-        if (TC_RULE) { const int two = 2 * sms / t < 4 ? 2 * sms / t : 4; s = s > two ? s : two; }
+        int two = 2 * sms / t < 4 ? 2 * sms / t : 4;
+        while (two > 2 && 4 * two * t > 7 * sms) --two;
+        if (s < two) s = two;
         if (s > 8) s = 8;                            // portable cluster size
         const int max_s = num_kb / 2 > 0 ? num_kb / 2 : 1;      // at least 2 k-blocks a slice
         if (s > max_s) s = max_s;

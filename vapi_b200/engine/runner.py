@@ -197,7 +197,8 @@ class ModelRunner:
             ctx.pos[pe.name] = pe.prepare(ctx)
         views = self.views(ctx)
         ctx.fused = (self._stream_form and self.device.type == "cuda" and self.dtype == torch.bfloat16 and ops.use_skinny
-                     and (ctx.n <= ops.stream_max_rows(ctx.max_q, self._layer_numbers) or 0 < ops.PROMPT_MIN_ROWS <= ctx.n))
+                     and (ctx.n <= ops.stream_max_rows(ctx.max_q, self._layer_numbers) or 0 < ops.PROMPT_MIN_ROWS <= ctx.n
+                          or (ctx.max_q <= 1 and ops.stream_decodes(ctx.n, self._layer_numbers))))
         if ctx.fused:
             return self._forward_few_rows(ctx, views)
         x = self._embed(ctx)

@@ -473,7 +473,8 @@ def skinny_linear(weight: torch.Tensor, *, act: Optional[torch.Tensor] = None,
 #: itself takes up to 256 rows, but it has one tile per block and pays its fixed costs (cluster
 #: reduction, epilogue) per launch: measured in the captured decode step of LFM2-1.2B sizes it
 #: beats the library's product plus separate norm / SwiGLU / add kernels at 32 rows (1.26 vs 1.33
-#: ms), loses narrowly at 64 (1.71 vs 1.68 ms) and clearly beyond (2-7x slower at 256 rows).
+#: ms) and, in the stream form of a decode step (STREAM_DECODE_MAX_ROWS), at 64; a product alone loses beyond 32 rows, and clearly so
+#: beyond 64 (2-7x slower at 256 rows).
 TC_MAX_ROWS = int(os.environ.get("VAPI_TC_MAX_ROWS", "32"))
 #: steps with a prompt portion run the stream form of their blocks (norms, SwiGLU and residual adds inside the products; LFM2's blocks have
 #: one) up to this many rows.  They are launched one by one, and what bounds them is the launches, of which this form has 81 where the other
@@ -483,12 +484,13 @@ TC_MAX_ROWS = int(os.environ.get("VAPI_TC_MAX_ROWS", "32"))
 #: 3.40 / 2.00; 60 decoding requests beside a portion of 60 1.92 / 1.61, 1.94 / 1.83, 3.20 / 3.15 against 2.16 / 1.21, 2.14 / 1.38, 3.62 / 2.28.  So
 #: it pays as far as the host is what a step waits for, and from about 50 rows on only that far: with weights much wider than these the
 #: device's share is what counts, and the other form is ahead.  From 129 rows on a product's tokens no longer fit beside a share of K (200
-#: tokens of the 700M size: 1.98 -> 4.37 ms), and captured decode steps, which cost no launches, stay with TC_MAX_ROWS (2.6B, 64
-#: requests: 1.93 ms a step on the library, 2.08 ms in this form).
+#: tokens of the 700M size: 1.98 -> 4.37 ms).  (Measured before the products' way from the partial sums to the output was shortened.)
 STREAM_PROMPT_MAX_ROWS = 128
 #: and this many numbers in a layer's matrices (40, 65 and 59 million in the sizes above)
 STREAM_PROMPT_MAX_LAYER = 80_000_000
-#: and decode steps, captured or not, up to this many
+#: Decode steps of such models run it up to this many rows, although a product alone is the library's above TC_MAX_ROWS (64 rows: 6,144 x 2,048 10.5
+#: against 7.1 us, the gate's with SwiGLU 17.7 against 12.2 + 2.4): what it saves are the norms, adds and gates between them.  Captured, four steps of 64
+#: requests of 128 to 2,048 tokens on the 2.6B size 7,756 us in the other form, 7,407 in this one.
 STREAM_DECODE_MAX_ROWS = int(os.environ.get("VAPI_STREAM_DECODE_MAX_ROWS", "64"))
 #: set False to keep products of 17..TC_MAX_ROWS rows on the library
 use_tc = os.environ.get("VAPI_TC", "1") != "0"
@@ -549,9 +551,13 @@ def stream_max_rows(max_q: int, layer: int) -> int:
     model with ``layer`` numbers in the matrices of a layer."""
     if not use_tc:
         return SKINNY_MAX_ROWS
-    if layer > STREAM_PROMPT_MAX_LAYER or TC_MAX_ROWS <= SKINNY_MAX_ROWS:
-        return TC_MAX_ROWS
-    return max(TC_MAX_ROWS, STREAM_DECODE_MAX_ROWS if max_q <= 1 else STREAM_PROMPT_MAX_ROWS)
+    decode_only = max_q <= 1 or layer > STREAM_PROMPT_MAX_LAYER or TC_MAX_ROWS <= SKINNY_MAX_ROWS
+    return TC_MAX_ROWS if decode_only else max(TC_MAX_ROWS, STREAM_PROMPT_MAX_ROWS)
+
+
+def stream_decodes(rows: int, layer: int) -> bool:
+    """Whether a decode step of more than TC_MAX_ROWS rows runs the stream form of its blocks too."""
+    return use_tc and SKINNY_MAX_ROWS < TC_MAX_ROWS < rows <= STREAM_DECODE_MAX_ROWS and layer <= STREAM_PROMPT_MAX_LAYER
 
 
 def tc_applies(rows: int, weight: torch.Tensor, most: Optional[int] = None) -> bool:
