@@ -549,16 +549,15 @@ VAPI_EXPORT int vapi_prompt_linear(const void* W, int N, int K, int M, int pro, 
     p.resid = resid; p.ss_out = ss_out; p.next_w = next_w; p.xw_out = (__nv_bfloat16*)xw_out;
     p.status = status; p.xielu = xielu_consts; p.glu = glu;
     const bool half_rows = epi == PL_EPI_SWIGLU || pair == 2;      // boxes of BN/2 weight rows
-    const CUtensorMap *ta, *tw;
-    int rc = kmajor_map(&tw, "prompt_linear", W, N, K, half_rows ? bn / 2 : bn, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    CUtensorMap ta, tw;
+    int rc = kmajor_map(&ta, "prompt_linear", tokens, M, K, PL_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, true);
     if (rc) return rc;
-    const CUtensorMap weights = *tw;                               // (the second call may empty the store)
-    rc = kmajor_map(&ta, "prompt_linear", tokens, M, K, PL_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    rc = kmajor_map(&tw, "prompt_linear", W, N, K, half_rows ? bn / 2 : bn, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, true);
     if (rc) return rc;
-    if (bn == 256 && pair == 2) return launch_pl<256, 2>(*ta, weights, p, stream);
-    if (bn == 128 && pair == 2) return launch_pl<128, 2>(*ta, weights, p, stream);
-    if (bn == 256 && pair == 1) return launch_pl<256, 1>(*ta, weights, p, stream);
-    if (bn == 128 && pair == 1) return launch_pl<128, 1>(*ta, weights, p, stream);
+    if (bn == 256 && pair == 2) return launch_pl<256, 2>(ta, tw, p, stream);
+    if (bn == 128 && pair == 2) return launch_pl<128, 2>(ta, tw, p, stream);
+    if (bn == 256 && pair == 1) return launch_pl<256, 1>(ta, tw, p, stream);
+    if (bn == 128 && pair == 1) return launch_pl<128, 1>(ta, tw, p, stream);
     return fail(-2, "prompt_linear: no kernel for tiles of %d features and %d blocks", bn, pair);
 }
 

@@ -458,17 +458,16 @@ VAPI_EXPORT int vapi_linear_tc(const void* W, int N, int K, int M, int pro, cons
     p.out_bf16 = (__nv_bfloat16*)out_bf16; p.out_f32 = out_f32; p.out_stride = out_stride; p.bias = bias;
     p.resid = resid; p.ss_out = ss_out; p.next_w = next_w; p.xw_out = (__nv_bfloat16*)xw_out;
     p.status = status; p.xielu = xielu_consts; p.glu = glu;
-    const CUtensorMap *tw, *ta;
-    int rc = kmajor_map(&tw, "linear_tc", W, N, K, epi == TC_EPI_SWIGLU ? 64 : TC_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    CUtensorMap tw, ta;
+    int rc = kmajor_map(&tw, "linear_tc", W, N, K, epi == TC_EPI_SWIGLU ? 64 : TC_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, true);
     if (rc) return rc;
-    const CUtensorMap weights = *tw;                               // (the second call may empty the store)
-    rc = kmajor_map(&ta, "linear_tc", tokens, M, K, bn, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    rc = kmajor_map(&ta, "linear_tc", tokens, M, K, bn, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, false);
     if (rc) return rc;
     switch (bn) {
-        case 32: return launch_tc<32>(weights, *ta, p, tiles, stream);
-        case 64: return launch_tc<64>(weights, *ta, p, tiles, stream);
-        case 128: return launch_tc<128>(weights, *ta, p, tiles, stream);
-        case 256: return launch_tc<256>(weights, *ta, p, tiles, stream);
+        case 32: return launch_tc<32>(tw, ta, p, tiles, stream);
+        case 64: return launch_tc<64>(tw, ta, p, tiles, stream);
+        case 128: return launch_tc<128>(tw, ta, p, tiles, stream);
+        case 256: return launch_tc<256>(tw, ta, p, tiles, stream);
     }
     return fail(-2, "linear_tc: no kernel for %d tokens", bn);
 }

@@ -151,12 +151,11 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// A [rows][K] bfloat16 matrix, K contiguous, tiled in boxes of 64 k x box_rows rows, 128-byte swizzle.  A map is a function of address,
-// shape and box alone; it is encoded once for each of these and thread (weights keep their address, and so, by and large, do the
-// activations that a step's allocator hands out): the driver's encoder takes about a microsecond, and a step of a few tokens is bound by
-// what its launches cost the host.
-static int kmajor_map(const CUtensorMap** out, const char* what, const void* ptr, long long rows, long long K, int box_rows,
-                      CUtensorMapL2promotion promotion) {
+// A [rows][K] bfloat16 matrix, K contiguous, tiled in boxes of 64 k x box_rows rows, 128-byte swizzle.  keep: the map, a function of address,
+// shape and box alone, is encoded once for each of these and thread, and not at every call (weights; the driver's encoder takes about
+// a microsecond, and a step of a few tokens is bound by what its launches cost the host).
+static int kmajor_map(CUtensorMap* out, const char* what, const void* ptr, long long rows, long long K, int box_rows,
+                      CUtensorMapL2promotion promotion, bool keep) {
     struct Key {
         const void* p; long long r, k; int b;
         bool operator==(const Key& o) const { return p == o.p && r == o.r && k == o.k && b == o.b; }
@@ -166,10 +165,12 @@ static int kmajor_map(const CUtensorMap** out, const char* what, const void* ptr
             return std::hash<const void*>()(k.p) ^ (std::hash<long long>()(k.r) * 31) ^ (std::hash<long long>()(k.k) * 131) ^ (size_t)k.b;
         }
     };
-    static thread_local std::unordered_map<Key, CUtensorMap, Hash> cache;
+    static thread_local std::unordered_map<Key, CUtensorMap, Hash> kept;
     const Key key{ptr, rows, K, box_rows};
-    auto it = cache.find(key);
-    if (it != cache.end()) { *out = &it->second; return 0; }
+    if (keep) {
+        const auto it = kept.find(key);
+        if (it != kept.end()) { *out = it->second; return 0; }
+    }
     EncodeTiledFn fn = encode_fn();
     if (!fn) return fail(-102, "%s: cuTensorMapEncodeTiled is not available from the driver", what);
     if (((uintptr_t)ptr & 15) != 0 || (K * 2) % 16 != 0)
@@ -178,12 +179,13 @@ static int kmajor_map(const CUtensorMap** out, const char* what, const void* ptr
     cuuint64_t strides[1] = {(cuuint64_t)K * 2};
     cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUtensorMap map;
-    CUresult r = fn(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(-103, "%s: cuTensorMapEncodeTiled failed with %d", what, (int)r);
-    if (cache.size() > 4096) cache.clear();
-    *out = &cache.emplace(key, map).first->second;
+    if (keep) {
+        if (kept.size() > 4096) kept.clear();
+        kept.emplace(key, *out);
+    }
     return 0;
 }
 
