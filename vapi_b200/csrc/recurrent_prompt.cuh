@@ -11,7 +11,8 @@
 // 2,000 tokens, 128 rows, one sequence, bfloat16: delta rule (16 heads of 128 columns) 655 us in gated_delta_kernel, 317
 // here; state space (64 heads of 64 columns) 726 us in state_space_kernel, 250 here.  Measured beside it: two columns a
 // thread for the delta rule (half the warps) 373 us; one column a thread for the state space 303 to 380 us; one block an SM
-// (more registers) within 2 % for one sequence, but 244 against 191 us for five of 300 tokens.
+// (more registers) within 2 % for one sequence, but 244 against 191 us for five of 300 tokens; the read-out by four more warps that
+// follow with a state of their own 303 against 289 us (captured): what is left is the chain itself.
 #pragma once
 #include "common.cuh"
 
