@@ -887,8 +887,13 @@ __global__ void postnorm_add_rmsnorm_vec_kernel(float* __restrict__ x, const T* 
     const T* yr = y ? y + (size_t)row * hidden : nullptr;
     const T* y2r = (y && y2) ? y2 + (size_t)row * hidden : nullptr;
     const int h4 = hidden >> 2;
-    float4 v[NORM_KMAX];
+    float4 v[NORM_KMAX], xq[NORM_KMAX];          // (the stream's row is on its way while the output's norm is worked out)
     float ssy = 0.f;
+#pragma unroll
+    for (int k = 0; k < NORM_KMAX; ++k) {
+        const int c = threadIdx.x + k * blockDim.x;
+        xq[k] = c < h4 ? Pack4<float>::load(xr + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     if (y2r) {                                   // two raw branches: their norms and their mean come first
         float4 u[NORM_KMAX];
         float sa = 0.f, sb = 0.f;
@@ -936,7 +941,7 @@ __global__ void postnorm_add_rmsnorm_vec_kernel(float* __restrict__ x, const T* 
     for (int k = 0; k < NORM_KMAX; ++k) {
         const int c = threadIdx.x + k * blockDim.x;
         if (c < h4) {
-            const float4 xv = Pack4<float>::load(xr + 4 * c);
+            const float4 xv = xq[k];
             if (yr) {
                 const float4 wp = Pack4<float>::load(w_post + 4 * c);
                 v[k].x = xv.x + mult * (v[k].x * inv_y * wp.x);
@@ -1093,6 +1098,51 @@ __global__ void gated_group_rmsnorm_kernel(const float* __restrict__ y, const T*
     }
 }
 
+// The same for groups of 32 PER columns: a lane's PER columns are asked for together and stay in registers, where the kernel above reads
+// y and z twice, column after column, and divides 64-bit numbers.  The sums in the same order.
+template <typename T, int PER>
+__global__ void __launch_bounds__(256)
+gated_group_rmsnorm_lane_kernel(const float* __restrict__ y, const T* __restrict__ z, long long z_stride, const float* __restrict__ w,
+                                int w_len, float eps, int gate_first, T* __restrict__ out, int items, int width,
+                                long long out_stride) {
+    constexpr int GROUP = 32 * PER;
+    const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    pdl_trigger();
+    const int groups = width / GROUP;
+    const int sig = gate_first & 2;
+    gate_first &= 1;
+    if (item >= items) {
+        pdl_wait();
+        return;
+    }
+    const int t = item / groups, g = item - t * groups;
+    const float* yr = y + (size_t)t * width + (size_t)g * GROUP + lane;
+    const T* zr = z + (size_t)t * z_stride + (size_t)g * GROUP + lane;
+    const float* wr = w + (g * GROUP) % w_len + lane;
+    float wv[PER], yv[PER], gate[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) wv[k] = wr[32 * k];
+    pdl_wait();
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        yv[k] = yr[32 * k];
+        gate[k] = to_f32(zr[32 * k]);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        gate[k] = norm_gate(gate[k], sig);
+        if (gate_first) yv[k] *= gate[k];
+        ss += yv[k] * yv[k];
+    }
+    ss = warp_sum(ss);
+    const float inv = rsqrtf(ss / (float)GROUP + eps);
+    T* orow = out + (size_t)t * out_stride + (size_t)g * GROUP + lane;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) orow[32 * k] = from_f32<T>(gate_first ? yv[k] * inv * wv[k] : yv[k] * inv * wv[k] * gate[k]);
+}
+
 // The same for wide groups (a whole row of a few thousand columns is one group): a block per (row, group).
 template <typename T>
 __global__ void gated_group_rmsnorm_wide_kernel(const float* __restrict__ y, const T* __restrict__ z, long long z_stride,
@@ -1203,6 +1253,17 @@ VAPI_EXPORT int vapi_gated_group_rmsnorm(const float* y, const void* z, long lon
         else
             e = launch(gated_group_rmsnorm_wide_kernel<__nv_bfloat16>, (int)items, threads, 0, stream, y, (const __nv_bfloat16*)z,
                        z_stride, w, w_len, eps, gate_first, (__nv_bfloat16*)out, n, width, group, out_stride);
+        return check_launch("gated_group_rmsnorm", e);
+    }
+    // (heads of these sizes, one weight for all heads or one for each column)
+    if ((group == 64 || group == 128 || group == 256) && w_len % group == 0 && items <= 0x7fffffffLL - 8 && (dtype == VAPI_F32 || dtype == VAPI_BF16)) {
+        const int lane_blocks = (int)((items + 7) / 8);
+#define GG_LANE(T, PER)                                                                                                       \
+    launch(gated_group_rmsnorm_lane_kernel<T, PER>, lane_blocks, 256, 0, stream, y, (const T*)z, z_stride, w, w_len, eps,     \
+           gate_first, (T*)out, (int)items, width, out_stride)
+        if (dtype == VAPI_F32) e = group == 64 ? GG_LANE(float, 2) : (group == 128 ? GG_LANE(float, 4) : GG_LANE(float, 8));
+        else e = group == 64 ? GG_LANE(__nv_bfloat16, 2) : (group == 128 ? GG_LANE(__nv_bfloat16, 4) : GG_LANE(__nv_bfloat16, 8));
+#undef GG_LANE
         return check_launch("gated_group_rmsnorm", e);
     }
     if (dtype == VAPI_F32)

@@ -391,6 +391,77 @@ __global__ void qk_norm_rope_write_split_kernel(T* __restrict__ qkv, long long r
     }
 }
 
+// The same for heads of 64: a lane has the elements `lane` and `lane + 32` in registers, and an element's partner in the rotation is
+// the neighbouring lane's (interleaved pairs) or its own other one (halves of 32), so nothing goes through shared memory, and a
+// warp's loads are all on their way at once.
+template <typename T>
+__global__ void __launch_bounds__(256)
+qk_norm_rope_write_split64_kernel(T* __restrict__ qkv, long long row_stride, const float* __restrict__ qw,
+                                  const float* __restrict__ kw, float eps, const float* __restrict__ cosr,
+                                  const float* __restrict__ sinr, int rot, int interleaved, T* __restrict__ cache,
+                                  const int* __restrict__ slot_mapping, int n, int nh, int nkv, int page_size, int num_pages,
+                                  int* __restrict__ status, const int* __restrict__ positions, float qt_coef, int qt_every) {
+    constexpr int D = 64;
+    const int lane = threadIdx.x & 31, heads = nh + 2 * nkv;
+    const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    pdl_trigger();
+    if (item >= n * heads) {
+        pdl_wait();
+        return;
+    }
+    const int t = item / heads, h = item - t * heads;
+    const int slot = (cache && h >= nh) ? slot_mapping[t] : 0;
+    const bool is_q = h < nh, is_k = !is_q && h < nh + nkv;
+    const float* w = is_q ? qw : (is_k ? kw : nullptr);
+    const bool rope = (is_q || is_k) && cosr != nullptr;
+    // a query temperature: q at position p is multiplied by 1 + coef * ln(floor((p + 1) / every) + 1)
+    const float q_mult = (is_q && qt_every > 0) ? 1.f + qt_coef * logf((float)((positions[t] + 1) / qt_every + 1)) : 1.f;
+    const float w0 = w ? w[lane] : 1.f, w1 = w ? w[lane + 32] : 1.f;
+    pdl_wait();
+    T* src = qkv + (size_t)t * row_stride + (size_t)h * D;
+    float v0 = to_f32(src[lane]), v1 = to_f32(src[lane + 32]);
+    const int half = rot >> 1;
+    // of element i: the pair's index, and whether it is the first of its pair
+    const int j0 = interleaved ? lane >> 1 : lane, j1 = interleaved ? (lane + 32) >> 1 : lane;
+    const bool r0 = rope && lane < rot, r1 = rope && lane + 32 < rot;
+    float c0 = 1.f, s0 = 0.f, c1 = 1.f, s1 = 0.f;
+    if (r0) { c0 = cosr[(size_t)t * half + j0]; s0 = sinr[(size_t)t * half + j0]; }
+    if (r1) { c1 = cosr[(size_t)t * half + j1]; s1 = sinr[(size_t)t * half + j1]; }
+    T* dst = nullptr;
+    if (is_q) {
+        if (!w && !rope && q_mult == 1.f) return;      // nothing changes a query that is neither normed, rotated nor scaled
+        dst = src;
+    } else if (cache) {
+        const int page = slot / page_size, off = slot - page * page_size;
+        if (slot < 0 || page >= num_pages) {
+            if (lane == 0 && status) atomicExch(status, 2);
+            return;
+        }
+        const size_t page_elems = (size_t)nkv * page_size * (2 * D);
+        dst = is_k ? cache + (size_t)page * page_elems + ((size_t)(h - nh) * page_size + off) * D
+                   : cache + (size_t)page * page_elems + (size_t)nkv * page_size * D + ((size_t)(h - nh - nkv) * page_size + off) * D;
+    }
+    if (!dst) return;
+    if (w) {
+        float ss = 0.f;
+        ss += v0 * v0;
+        ss += v1 * v1;
+        ss = warp_sum(ss);
+        const float inv = rsqrtf(ss / (float)D + eps);
+        v0 = v0 * inv * w0;
+        v1 = v1 * inv * w1;
+    }
+    if (rope) {                                        // (the same for the whole warp)
+        const float p0 = interleaved ? __shfl_xor_sync(0xffffffffu, v0, 1) : v1, p1 = interleaved ? __shfl_xor_sync(0xffffffffu, v1, 1) : v0;
+        const bool first0 = interleaved ? (lane & 1) == 0 : true, first1 = interleaved ? (lane & 1) == 0 : false;
+        const float a0 = first0 ? v0 * c0 - p0 * s0 : v0 * c0 + p0 * s0, a1 = first1 ? v1 * c1 - p1 * s1 : v1 * c1 + p1 * s1;
+        if (r0) v0 = a0;
+        if (r1) v1 = a1;
+    }
+    dst[lane] = from_f32<T>(v0 * q_mult);
+    dst[lane + 32] = from_f32<T>(v1 * q_mult);
+}
+
 // The same work where the RMS norm of q (and of k) runs over the whole projection of a token, all heads at
 // once, with a weight per element of the projection (qw [nh * dk], kw [nkv * dk]); eps inside the root.  One
 // block per token: every thread adds up its share of the squares of q and of k in a fixed order, the block
@@ -511,6 +582,15 @@ VAPI_EXPORT int vapi_qk_norm_rope_write_split(void* qkv, long long row_stride, i
         else
             return fail(-2, "qk_norm_rope_write_split: unsupported dtype %d", dtype);
         return check_launch("qk_norm_rope_write_split (whole projection)", e);
+    }
+    if (dk == 64 && dv == 64 && (!cosr || interleaved || rot == 64) && items <= 0x7fffffffLL - 8 && (dtype == VAPI_F32 || dtype == VAPI_BF16)) {
+        const int blocks64 = (int)((items + 7) / 8);
+#define QK_64(T)                                                                                                              \
+    launch(qk_norm_rope_write_split64_kernel<T>, blocks64, 256, 0, stream, (T*)qkv, row_stride, qw, kw, eps, cosr, sinr, rot, \
+           interleaved, (T*)cache, slot_mapping, n, nh, nkv, page_size, num_pages, status, positions, qt_coef, qt_every)
+        e = dtype == VAPI_F32 ? QK_64(float) : QK_64(__nv_bfloat16);
+#undef QK_64
+        return check_launch("qk_norm_rope_write_split", e);
     }
     if (dtype == VAPI_F32)
         e = launch(qk_norm_rope_write_split_kernel<float>, blocks, QK_WARPS * 32, 0, stream, (float*)qkv, row_stride, qw, kw, eps,
