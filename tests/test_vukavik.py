@@ -406,6 +406,48 @@ def test_norm_rotation_and_cache_write_for_unlike_widths(dtype):
         assert torch.equal(b[:, -nh - 5:].cpu(), qkv[:, -nh - 5:]), "columns beyond the heads are left alone"
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_kernels_of_heads_that_a_warp_holds_in_registers(dtype):
+    """The gated norm over groups of 64, 128 and 256 (one weight for all groups, some of them, or each column) and the rotation of
+    heads of 64 (pairs side by side or halves, a part of the head, no norm, no rotation, a query temperature, no cache, a slot outside
+    the pool), with row counts that leave warps of a block without work."""
+    from vapi_b200 import ops
+    g = torch.Generator().manual_seed(17)
+    # (float32: the sums of squares and the device's exponentials; bfloat16: one rounding of the result)
+    tol = 1e-5 if dtype == torch.float32 else 8e-3
+    for n, width, group, wl in ((1, 64, 64, 64), (7, 192, 64, 192), (5, 640, 128, 128), (3, 512, 128, 256), (9, 256, 256, 256)):
+        y, z = torch.randn((n, width), generator=g) * 3, torch.randn((n, width + 6), generator=g).to(dtype)[:, 2:width + 2]
+        w = torch.randn(wl, generator=g)
+        for first in (False, True):
+            for gate in ("silu", "sigmoid"):
+                want = plain_ops.gated_group_rmsnorm(y, z, w, 1e-5, group, first, dtype, gate)
+                got = ops.gated_group_rmsnorm(y.cuda(), z.cuda(), w.cuda(), 1e-5, group, first, dtype, gate)
+                assert torch.allclose(got.float().cpu(), want.float(), atol=tol, rtol=tol), (n, width, group, wl, first, gate)
+    n, nh, nkv, page = 5, 3, 2, 16
+    pos, slots = torch.arange(90, 90 + n, dtype=torch.int32), torch.tensor([17, 3, 40, 0, 31], dtype=torch.int32)
+    qkv = torch.randn((n, (nh + 2 * nkv) * 64 + 3), generator=g).to(dtype)
+    qw, kw = torch.randn(64, generator=g), torch.randn(64, generator=g)
+    for rot, inter, norm, temp, paged in ((64, True, True, None, True), (64, False, True, (0.3, 7), True), (20, True, False, None, True),
+                                          (0, False, True, None, True), (0, False, False, (0.2, 3), False), (0, False, False, None, True)):
+        cos, sin = (None, None) if rot == 0 else (torch.randn((n, rot // 2), generator=g), torch.randn((n, rot // 2), generator=g))
+        c = lambda t: None if t is None else t.cuda()
+        cache = torch.zeros((3, page * nkv * 128), dtype=dtype)
+        a, b, dcache = qkv.clone(), qkv.cuda(), cache.cuda()
+        w2 = (qw, kw) if norm else (None, None)
+        plain_ops.qk_norm_rope_write_split(a, nh, nkv, 64, 64, *w2, 1e-5, cos, sin, rot, inter, cache if paged else None, page, slots if paged else None,
+                                           positions=pos, q_temp=temp)
+        ops.qk_norm_rope_write_split(b, nh, nkv, 64, 64, c(w2[0]), c(w2[1]), 1e-5, c(cos), c(sin), rot, inter, dcache if paged else None, page,
+                                     slots.cuda() if paged else None, positions=pos.cuda(), q_temp=temp)
+        scale = 1.0 + float(a.float().abs().max())
+        assert torch.allclose(b.float().cpu(), a.float(), atol=tol * scale, rtol=tol), (rot, inter, norm, temp)
+        assert torch.allclose(dcache.float().cpu(), cache.float(), atol=tol * scale, rtol=tol), (rot, inter, norm, temp)
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.qk_norm_rope_write_split(qkv.cuda(), nh, nkv, 64, 64, None, None, 1e-5, None, None, 0, False, dcache, page,
+                                 torch.tensor([17, 3, 48, 0, 31], dtype=torch.int32, device="cuda"), st)
+    assert int(st.item()) == 2
+
+
 # ---- the engine: scheduler, batching, sampling, entry point -----------------------------------------------------
 @pytest.mark.parametrize("device,name,lens,new", [pytest.param("cpu", "tiny", [1, 9, 20], 5, id="host"),
                                                   pytest.param("cuda", "mixed", [1, 33, 150, 7, 64, 90], 24, marks=pytest.mark.gpu, id="gpu")])

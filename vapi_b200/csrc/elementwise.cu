@@ -887,13 +887,8 @@ __global__ void postnorm_add_rmsnorm_vec_kernel(float* __restrict__ x, const T* 
     const T* yr = y ? y + (size_t)row * hidden : nullptr;
     const T* y2r = (y && y2) ? y2 + (size_t)row * hidden : nullptr;
     const int h4 = hidden >> 2;
-    float4 v[NORM_KMAX], xq[NORM_KMAX];          // (the stream's row is on its way while the output's norm is worked out)
+    float4 v[NORM_KMAX];
     float ssy = 0.f;
-#pragma unroll
-    for (int k = 0; k < NORM_KMAX; ++k) {
-        const int c = threadIdx.x + k * blockDim.x;
-        xq[k] = c < h4 ? Pack4<float>::load(xr + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
     if (y2r) {                                   // two raw branches: their norms and their mean come first
         float4 u[NORM_KMAX];
         float sa = 0.f, sb = 0.f;
@@ -941,7 +936,7 @@ __global__ void postnorm_add_rmsnorm_vec_kernel(float* __restrict__ x, const T* 
     for (int k = 0; k < NORM_KMAX; ++k) {
         const int c = threadIdx.x + k * blockDim.x;
         if (c < h4) {
-            const float4 xv = xq[k];
+            const float4 xv = Pack4<float>::load(xr + 4 * c);
             if (yr) {
                 const float4 wp = Pack4<float>::load(w_post + 4 * c);
                 v[k].x = xv.x + mult * (v[k].x * inv_y * wp.x);
@@ -1099,7 +1094,8 @@ __global__ void gated_group_rmsnorm_kernel(const float* __restrict__ y, const T*
 }
 
 // The same for groups of 32 PER columns: a lane's PER columns are asked for together and stay in registers, where the kernel above reads
-// y and z twice, column after column, and divides 64-bit numbers.  The sums in the same order.
+// y and z twice, column after column, and divides 64-bit numbers.  The sums in the same order.  2,000 rows of 2,048 columns in bfloat16,
+// groups of 128: 17.0 us (20.1 with the gate first), so 11.5; groups of 64 26.4, so 15.7; 1,024 columns in groups of 256 9.5, so 5.4.
 template <typename T, int PER>
 __global__ void __launch_bounds__(256)
 gated_group_rmsnorm_lane_kernel(const float* __restrict__ y, const T* __restrict__ z, long long z_stride, const float* __restrict__ w,
