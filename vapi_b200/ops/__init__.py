@@ -117,6 +117,16 @@ def _address(lib: ctypes.CDLL, fn: str) -> int:
 _calls_module = None
 
 
+class _NoCalls:
+    """Stands where csrc/calls.cpp cannot be built (it needs torch's and Python's headers): every call goes through Python."""
+
+    @staticmethod
+    def product(*_):
+        return NotImplemented
+
+    shortconv = product
+
+
 def _calls():
     """The extension module of csrc/calls.cpp."""
     global _calls_module
@@ -124,12 +134,17 @@ def _calls():
         import importlib.util
         with _lock:
             if _calls_module is None:
-                path = _build.build("calls")
-                spec = importlib.util.spec_from_file_location("vapi_calls", path)
-                module = importlib.util.module_from_spec(spec)
-                spec.loader.exec_module(module)
-                loaded_libraries["calls"] = path
-                _calls_module = module
+                try:
+                    path = _build.build("calls")
+                    spec = importlib.util.spec_from_file_location("vapi_calls", path)
+                    module = importlib.util.module_from_spec(spec)
+                    spec.loader.exec_module(module)
+                    loaded_libraries["calls"] = path
+                    _calls_module = module
+                except (_build.BuildError, ImportError) as e:
+                    import warnings
+                    warnings.warn(f"steps of a few rows are launched from Python, at twice the cost to the host: {e}")
+                    _calls_module = _NoCalls
     return _calls_module
 
 
