@@ -350,6 +350,37 @@ def test_long_walks_give_the_bits_of_the_short_ones(dtype, rows, cols):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", [(64, 32), (128, 64)])
+@pytest.mark.parametrize("eps", [1e-6, 1e-30, 0.0])
+def test_long_walks_step_over_their_portion_and_no_further(dtype, rows, cols, eps):
+    """The long walks against the short ones (``max_q`` tells them apart) over portions that end in and between the eights that are
+    walked together, with states that hold infinities and negative zeros and any epsilon of the unit norms: a step over a token that is not
+    there would show in the state."""
+    from vapi_b200 import ops
+    g = torch.Generator().manual_seed(19)
+    qlens = [9, 17, 33, 1, 8, 16, 39, 23]
+    cu, pos, _, sl = _step_meta(qlens, [3] * len(qlens), list(range(len(qlens))), "cuda")
+    n, nh = sum(qlens), 2
+    A, dtb, D = torch.rand(nh, generator=g).cuda() * 2 - 1, torch.randn(nh, generator=g).cuda(), torch.randn(nh, generator=g).cuda()
+    ab = torch.randn((n, 2 * nh), generator=g).to(dtype).cuda()
+    state = torch.randn((len(qlens), nh * rows * cols), generator=g)
+    state[:, 5::97] = -0.0
+    state[::2, 7] = float("inf")
+    state = state.cuda()
+
+    def same(fn, width):
+        x = torch.randn((n, width), generator=g).to(dtype).cuda()
+        s0, s1 = state.clone(), state.clone()
+        for a, b in ((fn(x, s0, 1), fn(x, s1, max(qlens))), (s0, s1)):
+            assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(nan=0.0).view(torch.int32), b.nan_to_num(nan=0.0).view(torch.int32))
+        assert bool(s1[1].isfinite().all()), "a finite state stays finite"
+
+    same(lambda x, s, m: ops.gated_delta(x, ab, A, dtb, s, 0, sl, cu, pos, nh, 1, rows, cols, norm_eps=eps, max_q=m), 2 * rows + nh * cols)
+    same(lambda x, s, m: ops.state_space(x, ab[:, :nh], A, dtb, D, s, 0, sl, cu, pos, nh, 1, rows, cols, max_q=m), nh * cols + 2 * rows)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_norm_kernels_of_the_blocks_and_the_gated_group_norm(dtype):
     from vapi_b200 import ops
     g = torch.Generator().manual_seed(9)

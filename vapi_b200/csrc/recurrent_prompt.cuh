@@ -12,7 +12,8 @@
 // here; state space (64 heads of 64 columns) 726 us in state_space_kernel, 250 here.  Measured beside it: two columns a
 // thread for the delta rule (half the warps) 373 us; one column a thread for the state space 303 to 380 us; one block an SM
 // (more registers) within 2 % for one sequence, but 244 against 191 us for five of 300 tokens; the read-out by four more warps that
-// follow with a state of their own 303 against 289 us (captured): what is left is the chain itself.
+// follow with a state of their own 303 against 289 us (captured): what is left is the chain itself.  At the 128 registers that two
+// blocks leave a thread the delta rule keeps 16 to 56 bytes of it in local memory and the float state space of 128 rows 28.
 #pragma once
 #include "common.cuh"
 
@@ -120,25 +121,24 @@ gated_delta_prompt_kernel(const T* __restrict__ qkv, long long qkv_stride, int q
     const float decay_rate = expf(A_log[h]), bias = dt_bias[h], q_scale = rsqrtf((float)rows);
     auto fill = [&](Stage& st, int first) {
         const int tt = tid >> 3;
-        const bool there = first + tt < qlen;
-        const size_t t = (size_t)(t0 + first + (there ? tt : 0));
+        const size_t t = (size_t)(t0 + first + tt);
         const T* row = qkv + t * qkv_stride;
         WalkPiece<T, RT> kp, qp;
         float2 kv[RT / 2], qv[RT / 2];
         float vv[VPT], a = 0.f, b = 0.f;
-        kp.load(row + k_off + g * ROWS + sl * RT);
-        qp.load(row + q_off + g * ROWS + sl * RT);
+        kp.clear();
+        qp.clear();
 #pragma unroll
-        for (int c = 0; c < VPT; ++c) vv[c] = to_f32(row[v_off + h * cols + col0 + sl * VPT + c]);
-        if (sl == 1) {
-            a = to_f32(ab[t * ab_stride + h]);
-            b = to_f32(ab[t * ab_stride + nh + h]);
-        }
-        if (!there) {                                         // behind the portion: a step that leaves the state as it is
-            kp.clear();
-            qp.clear();
+        for (int c = 0; c < VPT; ++c) vv[c] = 0.f;
+        if (first + tt < qlen) {                              // (nothing steps over what is staged behind the portion)
+            kp.load(row + k_off + g * ROWS + sl * RT);
+            qp.load(row + q_off + g * ROWS + sl * RT);
 #pragma unroll
-            for (int c = 0; c < VPT; ++c) vv[c] = 0.f;
+            for (int c = 0; c < VPT; ++c) vv[c] = to_f32(row[v_off + h * cols + col0 + sl * VPT + c]);
+            if (sl == 1) {
+                a = to_f32(ab[t * ab_stride + h]);
+                b = to_f32(ab[t * ab_stride + nh + h]);
+            }
         }
         kp.store(&st.k[tt][sl * LANE]);
         qp.store(&st.q[tt][sl * LANE]);
@@ -147,7 +147,7 @@ gated_delta_prompt_kernel(const T* __restrict__ qkv, long long qkv_stride, int q
         kp.floats(kv);
         qp.floats(qv);
         if (sl == 1) {
-            st.unit[tt].x = there ? expf(-decay_rate * walk_softplus(a + bias)) : 1.f;
+            st.unit[tt].x = expf(-decay_rate * walk_softplus(a + bias));
             st.unit[tt].y = 1.f / (1.f + expf(-b));
         }
         float ssk = 0.f, ssq = 0.f, dot = 0.f;
@@ -193,62 +193,81 @@ gated_delta_prompt_kernel(const T* __restrict__ qkv, long long qkv_stride, int q
             WalkPiece<T, RT> kn, qn;
             kn.load(&st.k[0][sl * LANE]);
             float4 un = st.unit[0];
-            for (int t8 = 0; t8 < count; t8 += 8) {
+            // one token: its decay, read-out (this lane's share of it, `qp`) and write (`u`)
+            auto step = [&](int tt, int next, float (&qp)[NC], float (&u)[NC]) {
+                float2 kc[RT / 2], qc[RT / 2];
+                kn.floats(kc);
+                const float4 unit = un;
+                kn.load(&st.k[next][sl * LANE]);
+                qn.load(&st.q[tt][sl * LANE]);
+                un = st.unit[next];
+                const float2 g2 = make_float2(unit.x, unit.x);
+                float ksum[NC], vv[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    vv[c] = st.v[tt][c0 + c];
+                    float2 ks[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+                    for (int r4 = 0; r4 < RT / 4; ++r4) {
+                        S2[c][2 * r4] = __fmul2_rn(S2[c][2 * r4], g2);
+                        S2[c][2 * r4 + 1] = __fmul2_rn(S2[c][2 * r4 + 1], g2);
+                        ks[0] = __ffma2_rn(kc[2 * r4], S2[c][2 * r4], ks[0]);
+                        ks[1] = __ffma2_rn(kc[2 * r4 + 1], S2[c][2 * r4 + 1], ks[1]);
+                    }
+                    ksum[c] = (ks[0].x + ks[0].y) + (ks[1].x + ks[1].y);
+                }
+#pragma unroll
+                for (int c = 0; c < NC; ++c) ksum[c] = walk_sum8(ksum[c]) * unit.z;
+                // (the read-out of the decayed state: in the shadow of those shuffles)
+                qn.floats(qc);
+                float2 qs[NC][2];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) qs[c][0] = qs[c][1] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int r4 = 0; r4 < RT / 4; ++r4)
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        qs[c][0] = __ffma2_rn(qc[2 * r4], S2[c][2 * r4], qs[c][0]);
+                        qs[c][1] = __ffma2_rn(qc[2 * r4 + 1], S2[c][2 * r4 + 1], qs[c][1]);
+                    }
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    qp[c] = (qs[c][0].x + qs[c][0].y) + (qs[c][1].x + qs[c][1].y);
+                    u[c] = unit.y * (vv[c] - ksum[c]);
+                    const float2 uk = make_float2(u[c] * unit.z, u[c] * unit.z);
+#pragma unroll
+                    for (int r = 0; r < RT / 2; ++r) S2[c][r] = __ffma2_rn(kc[r], uk, S2[c][r]);
+                }
+            };
+            const int whole = count & ~7;
+            for (int done = 0; done < whole; done += 8) {
                 float qp[NC][8], mine[NC];                    // the lanes' shares of eight read-outs; u of this lane's token of the eight
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const int tt = t8 + j;
-                    float2 kc[RT / 2], qc[RT / 2];
-                    kn.floats(kc);
-                    const float4 unit = un;
-                    const int next = j < 7 ? tt + 1 : min(tt + 1, WALK_TC - 1);
-                    kn.load(&st.k[next][sl * LANE]);
-                    qn.load(&st.q[tt][sl * LANE]);
-                    un = st.unit[next];
-                    const float2 g2 = make_float2(unit.x, unit.x);
-                    float ksum[NC], vv[NC];
+                    float share[NC], u[NC];
+                    step(done + j, j < 7 ? done + j + 1 : min(done + j + 1, WALK_TC - 1), share, u);
 #pragma unroll
                     for (int c = 0; c < NC; ++c) {
-                        vv[c] = st.v[tt][c0 + c];
-                        float2 ks[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-                        for (int r4 = 0; r4 < RT / 4; ++r4) {
-                            S2[c][2 * r4] = __fmul2_rn(S2[c][2 * r4], g2);
-                            S2[c][2 * r4 + 1] = __fmul2_rn(S2[c][2 * r4 + 1], g2);
-                            ks[0] = __ffma2_rn(kc[2 * r4], S2[c][2 * r4], ks[0]);
-                            ks[1] = __ffma2_rn(kc[2 * r4 + 1], S2[c][2 * r4 + 1], ks[1]);
-                        }
-                        ksum[c] = (ks[0].x + ks[0].y) + (ks[1].x + ks[1].y);
-                    }
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) ksum[c] = walk_sum8(ksum[c]) * unit.z;
-                    // (the read-out of the decayed state: in the shadow of those shuffles)
-                    qn.floats(qc);
-                    float2 qs[NC][2];
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) qs[c][0] = qs[c][1] = make_float2(0.f, 0.f);
-#pragma unroll
-                    for (int r4 = 0; r4 < RT / 4; ++r4)
-#pragma unroll
-                        for (int c = 0; c < NC; ++c) {
-                            qs[c][0] = __ffma2_rn(qc[2 * r4], S2[c][2 * r4], qs[c][0]);
-                            qs[c][1] = __ffma2_rn(qc[2 * r4 + 1], S2[c][2 * r4 + 1], qs[c][1]);
-                        }
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        qp[c][j] = (qs[c][0].x + qs[c][0].y) + (qs[c][1].x + qs[c][1].y);
-                        const float u = unit.y * (vv[c] - ksum[c]);
-                        const float2 uk = make_float2(u * unit.z, u * unit.z);
-#pragma unroll
-                        for (int r = 0; r < RT / 2; ++r) S2[c][r] = __ffma2_rn(kc[r], uk, S2[c][r]);
-                        if (j == 0 || j == sl) mine[c] = u;
+                        qp[c][j] = share[c];
+                        if (j == 0 || j == sl) mine[c] = u[c];
                     }
                 }
-                const float qk = st.qk[t8 + sl], q_inv = st.unit[t8 + sl].w;
+                const float qk = st.qk[done + sl], q_inv = st.unit[done + sl].w;
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    out[((size_t)(t0 + first + done + sl) * nh + h) * cols + col0 + c0 + c] = fmaf(qk, mine[c], walk_sum8_each(qp[c], sl) * q_inv);
+            }
+            // The last few, fewer than eight, one by one: a step over a token that is not there would not leave the state as it is, whatever
+            // is staged for it (a unit norm over zeros with an epsilon of 0, an infinity in the state).  A sequence of one token beside a
+            // portion takes one step, not eight: 60 of them beside 17, 16 heads of 128 x 128, bfloat16 112 us, so 74.
+#pragma unroll 1
+            for (int done = whole; done < count; ++done) {
+                float share[NC], u[NC];
+                step(done, min(done + 1, WALK_TC - 1), share, u);
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    const float qsum = walk_sum8_each(qp[c], sl) * q_inv;
-                    if (t8 + sl < count) out[((size_t)(t0 + first + t8 + sl) * nh + h) * cols + col0 + c0 + c] = fmaf(qk, mine[c], qsum);
+                    const float qsum = walk_sum8(share[c]) * st.unit[done].w;
+                    if (sl == 0) out[((size_t)(t0 + first + done) * nh + h) * cols + col0 + c0 + c] = fmaf(st.qk[done], u[c], qsum);
                 }
             }
         }
