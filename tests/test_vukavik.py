@@ -379,6 +379,28 @@ def test_long_walks_step_over_their_portion_and_no_further(dtype, rows, cols, ep
     same(lambda x, s, m: ops.state_space(x, ab[:, :nh], A, dtb, D, s, 0, sl, cu, pos, nh, 1, rows, cols, max_q=m), nh * cols + 2 * rows)
 
 
+# around the rules of the launch: blocks that are all resident at once (296) and more, short and long portions, alone and beside single tokens
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("qlens", [[16] * 9, [16] * 10, [17] * 10, [23] * 10, [24] * 10, [1] * 9 + [16], [1] * 60 + [16], [1] * 60 + [24], [63] + [1] * 9,
+                                   [1] * 9 + [64], [1] * 8 + [200]])
+def test_which_kernel_walks_does_not_show(dtype, qlens):
+    from vapi_b200 import ops
+    g = torch.Generator().manual_seed(23)
+    rows = cols = 64
+    cu, pos, _, sl = _step_meta(qlens, [2] * len(qlens), list(range(len(qlens))), "cuda")
+    n = sum(qlens)
+
+    def same(fn, nh, width):
+        x, state = torch.randn((n, width), generator=g).to(dtype).cuda(), torch.randn((len(qlens), nh * rows * cols), generator=g).cuda()
+        A, dtb, ab = torch.rand(nh, generator=g).cuda(), torch.randn(nh, generator=g).cuda(), torch.randn((n, 2 * nh), generator=g).to(dtype).cuda()
+        s1 = state.clone()
+        assert torch.equal(fn(x, ab, A, dtb, state, 1), fn(x, ab, A, dtb, s1, max(qlens))) and torch.equal(state, s1)
+
+    same(lambda x, ab, A, dtb, s, m: ops.gated_delta(x, ab, A, dtb, s, 0, sl, cu, pos, 8, 2, rows, cols, max_q=m), 8, 4 * rows + 8 * cols)
+    same(lambda x, ab, A, dtb, s, m: ops.state_space(x, ab[:, :16], A, dtb, A, s, 0, sl, cu, pos, 16, 1, rows, cols, max_q=m), 16, 16 * cols + 2 * rows)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_norm_kernels_of_the_blocks_and_the_gated_group_norm(dtype):

@@ -559,10 +559,27 @@ state_space_kernel(const T* __restrict__ xbc, long long xbc_stride, const T* __r
 
 static inline int rec_lpc(int rows) { return rows <= 32 ? 4 : (rows <= 128 ? 8 : 16); }
 
+// Whether a step goes to the walks of recurrent_prompt.cuh (the same bits either way): from REC_TC tokens in its longest portion on, as long
+// as all blocks are resident at once, two a multiprocessor.  Where they come in rounds, a sequence of a token or two costs its state's way
+// there and back, and the smaller blocks of the kernels above have more of that in flight.  Captured, 60 single tokens beside a portion,
+// and equal portions, us above / in the walk: 16 heads of 128 x 128, float, 16 + 60 71 / 77, 48 + 60 82 / 85, 64 + 60 87 / 88, 64 of 17
+// 194 / 197, of 24 1.01 of the time, of 33 0.97; bfloat16 16 + 60 82 / 73, 64 of 16 178 / 158; 8 heads of 64 x 64, float, 16 + 60 16.3 / 20.1, 40 +
+// 60 22.6 / 23.0, 64 of 16 30.3 / 33.6, of 24 1.00, of 33 0.97; bfloat16 16 + 60 17.0 / 18.0, 17 + 60 18.2 / 18.5, 32 of 16 17.1 / 17.6, of 17 0.96.
+static bool delta_walk_pays(int max_q, int dtype, int rows, long long blocks, int n, int num_seqs) {
+    if (max_q < REC_TC) return false;
+    if (blocks <= 2LL * sm_count()) return true;
+    return dtype == VAPI_BF16 ? rows > 64 || max_q > REC_TC : max_q >= 4 * REC_TC || n / 24 >= num_seqs;
+}
+// The state space, 16 heads of 64 x 64: 16 + 60 float 20.5 / 23.1, bfloat16 22.5 / 23.3, 17 + 60 21.7 / 24.0 and 23.6 / 24.1, but 24 + 60 bfloat16
+// 25.0 / 24.0, 16 + 31 15.1 / 13.8; 64 heads of 128 x 64 16 + 60 1.01 and 0.90 of the time.
+static bool space_walk_pays(int max_q, int rows, long long blocks, int n, int num_seqs) {
+    return max_q >= REC_TC && (blocks <= 2LL * sm_count() || rows > 64 || 3LL * n >= 4LL * num_seqs);
+}
+
 VAPI_EXPORT int vapi_gated_delta(const void* qkv, long long qkv_stride, int q_off, int k_off, int v_off, const void* ab,
                                  long long ab_stride, int dtype, const float* A_log, const float* dt_bias, float* state,
                                  long long slot_stride, const int* state_slots, const int* cu_q, const int* positions,
-                                 float* out, int num_seqs, int nh, int nkv, int rows, int cols, int num_slots,
+                                 float* out, int n, int num_seqs, int nh, int nkv, int rows, int cols, int num_slots,
                                  float norm_eps, int max_q, int* status, cudaStream_t stream) {
     if (num_seqs <= 0) return 0;
     if (nh <= 0 || nkv <= 0 || nh % nkv || rows <= 0 || rows > 256 || cols <= 0)
@@ -572,10 +589,10 @@ VAPI_EXPORT int vapi_gated_delta(const void* qkv, long long qkv_stride, int q_of
     dim3 grid((cols + cpb - 1) / cpb, nh, num_seqs);
     const bool early = max_q < REC_TC;                     // decode steps may start beside the kernel before; long walks may not
     cudaError_t e = cudaSuccess;
-    // Portions of at least a buffer's half, full rows and whole blocks of columns, 16-byte pieces: the walk of recurrent_prompt.cuh
-    // (same bits).
+    // full rows and whole blocks of columns, 16-byte pieces
     constexpr int NC = 1, WW = 4;
-    if (!early && (rows == 64 || rows == 128) && cols % (4 * WW * NC) == 0 && walk_aligned(qkv, qkv_stride, dtype, q_off, k_off)) {
+    if ((rows == 64 || rows == 128) && cols % (4 * WW * NC) == 0 && walk_aligned(qkv, qkv_stride, dtype, q_off, k_off) &&
+        delta_walk_pays(max_q, dtype, rows, (long long)(cols / (4 * WW * NC)) * nh * num_seqs, n, num_seqs)) {
         grid.x = cols / (4 * WW * NC);
 #define GD_WALK(T, RT)                                                                                                     \
     launch_if(false, gated_delta_prompt_kernel<T, RT, NC, WW>, grid, WalkShape<T, RT, NC, WW>::THREADS, 0, stream,         \
@@ -603,7 +620,7 @@ VAPI_EXPORT int vapi_gated_delta(const void* qkv, long long qkv_stride, int q_of
 VAPI_EXPORT int vapi_state_space(const void* xbc, long long xbc_stride, const void* dt, long long dt_stride, int dtype,
                                  const float* A_log, const float* dt_bias, const float* D, float* state,
                                  long long slot_stride, const int* state_slots, const int* cu_q, const int* positions,
-                                 float* out, int num_seqs, int nh, int groups, int rows, int cols, int num_slots,
+                                 float* out, int n, int num_seqs, int nh, int groups, int rows, int cols, int num_slots,
                                  int max_q, int* status, cudaStream_t stream) {
     if (num_seqs <= 0) return 0;
     if (nh <= 0 || groups <= 0 || nh % groups || rows <= 0 || rows > 256 || cols <= 0)
@@ -614,7 +631,8 @@ VAPI_EXPORT int vapi_state_space(const void* xbc, long long xbc_stride, const vo
     const bool early = max_q < REC_TC;
     cudaError_t e = cudaSuccess;
     constexpr int NC = 2, WW = 4;                           // (as in vapi_gated_delta)
-    if (!early && (rows == 64 || rows == 128) && cols % (4 * WW * NC) == 0 && walk_aligned(xbc, xbc_stride, dtype, nh * cols, rows)) {
+    if ((rows == 64 || rows == 128) && cols % (4 * WW * NC) == 0 && walk_aligned(xbc, xbc_stride, dtype, nh * cols, rows) &&
+        space_walk_pays(max_q, rows, (long long)(cols / (4 * WW * NC)) * nh * num_seqs, n, num_seqs)) {
         grid.x = cols / (4 * WW * NC);
 #define SS_WALK(T, RT)                                                                                                     \
     launch_if(false, state_space_prompt_kernel<T, RT, NC, WW>, grid, WalkShape<T, RT, NC, WW>::THREADS, 0, stream,         \

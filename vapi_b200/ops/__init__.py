@@ -1813,7 +1813,7 @@ def gated_delta(qkv: torch.Tensor, ab: torch.Tensor, A_log: torch.Tensor, dt_bia
     _check(lib, lib.vapi_gated_delta(
         _p(qkv), ctypes.c_longlong(qkv.stride(0)), 0, nkv * dk, 2 * nkv * dk, _p(ab), ctypes.c_longlong(ab.stride(0)),
         _dt(qkv), _p(A_log), _p(dt_bias), ctypes.c_void_p(state.data_ptr() + 4 * int(state_offset)),
-        ctypes.c_longlong(state.stride(0)), _p(state_slots), _p(cu_q), _p(positions), _p(out), cu_q.numel() - 1, nh, nkv,
+        ctypes.c_longlong(state.stride(0)), _p(state_slots), _p(cu_q), _p(positions), _p(out), n, cu_q.numel() - 1, nh, nkv,
         dk, dv, state.shape[0], ctypes.c_float(norm_eps), int(min(max_q, 1 << 30)), _p(status), _stream()))
     return out
 
@@ -1847,7 +1847,7 @@ def state_space(xbc: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, dt_bia
     _check(lib, lib.vapi_state_space(
         _p(xbc), ctypes.c_longlong(xbc.stride(0)), _p(dt), ctypes.c_longlong(dt.stride(0)), _dt(xbc), _p(A_log),
         _p(dt_bias), _p(D), ctypes.c_void_p(state.data_ptr() + 4 * int(state_offset)), ctypes.c_longlong(state.stride(0)),
-        _p(state_slots), _p(cu_q), _p(positions), _p(out), cu_q.numel() - 1, nh, groups, n_state, head, state.shape[0],
+        _p(state_slots), _p(cu_q), _p(positions), _p(out), n, cu_q.numel() - 1, nh, groups, n_state, head, state.shape[0],
         int(min(max_q, 1 << 30)), _p(status), _stream()))
     return out
 
