@@ -199,7 +199,9 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         return p.epi == TC_EPI_RESID && m < p.M && f0 + 3 < p.N && (p.N & 3) == 0
                    ? *reinterpret_cast<const float4*>(p.resid + (size_t)m * p.N + f0) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
-    auto store_token = [&](const float4& v, const float4& old, int m) {          // phase B for token m, whole warp
+    // phase B for token m, whole warp; `old`: the stream's old values, where they have been asked for (asked for ahead in every form, also where the
+    // epilogue has none, 65,536 x 2,048 without slices of K took 57 us at 64 tokens and 72 at 128, where it takes 55 and 68.5)
+    auto store_token = [&](const float4& v, const float4* old, int m) {
         if (glu) {
             const long long f0 = (long long)n0 + 2 * lane;
             const float s0 = glu_gate_16(v.x, p.glu) * v.z, s1 = glu_gate_16(v.y, p.glu) * v.w;
@@ -241,7 +243,8 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             float* x = p.resid + (size_t)m * p.N + f0;
             float nv[4] = {0.f, 0.f, 0.f, 0.f};
             if (full && (p.N & 3) == 0) {
-                nv[0] = old.x + vv[0]; nv[1] = old.y + vv[1]; nv[2] = old.z + vv[2]; nv[3] = old.w + vv[3];
+                const float4 was = old ? *old : *reinterpret_cast<const float4*>(x);
+                nv[0] = was.x + vv[0]; nv[1] = was.y + vv[1]; nv[2] = was.z + vv[2]; nv[3] = was.w + vv[3];
                 *reinterpret_cast<float4*>(x) = make_float4(nv[0], nv[1], nv[2], nv[3]);
             } else {
 #pragma unroll
@@ -298,8 +301,14 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 #pragma unroll 4
                 for (int m = g0 + warp - 2; m < min(p.M, g0 + GROUP); m += 4) {
                     const float* f = fin + (m - g0) * TC_BM;
-                    const float2 lo = *reinterpret_cast<const float2*>(f + lane_off), hi = *reinterpret_cast<const float2*>(f + lane_off + (glu ? 64 : 2));
-                    store_token(make_float4(lo.x, lo.y, hi.x, hi.y), old_values(m), m);
+                    float4 v;
+                    if (glu) {
+                        const float2 g = *reinterpret_cast<const float2*>(f + lane_off), u = *reinterpret_cast<const float2*>(f + lane_off + 64);
+                        v = make_float4(g.x, g.y, u.x, u.y);
+                    } else {
+                        v = *reinterpret_cast<const float4*>(f + lane_off);
+                    }
+                    store_token(v, nullptr, m);
                 }
                 epi_bar();
             }
@@ -352,7 +361,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
                         if (f0 + 2 < p.N) w.z += p.bias[f0 + 2];
                         if (f0 + 3 < p.N) w.w += p.bias[f0 + 3];
                     }
-                    store_token(w, old[t], m[t]);
+                    store_token(w, &old[t], m[t]);
                 }
             }
         }
