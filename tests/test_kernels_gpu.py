@@ -1070,9 +1070,10 @@ def test_prompt_linear_plain_products(ops, prompt_tiles, M, N, K):
     assert int(st.item()) == 0
 
 
-# slices of K by the number of tiles: four and fewer up to two blocks a multiprocessor (64 and 65 tiles), two (98 to 148), one (149); a K of
-# few pieces, which cannot be cut so often
-@pytest.mark.parametrize("tiles,K", [(37, 512), (49, 512), (64, 520), (65, 512), (87, 384), (98, 512), (148, 512), (149, 512), (64, 128), (100, 192)])
+# slices of K by the number of tiles: four and fewer up to two blocks a multiprocessor (64 and 65 tiles), two (75 to 148, from 512, 1,024 or
+# 1,536 k on; above 96 tokens from 512 or 1,024), one (149); a K of few pieces, which cannot be cut so often
+@pytest.mark.parametrize("tiles,K", [(37, 512), (49, 512), (64, 520), (65, 512), (87, 384), (98, 512), (148, 512), (149, 512), (64, 128), (100, 192),
+                                     (98, 448), (99, 960), (129, 448), (129, 512), (130, 960), (129, 968), (130, 1032), (148, 1536)])
 def test_linear_tc_cuts_k_for_any_number_of_tiles(ops, tiles, K):
     g = torch.Generator(device="cuda").manual_seed(tiles)
     N = tiles * 128 - 5

@@ -427,10 +427,20 @@ VAPI_EXPORT int vapi_linear_tc_plan(int N, int K, int M, int epi, int* tiles, in
         // 48 tiles 9.0 / 11.4 / 15.7 us, so 8.7 / 10.5 / 13.9; 64 tiles 11.6 / 13.9 / 19.4, so 9.6 / 11.6 / 14.7; 80 tiles 15.3 / 19.0 / 27.0, so
         // 10.9 / 13.5 / 17.4; 128 tiles 17.7 / 21.3 / 29.7, so 16.6 / 19.3 / 24.5.  Not more than that: six slices of 48 tiles 13.0 / 17.0 us at
         // 19 / 64 (clusters that do not all find room at once), and three of 98 tiles 17.9 / 22.8, where two fill seven eighths of the places.
+        // Two slices instead of one want a K that is worth the exchange, 17 / 33 / 64 tokens, one slice / two: K = 256, 96 tiles 5.5 / 6.1, 6.5 / 7.0 and
+        // 8.3 / 8.2 us; K = 512, 96 tiles 7.0 / 6.9, 7.9 / 7.8 and 9.7 / 9.1, 112 tiles 7.2 / 7.4, 8.2 / 8.3 and 10.0 / 9.5, 128 tiles 7.3 / 7.9, 8.3 / 9.1 and 10.1 / 10.3; K = 1,024, 108 tiles 10.3 / 9.5, 11.5 / 10.6 and 13.2 / 11.9, 128 tiles 10.7 /
+        // 10.4, 11.8 / 11.2 and 13.6 / 12.9, 148 tiles 11.0 / 11.0, 12.1 / 12.3 and 13.9 / 13.5; K = 1,536, 148 tiles 14.0 / 13.9, 15.3 / 15.2 and 17.1 / 16.6.
+        // 65 / 128 tokens K = 512, 96 tiles 10.7 / 11.1 and 14.7 / 14.0, 128 tiles 1.00 and 0.95 of the time; K = 1,024, 148 tiles 15.1 / 14.1 and 19.2 /
+        // 18.0.  Three slices pay from K = 512 on: 76 tiles, 65 tokens 10.7 / 9.1.
+        int need = 16;
+        if (8 * t > 7 * sms) need = M > 64 ? 16 : 24;
+        else if (12 * t <= 7 * sms || M > 96 || (M <= 64 && 3 * t <= 2 * sms)) need = 8;
         s = sms / t;
-        int two = 2 * sms / t < 4 ? 2 * sms / t : 4;
-        while (two > 2 && 4 * two * t > 7 * sms) --two;
-        if (s < two) s = two;
+        if (s > 1 || num_kb >= need) {
+            int two = 2 * sms / t < 4 ? 2 * sms / t : 4;
+            while (two > 2 && 4 * two * t > 7 * sms) --two;
+            if (s < two) s = two;
+        }
         if (s > 8) s = 8;                            // portable cluster size
         const int max_s = num_kb / 2 > 0 ? num_kb / 2 : 1;      // at least 2 k-blocks a slice
         if (s > max_s) s = max_s;
