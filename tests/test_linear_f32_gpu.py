@@ -154,3 +154,14 @@ def test_gated_decode_product_is_the_product_and_its_gate(ops, N, K, act):
         x = a[:M].contiguous()
         want = ops.swiglu(ops.skinny_linear_f32(w, x), act)
         assert torch.equal(ops.linear_swiglu(x, w, act), want), M
+
+
+# shared K, staged rows, whole rows with a short and a long K: one launch but for the last, above eight tokens
+@pytest.mark.parametrize("N,K,M,launches", [(2048, 2048, 16, 1), (14336, 1024, 16, 1), (14336, 512, 9, 1), (14336, 516, 9, 2), (14336, 2048, 8, 1), (12288, 2048, 16, 2)])
+def test_where_the_gate_rides_on_the_product(ops, N, K, M, launches):
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w = (torch.randn(*s, generator=g, device="cuda") for s in ((M, K), (N, K)))
+    before = ops.launch_count
+    got = ops.linear_swiglu(x, w)
+    assert ops.launch_count == before + launches
+    assert torch.equal(got, ops.skinny_linear_f32(w, x, glu="silu")) and torch.equal(got, ops.swiglu(ops.skinny_linear_f32(w, x)))

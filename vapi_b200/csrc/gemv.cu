@@ -1135,6 +1135,23 @@ skinny_linear_f32_staged_kernel(const float* __restrict__ W, const float* __rest
         out[(size_t)m * out_stride + n0 + r] = GLU ? glu_gate(acc[0], glu) * up : acc[0] + (bias ? bias[n0 + r] : 0.f);
 }
 
+struct F32Form { bool whole, staged; };
+static F32Form f32_form(int N, int K, int M) {
+    F32Form f;
+    // Which order of addition (SHARE 4, or a warp for whole rows) is a matter of N and K alone, see above; where the lines lie, in us in a
+    // captured chain of products at 1 / 8 tokens, shared K against whole rows: 2,048 x 1,024 2.7 / 3.8 against 2.8 / 5.1, 3,072 x 1,024 4.0 /
+    // 6.0 against 3.7 / 6.5; 4,608 x 1,536 6.7 / 9.7 against 6.6 / 10.8, 6,144 x 1,536 8.1 / 12.4 against 7.5 / 12.1, x 2,048 10.1 / 15.2 against
+    // 10.2 / 16.2, x 4,096 21.1 / 27.1 against 19.1 / 30.6; 8,192 x 2,048 13.0 / 19.6 against 12.6 / 17.7, x 4,096 24.1 / 36.6 against 21.7 / 34.0.
+    f.whole = N >= 8192 || (K <= 1024 && N >= 3072) || (N >= 6144 && (K <= 1536 || K > 2048));
+    // Of the two forms for whole rows the unstaged one is ahead where K is a piece or two (65,536 x 128 at 1 / 8 tokens 10.9 / 14.2 against
+    // 12.2 / 29.6; 8,192 x 512 4.7 / 6.7 against 3.5 / 5.8) and above eight tokens (9 / 16 tokens: 4,096 x 512 5.7 / 6.6 against 8.2 / 8.3,
+    // 6,144 x 1,536 16 / 19 against 27 / 27, 13,824 x 4,096 73 / 91 against 91 / 91, 65,536 x 1,536 126 / 128 against 187 / 187), but for more than
+    // twelve whose blocks, three a multiprocessor, do not fill their rounds (8,192 x 4,096, two rounds to 0.58, 68 / 86 against 78 / 78).
+    const long long own = (N + F32_WARPS * F32_ROWS - 1) / (F32_WARPS * F32_ROWS), places = 3LL * sm_count(), rounds = (own + places - 1) / places;
+    f.staged = f.whole && K > 128 && (M <= 8 || (M > 12 && N >= 8192 && 4 * own < 3 * places * rounds));
+    return f;
+}
+
 // y[m][n] = sum_k act[m][k] * W[n][k] (+ bias[n]) in float, M <= 16, K a multiple of 4.
 static int skinny_linear_f32(const float* W, int N, int K, int M, const float* act, const float* bias, float* out, long long out_stride,
                              bool gated, int glu, cudaStream_t stream) {
@@ -1143,17 +1160,8 @@ static int skinny_linear_f32(const float* W, int N, int K, int M, const float* a
     if (N <= 0 || K <= 0 || K % 4 != 0) return fail(-1, "skinny_linear_f32: K=%d must be a positive multiple of 4 (N=%d)", K, N);
     if (!W || !act || !out) return fail(-1, "skinny_linear_f32: missing array");
     if ((((uintptr_t)W | (uintptr_t)act) & 15) != 0) return fail(-1, "skinny_linear_f32: operands must be 16-byte aligned");
-    // Which order of addition (SHARE 4, or a warp for whole rows) is a matter of N and K alone, see above; where the lines lie, in us in a
-    // captured chain of products at 1 / 8 tokens, shared K against whole rows: 2,048 x 1,024 2.7 / 3.8 against 2.8 / 5.1, 3,072 x 1,024 4.0 /
-    // 6.0 against 3.7 / 6.5; 4,608 x 1,536 6.7 / 9.7 against 6.6 / 10.8, 6,144 x 1,536 8.1 / 12.4 against 7.5 / 12.1, x 2,048 10.1 / 15.2 against
-    // 10.2 / 16.2, x 4,096 21.1 / 27.1 against 19.1 / 30.6; 8,192 x 2,048 13.0 / 19.6 against 12.6 / 17.7, x 4,096 24.1 / 36.6 against 21.7 / 34.0.
-    const bool whole = N >= 8192 || (K <= 1024 && N >= 3072) || (N >= 6144 && (K <= 1536 || K > 2048));
-    // Of the two forms for whole rows the unstaged one is ahead where K is a piece or two (65,536 x 128 at 1 / 8 tokens 10.9 / 14.2 against
-    // 12.2 / 29.6; 8,192 x 512 4.7 / 6.7 against 3.5 / 5.8) and above eight tokens (9 / 16 tokens: 4,096 x 512 5.7 / 6.6 against 8.2 / 8.3,
-    // 6,144 x 1,536 16 / 19 against 27 / 27, 13,824 x 4,096 73 / 91 against 91 / 91, 65,536 x 1,536 126 / 128 against 187 / 187), but for more than
-    // twelve whose blocks, three a multiprocessor, do not fill their rounds (8,192 x 4,096, two rounds to 0.58, 68 / 86 against 78 / 78).
-    const long long own = (N + F32_WARPS * F32_ROWS - 1) / (F32_WARPS * F32_ROWS), places = 3LL * sm_count(), rounds = (own + places - 1) / places;
-    const bool staged = whole && K > 128 && (M <= 8 || (M > 12 && N >= 8192 && 4 * own < 3 * places * rounds));
+    const F32Form form = f32_form(N, K, M);
+    const bool whole = form.whole, staged = form.staged;
     cudaError_t e;
 #define VAPI_F32(KERNEL, WARPS, ROWS)                                                                                                     \
     e = launch(KERNEL, (N + (ROWS) - 1) / (ROWS), (WARPS) * 32, 0, stream, W, act, bias, out, N, K, M, out_stride, glu)
@@ -1176,6 +1184,16 @@ static int skinny_linear_f32(const float* W, int N, int K, int M, const float* a
 VAPI_EXPORT int vapi_skinny_linear_f32(const float* W, int N, int K, int M, const float* act, const float* bias,
                                        float* out, long long out_stride, cudaStream_t stream) {
     return skinny_linear_f32(W, N, K, M, act, bias, out, out_stride, false, 0, stream);
+}
+
+// Whether the gate rides on the product, or is a launch behind it with the same values.  Above eight tokens, where a warp has whole rows that are
+// not staged, two gate and two up rows a warp take longer than four neighbouring rows, and with more than 512 k that is more than the launch
+// saved: 9 / 16 tokens, two launches / one: 13,824 x 512 14.7 / 13.7 and 16.8 / 16.1 us, x 1,024 23.3 / 23.4 and 28.0 / 29.4, x 2,048 41.1 / 43.4 and
+// 49.0 / 54.1, x 4,096 75.5 / 80.7 and 91.8 / 107.  Elsewhere one is ahead: staged, 8 / 16 tokens, 14,336 x 2,048 29.8 / 28.0 and 48.3 / 46.5, shared K,
+// 16 tokens, 3,072 x 2,048 14.1 / 12.5.
+VAPI_EXPORT int vapi_skinny_linear_f32_glu_pays(int N, int K, int M) {
+    const F32Form f = f32_form(N, K, M);
+    return M <= 8 || K <= 512 || !f.whole || f.staged;
 }
 
 // The same for a stack of gate and up rows, out[m][f] = gate(y[m][f]) * y[m][N / 2 + f] (`glu`: glu_gate's kind).

@@ -704,7 +704,7 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, act: str = "silu") -> t
             and few_rows_applies(rows, weight)):
         return few_rows_linear(weight, act=x, epilogue="swiglu", glu=act)      # a decode step: the gate rides on the product
     if (x.dtype == torch.float32 and weight.shape[0] % 2 == 0 and skinny_f32_applies(rows, weight) and x.is_contiguous()
-            and x.data_ptr() % 16 == 0):
+            and x.data_ptr() % 16 == 0 and (rows <= 8 or _lib("gemv").vapi_skinny_linear_f32_glu_pays(*weight.shape, rows))):
         return skinny_linear_f32(weight, x, glu=act)
     return swiglu(linear(x, weight), act)
 
