@@ -1,5 +1,5 @@
 """Builds the native sources of this package, one shared library per source: CUDA sources
-(``.cu``) for sm_100a with nvcc, host sources (``.cpp``: the host runtime) with the C++ compiler.
+(``.cu``) for sm_100a with nvcc, host sources (``.cpp``: the host runtime, the native calls) with the C++ compiler.
 
 Each ``<name>.cu`` / ``<name>.cpp`` becomes ``_build/lib<name>-<hash>.so`` next to it, where the hash covers
 the source, the shared headers and the compiler flags, so a stale library is never picked
@@ -7,8 +7,9 @@ up.  A library is built the first time something asks for it, which means a prog
 compiles what the model it runs needs.  While nvcc runs, a line is printed to stderr now and
 then so that a first call does not look hung.
 
-The build needs nothing but ``nvcc``: the libraries export plain C functions that take raw
-device pointers, and they are loaded with ``ctypes``.
+The kernels need nothing but ``nvcc`` and the host runtime nothing but the compiler: these libraries export plain C functions
+(the kernels' take raw device pointers) and are loaded with ``ctypes``.  ``calls.cpp`` is an extension module on torch's C++
+interface and needs torch's and Python's headers as well; without it the package does the same in Python.
 """
 from __future__ import annotations
 
@@ -21,6 +22,7 @@ import sys
 import tempfile
 import threading
 import time
+import warnings
 from typing import Dict, List, Optional
 
 CSRC_DIR = os.path.dirname(os.path.abspath(__file__))
@@ -31,6 +33,10 @@ COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--shared", "-Xcompiler", "-fP
 #: (tuning experiments: e.g. -DGV_STAGES_N=6)
 EXTRA: Dict[str, List[str]] = {}
 _ENV_FLAGS = os.environ.get("VAPI_NVCC_FLAGS", "").split()
+
+
+#: sources that the package can do without
+OPTIONAL = ("calls",)
 
 
 class BuildError(RuntimeError):
@@ -235,10 +241,10 @@ def build(name: str, verbose: bool = True) -> str:
 
 
 def build_all(verbose: bool = True, jobs: int = 4) -> Dict[str, str]:
-    """Build every source (in parallel) and return name -> path."""
+    """Build every source (in parallel) and return name -> path.  One of :data:`OPTIONAL` that cannot be built is warned of and left out."""
     names = sources()
     out: Dict[str, str] = {}
-    errs: List[str] = []
+    errs: Dict[str, str] = {}
     lock = threading.Lock()
     sem = threading.Semaphore(max(1, jobs))
 
@@ -250,15 +256,18 @@ def build_all(verbose: bool = True, jobs: int = 4) -> Dict[str, str]:
                     out[n] = p
             except BuildError as e:
                 with lock:
-                    errs.append(str(e))
+                    errs[n] = str(e)
 
     ths = [threading.Thread(target=one, args=(n,)) for n in names]
     for t in ths:
         t.start()
     for t in ths:
         t.join()
+    for n in OPTIONAL:
+        if n in errs:
+            warnings.warn(f"{n} could not be built, and the package does without: {errs.pop(n)}")
     if errs:
-        raise BuildError("\n".join(errs))
+        raise BuildError("\n".join(errs.values()))
     return out
 
 
