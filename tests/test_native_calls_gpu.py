@@ -98,3 +98,28 @@ def test_what_the_native_product_does_not_take_is_refused_or_done_as_before(ops)
         pass
 
     assert torch.equal(ops.linear_tc(w, act=x.as_subclass(Other)).as_subclass(torch.Tensor), ops.linear_tc(w, act=x))
+
+
+def test_a_call_that_has_been_made_is_not_made_again(ops, tmp_path):
+    """An exception out of the C function is an error: ``NotImplemented`` would send the caller through the same call once more, which
+    adds to the stream, or moves a state on, twice.  (The function here launches nothing.)"""
+    import ctypes
+    import subprocess
+    from vapi_b200.csrc import build
+    src = tmp_path / "throws.cpp"
+    src.write_text('#include <new>\n#include <stdexcept>\nextern "C" { int calls = 0; int plan(int, int, int, int, int* a, int* b, int* c) { *a = *b = *c = 1; return 0; }\n'
+                   'int memory() { ++calls; throw std::bad_alloc(); }\nint other() { ++calls; throw 1; } }\n')
+    subprocess.run([build.find_cxx(), "-shared", "-fPIC", "-o", str(tmp_path / "libthrows.so"), str(src)], check=True)
+    lib = ctypes.CDLL(str(tmp_path / "libthrows.so"))
+    at = lambda fn: ctypes.cast(getattr(lib, fn), ctypes.c_void_p).value
+    w, x, resid = torch.zeros(64, 32, device="cuda", dtype=BF), torch.zeros(20, 32, device="cuda", dtype=BF), torch.zeros(20, 64, device="cuda")
+    i = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    h3, state = torch.zeros(1, 24, device="cuda", dtype=BF), torch.zeros(1, 2, 8, device="cuda", dtype=BF)
+    for n, (fn, text) in enumerate((("memory", "bad_alloc"), ("other", "unknown"))):
+        with pytest.raises(RuntimeError, match=text):
+            ops._calls().product(at(fn), at("plan"), 0, w, x, None, None, 0.0, 2, None, resid, torch.ones(64, device="cuda"), None, None, 0, None)
+        with pytest.raises(RuntimeError, match=text):
+            ops._calls().shortconv(at(fn), h3, None, torch.zeros(3, 8, device="cuda"), None, state, i(0), i(0), i(0, 1), i(0), None, None)
+        assert ctypes.c_int.in_dll(lib, "calls").value == 2 * n + 2
+    assert ops._calls().product(at("memory"), at("plan"), 0, w.float(), x, None, None, 0.0, 2, None, resid, None, None, None, 0, None) is NotImplemented
+    assert ctypes.c_int.in_dll(lib, "calls").value == 4

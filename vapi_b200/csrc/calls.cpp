@@ -5,12 +5,16 @@
 //
 // A function here answers NotImplemented for anything but what the kernels take as it is (other types, layouts, devices or
 // tensor classes): its caller in ops then goes through the same steps in Python, which name what is wrong.  A negative number is the C
-// function's error code.  The C functions are given by address, so this library is linked with none of the kernels' ones.
+// function's error code.  Once the C function has been called there is no way back to Python's steps, which would add to the stream, or move
+// a state on, a second time: what goes wrong from there on is an error.  The C functions are given by address, so this library is linked
+// with none of the kernels' ones.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
 #include <ATen/ATen.h>
 #include <torch/csrc/autograd/python_variable.h>
+
+#include <string>
 
 namespace {
 
@@ -60,21 +64,40 @@ int size32(int64_t v) {
     if (v > 0x7fffffffLL) throw Bad{};
     return (int)v;
 }
-PyObject* wrap(const at::Tensor& t) {
+PyObject* wrap(const at::Tensor& t) {       // (null: a Python error)
     if (t.defined()) return THPVariable_Wrap(t);
     Py_RETURN_NONE;
 }
 
+// The interpreter's lock is given up while one of these lives, and taken again however its block is left.
+struct Unlocked {
+    PyThreadState* state = PyEval_SaveThread();
+    Unlocked() = default;
+    Unlocked(const Unlocked&) = delete;
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
+// body(called): sets `called` before it calls the C function
 template <typename F>
 PyObject* guarded(Py_ssize_t given, Py_ssize_t wanted, F&& body) {
     if (given != wanted) {
         PyErr_Format(PyExc_TypeError, "%zd arguments instead of %zd", given, wanted);
         return nullptr;
     }
+    bool called = false;
+    const char* what = "an unknown exception";
+    std::string text;
     try {
-        return body();
+        return body(called);
     } catch (const Bad&) {
-    } catch (const std::exception&) {       // (what torch objects to, the same calls in Python say)
+    } catch (const std::exception& e) {     // (what torch objects to, the same calls in Python say)
+        text = e.what();
+        what = text.c_str();
+    } catch (...) {
+    }
+    if (called) {
+        if (!PyErr_Occurred()) PyErr_Format(PyExc_RuntimeError, "a kernel's launch ended with an exception: %s", what);
+        return nullptr;
     }
     PyErr_Clear();
     Py_RETURN_NOTIMPLEMENTED;
@@ -88,7 +111,7 @@ enum { EPI_BF16 = 0, EPI_SWIGLU = 1, EPI_RESID = 2, EPI_F32 = 3 };
 // product(fn, plan, which of the plan's answers is the partial sums of squares, weight, act, xw, ss_in, eps, epilogue, bias, resid,
 //         next_weight, status, xielu, glu, stream): ops._fused_product
 PyObject* product(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
-    return guarded(nargs, 16, [&]() -> PyObject* {
+    return guarded(nargs, 16, [&](bool& called) -> PyObject* {
         const auto fn = reinterpret_cast<ProductFn>(address(a[0]));
         const auto plan = reinterpret_cast<PlanFn>(address(a[1]));
         const int answer = integer(a[2]), epi = integer(a[8]);
@@ -138,16 +161,19 @@ PyObject* product(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         void* stream = address(a[15]);
         const int glu = integer(a[14]);
         int rc;
-        Py_BEGIN_ALLOW_THREADS
-        rc = fn(w.data_ptr(), N, K, M, norm ? 1 : 0, x.data_ptr(), ss, parts_in, eps, epi, epi == EPI_F32 ? nullptr : o,
-                epi == EPI_F32 ? static_cast<float*>(o) : nullptr, stride, bias, resid, so, next_w, wo, status, stream, xielu, glu);
-        Py_END_ALLOW_THREADS
+        called = true;
+        {
+            Unlocked unlocked;
+            rc = fn(w.data_ptr(), N, K, M, norm ? 1 : 0, x.data_ptr(), ss, parts_in, eps, epi, epi == EPI_F32 ? nullptr : o,
+                    epi == EPI_F32 ? static_cast<float*>(o) : nullptr, stride, bias, resid, so, next_w, wo, status, stream, xielu, glu);
+        }
         if (rc != 0) return PyLong_FromLong(rc);
         if (epi != EPI_RESID) return wrap(out);
-        PyObject* pair = PyTuple_New(2);
-        if (!pair) return nullptr;
-        PyTuple_SET_ITEM(pair, 0, wrap(sums));
-        PyTuple_SET_ITEM(pair, 1, wrap(weighted));
+        PyObject* first = wrap(sums);
+        PyObject* second = first ? wrap(weighted) : nullptr;
+        PyObject* pair = second ? PyTuple_Pack(2, first, second) : nullptr;
+        Py_XDECREF(first);
+        Py_XDECREF(second);
         return pair;
     });
 }
@@ -157,7 +183,7 @@ typedef int (*ShortconvFn)(const void*, int, const float*, const float*, const f
 
 // shortconv(fn, h3, in_bias, taps, conv_bias, state, state_slots, tok_seq, cu_q, positions, status, stream): ops.shortconv in bfloat16
 PyObject* shortconv(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
-    return guarded(nargs, 12, [&]() -> PyObject* {
+    return guarded(nargs, 12, [&](bool& called) -> PyObject* {
         const auto fn = reinterpret_cast<ShortconvFn>(address(a[0]));
         const at::Tensor& h3 = need(a[1], at::kBFloat16, 2);
         const at::Tensor& taps = need(a[3], at::kFloat, 2);
@@ -181,11 +207,13 @@ PyObject* shortconv(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         void* stream = address(a[11]);
         at::Tensor out = at::empty({n, H}, h3.options());
         int rc;
-        Py_BEGIN_ALLOW_THREADS
-        rc = fn(h3.data_ptr(), 1, in_bias, static_cast<const float*>(taps.data_ptr()), conv_bias, L > 1 ? state->data_ptr() : nullptr,
-                slot_stride, state_slots, tok_seq, static_cast<const int*>(cu->data_ptr()), positions, out.data_ptr(), n, seqs, H, L, slots,
-                status, stream);
-        Py_END_ALLOW_THREADS
+        called = true;
+        {
+            Unlocked unlocked;
+            rc = fn(h3.data_ptr(), 1, in_bias, static_cast<const float*>(taps.data_ptr()), conv_bias, L > 1 ? state->data_ptr() : nullptr,
+                    slot_stride, state_slots, tok_seq, static_cast<const int*>(cu->data_ptr()), positions, out.data_ptr(), n, seqs, H, L,
+                    slots, status, stream);
+        }
         return rc != 0 ? PyLong_FromLong(rc) : wrap(out);
     });
 }

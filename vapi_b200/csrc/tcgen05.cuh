@@ -184,7 +184,7 @@ static int kmajor_map(CUtensorMap* out, const char* what, const void* ptr, long 
     if (r != CUDA_SUCCESS) return fail(-103, "%s: cuTensorMapEncodeTiled failed with %d", what, (int)r);
     if (keep) {
         if (kept.size() > 4096) kept.clear();
-        kept.emplace(key, *out);
+        try { kept.emplace(key, *out); } catch (...) {}      // (no memory for it: encoded again next time; callers in C know no exceptions)
     }
     return 0;
 }
