@@ -123,3 +123,30 @@ def test_a_call_that_has_been_made_is_not_made_again(ops, tmp_path):
         assert ctypes.c_int.in_dll(lib, "calls").value == 2 * n + 2
     assert ops._calls().product(at("memory"), at("plan"), 0, w.float(), x, None, None, 0.0, 2, None, resid, None, None, None, 0, None) is NotImplemented
     assert ctypes.c_int.in_dll(lib, "calls").value == 4
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_operands_that_are_too_short_are_refused(ops, monkeypatch, native):
+    """Every vector is at least as long as what the kernels read of it, by the native calls and by the same steps in Python."""
+    if not native:
+        monkeypatch.setattr(ops, "_calls", lambda: ops._NoCalls)
+    f = lambda *s: torch.zeros(*s, device="cuda")
+    i = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    w, x = f(64, 32).to(BF), f(20, 32).to(BF)
+    for which in (ops.linear_tc, ops.prompt_linear, lambda *a, act, resid=None, **kw: ops.skinny_linear(*a, act=act[:16], resid=None if resid is None else resid[:16], **kw)):
+        with pytest.raises(ops.KernelError, match="norm weight"):
+            which(w, act=x, epilogue="resid", resid=f(20, 64), next_weight=f(63))
+        with pytest.raises(ops.KernelError, match="activation"):
+            which(w, act=x, xielu=f(1))
+    with pytest.raises(ops.KernelError, match="activation"):
+        ops.xielu(x, f(1))
+    good = dict(h3=f(3, 24).to(BF), in_bias=f(24), taps=f(3, 8), conv_bias=f(8), state_layer=f(2, 2, 8).to(BF), state_slots=i(0, 1),
+                tok_seq=i(0, 0, 1), cu_q=i(0, 2, 3), positions=i(0, 1, 4))
+    assert ops.shortconv(**good).shape == (3, 8)
+    for key, short in (("in_bias", f(23)), ("conv_bias", f(7)), ("state_slots", i(0)), ("tok_seq", i(0, 0)), ("positions", i(0, 1)),
+                       ("state_slots", None), ("positions", None)):
+        with pytest.raises(ops.KernelError):
+            ops.shortconv(**{**good, key: short})
+    assert ops.shortconv(**{**good, "taps": f(1, 8), "state_layer": None, "state_slots": None, "positions": None}).shape == (3, 8)
+    # (longer ones are taken, as before)
+    assert ops.shortconv(**{**good, "in_bias": f(30), "positions": i(0, 1, 4, 5)}).shape == (3, 8)

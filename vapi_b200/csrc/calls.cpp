@@ -32,11 +32,11 @@ const at::Tensor& need(PyObject* o, at::ScalarType type, int64_t dim) {
     if (!t || t->scalar_type() != type || t->dim() != dim || !t->is_contiguous()) throw Bad{};
     return *t;
 }
-// a vector of `n` floats (-1: of any length), or none
-const float* floats(PyObject* o, int64_t n) {
+// a vector of floats, as many as the kernel reads or more (`most`: no more than that), or none
+const float* floats(PyObject* o, int64_t least, int64_t most = INT64_MAX) {
     const at::Tensor* t = tensor(o);
     if (!t) return nullptr;
-    if (t->scalar_type() != at::kFloat || !t->is_contiguous() || (n >= 0 && t->numel() != n)) throw Bad{};
+    if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->numel() < least || t->numel() > most) throw Bad{};
     return static_cast<const float*>(t->data_ptr());
 }
 const int* ints(PyObject* o, int64_t least) {
@@ -131,9 +131,9 @@ PyObject* product(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         } else if (a[6] != Py_None) {
             throw Bad{};
         }
-        const float* bias = floats(a[9], N);
-        const float* next_w = floats(a[11], -1);
-        const float* xielu = floats(a[13], -1);
+        const float* bias = floats(a[9], N, N);
+        const float* next_w = floats(a[11], N);
+        const float* xielu = floats(a[13], 2);
         float* resid = nullptr;
         at::Tensor out, sums, weighted;
         const auto options = w.options();
@@ -201,8 +201,8 @@ PyObject* shortconv(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         const at::Tensor* cu = tensor(a[8]);
         if (!cu || cu->scalar_type() != at::kInt || !cu->is_contiguous()) throw Bad{};
         const int seqs = size32(cu->numel() - 1);
-        const float *in_bias = floats(a[2], -1), *conv_bias = floats(a[4], -1);
-        const int *state_slots = ints(a[6], 0), *tok_seq = ints(a[7], 0), *positions = ints(a[9], 0);
+        const float *in_bias = floats(a[2], 3LL * H), *conv_bias = floats(a[4], H);
+        const int *state_slots = ints(a[6], seqs), *tok_seq = ints(a[7], n), *positions = ints(a[9], n);
         int* status = static_cast<int*>(address(a[10]));
         void* stream = address(a[11]);
         at::Tensor out = at::empty({n, H}, h3.options());

@@ -239,6 +239,12 @@ def _bias(t: Optional[torch.Tensor], n: int, what: str = "bias") -> None:
         raise KernelError(f"{what} of {tuple(t.shape)} does not fit {n} features")
 
 
+def _least(t: Optional[torch.Tensor], n: int, what: str) -> None:
+    """A vector that a kernel reads the first ``n`` numbers of."""
+    if t is not None and t.numel() < n:
+        raise KernelError(f"{what} of {tuple(t.shape)} holds fewer than {n} numbers")
+
+
 _sm_counts: Dict[int, int] = {}
 
 
@@ -455,6 +461,8 @@ def skinny_linear(weight: torch.Tensor, *, act: Optional[torch.Tensor] = None,
             raise KernelError("partial sums must be [parts, M]")
     _bias(bias, N)
     _f32(next_weight, "norm weight")
+    _least(next_weight, N, "norm weight")
+    _least(xielu, 2, "the activation's numbers")
     rpb = rows_per_block or 16
     out_bf16 = out_f32 = sso = xwo = None
     out_stride = N
@@ -623,6 +631,8 @@ def _fused_product(which: str, weight: torch.Tensor, act, xw, ss_in, eps: float,
             raise KernelError("partial sums must be [parts, M]")
     _bias(bias, N)
     _f32(next_weight, "norm weight")
+    _least(next_weight, N, "norm weight")
+    _least(xielu, 2, "the activation's numbers")
     if epilogue not in _EPI:
         raise KernelError(f"unknown epilogue {epilogue}")
     if which == "linear_tc":
@@ -721,6 +731,7 @@ def xielu(z: torch.Tensor, consts: torch.Tensor) -> torch.Tensor:
     _cuda(z, consts)
     _contig(z, "activations")
     _f32(consts, "the activation's numbers")
+    _least(consts, 2, "the activation's numbers")
     out = torch.empty_like(z)
     lib = _lib("elementwise")
     _check(lib, lib.vapi_xielu(_p(z), _p(out), _dt(z), _p(consts), ctypes.c_longlong(z.numel()), _stream()))
@@ -1220,8 +1231,16 @@ def shortconv(h3: torch.Tensor, in_bias: Optional[torch.Tensor], taps: torch.Ten
         if state_layer.stride(2) != 1 or state_layer.stride(1) != hidden:
             raise KernelError("state rows must be contiguous")
         slot_stride, num_slots = state_layer.stride(0), state_layer.shape[0]
-    out = torch.empty((n, hidden), dtype=h3.dtype, device=h3.device)
     num_seqs = cu_q.numel() - 1
+    _least(in_bias, 3 * hidden, "in_proj bias")
+    _least(conv_bias, hidden, "conv bias")
+    _least(tok_seq, n, "tok_seq")
+    if L > 1:
+        if state_slots is None or positions is None:
+            raise KernelError("a convolution with a state needs state slots and positions")
+        _least(state_slots, num_seqs, "state slots")
+        _least(positions, n, "positions")
+    out = torch.empty((n, hidden), dtype=h3.dtype, device=h3.device)
     lib = _lib("shortconv")
     _check(lib, lib.vapi_shortconv(
         _p(h3), _dt(h3), _p(in_bias), _p(taps), _p(conv_bias), _p(state_layer if L > 1 else None),
