@@ -150,3 +150,15 @@ def test_operands_that_are_too_short_are_refused(ops, monkeypatch, native):
     assert ops.shortconv(**{**good, "taps": f(1, 8), "state_layer": None, "state_slots": None, "positions": None}).shape == (3, 8)
     # (longer ones are taken, as before)
     assert ops.shortconv(**{**good, "in_bias": f(30), "positions": i(0, 1, 4, 5)}).shape == (3, 8)
+
+
+def test_tensor_maps_are_kept_for_weights_and_not_for_tokens(ops):
+    """Prompts at other addresses leave the table of kept maps as it is (a weight has one map for each tile that its products use)."""
+    maps, counts, alive = ops._lib("linear_prompt").vapi_prompt_linear_maps, [], []
+    w = torch.zeros(256, 64, device="cuda", dtype=BF)
+    for _ in range(2):
+        for n in (33, 130, 131, 257, 300, 301, 1000):
+            alive.append(torch.zeros(n, 64, device="cuda", dtype=BF))
+            assert ops.prompt_linear(w, act=alive[-1]).shape == (n, 256)
+        counts.append(maps())
+    assert counts[0] == counts[1] >= 1

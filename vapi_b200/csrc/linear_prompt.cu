@@ -550,7 +550,7 @@ VAPI_EXPORT int vapi_prompt_linear(const void* W, int N, int K, int M, int pro, 
     p.status = status; p.xielu = xielu_consts; p.glu = glu;
     const bool half_rows = epi == PL_EPI_SWIGLU || pair == 2;      // boxes of BN/2 weight rows
     CUtensorMap ta, tw;
-    int rc = kmajor_map(&ta, "prompt_linear", tokens, M, K, PL_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, true);
+    int rc = kmajor_map(&ta, "prompt_linear", tokens, M, K, PL_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, false);
     if (rc) return rc;
     rc = kmajor_map(&tw, "prompt_linear", W, N, K, half_rows ? bn / 2 : bn, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, true);
     if (rc) return rc;
@@ -560,5 +560,8 @@ VAPI_EXPORT int vapi_prompt_linear(const void* W, int N, int K, int M, int pro, 
     if (bn == 128 && pair == 1) return launch_pl<128, 1>(ta, tw, p, stream);
     return fail(-2, "prompt_linear: no kernel for tiles of %d features and %d blocks", bn, pair);
 }
+
+// How many tensor maps the calling thread keeps for this kernel's operands.
+VAPI_EXPORT int vapi_prompt_linear_maps() { return (int)kept_maps().size(); }
 
 VAPI_EXPORT const char* vapi_last_error() { return error_buffer(); }

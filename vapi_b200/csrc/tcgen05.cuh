@@ -151,22 +151,31 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// A [rows][K] bfloat16 matrix, K contiguous, tiled in boxes of 64 k x box_rows rows, 128-byte swizzle.  keep: the map, a function of address,
-// shape and box alone, is encoded once for each of these and thread, and not at every call (weights; the driver's encoder takes about
-// a microsecond, and a step of a few tokens is bound by what its launches cost the host).
+// A tensor map's arguments; the map is a function of these alone.
+struct MapKey {
+    const void* p;
+    long long rows, k;
+    int box, promotion;
+    bool operator==(const MapKey& o) const { return p == o.p && rows == o.rows && k == o.k && box == o.box && promotion == o.promotion; }
+};
+struct MapHash {
+    size_t operator()(const MapKey& m) const {
+        return std::hash<const void*>()(m.p) ^ (std::hash<long long>()(m.rows) * 31) ^ (std::hash<long long>()(m.k) * 131) ^
+               (size_t)(m.box * 8 + m.promotion);
+    }
+};
+static std::unordered_map<MapKey, CUtensorMap, MapHash>& kept_maps() {
+    static thread_local std::unordered_map<MapKey, CUtensorMap, MapHash> kept;
+    return kept;
+}
+
+// A [rows][K] bfloat16 matrix, K contiguous, tiled in boxes of 64 k x box_rows rows, 128-byte swizzle.  keep: for weights, the map is encoded
+// once for each thread and not at every call (the driver's encoder takes about a microsecond, and a step of a few tokens is bound by what
+// its launches cost the host).  Tokens lie at other addresses from step to step, in other numbers: kept, they would only fill the table.
 static int kmajor_map(CUtensorMap* out, const char* what, const void* ptr, long long rows, long long K, int box_rows,
                       CUtensorMapL2promotion promotion, bool keep) {
-    struct Key {
-        const void* p; long long r, k; int b;
-        bool operator==(const Key& o) const { return p == o.p && r == o.r && k == o.k && b == o.b; }
-    };
-    struct Hash {
-        size_t operator()(const Key& k) const {
-            return std::hash<const void*>()(k.p) ^ (std::hash<long long>()(k.r) * 31) ^ (std::hash<long long>()(k.k) * 131) ^ (size_t)k.b;
-        }
-    };
-    static thread_local std::unordered_map<Key, CUtensorMap, Hash> kept;
-    const Key key{ptr, rows, K, box_rows};
+    auto& kept = kept_maps();
+    const MapKey key{ptr, rows, K, box_rows, (int)promotion};
     if (keep) {
         const auto it = kept.find(key);
         if (it != kept.end()) { *out = it->second; return 0; }
