@@ -1,4 +1,4 @@
-"""What the package does where ``csrc/calls.cpp``, the one source that it can do without, cannot be built."""
+"""What the package does where ``csrc/calls.cpp``, the one source that it can do without, cannot be built; plans of products of nothing."""
 import warnings
 
 import pytest
@@ -37,3 +37,9 @@ def test_calls_that_cannot_be_built_are_answered_with_not_implemented(monkeypatc
         warnings.simplefilter("error")                       # (said once)
         assert ops._calls() is calls
     assert calls.product(*range(16)) is NotImplemented and calls.shortconv(*range(12)) is NotImplemented
+
+
+@pytest.mark.parametrize("N,K,epi", [(0, 64, 2), (64, 0, 2), (0, 0, 0), (1, 8, 1)])
+def test_a_product_of_nothing_has_a_plan(N, K, epi):
+    """The outputs are laid out by the plan before the call refuses such a product: no division by its tiles or its K."""
+    assert ops._tc_plan.__wrapped__(N, K, 20, epi)[:2] == ((N + 127) // 128 if epi != 1 else (N // 2 + 63) // 64, 1)

@@ -94,6 +94,11 @@ def test_what_the_native_product_does_not_take_is_refused_or_done_as_before(ops)
     with pytest.raises(ops.KernelError, match="more than 256"):          # (the C function's own refusal)
         ops.linear_tc(w, act=torch.zeros(257, 32, device="cuda", dtype=BF))
 
+    for n, k in ((0, 32), (64, 0)):                                      # (and products of nothing)
+        with pytest.raises(ops.KernelError, match="positive"):
+            ops.linear_tc(torch.zeros(n, k, device="cuda", dtype=BF), act=torch.zeros(20, k, device="cuda", dtype=BF), epilogue="resid",
+                          resid=torch.zeros(20, n, device="cuda"), next_weight=torch.ones(n, device="cuda"))
+
     class Other(torch.Tensor):
         pass
 

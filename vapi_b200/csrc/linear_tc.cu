@@ -421,7 +421,7 @@ VAPI_EXPORT int vapi_linear_tc_plan(int N, int K, int M, int epi, int* tiles, in
     const int num_kb = (K + TC_BK - 1) / TC_BK;
     int s = 1;
     const int sms = sm_count();
-    if (b <= 128 && t <= sms) {                      // (partials must fit the stages)
+    if (b <= 128 && t > 0 && t <= sms && num_kb > 0) {          // (partials must fit the stages; nothing to cut: the call refuses it)
         // Too few tiles for the multiprocessors: K is cut until they are one block each, or up to four slices as far as two blocks a
         // multiprocessor go, and both stream at once.  19 / 64 / 128 tokens, K = 2,048, one slice or as many as make one block, and then two:
         // 48 tiles 9.0 / 11.4 / 15.7 us, so 8.7 / 10.5 / 13.9; 64 tiles 11.6 / 13.9 / 19.4, so 9.6 / 11.6 / 14.7; 80 tiles 15.3 / 19.0 / 27.0, so
