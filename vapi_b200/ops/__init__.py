@@ -496,24 +496,26 @@ def skinny_linear(weight: torch.Tensor, *, act: Optional[torch.Tensor] = None,
 #: itself takes up to 256 rows, but it has one tile per block and pays its fixed costs (cluster
 #: reduction, epilogue) per launch: measured in the captured decode step of LFM2-1.2B sizes it
 #: beats the library's product plus separate norm / SwiGLU / add kernels at 32 rows (1.26 vs 1.33
-#: ms) and, in the stream form of a decode step (STREAM_DECODE_MAX_ROWS), at 64; a product alone loses beyond 32 rows, and clearly so
+#: ms) and, in the stream form of a decode step, up to 64 (STREAM_DECODE_MAX_ROWS); a product alone loses beyond 32 rows, and clearly so
 #: beyond 64 (2-7x slower at 256 rows).
 TC_MAX_ROWS = int(os.environ.get("VAPI_TC_MAX_ROWS", "32"))
 #: steps with a prompt portion run the stream form of their blocks (norms, SwiGLU and residual adds inside the products; LFM2's blocks have
 #: one) up to this many rows.  They are launched one by one, and what bounds them is the launches, of which this form has 81 where the other
-#: has 145 at 16 layers.  Steps one after the other, without a wait between them / the device's share, ms in this form against the other:
-#: 33 tokens of the 700M, 1.2B and 2.6B sizes 1.70 / 0.88, 1.71 / 1.03, 2.90 / 1.81 against 1.94 / 0.94, 1.96 / 1.05, 3.37 / 1.84; 64 1.67 / 0.99,
-#: 1.69 / 1.15, 2.90 / 2.02 against 1.94 / 0.96, 1.95 / 1.09, 3.38 / 1.86; 128 1.68 / 1.43, 1.69 / 1.61, 2.92 / 2.91 against 1.93 / 1.03, 1.95 / 1.14,
-#: 3.40 / 2.00; 60 decoding requests beside a portion of 60 1.92 / 1.61, 1.94 / 1.83, 3.20 / 3.15 against 2.16 / 1.21, 2.14 / 1.38, 3.62 / 2.28.  So
-#: it pays as far as the host is what a step waits for, and from about 50 rows on only that far: with weights much wider than these the
-#: device's share is what counts, and the other form is ahead.  From 129 rows on a product's tokens no longer fit beside a share of K (200
-#: tokens of the 700M size: 1.98 -> 4.37 ms).  (Measured before the products' way from the partial sums to the output was shortened.)
+#: has 145 at 16 layers.  Steps one after the other, without a wait between them / the same step as one graph (the device's share), ms in this form
+#: against the other: 33 tokens of the 700M, 1.2B and 2.6B sizes 1.10 / 0.75, 1.11 / 0.88, 1.76 / 1.51 against 1.93 / 0.77, 1.89 / 0.97, 3.23 / 1.71; 64
+#: 1.11 / 0.82, 1.11 / 0.95, 1.77 / 1.65 against 1.93 / 0.85, 1.89 / 0.99, 3.21 / 1.74; 96 1.12 / 1.03, 1.22 / 1.15, 2.15 / 2.04 against 1.94 / 0.88, 1.92 / 1.04,
+#: 3.32 / 1.84; 128 1.22 / 1.14, 1.36 / 1.29, 2.41 / 2.30 against 1.93 / 0.90, 1.92 / 1.05, 3.28 / 1.84; 60 decoding requests beside a portion of 60 1.40 /
+#: 1.25, 1.52 / 1.43, 2.62 / 2.48 against 2.10 / 1.01, 2.07 / 1.18, 3.46 / 2.01.  So it pays as far as the host is what a step waits for, and from about
+#: 64 rows on only that far: with weights much wider than these the device's share is what counts, and the other form is ahead.  From 129 rows on
+#: a product's tokens no longer fit beside a share of K (200 tokens of the 700M size: 1.98 -> 4.37 ms).
 STREAM_PROMPT_MAX_ROWS = 128
 #: and this many numbers in a layer's matrices (40, 65 and 59 million in the sizes above)
 STREAM_PROMPT_MAX_LAYER = 80_000_000
-#: Decode steps of such models run it up to this many rows, although a product alone is the library's above TC_MAX_ROWS (64 rows: 6,144 x 2,048 10.5
-#: against 7.1 us, the gate's with SwiGLU 17.7 against 12.2 + 2.4): what it saves are the norms, adds and gates between them.  Captured, four steps of 64
-#: requests of 128 to 2,048 tokens on the 2.6B size 7,756 us in the other form, 7,407 in this one.
+#: Decode steps of such models run it up to this many rows, the largest captured bucket, although a product alone is the library's above
+#: TC_MAX_ROWS (64 rows: 6,144 x 2,048 10.5 against 7.1 us, the gate's with SwiGLU 17.7 against 12.2 + 2.4): what it saves are the norms, adds and
+#: gates between them.  A step of 33 / 48 / 64 requests of 128 to 1,024 tokens, captured, us in the other form and in this one: 700M 903, 795 /
+#: 917, 825 / 944, 896; 1.2B 1,049, 918 / 1,004, 959 / 1,095, 1,020; 2.6B 1,802, 1,555 / 1,678, 1,622 / 1,738, 1,738 (of 128 to 2,048 tokens 1,939,
+#: 1,808); launched one by one 1,962 to 3,456 and 1,120 to 1,860.
 STREAM_DECODE_MAX_ROWS = int(os.environ.get("VAPI_STREAM_DECODE_MAX_ROWS", "64"))
 #: set False to keep products of 17..TC_MAX_ROWS rows on the library
 use_tc = os.environ.get("VAPI_TC", "1") != "0"
